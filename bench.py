@@ -94,7 +94,7 @@ def parse_args():
     ap.add_argument("--no-graph", action="store_true", help="time ordinary calls instead of CUDA-graph replays")
     ap.add_argument("--no-autotune", action="store_true", help="keep the default join launch shape")
     ap.add_argument("--join-kernel", type=int, choices=[0, 1, 2], default=None,
-                    help="force the join kernel (2: per-lane DFS with CTA-local slot regions, the default; 0: per-lane DFS "
+                    help="force the join kernel (2: per-lane DFS, one candidate per turn, the default; 0: per-lane DFS "
                          "with one work cursor; 1: warp-cooperative frontier) after any autotuning")
     ap.add_argument("--serving-only", action="store_true", help="run only the serving measurement (prints its JSON)")
     ap.add_argument("--shard", action="store_true",
@@ -282,7 +282,7 @@ def peaks():
     return 6650.0, "fallback"
 
 
-JOIN_KERNELS = {0: "k_join_masks", 1: "k_join_frontier", 2: "k_join_lanes"}  # sigmo_tuning.join_kernel
+JOIN_KERNELS = {0: "k_join_masks", 1: "k_join_frontier", 2: "k_join_dfs"}  # sigmo_tuning.join_kernel
 
 
 def traffic_for(kernel: str, workload: str, key: str = "bytes_per_launch"):
@@ -533,7 +533,7 @@ def run_sigmo(args, rank, world, local):
     jb = join_bytes(q, d, offsets, indices)
     join_ms = med("ms_join")
     achieved = jb / (join_ms / 1e3) / 1e9
-    jk = JOIN_KERNELS.get(queue.get_tuning()["join_kernel"], "k_join_lanes")
+    jk = JOIN_KERNELS.get(queue.get_tuning()["join_kernel"], "k_join_dfs")
     jkey = f"join:{jk}"
     l1, l2 = traffic_for(jkey, args.workload, "l1_hit_rate"), traffic_for(jkey, args.workload, "l2_hit_rate")
     roof = {"kernel": f"join stage: k_pair_masks + {jk} (side stream: k_join_fast for queries over 16 vertices, "

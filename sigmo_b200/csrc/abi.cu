@@ -209,6 +209,8 @@ void queue_free(Queue* q) {
   if (q->ev_aux_join) cudaEventDestroy(q->ev_aux_join);
   for (cudaEvent_t e : q->ev_masks)
     if (e) cudaEventDestroy(e);
+  for (cudaEvent_t e : q->ev_long)
+    if (e) cudaEventDestroy(e);
   if (q->ev_start) cudaEventDestroy(q->ev_start);
   if (q->ev_end) cudaEventDestroy(q->ev_end);
   if (q->pinned) cudaFreeHost(q->pinned);
@@ -276,6 +278,7 @@ int sigmo_queue_create(int device, const sigmo_options* opts, sigmo_queue_t* out
   if (st == cudaSuccess) st = cudaEventCreateWithFlags(&q->ev_aux_fork, cudaEventDisableTiming);
   if (st == cudaSuccess) st = cudaEventCreateWithFlags(&q->ev_aux_join, cudaEventDisableTiming);
   for (int i = 0; i < 2 && st == cudaSuccess; ++i) st = cudaEventCreateWithFlags(&q->ev_masks[i], cudaEventDisableTiming);
+  for (int i = 0; i < 2 && st == cudaSuccess; ++i) st = cudaEventCreateWithFlags(&q->ev_long[i], cudaEventDisableTiming);
   if (st == cudaSuccess) {
     // Keep freed stream-ordered allocations cached in the device's default pool
     // (per-call scratch is then reused instead of being remapped every call).
@@ -475,6 +478,8 @@ int sigmo_graph_destroy(sigmo_graph_t g) {
   dev_free(q, g->qorder);
   dev_free(q, g->qsel);
   dev_free(q, g->qsel_id);
+  dev_free(q, g->qmeta);
+  dev_free(q, g->qmeta_id);
   release_plane_program(g);
   if (g->ready) cudaEventDestroy(g->ready);
   delete g;

@@ -47,7 +47,8 @@ struct Queue {
   // join of the previous one), with its fork/join events and the events after
   // each stream's last level-mask pass
   cudaStream_t aux = nullptr;
-  cudaEvent_t ev_aux_fork = nullptr, ev_aux_join = nullptr, ev_masks[2] = {nullptr, nullptr};
+  // and after each chunk's long pairs
+  cudaEvent_t ev_aux_fork = nullptr, ev_aux_join = nullptr, ev_masks[2] = {nullptr, nullptr}, ev_long[2] = {nullptr, nullptr};
   // Join step budget (0: none) and the device status word the join kernels
   // raise when a lane runs out of it (kJoinStatusBudget).
   uint64_t join_budget = 0;
@@ -148,6 +149,11 @@ struct Graph {
   uint8_t* qorder = nullptr;       // [total_nodes] local id placed at level k
   uint64_t* qsel = nullptr;        // [total_nodes] adjacency to earlier levels
   uint64_t* qsel_id = nullptr;     // [total_nodes] same, identity order
+  // Query side of each level (queries of 2 to 16 vertices): two of its earlier
+  // neighbours (4 bits each; the same one twice if it has one), bit 8: it has
+  // two, bit 9: it has none or more than two.
+  uint16_t* qmeta = nullptr;       // [num_graphs][16]
+  uint16_t* qmeta_id = nullptr;    // [num_graphs][16] same, identity order
   std::vector<uint32_t> host_graph_offsets;  // host copy (sizes, dispatch)
   std::vector<uint64_t> label_hist;          // vertices per label (filled on first use, 256 entries)
   uint64_t stamp = 0;                        // unique per graph object (cache keys)

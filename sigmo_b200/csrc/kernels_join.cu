@@ -873,6 +873,7 @@ __global__ void __launch_bounds__(128) k_join_fast(
 // next = base[k+1] & (row(t) or ~row(t)) [& ~used]; base[k+2] is computed
 // once per descent.
 constexpr uint32_t kPhaseLevels = 16;
+constexpr uint32_t kDfsLevels = 10;  // most vertices of a query in k_join_dfs's short form
 constexpr uint32_t kPhaseThreads = 256;
 
 // Work layout: a warp takes 32 consecutive slots per round, one lane per slot
@@ -886,7 +887,8 @@ __global__ void __launch_bounds__(256) k_pair_masks(
     const uint8_t* __restrict__ qsym, const uint32_t* __restrict__ dgoff, const uint8_t* __restrict__ dsym,
     const uint32_t* __restrict__ indices, const uint32_t* __restrict__ pair_graph, uint64_t slot0, uint64_t count,
     uint64_t* __restrict__ masks, uint4* __restrict__ rec, uint32_t skip_below, uint32_t* __restrict__ overflow,
-    unsigned long long* __restrict__ overflow_len, uint64_t* __restrict__ counts) {
+    unsigned long long* __restrict__ overflow_len, uint32_t* __restrict__ longs, unsigned long long* __restrict__ longs_len,
+    uint64_t* __restrict__ counts, int zero_counts) {
   const unsigned lane = threadIdx.x & 31u;
   const uint64_t warp = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
@@ -905,12 +907,21 @@ __global__ void __launch_bounds__(256) k_pair_masks(
       // queries over kPhaseLevels vertices and molecules over 64 atoms (a
       // vertex set wider than one word) go to the generic kernel
       const bool generic = n > kPhaseLevels || dgoff[g + 1] - ds > 64u;
-      // the pair's setup record: first data vertex, query size | flags, query offset, data graph
-      rec[local] = make_uint4(ds, n | (ident ? 0x100u : 0u) | (generic ? 0x200u : 0u), qoff, g);
+      // the pair's setup record: first data vertex, query size | flags (0x100
+      // identity order, 0x200 generic, 0x400 long, 0x800 the literal join's),
+      // query offset, query graph
+      const bool lng = !generic && n > kDfsLevels;
+      rec[local] = make_uint4(ds, n | (ident ? 0x100u : 0u) | (generic ? 0x200u : 0u) | (lng ? 0x400u : 0u) |
+                                      (g < skip_below ? 0x800u : 0u), qoff, qg);
+      if (lng && g >= skip_below) {  // joined by k_join_dfs's long form, in parts
+        longs[atomicAdd(longs_len, 1ull)] = static_cast<uint32_t>(slot);
+        counts[slot] = 0;
+      }
       if (generic && g >= skip_below) {  // joined by the generic kernel, which accumulates into counts
         overflow[atomicAdd(overflow_len, 1ull)] = static_cast<uint32_t>(slot);
         counts[slot] = 0;
       }
+      if (zero_counts && g >= skip_below) counts[slot] = 0;  // the join adds up a pair's parts
       items = generic ? 0u : n;
     }
     uint32_t incl = items;
@@ -953,7 +964,7 @@ template <bool EXACT, uint32_t DAW>
 __global__ void __launch_bounds__(kPhaseThreads) k_join_masks(
     const uint64_t* __restrict__ masks, const uint4* __restrict__ rec, uint64_t slot0, uint64_t count,
     const uint64_t* __restrict__ qsel, const uint64_t* __restrict__ qsel_id, const uint64_t* __restrict__ dadj,
-    uint32_t skip_below, int find_first, uint32_t kChunk, unsigned long long* __restrict__ cursor,
+    int find_first, uint32_t kChunk, unsigned long long* __restrict__ cursor,
     uint64_t* __restrict__ counts, unsigned long long* __restrict__ d_total, JoinLimit lim) {
   extern __shared__ uint64_t sm[];
   uint64_t steps = 0;
@@ -1004,12 +1015,11 @@ __global__ void __launch_bounds__(kPhaseThreads) k_join_masks(
       }
       if (!pre) break;
       local = plocal;
-      const uint4 r = pr;  // first data vertex, query size | order flag, query offset, data graph
+      const uint4 r = pr;  // first data vertex, query size | flags, query offset, query graph
       const uint64_t m0 = pm0, m1 = pm1;
       fetch();
-      if (r.w < skip_below) continue;
+      if (r.y & 0xA00u) continue;  // the literal join's, or in the overflow list (generic kernel)
       n = r.y & 0xFFu;
-      if (r.y & 0x200u) continue;  // in the overflow list (generic kernel)
       s = r.x;
       selp = ((r.y & 0x100u) ? qsel_id : qsel) + r.z;
       AT(cand, 0) = m0;
@@ -1053,139 +1063,239 @@ __global__ void __launch_bounds__(kPhaseThreads) k_join_masks(
   if (lane == 0 && my_total) atomicAdd(d_total, static_cast<unsigned long long>(my_total));
 }
 
-// Join phase B, default form (sigmo_tuning.join_kernel = 2): the per-lane DFS
-// machine of k_join_masks with 9 bytes of shared state per level and lane,
-// base[j] (level j's candidates under the constraints of levels 0..j-2) and
-// pk[j] (level j's current pick).  The untried candidates of the current level
-// live in a register; a backtrack to level k recomputes them as base[k] AND
-// the constraint of pick[k-1]'s row, above pick[k].  Four 256-thread CTAs fit
-// on an SM.  A descent whose level-(k+2) base mask comes out empty is dropped:
-// every candidate of level k+1 would then extend to nothing, so the subtree
-// counts 0.  Work: each CTA first takes slots from its own contiguous region
-// of the chunk, so its lanes join neighbouring molecules whose adjacency rows
-// stay in L1 (measured: L1 hit rate 82 % against 33 % with one global work
-// cursor), then from a tail pool shared by all CTAs (pool16 sixteenths of the
-// chunk) that evens out the CTAs' finishing times.
-constexpr size_t kLaneBytesPerThread = kPhaseLevels * (8 + 1);
+// Join phase B, default form (sigmo_tuning.join_kernel = 2): a per-lane DFS in
+// which every turn is one candidate tried, by the same straight-line code, so
+// the 32 lanes of a warp stay together whatever their pairs are doing.
+//
+// What makes turns differ is the test of a level against all earlier picks
+// (one adjacency row per earlier level).  Here a lane keeps, for every vertex x
+// of its molecule, the number of placed levels whose row holds x, counted to 3
+// in two bit planes (b1 b0).  Level j with earlier neighbours S may take x
+// exactly when x is in the rows of S and in no other, i.e. in the rows of S and
+// counted |S| times; |S| is 1 or 2 at nearly every level of a molecular pattern
+// (otherwise the rows are walked):
+//     candidates = M[j] & row(S1) & row(S2) & (count == |S|)
+// Each level keeps its untried candidates, the planes before its pick and its
+// pick's row in shared memory, and a bit per level says where candidates are
+// left, so a turn starts at the deepest such level whatever the turn before
+// did: there are no separate moves back.  The last level is a popcount.
+// Trying candidates from the highest vertex down needs no bit reversal.
+//
+// Bound by the latency of the chain level -> candidate -> row -> candidates of
+// the next level at 15 warps per SM (ncu, 5.2 M pairs of queries up to 10
+// vertices: 55 % of the issue slots, 48 % of the integer pipe, 24 of 32 lanes
+// per instruction); the state is kept per level in shared memory rather than
+// recomputed because those loads use a pipe that is idle otherwise.  The form
+// before this one walked the earlier rows and went back level by level: 7 of 32
+// lanes per instruction; join stage of 100,000 molecules x 600 queries (6.86 M
+// pairs) 9.26 -> 4.79 ms find-all, of 10,007 ring systems x 100 automorphic
+// queries 14.8 -> 5.5 ms.
+//
+// A lane that ends its pair waits until `refill` lanes of its warp are idle, so
+// the (divergent) setup of new pairs is shared by several lanes.  Work: each
+// CTA first takes items from its own contiguous region of the chunk, so its
+// lanes join neighbouring molecules whose adjacency rows stay in L1, then from
+// a tail pool shared by all CTAs (pool16 sixteenths of the chunk).  An item is
+// one of the 1 << lparts parts of a pair (every 2^lparts-th root candidate):
+// pairs are split when there are fewer of them than lanes.
+//
+// LV: most vertices of a query (LV - 1 levels of state per lane).  Pairs of
+// longer queries are flagged and listed by k_pair_masks; with a list, the
+// items are its entries.  Queries of up to kDfsLevels vertices are 93 % of the
+// pairs and 97 % of the turns of the mixed query set, so the short form's
+// lanes carry 402 B instead of 654.  Its CTAs have 160 threads so that three
+// leave 60 KB of an SM to L1: with 192 (28 KB of L1) the rows fall out of it,
+// 5.9 instead of 4.8 ms.
+// Loads of data that is read once, kept out of L1 (which holds the adjacency
+// rows), and a hint that brings a later pair's data to L2.
+__device__ __forceinline__ uint4 load_once(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+struct Masks4 {
+  uint64_t m[4];
+};
+__device__ __forceinline__ Masks4 load_once(const Masks4* p) {  // 32-byte aligned
+  Masks4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(v.m[0]), "=l"(v.m[1]), "=l"(v.m[2]), "=l"(v.m[3]) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-template <bool EXACT, uint32_t DAW>
-__global__ void __launch_bounds__(kPhaseThreads, 4) k_join_lanes(
+template <uint32_t LV>
+constexpr uint32_t dfs_threads() { return LV <= kDfsLevels ? 160u : 96u; }
+template <uint32_t LV>
+constexpr size_t dfs_smem() { return dfs_threads<LV>() * (LV * 3 * 8 + (LV - 1) * (2 * 8 + 2)); }
+constexpr uint32_t kDfsAhead = 1024;  // slots ahead of the one taken that are brought to L2
+constexpr uint32_t kRefillAll = 12, kRefillFirst = 20;
+
+template <uint32_t LV, bool EXACT, uint32_t DAW>
+__global__ void __launch_bounds__(dfs_threads<LV>()) k_join_dfs(
     const uint64_t* __restrict__ masks, const uint4* __restrict__ rec, uint64_t slot0, uint64_t count,
-    const uint64_t* __restrict__ qsel, const uint64_t* __restrict__ qsel_id, const uint64_t* __restrict__ dadj,
-    uint32_t skip_below, int find_first, uint32_t pool16, unsigned long long* __restrict__ cursor,
-    uint64_t* __restrict__ counts, unsigned long long* __restrict__ d_total, JoinLimit lim) {
+    const uint32_t* __restrict__ list, const unsigned long long* __restrict__ list_len, uint32_t lparts,
+    const uint16_t* __restrict__ qmeta, const uint16_t* __restrict__ qmeta_id, const uint64_t* __restrict__ qsel,
+    const uint64_t* __restrict__ qsel_id, const uint64_t* __restrict__ dadj, int find_first,
+    uint32_t pool16, uint32_t refill, unsigned long long* __restrict__ cursor, uint64_t* __restrict__ counts,
+    unsigned long long* __restrict__ d_total, JoinLimit lim) {
   extern __shared__ uint64_t sm[];
-  __shared__ unsigned long long s_taken;  // slots of this CTA's region handed out so far
+  __shared__ unsigned long long s_taken;  // items of this CTA's region handed out so far
+  constexpr unsigned kAll = 0xFFFFFFFFu, T = dfs_threads<LV>(), D = LV - 1;
   const unsigned tid = threadIdx.x, lane = tid & 31u;
-  uint64_t* base = sm;
-  uint8_t* pk = reinterpret_cast<uint8_t*>(sm + kPhaseLevels * kPhaseThreads);
-#define AT(arr, lvl) arr[(lvl) * kPhaseThreads + tid]
-  const uint64_t shared_slots = count / 16u * (pool16 < 16u ? pool16 : 16u);
-  const uint64_t rlen = (count - shared_slots) / gridDim.x;
+  uint64_t* rest = sm + tid;                        // [LV][T] untried candidates of each level
+  uint64_t* p0 = sm + LV * T + tid;                 // [LV][T] planes before each level's pick (level 0: zero)
+  uint64_t* p1 = sm + 2 * LV * T + tid;
+  uint64_t* rows = sm + 3 * LV * T + tid;           // [LV - 1][T] row of each level's pick
+  uint64_t* nextm = sm + (3 * LV + D) * T + tid;    // [LV - 1][T] mask of the level after
+  uint16_t* meta = reinterpret_cast<uint16_t*>(sm + (3 * LV + 2 * D) * T) + tid;  // [LV - 1][T] query side of the level after
+  if (list) count = *list_len;
+  const uint64_t items = count << lparts;
+  const uint64_t shared_items = items / 16u * (pool16 < 16u ? pool16 : 16u);
+  const uint64_t rlen = (items - shared_items) / gridDim.x;
   const uint64_t pool0 = rlen * gridDim.x;
   const uint64_t r0 = static_cast<uint64_t>(blockIdx.x) * rlen;
   if (tid == 0) s_taken = 0;
+  p0[0] = p1[0] = 0;
   __syncthreads();
-  uint64_t steps = 0, my_total = 0, local = 0, cnt = 0, used = 0, rem = 0;
-  uint32_t n = 0, s = 0;
-  const uint64_t* selp = qsel;
-  int k = -1;
-  bool have = false;
-  // the next slot's record and first two level masks, loaded one pair ahead
-  uint4 pr = make_uint4(0, 0, 0, 0);
-  uint64_t pm0 = 0, pm1 = 0, plocal = 0;
-  bool pre = false;
-  auto fetch = [&]() {
-    pre = false;
-    if (join_stopped(lim)) return;
-    const unsigned am = __activemask();
-    const unsigned leader = __ffs(am) - 1, c = __popc(am);
-    const unsigned rank = __popc(am & ((1u << lane) - 1u));
-    unsigned long long rb = 0, pb = 0;
-    if (lane == leader) {
-      rb = atomicAdd(&s_taken, static_cast<unsigned long long>(c));
-      const uint64_t in_region = rb < rlen ? (rlen - rb < c ? rlen - rb : c) : 0ull;
-      if (c > in_region) pb = atomicAdd(cursor, static_cast<unsigned long long>(c - in_region));
-    }
-    rb = __shfl_sync(am, rb, leader);
-    pb = __shfl_sync(am, pb, leader);
-    const uint64_t in_region = rb < rlen ? (rlen - rb < c ? rlen - rb : c) : 0ull;
-    const uint64_t slot = rank < in_region ? r0 + rb + rank : pool0 + pb + (rank - in_region);
-    if (slot >= count) return;
-    plocal = slot;
-    pr = rec[slot];
-    pm0 = masks[slot * kPhaseLevels];
-    pm1 = masks[slot * kPhaseLevels + 1];
-    pre = true;
-  };
-  fetch();
+  uint64_t steps = 0, my_total = 0, slot = 0, cnt = 0;
+  uint32_t n = 0, qoff = 0;     // query size; query offset | identity-order flag << 31
+  uint32_t alive = 0;           // levels with untried candidates
+  const uint64_t* arow = dadj;  // adjacency rows of the lane's molecule
+  const bool limited = lim.budget != 0;
+  bool have = false, more = items != 0;  // more: the same for every lane of the warp
   for (;;) {
-    if (k < 0) {
-      if (have) {
+    const unsigned idle = __ballot_sync(kAll, alive == 0);
+    const unsigned nidle = __popc(idle);
+    if (nidle == 32u || (more && nidle >= refill)) {
+      if (alive == 0 && have) {
         if (find_first && cnt) cnt = 1;
-        counts[slot0 + local] = cnt;
-        my_total += cnt;
+        if (lparts == 0) {
+          counts[slot] = cnt;
+          my_total += cnt;
+        } else if (cnt) {  // counts[] zeroed by k_pair_masks
+          auto* at = reinterpret_cast<unsigned long long*>(counts + slot);
+          if (!find_first) atomicAdd(at, static_cast<unsigned long long>(cnt));
+          if (!find_first || atomicExch(at, 1ull) == 0ull) my_total += cnt;
+        }
         have = false;
       }
-      if (!pre) break;
-      local = plocal;
-      const uint4 r = pr;  // first data vertex, query size | flags, query offset, data graph
-      const uint64_t m0 = pm0, m1 = pm1;
-      fetch();
-      if (r.w < skip_below || (r.y & 0x200u)) continue;  // literal join, or the overflow list (generic kernel)
-      n = r.y & 0xFFu;
-      s = r.x;
-      selp = ((r.y & 0x100u) ? qsel_id : qsel) + r.z;
-      AT(base, 0) = m0;
-      AT(base, 1) = m1;
-      rem = m0;
-      used = 0;
-      cnt = 0;
-      k = 0;
-      have = true;
-      continue;
-    }
-    if (!rem) {  // back to level k-1: its untried candidates from its base and its parent's row
-      if (budget_spent(lim, steps)) break;
-      if (k == 0) {
-        k = -1;
-        continue;
+      if (more && __shfl_sync(kAll, join_stopped(lim) ? 1u : 0u, 0)) more = false;
+      if (!more) {
+        if (nidle == 32u) break;
+      } else {
+        unsigned long long rb = 0, pb = 0;
+        if (lane == 0) {
+          rb = atomicAdd(&s_taken, static_cast<unsigned long long>(nidle));
+          const uint64_t in_region = rb < rlen ? (rlen - rb < nidle ? rlen - rb : nidle) : 0ull;
+          if (nidle > in_region) pb = atomicAdd(cursor, static_cast<unsigned long long>(nidle - in_region));
+        }
+        rb = __shfl_sync(kAll, rb, 0);
+        pb = __shfl_sync(kAll, pb, 0);
+        const uint64_t in_region = rb < rlen ? (rlen - rb < nidle ? rlen - rb : nidle) : 0ull;
+        if (nidle > in_region && pool0 + pb + (nidle - in_region) >= items) more = false;
+        const unsigned rank = __popc(idle & ((1u << lane) - 1u));
+        const uint64_t item = rank < in_region ? r0 + rb + rank : pool0 + pb + (rank - in_region);
+        if (alive == 0 && item < items) {
+          uint64_t local = item >> lparts;
+          if (list) local = list[local] - slot0;
+          const uint64_t ahead = local + kDfsAhead;
+          if (!list && ahead < count) {
+            prefetch_l2(masks + ahead * kPhaseLevels);
+            prefetch_l2(rec + ahead);
+          }
+          const uint4 r = load_once(rec + local);  // first data vertex, query size | flags, query offset, query
+          // else the literal join's, or another list's
+          if (!(r.y & (0x800u | 0x200u)) && (LV > kDfsLevels || !(r.y & 0x400u))) {
+            n = r.y & 0xFFu;
+            slot = slot0 + local;
+            const bool ident = (r.y & 0x100u) != 0u;
+            qoff = r.z | (ident ? 0x80000000u : 0u);
+            arow = dadj + static_cast<uint64_t>(r.x) * DAW;
+            // all loads first, then the stores
+            const Masks4* mp = reinterpret_cast<const Masks4*>(masks + local * kPhaseLevels);
+            const uint4* qp = reinterpret_cast<const uint4*>((ident ? qmeta_id : qmeta) + static_cast<uint64_t>(r.w) * kPhaseLevels);
+            constexpr uint32_t kQuads = (LV + 3) / 4;
+            Masks4 mm[kQuads];
+            uint32_t qm[8];  // two levels each
+#pragma unroll
+            for (uint32_t j = 0; j < kQuads; ++j)
+              if (4 * j < n) mm[j] = load_once(mp + j);
+            const uint4 qa = load_once(qp);
+            uint4 qb = make_uint4(0, 0, 0, 0);
+            if (n > 8) qb = load_once(qp + 1);
+            qm[0] = qa.x, qm[1] = qa.y, qm[2] = qa.z, qm[3] = qa.w, qm[4] = qb.x, qm[5] = qb.y, qm[6] = qb.z, qm[7] = qb.w;
+            uint64_t root = mm[0].m[0];
+#pragma unroll
+            for (uint32_t j = 1; j < LV; ++j)
+              if (j < n) {
+                nextm[(j - 1) * T] = mm[j / 4].m[j % 4];
+                meta[(j - 1) * T] = static_cast<uint16_t>(qm[j / 2] >> (16u * (j % 2)));
+              }
+            if (lparts) {  // this part's root candidates: ranks = part mod 2^lparts
+              const uint32_t part = static_cast<uint32_t>(item) & ((1u << lparts) - 1u);
+              uint64_t keep = 0;
+              for (uint32_t i = 0; root; ++i, root &= root - 1)
+                if ((i & ((1u << lparts) - 1u)) == part) keep |= root & (0ull - root);
+              root = keep;
+            }
+            rest[0] = root;
+            alive = root ? 1u : 0u;
+            cnt = 0;
+            have = true;
+          }
+        }
       }
-      --k;
-      const uint32_t p = AT(pk, k);
-      if (EXACT) used &= ~(1ull << p);
-      uint64_t f = AT(base, k);
-      if (k > 0) {
-        const uint64_t rw = dadj[static_cast<uint64_t>(s + AT(pk, k - 1)) * DAW];
-        f &= ~(rw ^ (0ull - ((static_cast<uint32_t>(selp[k]) >> (k - 1)) & 1u)));
-        if (EXACT) f &= ~used;
+    }
+    if (alive == 0) continue;
+    // try the highest untried candidate t of the deepest level k that has one
+    const uint32_t k = 31u - __clz(alive);
+    uint64_t rem = rest[k * T];
+    const uint32_t hi = static_cast<uint32_t>(rem >> 32);
+    const uint32_t t = (31u - __clz(hi ? hi : static_cast<uint32_t>(rem))) + (hi ? 32u : 0u);
+    const uint64_t r = arow[t * DAW];
+    const uint64_t bit = 1ull << t;
+    rem ^= bit;
+    rest[k * T] = rem;
+    const uint64_t b0 = p0[k * T], b1 = p1[k * T];
+    uint64_t f = nextm[k * T];
+    const uint32_t q = meta[k * T];  // level k + 1's earlier neighbours i1, i2 (4 bits each), bit 8: two of them, bit 9: none or more than two
+    if (EXACT) meta[k * T] = static_cast<uint16_t>((q & 0x3FFu) | (t << 10));
+    uint64_t n0 = (b0 ^ r) | (b1 & b0), n1 = b1 | (b0 & r);  // count + 1 where r holds the vertex, at most 3
+    if (EXACT) {  // a placed vertex is never a candidate again
+      n0 |= bit;
+      n1 |= bit;
+    }
+    rows[k * T] = r;
+    if (!(q & 0x200u)) {
+      const uint64_t two = 0ull - static_cast<uint64_t>((q >> 8) & 1u);
+      f &= rows[(q & 15u) * T] & rows[((q >> 4) & 15u) * T];
+      f &= (n0 ^ two) & ~(n1 ^ two);
+    } else {
+      const uint64_t sel = ((qoff >> 31) ? qsel_id : qsel)[(qoff & 0x7FFFFFFFu) + k + 1u];
+      if (sel == 0) {
+        f &= ~(n0 | n1);
+      } else {
+        for (uint32_t i = 0; i <= k; ++i) {
+          f &= ~(rows[i * T] ^ (0ull - ((sel >> i) & 1ull)));
+          if (EXACT) f &= ~(1ull << (meta[i * T] >> 10));
+        }
       }
-      rem = f & ~((2ull << p) - 1ull);
-      continue;
     }
-    const uint32_t t = __ffsll(static_cast<long long>(rem)) - 1;
-    rem &= rem - 1;
-    const uint64_t rw = dadj[static_cast<uint64_t>(s + t) * DAW];
-    uint64_t nx = AT(base, k + 1) & ~(rw ^ (0ull - ((static_cast<uint32_t>(selp[k + 1]) >> k) & 1u)));
-    if (EXACT) nx &= ~(used | (1ull << t));
-    if (static_cast<uint32_t>(k + 2) >= n) {
-      cnt += __popcll(nx);
-      if (find_first && cnt) k = -1;
-      continue;
+    const bool last = k + 2u == n;
+    // level k + 1's state, used when it has candidates (of the last level: never)
+    rest[(k + 1u) * T] = f;
+    p0[(k + 1u) * T] = n0;
+    p1[(k + 1u) * T] = n1;
+    alive ^= (rem ? 0u : 1u << k) | (f && !last ? 2u << k : 0u);
+    const uint32_t found = last ? __popcll(f) : 0u;  // every candidate of the last level is a match
+    cnt += found;
+    if (find_first && found) alive = 0;
+    if (limited && !rem && budget_spent(lim, steps)) {
+      have = false;  // the count is incomplete
+      alive = 0;
     }
-    if (!nx) continue;
-    const uint32_t sl2 = static_cast<uint32_t>(selp[k + 2]);
-    uint64_t b2 = masks[local * kPhaseLevels + k + 2] & ~(rw ^ (0ull - ((sl2 >> k) & 1u)));
-    for (int i = 0; i < k && b2; ++i) b2 &= ~(dadj[static_cast<uint64_t>(s + AT(pk, i)) * DAW] ^ (0ull - ((sl2 >> i) & 1u)));
-    if (!b2) continue;  // level k+2 would be empty below every candidate of level k+1
-    AT(pk, k) = static_cast<uint8_t>(t);
-    if (EXACT) used |= 1ull << t;
-    AT(base, k + 2) = b2;
-    ++k;
-    rem = nx;
   }
-#undef AT
-  for (int o = 16; o; o >>= 1) my_total += __shfl_xor_sync(0xFFFFFFFFu, my_total, o);
+  for (int o = 16; o; o >>= 1) my_total += __shfl_xor_sync(kAll, my_total, o);
   if (lane == 0 && my_total) atomicAdd(d_total, static_cast<unsigned long long>(my_total));
 }
 
@@ -1243,7 +1353,7 @@ template <bool EXACT, uint32_t DAW>
 __global__ void __launch_bounds__(kFrontWarps * 32, 3) k_join_frontier(
     const uint64_t* __restrict__ masks, const uint4* __restrict__ rec, uint64_t slot0, uint64_t count,
     const uint64_t* __restrict__ qsel, const uint64_t* __restrict__ qsel_id, const uint64_t* __restrict__ dadj,
-    uint32_t skip_below, int find_first, uint32_t kChunk, unsigned long long* __restrict__ cursor,
+    int find_first, uint32_t kChunk, unsigned long long* __restrict__ cursor,
     uint64_t* __restrict__ counts, unsigned long long* __restrict__ d_total, JoinLimit lim) {
   extern __shared__ __align__(16) unsigned char front_raw[];
   uint64_t rounds = 0;
@@ -1290,8 +1400,8 @@ __global__ void __launch_bounds__(kFrontWarps * 32, 3) k_join_frontier(
         const uint32_t rank = __popc(F & lt);
         if (fr && rank < take) {
           const uint64_t local = next + rank;
-          const uint4 r = rec[local];  // first data vertex, query size | flags, query offset, data graph
-          if (r.w >= skip_below && !(r.y & 0x200u)) {
+          const uint4 r = rec[local];  // first data vertex, query size | flags, query offset, query graph
+          if (!(r.y & 0xA00u)) {
             const uint64_t c0 = masks[local * kPhaseLevels];
             if (c0) {
               w.pinfo[lane] = make_uint4(r.x, r.z | ((r.y & 0x100u) ? 0x80000000u : 0u), static_cast<uint32_t>(local), r.y & 0xFFu);
@@ -1553,24 +1663,31 @@ int launch_join_fast_planes(Queue* q, const Graph* query, const Graph* data, con
   const bool exact = q->opts.profile == kProfileExact;
   SIGMO_TRY(launch_query_order(const_cast<Graph*>(query)));
   const uint32_t skip = exact ? 0u : data->low_offset_graphs;
+  const sigmo_tuning& tn = q->tune;
+  const uint64_t chunk = std::min<uint64_t>(m->total, static_cast<uint64_t>(tn.mask_chunk_slots) << 20);
   void* buf = nullptr;
-  SIGMO_TRY(tmp_alloc(q, &buf, 256 + 4ull * m->total));
-  // [0] work cursor of the even chunks, [1] generic-join cursor, [2] overflow length, [3] odd chunks' cursor
+  SIGMO_TRY(tmp_alloc(q, &buf, 256 + 4ull * m->total + 8ull * chunk));
+  // [0] work cursor of the even chunks, [1] generic-join cursor, [2] overflow
+  // length, [3] odd chunks' cursor; then per chunk parity the long pairs'
+  // list length [4 + 2 i] and cursor [5 + 2 i]
   auto* ctr = static_cast<unsigned long long*>(buf);
   uint32_t* overflow = reinterpret_cast<uint32_t*>(static_cast<char*>(buf) + 256);
+  uint32_t* longs = overflow + m->total;  // [2][chunk]
   SIGMO_CUDA_TRY(cudaMemsetAsync(ctr, 0, 256, q->stream));
   auto* tot = reinterpret_cast<unsigned long long*>(d_total);
   // two-phase join, in chunks of slots, for the pairs of queries of <= 16
   // vertices and molecules of <= 64 atoms; the rest go to the overflow list
   int rc = SIGMO_OK;
-  bool two = false;
+  const bool frontier = tn.join_kernel == 1, dfs = tn.join_kernel == 2;
+  const bool has_long = dfs && query->max_nodes > kDfsLevels;
+  const bool has_overflow = query->max_nodes > kPhaseLevels || data->max_nodes > 64u;
+  // several chunks: even ones on the main stream, odd ones on the aux stream,
+  // each stream with its own mask buffer and work cursor, so one chunk's level
+  // masks run beside the previous chunk's persistent join
+  const bool two = m->total > chunk;
+  // the long pairs run beside the short ones
+  const cudaStream_t long_stream = two ? q->side : q->aux;
   {
-    const sigmo_tuning& tn = q->tune;
-    const uint64_t chunk = std::min<uint64_t>(m->total, static_cast<uint64_t>(tn.mask_chunk_slots) << 20);
-    // several chunks: even ones on the main stream, odd ones on the aux
-    // stream, each stream with its own mask buffer and work cursor, so one
-    // chunk's level masks run beside the previous chunk's persistent join
-    two = m->total > chunk;
     const size_t mbytes = 8ull * kPhaseLevels * chunk + 16ull * chunk;
     void* mbuf[2] = {nullptr, nullptr};
     rc = tmp_alloc(q, &mbuf[0], mbytes);
@@ -1579,18 +1696,21 @@ int launch_join_fast_planes(Queue* q, const Graph* query, const Graph* data, con
     if (!rc && two &&
         (cudaEventRecord(q->ev_aux_fork, q->stream) != cudaSuccess || cudaStreamWaitEvent(q->aux, q->ev_aux_fork, 0) != cudaSuccess))
       rc = fail(SIGMO_ERR_CUDA, "stream fork failed");
-    // the kernel for this batch's adjacency-row width and profile: the
-    // per-lane DFS machine, or the warp-cooperative frontier join
-    const bool frontier = tn.join_kernel == 1, lanes = tn.join_kernel == 2;
+    // the kernels for this batch's adjacency-row width and profile
     const size_t smem = frontier ? sizeof(FrontWarp) * kFrontWarps
-                        : lanes  ? kLaneBytesPerThread * kPhaseThreads
+                        : dfs    ? dfs_smem<kDfsLevels>()
                                  : static_cast<size_t>(kPhaseLevels) * kPhaseThreads * (2 * 8 + 1);
-    const unsigned block = frontier ? kFrontWarps * 32u : kPhaseThreads;
+    const unsigned block = frontier ? kFrontWarps * 32u : dfs ? dfs_threads<kDfsLevels>() : kPhaseThreads;
     void (*join_kernel)(const uint64_t*, const uint4*, uint64_t, uint64_t, const uint64_t*, const uint64_t*, const uint64_t*,
-                        uint32_t, int, uint32_t, unsigned long long*, uint64_t*, unsigned long long*, JoinLimit) = nullptr;
-#define SIGMO_PICK_JOIN(AWV)                                                                                \
-  join_kernel = frontier ? (exact ? k_join_frontier<true, AWV> : k_join_frontier<false, AWV>)              \
-                : lanes  ? (exact ? k_join_lanes<true, AWV> : k_join_lanes<false, AWV>)                    \
+                        int, uint32_t, unsigned long long*, uint64_t*, unsigned long long*, JoinLimit) = nullptr;
+    using DfsKernel = void (*)(const uint64_t*, const uint4*, uint64_t, uint64_t, const uint32_t*, const unsigned long long*,
+                               uint32_t, const uint16_t*, const uint16_t*, const uint64_t*, const uint64_t*, const uint64_t*,
+                               int, uint32_t, uint32_t, unsigned long long*, uint64_t*, unsigned long long*, JoinLimit);
+    DfsKernel dfs_short = nullptr, dfs_long = nullptr;
+#define SIGMO_PICK_JOIN(AWV)                                                                                     \
+  dfs_short = exact ? k_join_dfs<kDfsLevels, true, AWV> : k_join_dfs<kDfsLevels, false, AWV>;                    \
+  dfs_long = exact ? k_join_dfs<kPhaseLevels, true, AWV> : k_join_dfs<kPhaseLevels, false, AWV>;                 \
+  join_kernel = frontier ? (exact ? k_join_frontier<true, AWV> : k_join_frontier<false, AWV>)                   \
                          : (exact ? k_join_masks<true, AWV> : k_join_masks<false, AWV>)
     switch (data->adj_words) {
       case 1: SIGMO_PICK_JOIN(1); break;
@@ -1598,34 +1718,62 @@ int launch_join_fast_planes(Queue* q, const Graph* query, const Graph* data, con
       default: SIGMO_PICK_JOIN(4); break;
     }
 #undef SIGMO_PICK_JOIN
-    if (!rc) rc = allow_max_dynamic_smem(reinterpret_cast<const void*>(join_kernel), q->device);
+    if (!rc)
+      rc = allow_max_dynamic_smem(dfs ? reinterpret_cast<const void*>(dfs_short) : reinterpret_cast<const void*>(join_kernel), q->device);
+    if (!rc && has_long) rc = allow_max_dynamic_smem(reinterpret_cast<const void*>(dfs_long), q->device);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, q->device);
+    // persistent CTAs; `reserve` slots stay free for a kernel running beside
+    // them.  k_join_dfs keeps at most three resident: a fourth would start its
+    // region only when another CTA has ended
+    const unsigned full = static_cast<unsigned>(sms) * (dfs ? std::min(tn.join_blocks_per_sm, 3u) : tn.join_blocks_per_sm);
+    const unsigned grid = full > reserve + static_cast<unsigned>(sms) ? full - reserve : full;
+    // fewer pairs than lanes: every pair in up to 16 parts by root candidate
+    uint32_t lparts = 0;
+    while (dfs && lparts < 4 && (m->total << (lparts + 1)) <= static_cast<uint64_t>(grid) * block) ++lparts;
+    const uint32_t long_parts = find_first ? lparts : std::max(lparts, 1u);
     uint64_t c = 0;
     for (uint64_t slot0 = 0; slot0 < m->total && !rc; slot0 += chunk, ++c) {
       const uint64_t cnt = std::min<uint64_t>(chunk, m->total - slot0);
-      const cudaStream_t st = streams[c & 1];
-      auto* masks = static_cast<uint64_t*>(mbuf[c & 1]);
+      const uint32_t par = c & 1;
+      const cudaStream_t st = streams[par];
+      auto* masks = static_cast<uint64_t*>(mbuf[par]);
       auto* recs = reinterpret_cast<uint4*>(masks + kPhaseLevels * chunk);
-      unsigned long long* cursor = ctr + ((c & 1) ? 3 : 0);
+      unsigned long long* cursor = ctr + (par ? 3 : 0);
+      unsigned long long* lctr = ctr + 4 + 2 * par;
+      uint32_t* llist = longs + par * chunk;
+      if (c >= 2 && (cudaMemsetAsync(cursor, 0, 8, st) != cudaSuccess || cudaMemsetAsync(lctr, 0, 16, st) != cudaSuccess))
+        rc = fail(SIGMO_ERR_CUDA, "memset failed");
+      if (rc) break;
       k_pair_masks<<<grid_for(cnt, 256, 148u * 16u), 256, 0, st>>>(
           planes, planes_rows, data->adj_words, pp.prog_off, prog, pp.cls, query->graph_offsets, query->qorder, query->sym,
-          data->graph_offsets, data->sym, m->indices, m->pair_graph, slot0, cnt, masks, recs, skip, overflow, ctr + 2,
-          m->counts);
+          data->graph_offsets, data->sym, m->indices, m->pair_graph, slot0, cnt, masks, recs, skip, overflow, ctr + 2, llist,
+          lctr, m->counts, lparts != 0);
       rc = check_launch(q, "k_pair_masks");
-      if (!rc && cudaEventRecord(q->ev_masks[c & 1], st) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
-      if (!rc && cudaMemsetAsync(cursor, 0, 8, st) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "memset failed");
-      if (!rc) {
-        // persistent CTAs; `reserve` slots stay free for a kernel running beside them
-        const unsigned full = static_cast<unsigned>(sms) * tn.join_blocks_per_sm;
-        const unsigned grid = full > reserve + static_cast<unsigned>(sms) ? full - reserve : full;
-        // the per-lane machine and the frontier join take join_chunk slots per
-        // grab; k_join_lanes takes its pool share
-        join_kernel<<<grid, block, smem, st>>>(masks, recs, slot0, cnt, query->qsel, query->qsel_id, data->adj, skip,
-                                               find_first, lanes ? tn.join_pool : tn.join_chunk, cursor, m->counts, tot,
-                                               join_limit(q));
-        rc = check_launch(q, frontier ? "k_join_frontier" : lanes ? "k_join_lanes" : "k_join_masks");
+      if (!rc && cudaEventRecord(q->ev_masks[par], st) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
+      if (!rc && has_long) {
+        const unsigned lblock = dfs_threads<kPhaseLevels>();
+        if (cudaStreamWaitEvent(long_stream, q->ev_masks[par], 0) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "stream fork failed");
+        if (!rc) {
+          dfs_long<<<static_cast<unsigned>(sms), lblock, dfs_smem<kPhaseLevels>(), long_stream>>>(
+              masks, recs, slot0, cnt, llist, lctr, long_parts, query->qmeta, query->qmeta_id, query->qsel,
+              query->qsel_id, data->adj, find_first, 8u, find_first ? kRefillFirst : kRefillAll, lctr + 1, m->counts, tot, join_limit(q));
+          rc = check_launch(q, "k_join_dfs<long>");
+        }
+        if (!rc && cudaEventRecord(q->ev_long[par], long_stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
       }
+      if (!rc) {
+        if (dfs)
+          dfs_short<<<grid, block, smem, st>>>(masks, recs, slot0, cnt, nullptr, nullptr, lparts, query->qmeta, query->qmeta_id,
+                                               query->qsel, query->qsel_id, data->adj, find_first, tn.join_pool,
+                                               find_first ? kRefillFirst : kRefillAll, cursor, m->counts, tot, join_limit(q));
+        else  // join_chunk slots per grab
+          join_kernel<<<grid, block, smem, st>>>(masks, recs, slot0, cnt, query->qsel, query->qsel_id, data->adj, find_first,
+                                                 tn.join_chunk, cursor, m->counts, tot, join_limit(q));
+        rc = check_launch(q, frontier ? "k_join_frontier" : dfs ? "k_join_dfs" : "k_join_masks");
+      }
+      // the chunk's buffers are free again once its long pairs are joined too
+      if (has_long && cudaStreamWaitEvent(st, q->ev_long[par], 0) != cudaSuccess) rc = rc ? rc : fail(SIGMO_ERR_CUDA, "stream join failed");
     }
     // the aux stream joins the main one before its buffer is released
     if (two && (cudaEventRecord(q->ev_aux_join, q->aux) != cudaSuccess ||
@@ -1635,7 +1783,7 @@ int launch_join_fast_planes(Queue* q, const Graph* query, const Graph* data, con
     dev_free(q, mbuf[1]);
   }
   const cudaStream_t main_stream = q->stream;
-  const bool side = !q->tune.overflow_serial;
+  const bool side = has_overflow && !q->tune.overflow_serial;
   if (!rc && side) {
     // the overflow list is complete after the last Phase A of each stream: its
     // pairs run on the side stream, overlapping Phase B
@@ -1644,7 +1792,7 @@ int launch_join_fast_planes(Queue* q, const Graph* query, const Graph* data, con
       rc = fail(SIGMO_ERR_CUDA, "stream fork failed");
     q->stream = q->side;
   }
-  if (!rc) {
+  if (!rc && has_overflow) {
     // the overflow list through the generic kernel
     const unsigned block = 128;
     const unsigned grid = q->tune.overflow_blocks;
