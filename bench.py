@@ -536,8 +536,8 @@ def run_sigmo(args, rank, world, local):
     jk = JOIN_KERNELS.get(queue.get_tuning()["join_kernel"], "k_join_dfs")
     jkey = f"join:{jk}"
     l1, l2 = traffic_for(jkey, args.workload, "l1_hit_rate"), traffic_for(jkey, args.workload, "l2_hit_rate")
-    roof = {"kernel": f"join stage: k_pair_masks + {jk} (side stream: k_join_fast for queries over 16 vertices, "
-                      "k_join_literal_small for the data graphs starting below vertex 256)",
+    roof = {"kernel": f"join stage: k_pair_masks + {jk} (beside it: k_join_wide for queries over 16 vertices, "
+                      "k_join_literal_sets for the data graphs starting below vertex 256)",
             "bound": "hbm", "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
             "frac": round(achieved / hbm, 4), "traffic": traffic_for(jkey, args.workload),
             "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs, burst copy)" if peak_kind == "measured" else peak_kind,

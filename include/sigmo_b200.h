@@ -127,11 +127,12 @@ typedef struct sigmo_tuning {
                                     keeps at most 3 resident)                                   */
   uint32_t join_chunk;           /* GMCR slots a lane takes per work grab, 1..64 (4; join_kernel
                                     0 and 1)                                                    */
-  uint32_t overflow_blocks;      /* CTAs of the join for queries over 16 vertices (1184)        */
+  uint32_t overflow_blocks;      /* CTAs of the join for queries over 16 vertices and molecules
+                                    over 64 atoms (1184)                                        */
   uint32_t overflow_serial;      /* 0 (default): run those beside the main join; 1: after it       */
   uint32_t mask_chunk_slots;     /* GMCR slots per level-mask pass, in 2^20 units, 1..64 (8)     */
-  uint32_t overflow_split;       /* work items per pair of those queries, each taking every
-                                    split-th root candidate, 1..64 (16)                          */
+  uint32_t overflow_split;       /* accepted, 1..64 (16), and without effect: every root candidate
+                                    of those pairs is a work item of its own                     */
   uint32_t join_kernel;          /* 2 (default): per-lane DFS whose turns are all alike (one
                                     candidate each, neighbour counts instead of a walk over the
                                     earlier levels) with CTA-local slot regions; 0: per-lane DFS

@@ -806,7 +806,26 @@ int sigmo_join_candidates(sigmo_queue_t q, sigmo_graph_t query, sigmo_graph_t da
   SIGMO_TRY(dev_alloc(q, reinterpret_cast<void**>(&d_total), 8));
   SIGMO_CUDA_TRY(cudaMemsetAsync(d_total, 0, 8, q->stream));
   int rc = join_status_reset(q);
-  if (!rc) rc = launch_join_literal(q, query, data, c, m, find_first, 0, data->num_graphs, d_total, 0, 0xFFFFFFFFu);
+  MaskSource src;
+  src.bits = c->bits;
+  src.Wp = c->Wp;
+  src.prof = q->opts.profile;
+  if (!rc) {
+    // The reference's search is restated step by step where its result depends
+    // on the order of the steps: under REF_X86, under REF_PTX for graphs that
+    // start below vertex 256, and for graphs too large for the local sets.
+    // Elsewhere the count is the number of tuples, and the batched form's join
+    // takes the pairs (bits as its source of candidates).
+    const bool sets = q->opts.profile != kProfileX86 && data->max_nodes <= 64u * kMaxAdjWords && query->max_nodes <= kMaxQueryNodes;
+    uint32_t low = data->num_graphs;
+    if (sets) {
+      low = 0;
+      if (q->opts.profile == kProfilePtx)
+        while (low < data->num_graphs && data->host_graph_offsets[low] < kLowOffsetLimit) ++low;
+    }
+    rc = sets ? launch_join(q, query, data, src, m, find_first, low, d_total)
+              : launch_join_literal(q, query, data, src, m, find_first, 0, low, d_total, 0, 0xFFFFFFFFu);
+  }
   if (!rc) rc = stage_end(q);
   if (!rc) rc = join_status_fetch(q);
   if (!rc) {

@@ -432,19 +432,6 @@ struct Events {
   }
 };
 
-// The literal join of graphs [0, L): one launch over every admitted query, or
-// (serving) one per request's query range, so a request's counts do not
-// depend on the other requests of its batch (the reference's work-items
-// carry DFS state from one pair to the next, isomorphism.hpp:309).
-int join_literal_ranges(Queue* q, Graph* query, Graph* data, const Candidates* c, Gmcr* m, int find_first, uint32_t L,
-                        uint64_t* d_total, const BatchedRun& run) {
-  if (!run.query_ranges || run.nranges == 0)
-    return launch_join_literal(q, query, data, c, m, find_first, 0, L, d_total, 0, 0xFFFFFFFFu);
-  for (uint32_t r = 0; r < run.nranges; ++r)
-    SIGMO_TRY(launch_join_literal(q, query, data, c, m, find_first, 0, L, d_total, run.query_ranges[r], run.query_ranges[r + 1]));
-  return SIGMO_OK;
-}
-
 // The bitset route: fused filter writes the final bitset (all words), GMCR
 // and the join read it.  Used when the caller asks for the bitset, or when a
 // batch does not fit the plane route.
@@ -467,9 +454,13 @@ int batched_bitset(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
   if (!rc) rc = launch_gmcr(q, query, data, c, m, true, 0);
   if (!rc && cudaEventRecord(ev.e[3], q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
   const bool exact = q->opts.profile == kProfileExact;
-  if (!rc && !exact) rc = join_literal_ranges(q, query, data, c, m, find_first, std::min(data->low_offset_graphs, data->num_graphs),
-                                             d_total, run);
-  if (!rc) rc = launch_join_fast(q, query, data, c, m, find_first, d_total);
+  MaskSource src;
+  src.bits = c->bits;
+  src.Wp = c->Wp;
+  src.prof = q->opts.profile;
+  if (!rc)
+    rc = launch_join(q, query, data, src, m, find_first, exact ? 0u : std::min(data->low_offset_graphs, data->num_graphs), d_total,
+                     run.query_ranges, run.nranges);
   dev_free(q, buf);
   return rc;
 }
@@ -483,13 +474,10 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
     return cudaEventRecord(ev.e[i], q->stream) == cudaSuccess ? SIGMO_OK : fail(SIGMO_ERR_CUDA, "event record failed");
   };
   PlaneProgram& pp = query->pp;
-  const uint64_t N = data->total_nodes, Qn = query->total_nodes;
+  const uint64_t N = data->total_nodes;
   const uint32_t G = data->num_graphs, GW = (G + 31u) / 32u, AW = data->adj_words;
   const bool exact = q->opts.profile == kProfileExact;
   const uint32_t L = exact ? 0u : std::min(data->low_offset_graphs, G);
-  // words of the bitset the literal join reads (graphs [0, L))
-  const uint64_t Wlow = L ? (static_cast<uint64_t>(data->host_graph_offsets[L]) + 31) / 32 : 0;
-  const uint64_t Wlp = (Wlow + 31) / 32 * 32;
   auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
   const ResidentPlanes* rp = run.resident;
   const uint64_t b_dsig = run.dsig ? 0 : 8ull * R * N, b_planes = rp ? 0 : 8ull * GW * pp.K * AW * 32,
@@ -514,9 +502,8 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
     for (size_t i = 0; i < rprog.size(); ++i) rprog[i] = static_cast<uint16_t>(row_map[pp.h_prog[i]]);
   }
   const uint64_t b_map = 4ull * row_map.size() + 2ull * rprog.size();
-  const uint64_t b_lplanes = 16ull * 16 * R * Wlp, b_lbits = 4ull * Qn * Wlp;
   void* buf = nullptr;
-  SIGMO_TRY(tmp_alloc(q, &buf, al(b_dsig) + al(b_planes) + al(b_ne) + al(b_lplanes) + al(b_lbits) + al(b_map) + 256));
+  SIGMO_TRY(tmp_alloc(q, &buf, al(b_dsig) + al(b_planes) + al(b_ne) + al(b_map) + 256));
   char* p = static_cast<char*>(buf);
   uint64_t* dsig = run.dsig ? const_cast<uint64_t*>(run.dsig) : reinterpret_cast<uint64_t*>(p);
   p += al(b_dsig);
@@ -525,10 +512,6 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
   uint32_t* admit = reinterpret_cast<uint32_t*>(p);  // [query graphs][GW], then per-graph counts [G]
   uint32_t* adm_counts = admit + static_cast<uint64_t>(query->num_graphs) * GW;
   p += al(b_ne);
-  uint32_t* lplanes = reinterpret_cast<uint32_t*>(p);
-  p += al(b_lplanes);
-  uint32_t* lbits = reinterpret_cast<uint32_t*>(p);
-  p += al(b_lbits);
   uint32_t* d_row_map = reinterpret_cast<uint32_t*>(p);
   uint16_t* d_rprog = reinterpret_cast<uint16_t*>(d_row_map + row_map.size());
   int rc = run.dsig ? SIGMO_OK : launch_sig_all(q, data, R, dsig);
@@ -553,43 +536,16 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
   // arrays (the replay checks that it did not change)
   if (!rc) rc = launch_gmcr_from_admit(q, query, data, admit, adm_counts, m, !run.capture, run.capture ? m->total : 0);
   if (!rc) rc = mark(3);
-  const bool literal = !rc && L && m->total;
-  uint32_t reserve = 0;
-  bool forked = false;  // the side stream joined this call's work
-  if (literal) {
-    // REF_PTX: graphs starting below vertex 256 keep the reference's live
-    // `visited` bitset, so they take the literal join on the bitset words it
-    // reads.  The words are computed here (a few KB per query vertex); the
-    // literal join then runs on the side stream, overlapping the fast join,
-    // which leaves one CTA slot per literal block free so that the literal
-    // join does not wait behind its persistent CTAs.
-    for (uint32_t r = 0; r < R && !rc; ++r)
-      rc = launch_sig_planes(q, dsig + static_cast<uint64_t>(r) * N, N, Wlp, lplanes + static_cast<uint64_t>(r) * 16 * 4 * Wlp);
-    if (!rc) rc = launch_fused_filter_raw(q, query->node_labels, pp.qsig_all, Qn, data->node_labels, N, lplanes, Wlp, R, lbits);
-    const cudaStream_t main_stream = q->stream;
-    if (!rc && (cudaEventRecord(q->ev_fork, main_stream) != cudaSuccess || cudaStreamWaitEvent(q->side, q->ev_fork, 0) != cudaSuccess))
-      rc = fail(SIGMO_ERR_CUDA, "stream fork failed");
-    forked = !rc;
-    q->stream = q->side;
-    reserve = std::min<uint32_t>(L, 148u);
-    Candidates view;
-    view.q = q;
-    view.rows = Qn;
-    view.targets = N;
-    view.W = Wlow;
-    view.Wp = Wlp;
-    view.bits = lbits;
-    if (!rc) rc = join_literal_ranges(q, query, data, &view, m, find_first, L, d_total, run);
-    q->stream = main_stream;
-  }
-  if (!rc)
-    rc = rp ? launch_join_fast_planes(q, query, data, pp, rp->planes, rp->rows, d_rprog, m, find_first, d_total, reserve)
-            : launch_join_fast_planes(q, query, data, pp, planes, pp.K, pp.prog, m, find_first, d_total, reserve);
-  // join the side stream back before the scratch is released and the total
-  // read (only when this call forked it: a CUDA-graph capture may wait only
-  // on events of streams that joined the capture)
-  if (forked && (cudaEventRecord(q->ev_join, q->side) != cudaSuccess || cudaStreamWaitEvent(q->stream, q->ev_join, 0) != cudaSuccess))
-    rc = rc ? rc : fail(SIGMO_ERR_CUDA, "stream join failed");
+  // REF_PTX: graphs starting below vertex 256 keep the reference's live
+  // `visited` bitset, so they take the literal join
+  MaskSource src;
+  src.prof = q->opts.profile;
+  src.planes = rp ? rp->planes : planes;
+  src.K = rp ? rp->rows : pp.K;
+  src.prog_off = pp.prog_off;
+  src.prog = rp ? d_rprog : pp.prog;
+  src.cls = pp.cls;
+  if (!rc) rc = launch_join(q, query, data, src, m, find_first, L, d_total, run.query_ranges, run.nranges);
   dev_free(q, buf);
   return rc;
 }
@@ -839,7 +795,6 @@ extern "C" int sigmo_autotune(sigmo_queue_t q, sigmo_graph_t query, sigmo_graph_
       {&sigmo_tuning::join_chunk, {1, 2, 4, 8, 16}},
       {&sigmo_tuning::overflow_blocks, {148, 296, 592, 1184, 2368}},
       {&sigmo_tuning::mask_chunk_slots, {2, 8, 32}},
-      {&sigmo_tuning::overflow_split, {1, 4, 16, 32}},
   };
   for (const Axis& ax : axes) {
     for (uint32_t v : ax.values) {

@@ -247,19 +247,35 @@ int launch_fused_filter(Queue* q, const Graph* query, const Graph* data, uint32_
                         const uint32_t* planes_all, Candidates* c);
 int launch_gmcr(Queue* q, const Graph* query, const Graph* data, const Candidates* c, Gmcr* m, bool sync_total,
                 uint64_t capacity_hint);
+// Where a join takes a pair's candidate sets from: the candidate bitset, or
+// the batched form's planes (planes: [graph / 32][K][AW][32]; prog: the class
+// programs as row indices into it, pp.prog for the per-batch planes).
+struct MaskSource {
+  const uint32_t* bits = nullptr;
+  uint64_t Wp = 0;
+  int prof = 0;  // range masks of the bitset's words
+  const uint64_t* planes = nullptr;
+  uint32_t K = 0;
+  const uint32_t* prog_off = nullptr;
+  const uint16_t* prog = nullptr;
+  const uint32_t* cls = nullptr;
+};
 // Query graphs [q_begin, q_end) of each segment only (the full range: 0, ~0u).
-int launch_join_literal(Queue* q, const Graph* query, const Graph* data, const Candidates* c, Gmcr* m, int find_first,
+int launch_join_literal(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first,
                         uint32_t graph_begin, uint32_t graph_end, uint64_t* d_total, uint32_t q_begin, uint32_t q_end);
-int launch_join_fast(Queue* q, const Graph* query, const Graph* data, const Candidates* c, Gmcr* m, int find_first,
-                     uint64_t* d_total);
 int launch_join_wildcard(Queue* q, const Graph* query, const Graph* data, const Candidates* c, Gmcr* m, int find_first,
                          uint64_t* d_total);
-// planes: [graph / 32][planes_rows][AW][32]; prog: the class programs as
-// row indices into it (pp.prog for the per-batch planes).
-// reserve: persistent join CTA slots left free for a kernel running beside it
-int launch_join_fast_planes(Queue* q, const Graph* query, const Graph* data, const PlaneProgram& pp, const uint64_t* planes,
-                            uint32_t planes_rows, const uint16_t* prog, Gmcr* m, int find_first, uint64_t* d_total,
-                            uint32_t reserve = 0);
+// Every pair of data graphs from `skip` on (molecules of up to 64 * kMaxAdjWords
+// vertices; REF_PTX: starting at vertex 256 or above, where the reference's
+// count does not depend on the order of its search).  reserve: persistent join
+// CTA slots left free for a kernel running beside it.
+int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first, uint32_t skip,
+                      uint64_t* d_total, uint32_t reserve = 0);
+// Every pair: the literal join of data graphs [0, literal) on the side stream
+// (once per range of query graphs when `ranges` holds nranges + 1 boundaries),
+// beside launch_join_pairs for the rest; the main stream waits for both.
+int launch_join(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first, uint32_t literal,
+                uint64_t* d_total, const uint32_t* ranges = nullptr, uint32_t nranges = 0);
 int launch_gmcr_from_ne(Queue* q, const Graph* query, const Graph* data, const uint32_t* NE, const uint32_t* cls, Gmcr* m,
                         bool sync_total, uint64_t capacity_hint);
 int launch_planes_admit(Queue* q, const Graph* query, const Graph* data, const uint64_t* sig_all, uint32_t R,
@@ -282,8 +298,6 @@ int launch_gmcr_from_admit(Queue* q, const Graph* query, const Graph* data, cons
                            Gmcr* m, bool sync_total, uint64_t capacity_hint);
 // Vertices per label of a graph batch (host copy, computed once).
 int ensure_label_hist(Queue* q, Graph* g);
-int launch_fused_filter_raw(Queue* q, const uint8_t* qlab, const uint64_t* qsig_all, uint64_t Qn, const uint8_t* dlab,
-                            uint64_t N, const uint32_t* planes_all, uint64_t Wstride, uint32_t R, uint32_t* bits);
 int launch_row_counts(Queue* q, const Candidates* c, uint32_t* d_counts);
 int build_plane_program(Queue* q, Graph* query, uint32_t R);
 // Fills zero fields of a tuning with the defaults and checks the ranges.

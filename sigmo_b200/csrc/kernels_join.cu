@@ -85,6 +85,50 @@ __device__ __forceinline__ bool data_neighbor(uint32_t a, uint32_t b, uint32_t s
   return false;
 }
 
+// Graph-local candidate set of one bitset row for data graph [s, e): bit t =
+// global candidate s + t, after the profile's range masks.
+template <int AW>
+__device__ __forceinline__ void extract_local(const uint32_t* __restrict__ row, uint32_t s, uint32_t e, int prof, uint64_t* out) {
+#pragma unroll
+  for (int k = 0; k < AW; ++k) out[k] = 0;
+  const uint32_t i0 = s >> 5, i1 = (e + 31u) >> 5;
+  for (uint32_t i = i0; i < i1; ++i) {
+    uint32_t wv = row[i] & range_mask(i, s, e, prof);
+    if (!wv) continue;
+    int32_t off = static_cast<int32_t>(i << 5) - static_cast<int32_t>(s);
+    if (off < 0) {
+      wv >>= static_cast<uint32_t>(-off);
+      off = 0;
+    }
+    const uint32_t k = static_cast<uint32_t>(off) >> 6, sh = static_cast<uint32_t>(off) & 63u;
+#pragma unroll
+    for (int kk = 0; kk < AW; ++kk) {
+      if (static_cast<uint32_t>(kk) == k) out[kk] |= static_cast<uint64_t>(wv) << sh;
+      if (sh > 32u && static_cast<uint32_t>(kk) == k + 1) out[kk] |= static_cast<uint64_t>(wv) >> (64u - sh);
+    }
+  }
+}
+
+// Candidate set of query vertex v (global id) in data graph g = [s, e) from
+// either source.  AW words are written; dAW is the planes' words per set.
+template <int AW>
+__device__ __forceinline__ void source_mask(const MaskSource& src, uint32_t dAW, uint32_t v, uint32_t g, uint32_t s, uint32_t e,
+                                            uint64_t* out) {
+  if (!src.planes) {
+    extract_local<AW>(src.bits + static_cast<uint64_t>(v) * src.Wp, s, e, src.prof, out);
+    return;
+  }
+  const uint64_t* base = src.planes + static_cast<uint64_t>(g >> 5) * src.K * dAW * 32 + (g & 31u);
+#pragma unroll
+  for (int w = 0; w < AW; ++w) out[w] = ~0ull;
+  const uint32_t c = src.cls[v], e1 = src.prog_off[c + 1];
+  for (uint32_t i = src.prog_off[c]; i < e1; ++i) {
+    const uint64_t* row = base + static_cast<uint64_t>(src.prog[i]) * dAW * 32;
+#pragma unroll
+    for (int w = 0; w < AW; ++w) out[w] &= row[32 * w];
+  }
+}
+
 struct Frame {
   uint32_t depth;
   uint32_t idx;
@@ -133,7 +177,6 @@ struct PairCands {
   }
 };
 
-template <bool EXACT>
 __global__ void k_join_literal(const uint32_t* __restrict__ bits, uint64_t Wp, int prof,
                                const uint32_t* __restrict__ qgoff, const uint64_t* __restrict__ qadj,
                                const uint32_t* __restrict__ dgoff, const uint64_t* __restrict__ dadj, uint32_t dAW,
@@ -215,7 +258,7 @@ __global__ void k_join_literal(const uint32_t* __restrict__ bits, uint64_t Wp, i
       Frame stack[kMaxQueryNodes + 2];
       uint32_t top = 0;
       stack[top++] = {0u, 0u};
-      if (!EXACT) {
+      {
         uint64_t visited = 0;  // Bitset<uint64_t>{offset = s}
         while (top > 0) {
           const Frame fr = stack[top - 1];
@@ -278,47 +321,6 @@ __global__ void k_join_literal(const uint32_t* __restrict__ bits, uint64_t Wp, i
             push_mask(qn + 1);
           }
         }
-      } else {
-        // Injective DFS with clean backtracking (graphs <= 256 vertices).
-        uint64_t used[kMaxAdjWords] = {0, 0, 0, 0};
-        uint32_t placed[kMaxQueryNodes + 1];
-#pragma unroll 1
-        for (uint32_t k = 0; k <= n; ++k) placed[k] = 0xFFFFFFFFu;
-        while (top > 0) {
-          const Frame fr = stack[top - 1];
-          const uint32_t qn = fr.depth;
-          if (qn == n) {
-            ++found;
-            --top;
-            if (find_first) break;
-            continue;
-          }
-          if (placed[qn] != 0xFFFFFFFFu) {
-            const uint32_t t = placed[qn] - s;
-            used[t >> 6] &= ~(1ull << (t & 63u));
-            placed[qn] = 0xFFFFFFFFu;
-          }
-          if (fr.idx >= count_of(qn)) {
-            --top;
-            if (budget_spent(lim, steps)) {
-              stop = true;
-              break;
-            }
-            continue;
-          }
-          const uint32_t cand = cand_of(qn, fr.idx);
-          stack[top - 1].idx++;
-          const uint32_t t = cand - s;
-          if ((used[t >> 6] >> (t & 63u)) & 1ull) continue;
-          if (valid(qn, cand)) {
-            mapping[qn] = cand;
-            if (small) rowc[qn] = dadj[static_cast<uint64_t>(cand) * dAW];
-            placed[qn] = cand;
-            used[t >> 6] |= 1ull << (t & 63u);
-            stack[top++] = {qn + 1, 0u};
-            push_mask(qn + 1);
-          }
-        }
       }
       if (stop) break;
       counts[seg0 + it] = found;
@@ -338,12 +340,13 @@ __global__ void k_join_literal(const uint32_t* __restrict__ bits, uint64_t Wp, i
   }
 }
 
-// k_join_literal for its common case: every data graph of the launch has at
-// most 64 vertices and every query at most kLitLevels.  The same DFS, step for
-// step, with the per-level state of each thread in shared memory
-// ([level][thread], no local-memory stack):
+// k_join_literal for graphs of at most 64 * AW vertices (and, under REF_X86, of
+// at most 64).  The same DFS, step for step, on graph-local sets, with the
+// per-level state of each thread in shared memory ([level][thread]) for AW = 1
+// and queries of at most kLitLevels vertices (SMEM), else in local memory:
 //   cm[j]   the pair's range-masked candidates of query vertex j as graph-local
-//           bits (candidates.hpp:86-162; at most 3 bitset words per graph);
+//           bits (candidates.hpp:86-162), from the candidate bitset or from the
+//           batched form's planes (the same sets);
 //   rem[j]  the candidates the frame at depth j has still to try, taken in
 //           ascending order like getCandidateAt(idx) for idx = 0, 1, ...
 //           Only those passing isValidMapping are kept (its result depends on
@@ -353,33 +356,43 @@ __global__ void k_join_literal(const uint32_t* __restrict__ bits, uint64_t Wp, i
 //   map[j]  mapping[j] as a local id, carried across the thread's pairs of a
 //           data graph like the reference's private array (isomorphism.hpp:309);
 //           a fresh work-item's mapping[] holds global vertex 0, which is
-//           local 0 of a graph starting at vertex 0 and kLitOutside (no
-//           bit of the graph) otherwise.
-// REF_PTX keeps the reference's `visited` bookkeeping (utils.hpp:64-96,
-// isomorphism.hpp:346-369): a frame that runs out unsets only mapping[depth]
-// (perhaps stale), and the set is cleared when the DFS is back at depth 0.
-// EXACT runs the injective DFS: the pick of a frame is unset when its child
-// frame runs out.  The last query vertex is placed in one step, as in
+//           local 0 of a graph starting at vertex 0 and kLitOutside (a local
+//           id that never has a bit in the visited set) otherwise.
+// The reference's `visited` bookkeeping (utils.hpp:64-96,
+// isomorphism.hpp:346-369) is kept: a frame that runs out unsets only
+// mapping[depth] (perhaps stale), and the set is cleared when the DFS is back
+// at depth 0.  Its 64 bits hold local ids below 64 (REF_PTX: whose global id is
+// below 256).  The last query vertex is placed in one step, as in
 // k_join_literal.
+//
+// A serial chain per pair: bound by the latency of a step, so the sets are
+// taken from the planes where the caller has them.  (Writing them as bitset
+// words first took seven more launches, 130 us before the join of a batch of
+// any size.)  Molecules over 64 atoms and queries over 32 vertices used to
+// take k_join_literal's candidate-by-candidate form: 3.7 ms for the first ten
+// molecules of 60,000 x 500 uneven pairs, against 0.5 ms here.
 constexpr uint32_t kLitLevels = 32;
 constexpr uint8_t kLitOutside = 0xFFu;
-// 17 B per level and thread: 68 KB for the default 128 threads, so a block
-// fits beside two persistent k_join_masks CTAs on one SM.
 constexpr size_t kLitBytesPerThread = kLitLevels * (2 * sizeof(uint64_t) + 1);
 
-template <bool EXACT>
-__global__ void k_join_literal_small(const uint32_t* __restrict__ bits, uint64_t Wp, int prof,
-                                     const uint32_t* __restrict__ qgoff, const uint64_t* __restrict__ qadj,
-                                     const uint32_t* __restrict__ dgoff, const uint64_t* __restrict__ dadj, uint32_t dAW,
-                                     const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ indices, uint32_t g0,
-                                     uint32_t g1, uint32_t q_begin, uint32_t q_end, int find_first,
-                                     uint64_t* __restrict__ counts, unsigned long long* __restrict__ d_total, JoinLimit lim) {
+template <int AW, bool SMEM>
+__global__ void k_join_literal_sets(MaskSource src, int prof, const uint32_t* __restrict__ qgoff, const uint64_t* __restrict__ qadj,
+                                    const uint32_t* __restrict__ dgoff, const uint64_t* __restrict__ dadj, uint32_t dAW,
+                                    const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ indices, uint32_t g0,
+                                    uint32_t g1, uint32_t q_begin, uint32_t q_end, int find_first, uint64_t* __restrict__ counts,
+                                    unsigned long long* __restrict__ d_total, JoinLimit lim) {
   extern __shared__ uint64_t lit_sm[];
   const uint32_t wg = blockDim.x, lid = threadIdx.x;
-  uint64_t* cm = lit_sm;
-  uint64_t* rem = lit_sm + kLitLevels * wg;
-  uint8_t* map = reinterpret_cast<uint8_t*>(lit_sm + 2 * kLitLevels * wg);
-#define LV(arr, l) arr[(l) * wg + lid]
+  uint64_t* cm_s = lit_sm + lid;
+  uint64_t* rem_s = lit_sm + kLitLevels * wg + lid;
+  uint8_t* map_s = reinterpret_cast<uint8_t*>(lit_sm + 2 * kLitLevels * wg) + lid;
+  constexpr uint32_t kLocal = SMEM ? 1 : kMaxQueryNodes;
+  uint64_t cm_l[kLocal * AW], rem_l[kLocal * AW];
+  uint8_t map_l[kLocal];
+#define CM(j, w) (SMEM ? cm_s[(j) * wg] : cm_l[(j) * AW + (w)])
+#define REM(j, w) (SMEM ? rem_s[(j) * wg] : rem_l[(j) * AW + (w)])
+#define MAP(j) (SMEM ? map_s[(j) * wg] : map_l[(j)])
+  constexpr uint32_t kLevels = SMEM ? kLitLevels : kMaxQueryNodes;
   uint64_t my_total = 0, steps = 0;
   bool stop = false;
   for (uint32_t g = g0 + blockIdx.x; g < g1 && !stop; g += gridDim.x) {
@@ -403,7 +416,7 @@ __global__ void k_join_literal_small(const uint32_t* __restrict__ bits, uint64_t
     }
     const uint8_t map0 = s == 0 ? 0 : kLitOutside;
 #pragma unroll 1
-    for (uint32_t k = 0; k < kLitLevels; ++k) LV(map, k) = map0;  // mapping[] of a fresh work-item
+    for (uint32_t k = 0; k < kLevels; ++k) MAP(k) = map0;  // mapping[] of a fresh work-item
     // graph-local bits the reference's uint8-indexed visited set can hold:
     // under REF_PTX those whose global id is below 256; under REF_X86 all
     // (the count modulo 64 is the local id).  A fresh work-item's mapping[]
@@ -411,7 +424,6 @@ __global__ void k_join_literal_small(const uint32_t* __restrict__ bits, uint64_t
     const uint64_t low = prof == kProfileX86 ? ~0ull
                          : (s >= 256u ? 0ull : (256u - s >= 64u ? ~0ull : ((1ull << (256u - s)) - 1ull)));
     const uint64_t outside_bit = prof == kProfileX86 ? (1ull << ((0u - s) & 63u)) : 0ull;
-    const uint32_t i0 = s >> 5, nw = ((e + 31u) >> 5) - i0, sh = s & 31u;
     for (uint32_t it = lid; it < seg1 - seg0; it += wg) {
       if (join_stopped(lim)) {
         stop = true;
@@ -420,62 +432,80 @@ __global__ void k_join_literal_small(const uint32_t* __restrict__ bits, uint64_t
       const uint32_t qg = indices[seg0 + it];
       const uint32_t qoff = qgoff[qg], n = qgoff[qg + 1] - qoff;
       for (uint32_t j = 0; j < n; ++j) {
-        const uint32_t* r = bits + static_cast<uint64_t>(qoff + j) * Wp;
-        uint32_t w[3];
+        uint64_t m[AW];
+        source_mask<AW>(src, dAW, qoff + j, g, s, e, m);
 #pragma unroll
-        for (uint32_t k = 0; k < 3; ++k) w[k] = k < nw ? (r[i0 + k] & range_mask(i0 + k, s, e, prof)) : 0u;
-        const uint64_t lo64 = static_cast<uint64_t>(w[0]) | (static_cast<uint64_t>(w[1]) << 32);
-        LV(cm, j) = (lo64 >> sh) | (sh ? (static_cast<uint64_t>(w[2]) << (64u - sh)) : 0ull);
+        for (int w = 0; w < AW; ++w) CM(j, w) = m[w];
       }
       uint64_t found = 0, visited = 0;
       uint32_t top = 1;  // frames at depths 0 .. top-1
-      LV(rem, 0) = LV(cm, 0);
+#pragma unroll
+      for (int w = 0; w < AW; ++w) REM(0, w) = CM(0, w);
       while (top > 0) {
         const uint32_t qn = top - 1;
         if (qn + 1 == n) {
           // the last query vertex in one step: the frame was just pushed
-          uint64_t place = LV(rem, qn) & ~visited;
-          if (place) {
-            if (find_first) place &= 0ull - place;
-            found += __popcll(place);
-            if (!EXACT) {
-              visited |= place & low;
-              LV(map, qn) = static_cast<uint8_t>(63 - __clzll(static_cast<long long>(place)));
+          uint32_t placed = 0, first = 0, final = 0;
+#pragma unroll
+          for (int w = 0; w < AW; ++w) {
+            const uint64_t p = REM(qn, w) & (w ? ~0ull : ~visited);
+            if (!p) continue;
+            if (!placed) first = 64u * w + __ffsll(static_cast<long long>(p)) - 1u;
+            placed += __popcll(p);
+            final = 64u * w + 63u - __clzll(static_cast<long long>(p));
+            if (w == 0 && !find_first) visited |= p & low;
+          }
+          if (placed) {
+            if (find_first) {
+              found = 1;
+              MAP(qn) = static_cast<uint8_t>(first);
+              break;
             }
-            if (find_first) break;
+            found += placed;
+            MAP(qn) = static_cast<uint8_t>(final);
           }
         } else {
-          const uint64_t r = LV(rem, qn);
-          if (r) {
-            const uint32_t t = __ffsll(static_cast<long long>(r)) - 1;
-            LV(rem, qn) = r & (r - 1);
-            const uint64_t bit = 1ull << t;
-            if (EXACT ? (visited & bit) : (visited & bit & low)) continue;
+          uint32_t t = 0xFFFFFFFFu;
+#pragma unroll
+          for (int w = 0; w < AW; ++w) {
+            const uint64_t r = REM(qn, w);
+            if (t == 0xFFFFFFFFu && r) {
+              t = 64u * w + __ffsll(static_cast<long long>(r)) - 1u;
+              REM(qn, w) = r & (r - 1);
+            }
+          }
+          if (t != 0xFFFFFFFFu) {
+            const uint64_t bit = t < 64u ? (1ull << t) & low : 0ull;
+            if (visited & bit) continue;
             // place t at depth qn and push the frame of depth qn + 1
-            LV(map, qn) = static_cast<uint8_t>(t);
-            visited |= EXACT ? bit : (bit & low);
+            MAP(qn) = static_cast<uint8_t>(t);
+            visited |= bit;
             // isValidMapping for depth d = qn + 1 against mapping[0..qn]: the
             // data rows of the picks (graph-local adjacency words) must equal
             // the query's adjacency to d, bit for bit
             const uint32_t d = qn + 1;
             const uint64_t qcol = qadj[qoff + d];  // bit i: query vertices i and d adjacent
-            uint64_t vm = LV(cm, d) & ~(dadj[static_cast<uint64_t>(s + t) * dAW] ^ (0ull - ((qcol >> qn) & 1ull)));
-            for (uint32_t i = 0; i < qn; ++i)
-              vm &= ~(dadj[static_cast<uint64_t>(s + LV(map, i)) * dAW] ^ (0ull - ((qcol >> i) & 1ull)));
-            LV(rem, d) = vm;
+            uint64_t vm[AW];
+#pragma unroll
+            for (int w = 0; w < AW; ++w)
+              vm[w] = CM(d, w) & ~(dadj[static_cast<uint64_t>(s + t) * dAW + w] ^ (0ull - ((qcol >> qn) & 1ull)));
+            for (uint32_t i = 0; i < qn; ++i) {
+              const uint64_t* row = dadj + static_cast<uint64_t>(s + MAP(i)) * dAW;
+              const uint64_t want = 0ull - ((qcol >> i) & 1ull);
+#pragma unroll
+              for (int w = 0; w < AW; ++w) vm[w] &= ~(row[w] ^ want);
+            }
+#pragma unroll
+            for (int w = 0; w < AW; ++w) REM(d, w) = vm[w];
             ++top;
             continue;
           }
         }
         // the frame at depth qn is used up
         --top;
-        if (EXACT) {
-          if (top) visited &= ~(1ull << LV(map, top - 1));  // the parent's pick
-        } else {
-          const uint32_t mq = LV(map, qn);  // mapping[qn], perhaps stale
-          visited &= ~(mq < 64u ? ((1ull << mq) & low) : outside_bit);
-          if (top == 1) visited = 0;
-        }
+        const uint32_t mq = MAP(qn);  // mapping[qn], perhaps stale
+        visited &= ~(mq < 64u ? ((1ull << mq) & low) : (mq == kLitOutside ? outside_bit : 0ull));
+        if (top == 1) visited = 0;
         if (budget_spent(lim, steps)) {
           stop = true;
           break;
@@ -486,7 +516,9 @@ __global__ void k_join_literal_small(const uint32_t* __restrict__ bits, uint64_t
       my_total += found;
     }
   }
-#undef LV
+#undef CM
+#undef REM
+#undef MAP
   for (int o = 16; o; o >>= 1) my_total += __shfl_xor_sync(0xFFFFFFFFu, my_total, o);
   __shared__ uint64_t part[32];
   if ((lid & 31u) == 0) part[lid >> 5] = my_total;
@@ -650,214 +682,213 @@ __global__ void k_join_wildcard(const uint32_t* __restrict__ bits, uint64_t Wp, 
   if (lane == 0 && my_total) atomicAdd(d_total, static_cast<unsigned long long>(my_total));
 }
 
-// Graph-local candidate set of one bitset row for data graph [s, e): bit t =
-// global candidate s + t, after the profile's range masks.
-template <int AW>
-__device__ __forceinline__ void extract_local(const uint32_t* __restrict__ row, uint32_t s, uint32_t e, int prof, uint64_t* out) {
-#pragma unroll
-  for (int k = 0; k < AW; ++k) out[k] = 0;
-  const uint32_t i0 = s >> 5, i1 = (e + 31u) >> 5;
-  for (uint32_t i = i0; i < i1; ++i) {
-    uint32_t wv = row[i] & range_mask(i, s, e, prof);
-    if (!wv) continue;
-    int32_t off = static_cast<int32_t>(i << 5) - static_cast<int32_t>(s);
-    if (off < 0) {
-      wv >>= static_cast<uint32_t>(-off);
-      off = 0;
-    }
-    const uint32_t k = static_cast<uint32_t>(off) >> 6, sh = static_cast<uint32_t>(off) & 63u;
-#pragma unroll
-    for (int kk = 0; kk < AW; ++kk) {
-      if (static_cast<uint32_t>(kk) == k) out[kk] |= static_cast<uint64_t>(wv) << sh;
-      if (sh > 32u && static_cast<uint32_t>(kk) == k + 1) out[kk] |= static_cast<uint64_t>(wv) >> (64u - sh);
-    }
-  }
+// The join of the pairs listed by k_pair_masks as too large for the two-phase
+// join: queries of up to kMaxQueryNodes vertices, molecules of up to 64 * AW
+// atoms.  A warp takes a batch of up to `batch` pairs, builds their level masks
+// in shared memory with all lanes busy (an item per (pair, level), as in
+// k_pair_masks), and then its lanes run k_join_dfs's turns, each lane on one
+// root candidate of one pair at a time, so a heavy pair is spread over the
+// warp.  The per-level state is in local memory (the pairs are few).  The
+// one-lane-per-part form that this replaced rebuilt every mask in every part:
+// 1.43 ms for the 0.4 % of 6.86 M pairs with queries over 16 vertices.
+constexpr uint32_t kWideWarps = 4;
+constexpr uint32_t kWideBatch = 8;
+constexpr size_t kWideMaskBytes = 8192;  // level masks of one warp's batch, at most
+struct WideEntry {
+  uint64_t cnt;
+  uint32_t qoff, n, s, slot;  // qoff: identity-order flag in bit 31
+};
+// [batch] entries, [batch][AW] root candidates, [batch][stride] masks per warp
+inline size_t wide_smem(uint32_t batch, uint32_t aw, uint32_t stride) {
+  return kWideWarps * batch * (sizeof(WideEntry) + 8ull * aw + 8ull * stride);
 }
 
-// Candidate set of query vertex v (global id) in data graph g from the plane
-// tiles: the AND of the planes of v's class program.
-template <int AW>
-__device__ __forceinline__ void mask_from_planes(const uint64_t* __restrict__ planes, uint32_t K, uint32_t g, uint32_t cls_v,
-                                                 const uint32_t* __restrict__ prog_off, const uint16_t* __restrict__ prog,
-                                                 uint64_t* out) {
-  const uint64_t* base = planes + static_cast<uint64_t>(g >> 5) * K * AW * 32 + (g & 31u);
+template <int AW, bool EXACT>
+__global__ void __launch_bounds__(kWideWarps * 32) k_join_wide(
+    MaskSource src, const uint32_t* __restrict__ qgoff, const uint8_t* __restrict__ qorder, const uint64_t* __restrict__ qsel,
+    const uint64_t* __restrict__ qsel_id, const uint8_t* __restrict__ qsym, const uint32_t* __restrict__ dgoff,
+    const uint64_t* __restrict__ dadj, const uint8_t* __restrict__ dsym, const uint32_t* __restrict__ indices,
+    const uint32_t* __restrict__ pair_graph, const uint32_t* __restrict__ list, const unsigned long long* __restrict__ list_len,
+    uint32_t batch, uint32_t stride, int find_first, unsigned long long* __restrict__ cursor, uint64_t* __restrict__ counts,
+    unsigned long long* __restrict__ d_total, JoinLimit lim) {
+  extern __shared__ __align__(16) unsigned char wide_raw[];
+  constexpr unsigned kAll = 0xFFFFFFFFu;
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  unsigned char* base = wide_raw + static_cast<size_t>(warp) * batch * (sizeof(WideEntry) + 8u * AW + 8ull * stride);
+  WideEntry* ent = reinterpret_cast<WideEntry*>(base);
+  unsigned long long* roots = reinterpret_cast<unsigned long long*>(ent + batch);
+  uint64_t* masks = reinterpret_cast<uint64_t*>(roots + batch * AW);
+  uint64_t rest[kMaxQueryNodes][AW], p0[kMaxQueryNodes][AW], p1[kMaxQueryNodes][AW];
+  uint8_t pick[kMaxQueryNodes];
 #pragma unroll
-  for (int w = 0; w < AW; ++w) out[w] = ~0ull;
-  const uint32_t e1 = prog_off[cls_v + 1];
-  for (uint32_t e = prog_off[cls_v]; e < e1; ++e) {
-    const uint32_t k = prog[e];
-#pragma unroll
-    for (int w = 0; w < AW; ++w) out[w] &= base[(static_cast<uint64_t>(k) * AW + w) * 32];
-  }
-}
-
-// Persistent join over GMCR slots.  Each lane runs its own DFS as a flat
-// state machine — one loop iteration expands one node — and pulls a new pair
-// when its current one is finished, so lanes of a warp stay busy regardless of
-// how uneven the pairs are.  Lanes needing work take kChunk consecutive slots
-// each with one warp-aggregated atomic.
-template <int AW, bool EXACT, bool FROM_PLANES>
-__global__ void __launch_bounds__(128) k_join_fast(
-    const uint32_t* __restrict__ bits, uint64_t Wp, const uint64_t* __restrict__ planes, uint32_t K,
-    const uint32_t* __restrict__ prog_off, const uint16_t* __restrict__ prog, const uint32_t* __restrict__ cls,
-    int prof, const uint32_t* __restrict__ qgoff,
-    const uint8_t* __restrict__ qorder, const uint64_t* __restrict__ qsel, const uint64_t* __restrict__ qsel_id,
-    const uint8_t* __restrict__ qsym, const uint32_t* __restrict__ dgoff, const uint64_t* __restrict__ dadj,
-    const uint8_t* __restrict__ dsym, const uint32_t* __restrict__ indices, const uint32_t* __restrict__ pair_graph,
-    const uint32_t* __restrict__ list, const unsigned long long* __restrict__ list_len, uint64_t total_slots,
-    uint32_t skip_below, int find_first, uint32_t split, unsigned long long* __restrict__ cursor,
-    uint64_t* __restrict__ counts, unsigned long long* __restrict__ d_total, JoinLimit lim) {
-  constexpr uint32_t kChunk = 8;
-  uint64_t steps = 0;
-  // entries to walk (list or all slots); with split > 1 every entry is split
-  // into `split` work items, item p taking the root candidates of rank = p mod
-  // split, and the items' counts are merged into counts[] (zeroed beforehand)
-  const uint64_t total = (list ? *list_len : total_slots) * split;
-  const unsigned lane = threadIdx.x & 31u;
-  uint64_t my_total = 0;
-  uint64_t M[kMaxQueryNodes][AW];     // candidates of each level (graph-local)
-  uint64_t cand[kMaxQueryNodes][AW];  // untried candidates of each level
-  uint64_t rows[kMaxQueryNodes][AW];  // adjacency row of each level's pick
-  uint32_t pick[kMaxQueryNodes];
-  uint64_t next = 0, end = 0;  // this lane's claimed slot range
-  uint64_t slot = 0;
-  uint32_t part = 0;
-  uint64_t cnt = 0;
-  uint32_t n = 0, s = 0;
-  const uint64_t* selp = nullptr;
-  int k = -1;  // DFS level; -1 = no pair in progress
-  bool have = false;
+  for (int w = 0; w < AW; ++w) p0[0][w] = p1[0][w] = 0;
+  const uint64_t total = *list_len;
+  uint64_t my_total = 0, steps = 0;
   for (;;) {
-    if (k < 0) {
-      if (have) {
-        if (find_first && cnt) cnt = 1;
-        if (split == 1) {
-          counts[slot] = cnt;
-          my_total += cnt;
-        } else if (cnt) {
-          if (!find_first) {
-            atomicAdd(reinterpret_cast<unsigned long long*>(counts + slot), static_cast<unsigned long long>(cnt));
-            my_total += cnt;
-          } else if (atomicCAS(reinterpret_cast<unsigned long long*>(counts + slot), 0ull, 1ull) == 0ull) {
-            my_total += 1;
-          }
-        }
-        have = false;
-      }
-      // claim the next slot of a pair this kernel handles
-      bool done = false;
-      for (;;) {
-        if (next >= end) {
-          if (join_stopped(lim)) {
-            done = true;
-            break;
-          }
-          const unsigned am = __activemask();
-          const unsigned leader = __ffs(am) - 1;
-          const unsigned rank = __popc(am & ((1u << lane) - 1u));
-          unsigned long long base = 0;
-          if (lane == leader) base = atomicAdd(cursor, static_cast<unsigned long long>(__popc(am)) * kChunk);
-          base = __shfl_sync(am, base, leader);
-          next = base + static_cast<uint64_t>(rank) * kChunk;
-          end = next + kChunk < total ? next + kChunk : total;
-          if (next >= total) {
-            done = true;
-            break;
-          }
-        }
-        const uint64_t entry = next / split;
-        part = static_cast<uint32_t>(next % split);
-        slot = list ? list[entry] : entry;
-        ++next;
-        if (pair_graph[slot] >= skip_below) break;
-      }
-      if (done) break;
-      const uint32_t g = pair_graph[slot];
+    unsigned long long b = total;
+    if (lane == 0 && !join_stopped(lim)) b = atomicAdd(cursor, static_cast<unsigned long long>(batch));
+    b = __shfl_sync(kAll, b, 0);
+    if (b >= total) break;
+    const uint32_t ne = static_cast<uint32_t>(total - b < batch ? total - b : batch);
+    // the batch's pairs, one lane each
+    uint32_t n = 0, qoff = 0, g = 0, s = 0, e = 0;
+    bool ident = true;
+    if (lane < ne) {
+      const uint32_t slot = list[b + lane];
       const uint32_t qg = indices[slot];
-      const uint32_t qoff = qgoff[qg];
+      qoff = qgoff[qg];
       n = qgoff[qg + 1] - qoff;
+      g = pair_graph[slot];
       s = dgoff[g];
-      const uint32_t e = dgoff[g + 1];
-      const bool ident = !(qsym[qg] && dsym[g]);
-      selp = (ident ? qsel_id : qsel) + qoff;
-      for (uint32_t j = 0; j < n; ++j) {
-        const uint32_t v = ident ? j : qorder[qoff + j];
-        if (FROM_PLANES) mask_from_planes<AW>(planes, K, g, cls[qoff + v], prog_off, prog, M[j]);
-        else extract_local<AW>(bits + static_cast<uint64_t>(qoff + v) * Wp, s, e, prof, M[j]);
+      e = dgoff[g + 1];
+      ident = !(qsym[qg] && dsym[g]);
+      ent[lane] = WideEntry{0, qoff | (ident ? 0x80000000u : 0u), n, s, slot};
+    }
+    uint32_t incl = n;
+#pragma unroll
+    for (unsigned o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(kAll, incl, o);
+      if (lane >= o) incl += v;
+    }
+    const uint32_t excl = incl - n, items = __shfl_sync(kAll, incl, 31);
+    for (uint32_t i0 = 0; i0 < items; i0 += 32) {
+      const uint32_t it = i0 + lane;
+      uint32_t pos = 0;  // the last pair whose first item is <= it
+      for (uint32_t k = 1; k < ne; ++k)
+        if (__shfl_sync(kAll, excl, k) <= it) pos = k;
+      const uint32_t j = it - __shfl_sync(kAll, excl, pos), oq = __shfl_sync(kAll, qoff, pos), og = __shfl_sync(kAll, g, pos);
+      const uint32_t os = __shfl_sync(kAll, s, pos), oe = __shfl_sync(kAll, e, pos);
+      const bool oi = __shfl_sync(kAll, static_cast<unsigned>(ident), pos) != 0u;
+      if (it < items) source_mask<AW>(src, AW, oq + (oi ? j : qorder[oq + j]), og, os, oe, masks + pos * stride + j * AW);
+    }
+    __syncwarp();
+    for (uint32_t i = lane; i < ne * AW; i += 32) roots[i] = masks[(i / AW) * stride + i % AW];
+    __syncwarp();
+    // the lanes' searches
+    uint64_t alive = 0, cnt = 0;  // alive: levels with untried candidates
+    uint32_t my = 0;              // this lane's pair within the batch
+    const uint64_t* selp = qsel;
+    const uint64_t* M = masks;
+    const uint64_t* arow = dadj;
+    bool dry = false;  // no root candidate left for this lane
+    for (;;) {
+      if (!alive && cnt) {
+        auto* at = reinterpret_cast<unsigned long long*>(&ent[my].cnt);
+        if (find_first) atomicExch(at, 1ull);
+        else atomicAdd(at, static_cast<unsigned long long>(cnt));
+        cnt = 0;
       }
+      if (!alive && !dry) {
+        dry = true;
+        for (uint32_t i = 0; i < ne && dry; ++i) {
+          const uint32_t c = (lane + i) % ne;
+          if (find_first && *reinterpret_cast<volatile uint64_t*>(&ent[c].cnt)) continue;
+          for (uint32_t w = 0; w < AW && dry; ++w) {
+            unsigned long long v = *reinterpret_cast<volatile unsigned long long*>(&roots[c * AW + w]);
+            while (v && dry) {
+              const unsigned long long bit = v & (0ull - v);
+              const unsigned long long old = atomicAnd(&roots[c * AW + w], ~bit);
+              if (old & bit) {
+                dry = false;
+                my = c;
 #pragma unroll
-      for (int w = 0; w < AW; ++w) cand[0][w] = M[0][w];
-      if (split > 1) {  // keep the root candidates of rank = part mod split
-        uint32_t rank = 0;
-#pragma unroll
-        for (int w = 0; w < AW; ++w) {
-          uint64_t bitsw = cand[0][w], keep = 0;
-          while (bitsw) {
-            const uint64_t low = bitsw & (0ull - bitsw);
-            if (rank % split == part) keep |= low;
-            ++rank;
-            bitsw ^= low;
+                for (uint32_t x = 0; x < AW; ++x) rest[0][x] = x == w ? bit : 0ull;
+              }
+              v = old & ~bit;
+            }
           }
-          cand[0][w] = keep;
+        }
+        if (!dry) {
+          const WideEntry& en = ent[my];
+          n = en.n;
+          selp = ((en.qoff >> 31) ? qsel_id : qsel) + (en.qoff & 0x7FFFFFFFu);
+          arow = dadj + static_cast<uint64_t>(en.s) * AW;
+          M = masks + my * stride;
+          alive = 1;
         }
       }
-      cnt = 0;
-      k = 0;
-      have = true;
-      continue;
-    }
-    // one DFS node at level k
-    bool empty = true;
+      if (!__any_sync(kAll, alive != 0)) break;
+      if (!alive) continue;
+      if (find_first && *reinterpret_cast<volatile uint64_t*>(&ent[my].cnt)) {
+        alive = 0;
+        continue;
+      }
+      // one turn of k_join_dfs on AW-word sets
+      const uint32_t k = 63u - __clzll(static_cast<long long>(alive));
+      uint32_t t = 0;
+      uint64_t left = 0;
 #pragma unroll
-    for (int w = 0; w < AW; ++w) empty &= cand[k][w] == 0;
-    if (empty) {
-      --k;
-      if (budget_spent(lim, steps)) break;
-      continue;
-    }
-    uint32_t t = 0;
+      for (int w = 0; w < AW; ++w)
+        if (rest[k][w]) t = 64u * w + 63u - __clzll(static_cast<long long>(rest[k][w]));
 #pragma unroll
-    for (int w = AW - 1; w >= 0; --w)
-      if (cand[k][w]) t = 64u * w + (__ffsll(static_cast<long long>(cand[k][w])) - 1);
-    cand[k][t >> 6] &= cand[k][t >> 6] - 1;
-    pick[k] = t;
-    const uint64_t* r = dadj + static_cast<uint64_t>(s + t) * AW;
+      for (int w = 0; w < AW; ++w) {
+        if ((t >> 6) == static_cast<uint32_t>(w)) rest[k][w] ^= 1ull << (t & 63u);
+        left |= rest[k][w];
+      }
+      if (!left) alive ^= 1ull << k;
+      pick[k] = static_cast<uint8_t>(t);
+      const uint64_t sel = selp[k + 1];
+      const uint32_t cn = __popcll(sel);
+      uint64_t n0[AW], n1[AW], f[AW];
 #pragma unroll
-    for (int w = 0; w < AW; ++w) rows[k][w] = r[w];
-    const uint64_t sl = selp[k + 1];
-    uint64_t nx[AW], excl[AW];
+      for (int w = 0; w < AW; ++w) {
+        const uint64_t r = arow[t * AW + w], b0 = p0[k][w], b1 = p1[k][w];
+        const uint64_t bit = EXACT && (t >> 6) == static_cast<uint32_t>(w) ? 1ull << (t & 63u) : 0ull;
+        n0[w] = (b0 ^ r) | (b1 & b0) | bit;
+        n1[w] = b1 | (b0 & r) | bit;
+        f[w] = M[(k + 1) * AW + w];
+      }
+      if (cn <= 2u) {
+        for (uint64_t m = sel; m; m &= m - 1) {
+          const uint64_t* row = arow + static_cast<uint32_t>(pick[__ffsll(static_cast<long long>(m)) - 1]) * AW;
 #pragma unroll
-    for (int w = 0; w < AW; ++w) {
-      nx[w] = M[k + 1][w];
-      excl[w] = 0;
-    }
-    for (int i = 0; i <= k; ++i) {
-      const uint64_t keep_set = 0ull - ((sl >> i) & 1ull);  // all ones when adjacent in the query
+          for (int w = 0; w < AW; ++w) f[w] &= row[w];
+        }
+        const uint64_t e0 = cn == 1u ? ~0ull : 0ull, e1 = cn == 2u ? ~0ull : 0ull;
 #pragma unroll
-      for (int w = 0; w < AW; ++w) nx[w] &= ~(rows[i][w] ^ keep_set) ;
-      if (EXACT) {
+        for (int w = 0; w < AW; ++w) f[w] &= ~((n0[w] ^ e0) | (n1[w] ^ e1));
+      } else {
+        for (uint32_t i = 0; i <= k; ++i) {
+          const uint64_t* row = arow + static_cast<uint32_t>(pick[i]) * AW;
+          const uint64_t want = 0ull - ((sel >> i) & 1ull);
 #pragma unroll
-        for (int w = 0; w < AW; ++w)
-          if ((pick[i] >> 6) == static_cast<uint32_t>(w)) excl[w] |= 1ull << (pick[i] & 63u);
+          for (int w = 0; w < AW; ++w) {
+            f[w] &= ~(row[w] ^ want);
+            if (EXACT && (pick[i] >> 6) == w) f[w] &= ~(1ull << (pick[i] & 63u));
+          }
+        }
+      }
+      uint32_t c = 0;
+#pragma unroll
+      for (int w = 0; w < AW; ++w) c += __popcll(f[w]);
+      if (c) {
+        if (k + 2u == n) {  // the last level: every candidate is a match
+          cnt += c;
+          if (find_first) alive = 0;
+        } else {
+#pragma unroll
+          for (int w = 0; w < AW; ++w) {
+            rest[k + 1][w] = f[w];
+            p0[k + 1][w] = n0[w];
+            p1[k + 1][w] = n1[w];
+          }
+          alive |= 2ull << k;
+        }
+      }
+      if (!left && budget_spent(lim, steps)) {
+        alive = 0;
+        dry = true;
       }
     }
-    if (EXACT) {
-#pragma unroll
-      for (int w = 0; w < AW; ++w) nx[w] &= ~excl[w];
+    __syncwarp();
+    if (lane < ne) {
+      const uint64_t c = ent[lane].cnt;
+      counts[ent[lane].slot] = c;
+      my_total += c;
     }
-    if (static_cast<uint32_t>(k + 1) == n - 1) {
-      uint32_t pc = 0;
-#pragma unroll
-      for (int w = 0; w < AW; ++w) pc += __popcll(nx[w]);
-      cnt += pc;
-      if (find_first && cnt) k = -1;
-      continue;
-    }
-    ++k;
-#pragma unroll
-    for (int w = 0; w < AW; ++w) cand[k][w] = nx[w];
+    __syncwarp();
   }
-  for (int o = 16; o; o >>= 1) my_total += __shfl_xor_sync(0xFFFFFFFFu, my_total, o);
+  for (int o = 16; o; o >>= 1) my_total += __shfl_xor_sync(kAll, my_total, o);
   if (lane == 0 && my_total) atomicAdd(d_total, static_cast<unsigned long long>(my_total));
 }
 
@@ -880,10 +911,9 @@ constexpr uint32_t kPhaseThreads = 256;
 // for the slot's metadata and setup record, then the round's sum of query
 // sizes (slot, level) items with every lane busy; an item finds its slot by a
 // binary search over the lanes' exclusive prefix sums (warp shuffles).
+template <bool FROM_PLANES>
 __global__ void __launch_bounds__(256) k_pair_masks(
-    const uint64_t* __restrict__ planes, uint32_t K, uint32_t AW, const uint32_t* __restrict__ prog_off,
-    const uint16_t* __restrict__ prog,
-    const uint32_t* __restrict__ cls, const uint32_t* __restrict__ qgoff, const uint8_t* __restrict__ qorder,
+    MaskSource src, uint32_t AW, const uint32_t* __restrict__ qgoff, const uint8_t* __restrict__ qorder,
     const uint8_t* __restrict__ qsym, const uint32_t* __restrict__ dgoff, const uint8_t* __restrict__ dsym,
     const uint32_t* __restrict__ indices, const uint32_t* __restrict__ pair_graph, uint64_t slot0, uint64_t count,
     uint64_t* __restrict__ masks, uint4* __restrict__ rec, uint32_t skip_below, uint32_t* __restrict__ overflow,
@@ -894,7 +924,7 @@ __global__ void __launch_bounds__(256) k_pair_masks(
   const uint64_t nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
   for (uint64_t s0 = warp * 32; s0 < count; s0 += nwarps * 32) {
     const uint64_t local = s0 + lane;
-    uint32_t n = 0, qoff = 0, g = 0, items = 0;
+    uint32_t n = 0, qoff = 0, g = 0, items = 0, ds = 0, de = 0;
     bool ident = true;
     if (local < count) {
       const uint64_t slot = slot0 + local;
@@ -903,10 +933,11 @@ __global__ void __launch_bounds__(256) k_pair_masks(
       n = qgoff[qg + 1] - qoff;
       g = pair_graph[slot];
       ident = !(qsym[qg] && dsym[g]);
-      const uint32_t ds = dgoff[g];
+      ds = dgoff[g];
+      de = dgoff[g + 1];
       // queries over kPhaseLevels vertices and molecules over 64 atoms (a
-      // vertex set wider than one word) go to the generic kernel
-      const bool generic = n > kPhaseLevels || dgoff[g + 1] - ds > 64u;
+      // vertex set wider than one word) go to k_join_wide
+      const bool generic = n > kPhaseLevels || de - ds > 64u;
       // the pair's setup record: first data vertex, query size | flags (0x100
       // identity order, 0x200 generic, 0x400 long, 0x800 the literal join's),
       // query offset, query graph
@@ -917,9 +948,8 @@ __global__ void __launch_bounds__(256) k_pair_masks(
         longs[atomicAdd(longs_len, 1ull)] = static_cast<uint32_t>(slot);
         counts[slot] = 0;
       }
-      if (generic && g >= skip_below) {  // joined by the generic kernel, which accumulates into counts
+      if (generic && g >= skip_below) {
         overflow[atomicAdd(overflow_len, 1ull)] = static_cast<uint32_t>(slot);
-        counts[slot] = 0;
       }
       if (zero_counts && g >= skip_below) counts[slot] = 0;  // the join adds up a pair's parts
       items = generic ? 0u : n;
@@ -946,14 +976,23 @@ __global__ void __launch_bounds__(256) k_pair_masks(
       const uint32_t o_qoff = __shfl_sync(0xFFFFFFFFu, qoff, pos);
       const uint32_t o_g = __shfl_sync(0xFFFFFFFFu, g, pos);
       const bool o_ident = __shfl_sync(0xFFFFFFFFu, static_cast<unsigned>(ident), pos) != 0u;
+      uint32_t o_s = 0, o_e = 0;
+      if (!FROM_PLANES) {
+        o_s = __shfl_sync(0xFFFFFFFFu, ds, pos);
+        o_e = __shfl_sync(0xFFFFFFFFu, de, pos);
+      }
       if (it >= total) continue;
       const uint32_t j = it - o_excl;
-      const uint32_t c = cls[o_qoff + (o_ident ? j : qorder[o_qoff + j])];
-      // word 0 of each plane: the graph's vertex set fits one word
-      const uint64_t* pb = planes + static_cast<uint64_t>(o_g >> 5) * K * AW * 32 + (o_g & 31u);
+      const uint32_t v = o_qoff + (o_ident ? j : qorder[o_qoff + j]);
+      // one word: the graph's vertex set fits it (word 0 of each plane)
       uint64_t m = ~0ull;
-      const uint32_t e1 = prog_off[c + 1];
-      for (uint32_t e = prog_off[c]; e < e1; ++e) m &= pb[static_cast<uint64_t>(prog[e]) * AW * 32];
+      if (FROM_PLANES) {
+        const uint64_t* pb = src.planes + static_cast<uint64_t>(o_g >> 5) * src.K * AW * 32 + (o_g & 31u);
+        const uint32_t c = src.cls[v], e1 = src.prog_off[c + 1];
+        for (uint32_t e = src.prog_off[c]; e < e1; ++e) m &= pb[static_cast<uint64_t>(src.prog[e]) * AW * 32];
+      } else {
+        extract_local<1>(src.bits + static_cast<uint64_t>(v) * src.Wp, o_s, o_e, src.prof, &m);
+      }
       masks[(s0 + pos) * kPhaseLevels + j] = m;
     }
   }
@@ -1551,45 +1590,43 @@ __global__ void __launch_bounds__(kFrontWarps * 32, 3) k_join_frontier(
 
 }  // namespace
 
-int launch_join_literal(Queue* q, const Graph* query, const Graph* data, const Candidates* c, Gmcr* m, int find_first,
+int launch_join_literal(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first,
                         uint32_t graph_begin, uint32_t graph_end, uint64_t* d_total, uint32_t q_begin, uint32_t q_end) {
   if (graph_end <= graph_begin) return SIGMO_OK;
   if (query->max_nodes > kMaxQueryNodes)
     return fail(SIGMO_ERR_DOMAIN, "query graphs of up to %u vertices are supported (largest: %u)", kMaxQueryNodes, query->max_nodes);
-  const bool exact = q->opts.profile == kProfileExact;
-  if (exact && data->max_nodes > 64u * kMaxAdjWords)
+  if (q->opts.profile == kProfileExact)
     return fail(SIGMO_ERR_DOMAIN, "exact profile supports data graphs of at most %u vertices", 64u * kMaxAdjWords);
   const uint32_t wg = q->opts.join_work_group_size ? q->opts.join_work_group_size : 128u;
   if (wg > 1024u || (wg & 31u)) return fail(SIGMO_ERR_INVALID, "join work-group size %u must be a multiple of 32 <= 1024", wg);
   const unsigned grid = std::min<uint32_t>(graph_end - graph_begin, 148u * 64u);
   auto* tot = reinterpret_cast<unsigned long long*>(d_total);
-  // the common case (graphs of <= 64 vertices, queries of <= kLitLevels) keeps
-  // its per-level state in shared memory
   uint32_t range_max = data->max_nodes;
   if (range_max > 64u) {
     range_max = 0;
     for (uint32_t g = graph_begin; g < graph_end; ++g)
       range_max = std::max(range_max, data->host_graph_offsets[g + 1] - data->host_graph_offsets[g]);
   }
-  if (range_max <= 64u && query->max_nodes <= kLitLevels && wg <= 256u) {
-    const size_t smem = kLitBytesPerThread * wg;
-    auto kern = exact ? k_join_literal_small<true> : k_join_literal_small<false>;
-    SIGMO_TRY(allow_max_dynamic_smem(reinterpret_cast<const void*>(kern), q->device));
-    kern<<<grid, wg, smem, q->stream>>>(c->bits, c->Wp, q->opts.profile, query->graph_offsets, query->adj,
-                                        data->graph_offsets, data->adj, data->adj_words, m->offsets, m->indices, graph_begin,
-                                        graph_end, q_begin, q_end, find_first, m->counts, tot, join_limit(q));
-    return check_launch(q, "k_join_literal_small");
+  // one word per set where the range's graphs allow it; its state fits shared
+  // memory up to kLitLevels levels and 256 threads
+  const bool one = range_max <= 64u, smem_fits = one && query->max_nodes <= kLitLevels && wg <= 256u;
+  if (one || (q->opts.profile == kProfilePtx && range_max <= 64u * kMaxAdjWords)) {
+    const size_t smem = smem_fits ? kLitBytesPerThread * wg : 0;
+    auto kern = smem_fits ? k_join_literal_sets<1, true>
+                : one     ? k_join_literal_sets<1, false>
+                : data->adj_words == 2 ? k_join_literal_sets<2, false>
+                                       : k_join_literal_sets<4, false>;
+    if (smem) SIGMO_TRY(allow_max_dynamic_smem(reinterpret_cast<const void*>(kern), q->device));
+    kern<<<grid, wg, smem, q->stream>>>(src, q->opts.profile, query->graph_offsets, query->adj, data->graph_offsets, data->adj,
+                                        data->adj_words, m->offsets, m->indices, graph_begin, graph_end, q_begin, q_end,
+                                        find_first, m->counts, tot, join_limit(q));
+    return check_launch(q, "k_join_literal_sets");
   }
-  if (exact)
-    k_join_literal<true><<<grid, wg, 0, q->stream>>>(c->bits, c->Wp, q->opts.profile, query->graph_offsets, query->adj,
-                                                      data->graph_offsets, data->adj, data->adj_words, data->row_offsets,
-                                                      data->column_indices, m->offsets, m->indices, graph_begin, graph_end,
-                                                      q_begin, q_end, find_first, m->counts, tot, join_limit(q));
-  else
-    k_join_literal<false><<<grid, wg, 0, q->stream>>>(c->bits, c->Wp, q->opts.profile, query->graph_offsets, query->adj,
-                                                       data->graph_offsets, data->adj, data->adj_words, data->row_offsets,
-                                                       data->column_indices, m->offsets, m->indices, graph_begin, graph_end,
-                                                       q_begin, q_end, find_first, m->counts, tot, join_limit(q));
+  if (!src.bits) return fail(SIGMO_ERR_INVALID, "internal: the literal join of graphs over %u vertices reads the bitset", 64u * kMaxAdjWords);
+  k_join_literal<<<grid, wg, 0, q->stream>>>(src.bits, src.Wp, q->opts.profile, query->graph_offsets, query->adj,
+                                             data->graph_offsets, data->adj, data->adj_words, data->row_offsets,
+                                             data->column_indices, m->offsets, m->indices, graph_begin, graph_end, q_begin,
+                                             q_end, find_first, m->counts, tot, join_limit(q));
   return check_launch(q, "k_join_literal");
 }
 
@@ -1621,48 +1658,13 @@ int launch_join_wildcard(Queue* q, const Graph* query, const Graph* data, const 
   return check_launch(q, "k_join_wildcard");
 }
 
-int launch_join_fast(Queue* q, const Graph* query, const Graph* data, const Candidates* c, Gmcr* m, int find_first,
-                     uint64_t* d_total) {
-  if (!m->total) return SIGMO_OK;
-  if (query->max_nodes > kMaxQueryNodes)
-    return fail(SIGMO_ERR_DOMAIN, "query graphs of up to %u vertices are supported (largest: %u)", kMaxQueryNodes, query->max_nodes);
-  const bool exact = q->opts.profile == kProfileExact;
-  if (data->max_nodes > 64u * kMaxAdjWords)
-    return fail(SIGMO_ERR_DOMAIN, "the batched join supports data graphs of at most %u vertices", 64u * kMaxAdjWords);
-  SIGMO_TRY(launch_query_order(const_cast<Graph*>(query)));
-  void* scratch = nullptr;
-  SIGMO_TRY(queue_scratch(q, 256, &scratch));
-  auto* cursor = static_cast<unsigned long long*>(scratch);
-  SIGMO_CUDA_TRY(cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), q->stream));
-  const uint32_t skip = exact ? 0u : data->low_offset_graphs;
-  const unsigned block = 128;
-  const unsigned grid = grid_for((m->total + 31) / 32 * 32, block, 148u * 16u);
-  auto* tot = reinterpret_cast<unsigned long long*>(d_total);
-#define SIGMO_JOIN_FAST(AWV, EX)                                                                                    \
-  k_join_fast<AWV, EX, false><<<grid, block, 0, q->stream>>>(c->bits, c->Wp, nullptr, 0, nullptr, nullptr, nullptr,         \
-                                                       q->opts.profile, query->graph_offsets, query->qorder,             \
-                                                       query->qsel, query->qsel_id, query->sym, data->graph_offsets,     \
-                                                       data->adj, data->sym, m->indices, m->pair_graph, nullptr, nullptr, \
-                                                       m->total, skip, find_first, 1u, cursor, m->counts, tot, \
-                                                       join_limit(q))
-  switch (data->adj_words) {
-    case 1: if (exact) SIGMO_JOIN_FAST(1, true); else SIGMO_JOIN_FAST(1, false); break;
-    case 2: if (exact) SIGMO_JOIN_FAST(2, true); else SIGMO_JOIN_FAST(2, false); break;
-    default: if (exact) SIGMO_JOIN_FAST(4, true); else SIGMO_JOIN_FAST(4, false); break;
-  }
-#undef SIGMO_JOIN_FAST
-  return check_launch(q, "k_join_fast");
-}
-
-int launch_join_fast_planes(Queue* q, const Graph* query, const Graph* data, const PlaneProgram& pp, const uint64_t* planes,
-                            uint32_t planes_rows, const uint16_t* prog, Gmcr* m, int find_first, uint64_t* d_total,
-                            uint32_t reserve) {
+int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first, uint32_t skip,
+                      uint64_t* d_total, uint32_t reserve) {
   if (!m->total) return SIGMO_OK;
   if (query->max_nodes > kMaxQueryNodes)
     return fail(SIGMO_ERR_DOMAIN, "query graphs of up to %u vertices are supported (largest: %u)", kMaxQueryNodes, query->max_nodes);
   const bool exact = q->opts.profile == kProfileExact;
   SIGMO_TRY(launch_query_order(const_cast<Graph*>(query)));
-  const uint32_t skip = exact ? 0u : data->low_offset_graphs;
   const sigmo_tuning& tn = q->tune;
   const uint64_t chunk = std::min<uint64_t>(m->total, static_cast<uint64_t>(tn.mask_chunk_slots) << 20);
   void* buf = nullptr;
@@ -1745,8 +1747,8 @@ int launch_join_fast_planes(Queue* q, const Graph* query, const Graph* data, con
       if (c >= 2 && (cudaMemsetAsync(cursor, 0, 8, st) != cudaSuccess || cudaMemsetAsync(lctr, 0, 16, st) != cudaSuccess))
         rc = fail(SIGMO_ERR_CUDA, "memset failed");
       if (rc) break;
-      k_pair_masks<<<grid_for(cnt, 256, 148u * 16u), 256, 0, st>>>(
-          planes, planes_rows, data->adj_words, pp.prog_off, prog, pp.cls, query->graph_offsets, query->qorder, query->sym,
+      (src.planes ? k_pair_masks<true> : k_pair_masks<false>)<<<grid_for(cnt, 256, 148u * 16u), 256, 0, st>>>(
+          src, data->adj_words, query->graph_offsets, query->qorder, query->sym,
           data->graph_offsets, data->sym, m->indices, m->pair_graph, slot0, cnt, masks, recs, skip, overflow, ctr + 2, llist,
           lctr, m->counts, lparts != 0);
       rc = check_launch(q, "k_pair_masks");
@@ -1793,30 +1795,52 @@ int launch_join_fast_planes(Queue* q, const Graph* query, const Graph* data, con
     q->stream = q->side;
   }
   if (!rc && has_overflow) {
-    // the overflow list through the generic kernel
-    const unsigned block = 128;
-    const unsigned grid = q->tune.overflow_blocks;
-    const uint32_t* list = overflow;
-    const uint32_t split = q->tune.overflow_split;
-    const unsigned long long* list_len = ctr + 2;
-#define SIGMO_JOIN_PLANES(AWV, EX)                                                                                      \
-  k_join_fast<AWV, EX, true><<<grid, block, 0, q->stream>>>(nullptr, 0, planes, planes_rows, pp.prog_off, prog, pp.cls,  \
-                                                            q->opts.profile, query->graph_offsets, query->qorder,        \
-                                                            query->qsel, query->qsel_id, query->sym, data->graph_offsets, \
-                                                            data->adj, data->sym, m->indices, m->pair_graph, list,       \
-                                                            list_len, m->total, skip, find_first, split, ctr + 1, m->counts, \
-                                                            tot, join_limit(q))
-    switch (data->adj_words) {
-      case 1: if (exact) SIGMO_JOIN_PLANES(1, true); else SIGMO_JOIN_PLANES(1, false); break;
-      case 2: if (exact) SIGMO_JOIN_PLANES(2, true); else SIGMO_JOIN_PLANES(2, false); break;
-      default: if (exact) SIGMO_JOIN_PLANES(4, true); else SIGMO_JOIN_PLANES(4, false); break;
+    // the overflow list; a warp's batch is as large as its masks' shared memory allows
+    const uint32_t aw = data->adj_words, stride = query->max_nodes * aw;
+    const uint32_t batch = std::max(1u, std::min<uint32_t>(kWideBatch, static_cast<uint32_t>(kWideMaskBytes / (8ull * stride))));
+    const size_t smem = wide_smem(batch, aw, stride);
+    auto kern = aw == 1   ? (exact ? k_join_wide<1, true> : k_join_wide<1, false>)
+                : aw == 2 ? (exact ? k_join_wide<2, true> : k_join_wide<2, false>)
+                          : (exact ? k_join_wide<4, true> : k_join_wide<4, false>);
+    rc = allow_max_dynamic_smem(reinterpret_cast<const void*>(kern), q->device);
+    if (!rc) {
+      kern<<<q->tune.overflow_blocks, kWideWarps * 32, smem, q->stream>>>(
+          src, query->graph_offsets, query->qorder, query->qsel, query->qsel_id, query->sym, data->graph_offsets, data->adj,
+          data->sym, m->indices, m->pair_graph, overflow, ctr + 2, batch, stride, find_first, ctr + 1, m->counts, tot,
+          join_limit(q));
+      rc = check_launch(q, "k_join_wide");
     }
-#undef SIGMO_JOIN_PLANES
-    rc = check_launch(q, "k_join_fast<planes>");
   }
   q->stream = main_stream;
   if (side && cudaEventRecord(q->ev_join, q->side) == cudaSuccess) cudaStreamWaitEvent(q->stream, q->ev_join, 0);
   dev_free(q, buf);
+  return rc;
+}
+
+int launch_join(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first, uint32_t literal,
+                uint64_t* d_total, const uint32_t* ranges, uint32_t nranges) {
+  if (!m->total) return SIGMO_OK;
+  uint32_t reserve = 0;
+  int rc = SIGMO_OK;
+  if (literal) {
+    // the persistent join leaves one CTA slot per literal block free, so that
+    // the literal join does not wait behind it
+    if (cudaEventRecord(q->ev_fork, q->stream) != cudaSuccess || cudaStreamWaitEvent(q->side, q->ev_fork, 0) != cudaSuccess)
+      return fail(SIGMO_ERR_CUDA, "stream fork failed");
+    const cudaStream_t main_stream = q->stream;
+    q->stream = q->side;
+    reserve = std::min<uint32_t>(literal, 148u);
+    if (!ranges || nranges == 0)
+      rc = launch_join_literal(q, query, data, src, m, find_first, 0, literal, d_total, 0, 0xFFFFFFFFu);
+    for (uint32_t r = 0; ranges && r < nranges && !rc; ++r)
+      rc = launch_join_literal(q, query, data, src, m, find_first, 0, literal, d_total, ranges[r], ranges[r + 1]);
+    q->stream = main_stream;
+  }
+  if (!rc && literal < data->num_graphs) rc = launch_join_pairs(q, query, data, src, m, find_first, literal, d_total, reserve);
+  // join the side stream back (only when this call forked it: a CUDA-graph
+  // capture may wait only on events of streams that joined the capture)
+  if (literal && (cudaEventRecord(q->ev_join, q->side) != cudaSuccess || cudaStreamWaitEvent(q->stream, q->ev_join, 0) != cudaSuccess))
+    rc = rc ? rc : fail(SIGMO_ERR_CUDA, "stream join failed");
   return rc;
 }
 
