@@ -549,7 +549,10 @@ __device__ __forceinline__ uint8_t csr_edge_label(uint32_t a, uint32_t b, const 
 // the DFS is back at depth 1) or, for EXACT, an injective set with clean
 // backtracking.  find_first ends a lane's DFS at its first match.  mapping[]
 // (per query vertex) starts zeroed per lane and carries over between its DFS
-// runs, as the reference's private array does.
+// runs, as the reference's private array does.  Like the driver's join, the
+// count depends on these steps only where the visited set is live: this kernel
+// takes the graphs starting below vertex 256 (REF_PTX) and those over 256
+// vertices; k_join_wide<.., BONDS> takes the others.
 template <bool EXACT>
 __global__ void k_join_wildcard(const uint32_t* __restrict__ bits, uint64_t Wp, int prof, const uint32_t* __restrict__ qgoff,
                                 const uint64_t* __restrict__ qadj, const uint32_t* __restrict__ qroff,
@@ -697,15 +700,53 @@ constexpr size_t kWideMaskBytes = 8192;  // level masks of one warp's batch, at 
 struct WideEntry {
   uint64_t cnt;
   uint32_t qoff, n, s, slot;  // qoff: identity-order flag in bit 31
+  uint32_t root, pad;         // BONDS: the query vertex placed first
 };
 // [batch] entries, [batch][AW] root candidates, [batch][stride] masks per warp
 inline size_t wide_smem(uint32_t batch, uint32_t aw, uint32_t stride) {
   return kWideWarps * batch * (sizeof(WideEntry) + 8ull * aw + 8ull * stride);
 }
 
-template <int AW, bool EXACT>
+//
+// BONDS: joinWildcardCandidates for every slot of the data graphs from
+// `first_graph` on (no list): the root is the query vertex (of the first 32)
+// with the most candidates, highest id on ties, the others follow in id order,
+// an earlier neighbour's row holds only the bonds with the query edge's label,
+// and with find_first every root candidate that extends to a match counts 1.
+// (k_join_wildcard on all slots: 5.09 ms for 22,323 pairs of 2,003 molecules x
+// 40 queries, one lane per root candidate and a walk over the earlier levels
+// and CSR rows for every candidate.)
+struct BondGraphs {
+  const uint64_t* qadj = nullptr;
+  const uint32_t *qroff = nullptr, *qcol = nullptr, *droff = nullptr, *dcol = nullptr, *doffsets = nullptr;
+  const uint8_t *qel = nullptr, *del = nullptr;
+  uint32_t first_graph = 0;
+  uint64_t total_slots = 0;
+};
+
+// Neighbours of data vertex a (graph [s, s + 64 AW)) over bonds of label l; the
+// first CSR entry of a neighbour gives its label (graph.hpp:88-93).
+template <int AW>
+__device__ __forceinline__ void bond_row(const BondGraphs& bg, uint32_t a, uint32_t s, uint8_t l, uint64_t* out) {
+  uint64_t seen[AW];
+#pragma unroll
+  for (int w = 0; w < AW; ++w) seen[w] = out[w] = 0;
+  const uint32_t i1 = bg.droff[a + 1];
+  for (uint32_t i = bg.droff[a]; i < i1; ++i) {
+    const uint32_t t = bg.dcol[i] - s;
+    const bool same = bg.del[i] == l;
+#pragma unroll
+    for (int w = 0; w < AW; ++w) {
+      const uint64_t bit = (t >> 6) == static_cast<uint32_t>(w) ? 1ull << (t & 63u) : 0ull;
+      if (same) out[w] |= bit & ~seen[w];
+      seen[w] |= bit;
+    }
+  }
+}
+
+template <int AW, bool EXACT, bool BONDS>
 __global__ void __launch_bounds__(kWideWarps * 32) k_join_wide(
-    MaskSource src, const uint32_t* __restrict__ qgoff, const uint8_t* __restrict__ qorder, const uint64_t* __restrict__ qsel,
+    MaskSource src, BondGraphs bg, const uint32_t* __restrict__ qgoff, const uint8_t* __restrict__ qorder, const uint64_t* __restrict__ qsel,
     const uint64_t* __restrict__ qsel_id, const uint8_t* __restrict__ qsym, const uint32_t* __restrict__ dgoff,
     const uint64_t* __restrict__ dadj, const uint8_t* __restrict__ dsym, const uint32_t* __restrict__ indices,
     const uint32_t* __restrict__ pair_graph, const uint32_t* __restrict__ list, const unsigned long long* __restrict__ list_len,
@@ -722,7 +763,8 @@ __global__ void __launch_bounds__(kWideWarps * 32) k_join_wide(
   uint8_t pick[kMaxQueryNodes];
 #pragma unroll
   for (int w = 0; w < AW; ++w) p0[0][w] = p1[0][w] = 0;
-  const uint64_t total = *list_len;
+  const uint64_t first = BONDS ? bg.doffsets[bg.first_graph] : 0;
+  const uint64_t total = BONDS ? bg.total_slots - first : *list_len;
   uint64_t my_total = 0, steps = 0;
   for (;;) {
     unsigned long long b = total;
@@ -734,15 +776,15 @@ __global__ void __launch_bounds__(kWideWarps * 32) k_join_wide(
     uint32_t n = 0, qoff = 0, g = 0, s = 0, e = 0;
     bool ident = true;
     if (lane < ne) {
-      const uint32_t slot = list[b + lane];
+      const uint32_t slot = BONDS ? static_cast<uint32_t>(first + b + lane) : list[b + lane];
       const uint32_t qg = indices[slot];
       qoff = qgoff[qg];
       n = qgoff[qg + 1] - qoff;
       g = pair_graph[slot];
       s = dgoff[g];
       e = dgoff[g + 1];
-      ident = !(qsym[qg] && dsym[g]);
-      ent[lane] = WideEntry{0, qoff | (ident ? 0x80000000u : 0u), n, s, slot};
+      ident = BONDS || !(qsym[qg] && dsym[g]);
+      ent[lane] = WideEntry{0, qoff | (ident ? 0x80000000u : 0u), n, s, slot, 0, 0};
     }
     uint32_t incl = n;
 #pragma unroll
@@ -762,7 +804,21 @@ __global__ void __launch_bounds__(kWideWarps * 32) k_join_wide(
       if (it < items) source_mask<AW>(src, AW, oq + (oi ? j : qorder[oq + j]), og, os, oe, masks + pos * stride + j * AW);
     }
     __syncwarp();
-    for (uint32_t i = lane; i < ne * AW; i += 32) roots[i] = masks[(i / AW) * stride + i % AW];
+    if (BONDS) {  // the root of each pair (defineMatchingOrder, isomorphism.hpp:383-408)
+      for (uint32_t c = 0; c < ne; ++c) {
+        const uint32_t m = ent[c].n < 32u ? ent[c].n : 32u;
+        uint32_t mine = 0;
+        if (lane < m)
+#pragma unroll
+          for (int w = 0; w < AW; ++w) mine += __popcll(masks[c * stride + lane * AW + w]);
+        const uint32_t most = __reduce_max_sync(kAll, mine);
+        const uint32_t root = __reduce_max_sync(kAll, lane < m && mine == most ? lane : 0u);
+        if (lane == 0) ent[c].root = root;
+      }
+      __syncwarp();
+    }
+    for (uint32_t i = lane; i < ne * AW; i += 32)
+      roots[i] = masks[(i / AW) * stride + (BONDS ? ent[i / AW].root * AW : 0u) + i % AW];
     __syncwarp();
     // the lanes' searches
     uint64_t alive = 0, cnt = 0;  // alive: levels with untried candidates
@@ -770,19 +826,20 @@ __global__ void __launch_bounds__(kWideWarps * 32) k_join_wide(
     const uint64_t* selp = qsel;
     const uint64_t* M = masks;
     const uint64_t* arow = dadj;
+    uint32_t root = 0, v0 = 0;    // BONDS: the root, and the query's first vertex
     bool dry = false;  // no root candidate left for this lane
     for (;;) {
       if (!alive && cnt) {
         auto* at = reinterpret_cast<unsigned long long*>(&ent[my].cnt);
-        if (find_first) atomicExch(at, 1ull);
-        else atomicAdd(at, static_cast<unsigned long long>(cnt));
+        if (find_first && !BONDS) atomicExch(at, 1ull);
+        else atomicAdd(at, static_cast<unsigned long long>(find_first ? 1ull : cnt));
         cnt = 0;
       }
       if (!alive && !dry) {
         dry = true;
         for (uint32_t i = 0; i < ne && dry; ++i) {
           const uint32_t c = (lane + i) % ne;
-          if (find_first && *reinterpret_cast<volatile uint64_t*>(&ent[c].cnt)) continue;
+          if (find_first && !BONDS && *reinterpret_cast<volatile uint64_t*>(&ent[c].cnt)) continue;
           for (uint32_t w = 0; w < AW && dry; ++w) {
             unsigned long long v = *reinterpret_cast<volatile unsigned long long*>(&roots[c * AW + w]);
             while (v && dry) {
@@ -804,12 +861,15 @@ __global__ void __launch_bounds__(kWideWarps * 32) k_join_wide(
           selp = ((en.qoff >> 31) ? qsel_id : qsel) + (en.qoff & 0x7FFFFFFFu);
           arow = dadj + static_cast<uint64_t>(en.s) * AW;
           M = masks + my * stride;
+          root = en.root;
+          v0 = en.qoff & 0x7FFFFFFFu;
+          s = en.s;
           alive = 1;
         }
       }
       if (!__any_sync(kAll, alive != 0)) break;
       if (!alive) continue;
-      if (find_first && *reinterpret_cast<volatile uint64_t*>(&ent[my].cnt)) {
+      if (find_first && !BONDS && *reinterpret_cast<volatile uint64_t*>(&ent[my].cnt)) {
         alive = 0;
         continue;
       }
@@ -827,7 +887,14 @@ __global__ void __launch_bounds__(kWideWarps * 32) k_join_wide(
       }
       if (!left) alive ^= 1ull << k;
       pick[k] = static_cast<uint8_t>(t);
-      const uint64_t sel = selp[k + 1];
+      // the next level's query vertex and its earlier neighbours (by level)
+      const uint32_t v = !BONDS ? k + 1u : (k + 1u <= root ? k : k + 1u);
+      uint64_t sel = selp[v];
+      if (BONDS) {
+        const uint64_t below = (1ull << root) - 1ull;
+        const uint64_t to_root = (bg.qadj[v0 + root] >> v) & 1ull;
+        sel = to_root | ((sel & below) << 1) | (sel & ~((below << 1) | 1ull));
+      }
       const uint32_t cn = __popcll(sel);
       uint64_t n0[AW], n1[AW], f[AW];
 #pragma unroll
@@ -836,10 +903,20 @@ __global__ void __launch_bounds__(kWideWarps * 32) k_join_wide(
         const uint64_t bit = EXACT && (t >> 6) == static_cast<uint32_t>(w) ? 1ull << (t & 63u) : 0ull;
         n0[w] = (b0 ^ r) | (b1 & b0) | bit;
         n1[w] = b1 | (b0 & r) | bit;
-        f[w] = M[(k + 1) * AW + w];
+        f[w] = M[v * AW + w];
+      }
+      if (BONDS) {  // bond labels of the earlier neighbours
+        for (uint64_t m = sel; m; m &= m - 1) {
+          const uint32_t i = __ffsll(static_cast<long long>(m)) - 1;
+          const uint32_t u = i == 0 ? root : (i <= root ? i - 1u : i);
+          uint64_t row[AW];
+          bond_row<AW>(bg, s + pick[i], s, csr_edge_label(v0 + u, v0 + v, bg.qroff, bg.qcol, bg.qel), row);
+#pragma unroll
+          for (int w = 0; w < AW; ++w) f[w] &= row[w];
+        }
       }
       if (cn <= 2u) {
-        for (uint64_t m = sel; m; m &= m - 1) {
+        for (uint64_t m = BONDS ? 0ull : sel; m; m &= m - 1) {
           const uint64_t* row = arow + static_cast<uint32_t>(pick[__ffsll(static_cast<long long>(m)) - 1]) * AW;
 #pragma unroll
           for (int w = 0; w < AW; ++w) f[w] &= row[w];
@@ -1640,22 +1717,65 @@ int launch_join_wildcard(Queue* q, const Graph* query, const Graph* data, const 
   const uint32_t wg = q->opts.join_work_group_size ? q->opts.join_work_group_size : 128u;
   if (wg > 1024u || (wg & 31u)) return fail(SIGMO_ERR_INVALID, "join work-group size %u must be a multiple of 32 <= 1024", wg);
   const uint32_t G = data->num_graphs;
-  if (!G) return SIGMO_OK;
-  const unsigned grid = std::min<uint32_t>(G, 148u * 64u);
+  if (!G || !m->total) return SIGMO_OK;
   auto* tot = reinterpret_cast<unsigned long long*>(d_total);
-  if (exact)
-    k_join_wildcard<true><<<grid, wg, 0, q->stream>>>(c->bits, c->Wp, q->opts.profile, query->graph_offsets, query->adj,
-                                                      query->row_offsets, query->column_indices, query->edge_labels,
-                                                      data->graph_offsets, data->adj, data->adj_words, data->row_offsets,
-                                                      data->column_indices, data->edge_labels, m->offsets, m->indices, G,
-                                                      find_first, m->counts, tot);
-  else
-    k_join_wildcard<false><<<grid, wg, 0, q->stream>>>(c->bits, c->Wp, q->opts.profile, query->graph_offsets, query->adj,
-                                                       query->row_offsets, query->column_indices, query->edge_labels,
-                                                       data->graph_offsets, data->adj, data->adj_words, data->row_offsets,
-                                                       data->column_indices, data->edge_labels, m->offsets, m->indices, G,
-                                                       find_first, m->counts, tot);
-  return check_launch(q, "k_join_wildcard");
+  // graphs [0, literal): step by step, on the side stream; the others by sets
+  uint32_t literal = G;
+  if (data->max_nodes <= 64u * kMaxAdjWords) {
+    literal = 0;
+    while (!exact && literal < G && data->host_graph_offsets[literal] < kLowOffsetLimit) ++literal;
+  }
+  if (literal) {
+    if (cudaEventRecord(q->ev_fork, q->stream) != cudaSuccess || cudaStreamWaitEvent(q->side, q->ev_fork, 0) != cudaSuccess)
+      return fail(SIGMO_ERR_CUDA, "stream fork failed");
+    const unsigned grid = std::min<uint32_t>(literal, 148u * 64u);
+    auto kern = exact ? k_join_wildcard<true> : k_join_wildcard<false>;
+    kern<<<grid, wg, 0, q->side>>>(c->bits, c->Wp, q->opts.profile, query->graph_offsets, query->adj, query->row_offsets,
+                                   query->column_indices, query->edge_labels, data->graph_offsets, data->adj, data->adj_words,
+                                   data->row_offsets, data->column_indices, data->edge_labels, m->offsets, m->indices, literal,
+                                   find_first, m->counts, tot);
+    SIGMO_TRY(check_launch(q, "k_join_wildcard"));
+  }
+  int rc = SIGMO_OK;
+  if (literal < G) {
+    rc = launch_query_order(const_cast<Graph*>(query));
+    void* cursor = nullptr;
+    if (!rc) rc = tmp_alloc(q, &cursor, 8);
+    if (!rc && cudaMemsetAsync(cursor, 0, 8, q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "memset failed");
+    MaskSource src;
+    src.bits = c->bits;
+    src.Wp = c->Wp;
+    src.prof = q->opts.profile;
+    BondGraphs bg;
+    bg.qadj = query->adj;
+    bg.qroff = query->row_offsets;
+    bg.qcol = query->column_indices;
+    bg.qel = query->edge_labels;
+    bg.droff = data->row_offsets;
+    bg.dcol = data->column_indices;
+    bg.del = data->edge_labels;
+    bg.doffsets = m->offsets;
+    bg.first_graph = literal;
+    bg.total_slots = m->total;
+    const uint32_t aw = data->adj_words, stride = query->max_nodes * aw;
+    const uint32_t batch = std::max(1u, std::min<uint32_t>(kWideBatch, static_cast<uint32_t>(kWideMaskBytes / (8ull * stride))));
+    const size_t smem = wide_smem(batch, aw, stride);
+    auto kern = aw == 1   ? (exact ? k_join_wide<1, true, true> : k_join_wide<1, false, true>)
+                : aw == 2 ? (exact ? k_join_wide<2, true, true> : k_join_wide<2, false, true>)
+                          : (exact ? k_join_wide<4, true, true> : k_join_wide<4, false, true>);
+    if (!rc) rc = allow_max_dynamic_smem(reinterpret_cast<const void*>(kern), q->device);
+    if (!rc) {
+      kern<<<grid_for(m->total, kWideWarps * batch, q->tune.overflow_blocks), kWideWarps * 32, smem, q->stream>>>(
+          src, bg, query->graph_offsets, query->qorder, query->qsel_id, query->qsel_id, query->sym, data->graph_offsets, data->adj,
+          data->sym, m->indices, m->pair_graph, nullptr, nullptr, batch, stride, find_first,
+          static_cast<unsigned long long*>(cursor), m->counts, tot, JoinLimit{0, q->d_status});
+      rc = check_launch(q, "k_join_wide<bonds>");
+    }
+    dev_free(q, cursor);
+  }
+  if (literal && (cudaEventRecord(q->ev_join, q->side) != cudaSuccess || cudaStreamWaitEvent(q->stream, q->ev_join, 0) != cudaSuccess))
+    rc = rc ? rc : fail(SIGMO_ERR_CUDA, "stream join failed");
+  return rc;
 }
 
 int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first, uint32_t skip,
@@ -1799,14 +1919,14 @@ int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const Mas
     const uint32_t aw = data->adj_words, stride = query->max_nodes * aw;
     const uint32_t batch = std::max(1u, std::min<uint32_t>(kWideBatch, static_cast<uint32_t>(kWideMaskBytes / (8ull * stride))));
     const size_t smem = wide_smem(batch, aw, stride);
-    auto kern = aw == 1   ? (exact ? k_join_wide<1, true> : k_join_wide<1, false>)
-                : aw == 2 ? (exact ? k_join_wide<2, true> : k_join_wide<2, false>)
-                          : (exact ? k_join_wide<4, true> : k_join_wide<4, false>);
+    auto kern = aw == 1   ? (exact ? k_join_wide<1, true, false> : k_join_wide<1, false, false>)
+                : aw == 2 ? (exact ? k_join_wide<2, true, false> : k_join_wide<2, false, false>)
+                          : (exact ? k_join_wide<4, true, false> : k_join_wide<4, false, false>);
     rc = allow_max_dynamic_smem(reinterpret_cast<const void*>(kern), q->device);
     if (!rc) {
       kern<<<q->tune.overflow_blocks, kWideWarps * 32, smem, q->stream>>>(
-          src, query->graph_offsets, query->qorder, query->qsel, query->qsel_id, query->sym, data->graph_offsets, data->adj,
-          data->sym, m->indices, m->pair_graph, overflow, ctr + 2, batch, stride, find_first, ctr + 1, m->counts, tot,
+          src, BondGraphs{}, query->graph_offsets, query->qorder, query->qsel, query->qsel_id, query->sym, data->graph_offsets,
+          data->adj, data->sym, m->indices, m->pair_graph, overflow, ctr + 2, batch, stride, find_first, ctr + 1, m->counts, tot,
           join_limit(q));
       rc = check_launch(q, "k_join_wide");
     }

@@ -90,3 +90,27 @@ def test_levels_with_any_number_of_earlier_neighbours(prof, ff):
     q, d = sb.io.parse("\n".join(queries) + "\n"), sb.io.parse("\n".join(graphs) + "\n")
     ref = _check(q, d, 2, prof, ff)
     assert ref["total"] > 0
+
+
+@pytest.mark.parametrize("prof,ff", MODES)
+@pytest.mark.parametrize("qlo,qhi,dlo,dhi,count", [(2, 6, 3, 64, 150), (10, 40, 20, 130, 200), (20, 48, 120, 256, 60)])
+def test_bond_label_join_sizes(qlo, qhi, dlo, dhi, count, prof, ff):
+    d = sb.generate_molecules(count, dlo, dhi, seed=3201 + dhi, kind=1, median=(dlo + dhi) / 2)
+    q = sb.generate_queries(16, qlo, qhi, seed=3202 + qhi).concat(sb.generate_queries(4, 2, 4, seed=3203))
+    queue = sb.Queue(0, profile=prof)
+    qg, dg = sb.createDeviceCSRGraph(queue, q), sb.createDeviceCSRGraph(queue, d)
+    cand = sb.Candidates(queue, qg.total_nodes, dg.total_nodes)
+    sig = sb.Signature(queue, dg.total_nodes, qg.total_nodes)
+    sb.filterCandidates(queue, qg, dg, sig, cand)  # labels only: many candidates per vertex
+    sig.generateDataSignatures(dg)
+    sig.generateQuerySignatures(qg)
+    sig.refineDataSignatures(dg, 1)
+    sig.refineQuerySignatures(qg, 1)
+    sb.refineCandidates(queue, qg, dg, sig, cand)
+    gm = sb.GMCR(queue)
+    gm.generateGMCR(qg, dg, cand)
+    off, idx = gm.getGMCR()
+    want_total, want_per = oracle.join_wildcard(q, d, cand.getHostCandidates(), off, idx, PROF[prof], ff)
+    total = np.zeros(1, np.uint64)
+    _, per = sb.joinWildcardCandidates(queue, qg, dg, cand, gm, total, ff, per_pair=True)
+    assert len(idx) > 0 and np.array_equal(per, want_per) and int(total[0]) == want_total
