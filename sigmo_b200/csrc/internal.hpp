@@ -267,10 +267,9 @@ int launch_join_wildcard(Queue* q, const Graph* query, const Graph* data, const 
                          uint64_t* d_total);
 // Every pair of data graphs from `skip` on (molecules of up to 64 * kMaxAdjWords
 // vertices; REF_PTX: starting at vertex 256 or above, where the reference's
-// count does not depend on the order of its search).  reserve: persistent join
-// CTA slots left free for a kernel running beside it.
+// count does not depend on the order of its search).
 int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first, uint32_t skip,
-                      uint64_t* d_total, uint32_t reserve = 0);
+                      uint64_t* d_total);
 // Every pair: the literal join of data graphs [0, literal) on the side stream
 // (once per range of query graphs when `ranges` holds nranges + 1 boundaries),
 // beside launch_join_pairs for the rest; the main stream waits for both.

@@ -8,11 +8,11 @@
 // (isomorphism.hpp:150-168).  mapping[] starts zeroed per thread and is
 // carried across the pairs the thread handles, as in the reference.  Under
 // REF_PTX the visited bitset is inert for any data graph whose first vertex is
-// >= 256; the batched form therefore runs this kernel only for the few graphs
-// below that.
+// >= 256; the literal search therefore runs only for the few graphs below that
+// (k_join_literal_sets), for REF_X86, and for graphs over 256 vertices.
 //
-// k_join_fast counts the same matches with graph-local bit sets.  For the
-// pairs it handles, the reference's count is order independent:
+// The other kernels count the same matches with graph-local bit sets.  For the
+// pairs they handle, the reference's count is order independent:
 //   REF_PTX (visited inert): #{(d_0..d_{n-1}) in prod C_i : for all i<j,
 //       adjQ(i,j) == adjD(d_i,d_j)}  (non-adjacent query vertices may share a
 //       data vertex);
@@ -353,6 +353,9 @@ __global__ void k_join_literal(const uint32_t* __restrict__ bits, uint64_t Wp, i
 //           mapping[0..j-1], fixed while the frame runs, so it is one AND
 //           when the frame is pushed); the others are skipped by the
 //           reference with no effect, so the placements are the same;
+//           As in k_join_dfs, the test is the rows of the earlier neighbours
+//           and a count: p0[j], p1[j] are the bit planes (to 3) of the number
+//           of rows of mapping[0..j-1] that hold a vertex;
 //   map[j]  mapping[j] as a local id, carried across the thread's pairs of a
 //           data graph like the reference's private array (isomorphism.hpp:309);
 //           a fresh work-item's mapping[] holds global vertex 0, which is
@@ -365,38 +368,67 @@ __global__ void k_join_literal(const uint32_t* __restrict__ bits, uint64_t Wp, i
 // below 256).  The last query vertex is placed in one step, as in
 // k_join_literal.
 //
-// A serial chain per pair: bound by the latency of a step, so the sets are
-// taken from the planes where the caller has them.  (Writing them as bitset
-// words first took seven more launches, 130 us before the join of a batch of
-// any size.)  Molecules over 64 atoms and queries over 32 vertices used to
-// take k_join_literal's candidate-by-candidate form: 3.7 ms for the first ten
-// molecules of 60,000 x 500 uneven pairs, against 0.5 ms here.
+// A serial chain per pair (and per work-item), and few of them: bound by the
+// latency of a step.  So the sets are taken from the planes where the caller
+// has them (writing them as bitset words first took seven more launches, 130 us
+// before the join of a batch of any size), the graph's rows are staged in
+// shared memory, a round's masks are built by the whole block, and the
+// work-items of a graph are spread over blocks of kLitItems: a warp steps through its lanes' different moves in turn, so four
+// lanes take less time than 32, and blocks of 9 KB fit beside the persistent
+// join's.  (One block of 128 work-items per graph, walking the earlier rows at
+// each step: 1.02 ms for the first ten molecules of 100,000 x 600 pairs, 112 us
+// of 1,000 x 20; this form 190 and 74 us.)  Launches over many graphs (REF_X86)
+// keep one block per graph.  Molecules over 64 atoms and queries over
+// 32 vertices used to take k_join_literal's candidate-by-candidate form: 3.7 ms
+// for the first ten molecules of 60,000 x 500 uneven pairs.
 constexpr uint32_t kLitLevels = 32;
 constexpr uint8_t kLitOutside = 0xFFu;
-constexpr size_t kLitBytesPerThread = kLitLevels * (2 * sizeof(uint64_t) + 1);
+constexpr uint32_t kLitItems = 4;
+constexpr size_t kLitBytesPerThread = kLitLevels * (4 * sizeof(uint64_t) + 1);
 
+// wg: work-items of a graph (the reference's work-group size); bt of them per
+// block, one thread each.  With SMEM the block may have more threads, which only
+// help to build the level masks.
 template <int AW, bool SMEM>
-__global__ void k_join_literal_sets(MaskSource src, int prof, const uint32_t* __restrict__ qgoff, const uint64_t* __restrict__ qadj,
+__global__ void k_join_literal_sets(MaskSource src, int prof, const uint32_t* __restrict__ qgoff, const uint64_t* __restrict__ qsel_id,
                                     const uint32_t* __restrict__ dgoff, const uint64_t* __restrict__ dadj, uint32_t dAW,
                                     const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ indices, uint32_t g0,
-                                    uint32_t g1, uint32_t q_begin, uint32_t q_end, int find_first, uint64_t* __restrict__ counts,
-                                    unsigned long long* __restrict__ d_total, JoinLimit lim) {
+                                    uint32_t g1, uint32_t wg, uint32_t bt, uint32_t q_begin, uint32_t q_end, int find_first,
+                                    uint64_t* __restrict__ counts, unsigned long long* __restrict__ d_total, JoinLimit lim) {
   extern __shared__ uint64_t lit_sm[];
-  const uint32_t wg = blockDim.x, lid = threadIdx.x;
-  uint64_t* cm_s = lit_sm + lid;
-  uint64_t* rem_s = lit_sm + kLitLevels * wg + lid;
-  uint8_t* map_s = reinterpret_cast<uint8_t*>(lit_sm + 2 * kLitLevels * wg) + lid;
+  __shared__ uint64_t s_row[SMEM ? 64 : 1];  // the graph's adjacency rows (word 0)
+  const uint32_t tid = threadIdx.x;
+  uint64_t* cm_s = lit_sm + tid;  // the threads past bt - 1 do not search
+  uint64_t* rem_s = lit_sm + kLitLevels * bt + tid;
+  uint64_t* p0_s = lit_sm + 2 * kLitLevels * bt + tid;
+  uint64_t* p1_s = lit_sm + 3 * kLitLevels * bt + tid;
+  uint8_t* map_s = reinterpret_cast<uint8_t*>(lit_sm + 4 * kLitLevels * bt) + tid;
   constexpr uint32_t kLocal = SMEM ? 1 : kMaxQueryNodes;
-  uint64_t cm_l[kLocal * AW], rem_l[kLocal * AW];
+  uint64_t cm_l[kLocal * AW], rem_l[kLocal * AW], p0_l[kLocal * AW], p1_l[kLocal * AW];
   uint8_t map_l[kLocal];
-#define CM(j, w) (SMEM ? cm_s[(j) * wg] : cm_l[(j) * AW + (w)])
-#define REM(j, w) (SMEM ? rem_s[(j) * wg] : rem_l[(j) * AW + (w)])
-#define MAP(j) (SMEM ? map_s[(j) * wg] : map_l[(j)])
+#define CM(j, w) (SMEM ? cm_s[(j) * bt] : cm_l[(j) * AW + (w)])
+#define REM(j, w) (SMEM ? rem_s[(j) * bt] : rem_l[(j) * AW + (w)])
+#define P0(j, w) (SMEM ? p0_s[(j) * bt] : p0_l[(j) * AW + (w)])
+#define P1(j, w) (SMEM ? p1_s[(j) * bt] : p1_l[(j) * AW + (w)])
+#define MAP(j) (SMEM ? map_s[(j) * bt] : map_l[(j)])
   constexpr uint32_t kLevels = SMEM ? kLitLevels : kMaxQueryNodes;
+  const uint32_t parts = (wg + bt - 1u) / bt;  // blocks per graph
+  const uint64_t blocks = static_cast<uint64_t>(g1 - g0) * parts;
   uint64_t my_total = 0, steps = 0;
   bool stop = false;
-  for (uint32_t g = g0 + blockIdx.x; g < g1 && !stop; g += gridDim.x) {
+#pragma unroll
+  for (int w = 0; w < AW; ++w)
+    if (tid < bt) P0(0, w) = P1(0, w) = 0;
+  for (uint64_t blk = blockIdx.x; blk < blocks; blk += gridDim.x) {
+    const uint32_t g = g0 + static_cast<uint32_t>(blk / parts), lid = static_cast<uint32_t>(blk % parts) * bt + tid;
     const uint32_t s = dgoff[g], e = dgoff[g + 1];
+    if (SMEM) {
+      __syncthreads();  // the previous graph's rows are no longer read
+      for (uint32_t i = tid; i < e - s; i += blockDim.x) s_row[i] = dadj[static_cast<uint64_t>(s + i) * dAW];
+      __syncthreads();
+    }
+    const bool searches = tid < bt && lid < wg;
+    auto row_of = [&](uint32_t t, int w) -> uint64_t { return SMEM ? s_row[t] : dadj[static_cast<uint64_t>(s + t) * dAW + w]; };
     uint32_t seg0 = offsets[g], seg1 = offsets[g + 1];
     if (q_begin != 0 || q_end != 0xFFFFFFFFu) {  // the segment's slots with query graph in [q_begin, q_end)
       uint32_t lo = seg0, hi = seg1;
@@ -416,7 +448,7 @@ __global__ void k_join_literal_sets(MaskSource src, int prof, const uint32_t* __
     }
     const uint8_t map0 = s == 0 ? 0 : kLitOutside;
 #pragma unroll 1
-    for (uint32_t k = 0; k < kLevels; ++k) MAP(k) = map0;  // mapping[] of a fresh work-item
+    for (uint32_t k = 0; searches && k < kLevels; ++k) MAP(k) = map0;  // mapping[] of a fresh work-item
     // graph-local bits the reference's uint8-indexed visited set can hold:
     // under REF_PTX those whose global id is below 256; under REF_X86 all
     // (the count modulo 64 is the local id).  A fresh work-item's mapping[]
@@ -424,14 +456,26 @@ __global__ void k_join_literal_sets(MaskSource src, int prof, const uint32_t* __
     const uint64_t low = prof == kProfileX86 ? ~0ull
                          : (s >= 256u ? 0ull : (256u - s >= 64u ? ~0ull : ((1ull << (256u - s)) - 1ull)));
     const uint64_t outside_bit = prof == kProfileX86 ? (1ull << ((0u - s) & 63u)) : 0ull;
-    for (uint32_t it = lid; it < seg1 - seg0; it += wg) {
+    const uint32_t lid0 = lid - tid;  // the block's first work-item
+    for (uint32_t it = lid; lid0 < wg && it - tid < seg1 - seg0; it += wg) {
+      if (SMEM) {  // the masks of the round's pairs, (work-item, level) per thread
+        __syncthreads();  // the round before is done
+        for (uint32_t x = tid; x < bt * kLitLevels; x += blockDim.x) {
+          const uint32_t i = x % bt, j = x / bt, slot = it - tid + i;
+          if (lid0 + i >= wg || slot >= seg1 - seg0) continue;
+          const uint32_t q0 = qgoff[indices[seg0 + slot]];
+          if (q0 + j < qgoff[indices[seg0 + slot] + 1]) source_mask<AW>(src, dAW, q0 + j, g, s, e, lit_sm + j * bt + i);
+        }
+        __syncthreads();
+      }
+      if (stop || !searches || it >= seg1 - seg0) continue;
       if (join_stopped(lim)) {
         stop = true;
-        break;
+        continue;
       }
       const uint32_t qg = indices[seg0 + it];
       const uint32_t qoff = qgoff[qg], n = qgoff[qg + 1] - qoff;
-      for (uint32_t j = 0; j < n; ++j) {
+      for (uint32_t j = 0; !SMEM && j < n; ++j) {
         uint64_t m[AW];
         source_mask<AW>(src, dAW, qoff + j, g, s, e, m);
 #pragma unroll
@@ -480,23 +524,30 @@ __global__ void k_join_literal_sets(MaskSource src, int prof, const uint32_t* __
             // place t at depth qn and push the frame of depth qn + 1
             MAP(qn) = static_cast<uint8_t>(t);
             visited |= bit;
-            // isValidMapping for depth d = qn + 1 against mapping[0..qn]: the
-            // data rows of the picks (graph-local adjacency words) must equal
-            // the query's adjacency to d, bit for bit
+            // isValidMapping for depth d = qn + 1 against mapping[0..qn]: a
+            // candidate is in the rows of d's earlier neighbours and no other
             const uint32_t d = qn + 1;
-            const uint64_t qcol = qadj[qoff + d];  // bit i: query vertices i and d adjacent
-            uint64_t vm[AW];
+            const uint64_t sel = qsel_id[qoff + d];  // bit i: query vertex i < d has d in its row
+            const uint32_t cn = __popcll(sel);
+            const uint32_t i1 = cn ? __ffsll(static_cast<long long>(sel)) - 1u : 0u, i2 = cn ? 63u - __clzll(static_cast<long long>(sel)) : 0u;
+            const uint32_t t1 = i1 == qn ? t : MAP(i1), t2 = i2 == qn ? t : MAP(i2);
+            const uint64_t e0 = cn == 1u ? ~0ull : 0ull, e1 = cn == 2u ? ~0ull : 0ull;
 #pragma unroll
-            for (int w = 0; w < AW; ++w)
-              vm[w] = CM(d, w) & ~(dadj[static_cast<uint64_t>(s + t) * dAW + w] ^ (0ull - ((qcol >> qn) & 1ull)));
-            for (uint32_t i = 0; i < qn; ++i) {
-              const uint64_t* row = dadj + static_cast<uint64_t>(s + MAP(i)) * dAW;
-              const uint64_t want = 0ull - ((qcol >> i) & 1ull);
-#pragma unroll
-              for (int w = 0; w < AW; ++w) vm[w] &= ~(row[w] ^ want);
+            for (int w = 0; w < AW; ++w) {
+              const uint64_t r = row_of(t, w), b0 = P0(qn, w), b1 = P1(qn, w);
+              const uint64_t n0 = (b0 ^ r) | (b1 & b0), n1 = b1 | (b0 & r);
+              uint64_t vm = CM(d, w);
+              if (cn <= 2u) {
+                if (cn) vm &= row_of(t1, w) & row_of(t2, w);
+                vm &= ~((n0 ^ e0) | (n1 ^ e1));
+              } else {
+                for (uint32_t i = 0; i <= qn; ++i)
+                  vm &= ~(row_of(i == qn ? t : MAP(i), w) ^ (0ull - ((sel >> i) & 1ull)));
+              }
+              REM(d, w) = vm;
+              P0(d, w) = n0;
+              P1(d, w) = n1;
             }
-#pragma unroll
-            for (int w = 0; w < AW; ++w) REM(d, w) = vm[w];
             ++top;
             continue;
           }
@@ -511,23 +562,22 @@ __global__ void k_join_literal_sets(MaskSource src, int prof, const uint32_t* __
           break;
         }
       }
-      if (stop) break;
+      if (stop) continue;
       counts[seg0 + it] = found;
       my_total += found;
     }
   }
 #undef CM
 #undef REM
+#undef P0
+#undef P1
 #undef MAP
-  for (int o = 16; o; o >>= 1) my_total += __shfl_xor_sync(0xFFFFFFFFu, my_total, o);
-  __shared__ uint64_t part[32];
-  if ((lid & 31u) == 0) part[lid >> 5] = my_total;
+  __shared__ unsigned long long s_total;
+  if (tid == 0) s_total = 0;
   __syncthreads();
-  if (lid < 32) {
-    uint64_t v = lid < ((wg + 31u) >> 5) ? part[lid] : 0ull;
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    if (lid == 0 && v) atomicAdd(d_total, static_cast<unsigned long long>(v));
-  }
+  if (my_total) atomicAdd(&s_total, static_cast<unsigned long long>(my_total));
+  __syncthreads();
+  if (tid == 0 && s_total) atomicAdd(d_total, s_total);
 }
 
 // getEdgeLabel (graph.hpp:88-93): label of the CSR entry a -> b, or 255.
@@ -1134,7 +1184,7 @@ __global__ void __launch_bounds__(kPhaseThreads) k_join_masks(
       const uint4 r = pr;  // first data vertex, query size | flags, query offset, query graph
       const uint64_t m0 = pm0, m1 = pm1;
       fetch();
-      if (r.y & 0xA00u) continue;  // the literal join's, or in the overflow list (generic kernel)
+      if (r.y & 0xA00u) continue;  // the literal join's, or in the overflow list
       n = r.y & 0xFFu;
       s = r.x;
       selp = ((r.y & 0x100u) ? qsel_id : qsel) + r.z;
@@ -1676,7 +1726,8 @@ int launch_join_literal(Queue* q, const Graph* query, const Graph* data, const M
     return fail(SIGMO_ERR_DOMAIN, "exact profile supports data graphs of at most %u vertices", 64u * kMaxAdjWords);
   const uint32_t wg = q->opts.join_work_group_size ? q->opts.join_work_group_size : 128u;
   if (wg > 1024u || (wg & 31u)) return fail(SIGMO_ERR_INVALID, "join work-group size %u must be a multiple of 32 <= 1024", wg);
-  const unsigned grid = std::min<uint32_t>(graph_end - graph_begin, 148u * 64u);
+  SIGMO_TRY(launch_query_order(const_cast<Graph*>(query)));
+  const uint32_t graphs = graph_end - graph_begin;
   auto* tot = reinterpret_cast<unsigned long long*>(d_total);
   uint32_t range_max = data->max_nodes;
   if (range_max > 64u) {
@@ -1686,21 +1737,25 @@ int launch_join_literal(Queue* q, const Graph* query, const Graph* data, const M
   }
   // one word per set where the range's graphs allow it; its state fits shared
   // memory up to kLitLevels levels and 256 threads
-  const bool one = range_max <= 64u, smem_fits = one && query->max_nodes <= kLitLevels && wg <= 256u;
+  const bool one = range_max <= 64u;
+  // few graphs (those below vertex 256): small blocks, else a block per graph
+  const uint32_t block = graphs <= kLowOffsetLimit ? kLitItems : wg;
+  const bool smem_fits = one && query->max_nodes <= kLitLevels && kLitBytesPerThread * block <= 200u * 1024u;
+  const uint64_t want = static_cast<uint64_t>(graphs) * ((wg + block - 1u) / block);
   if (one || (q->opts.profile == kProfilePtx && range_max <= 64u * kMaxAdjWords)) {
-    const size_t smem = smem_fits ? kLitBytesPerThread * wg : 0;
+    const size_t smem = smem_fits ? kLitBytesPerThread * block : 0;
     auto kern = smem_fits ? k_join_literal_sets<1, true>
                 : one     ? k_join_literal_sets<1, false>
                 : data->adj_words == 2 ? k_join_literal_sets<2, false>
                                        : k_join_literal_sets<4, false>;
     if (smem) SIGMO_TRY(allow_max_dynamic_smem(reinterpret_cast<const void*>(kern), q->device));
-    kern<<<grid, wg, smem, q->stream>>>(src, q->opts.profile, query->graph_offsets, query->adj, data->graph_offsets, data->adj,
-                                        data->adj_words, m->offsets, m->indices, graph_begin, graph_end, q_begin, q_end,
-                                        find_first, m->counts, tot, join_limit(q));
+    kern<<<grid_for(want, 1, 148u * 64u), smem_fits ? std::max(block, 32u) : block, smem, q->stream>>>(
+        src, q->opts.profile, query->graph_offsets, query->qsel_id, data->graph_offsets, data->adj, data->adj_words, m->offsets,
+        m->indices, graph_begin, graph_end, wg, block, q_begin, q_end, find_first, m->counts, tot, join_limit(q));
     return check_launch(q, "k_join_literal_sets");
   }
   if (!src.bits) return fail(SIGMO_ERR_INVALID, "internal: the literal join of graphs over %u vertices reads the bitset", 64u * kMaxAdjWords);
-  k_join_literal<<<grid, wg, 0, q->stream>>>(src.bits, src.Wp, q->opts.profile, query->graph_offsets, query->adj,
+  k_join_literal<<<std::min<uint32_t>(graphs, 148u * 64u), wg, 0, q->stream>>>(src.bits, src.Wp, q->opts.profile, query->graph_offsets, query->adj,
                                              data->graph_offsets, data->adj, data->adj_words, data->row_offsets,
                                              data->column_indices, m->offsets, m->indices, graph_begin, graph_end, q_begin,
                                              q_end, find_first, m->counts, tot, join_limit(q));
@@ -1779,7 +1834,7 @@ int launch_join_wildcard(Queue* q, const Graph* query, const Graph* data, const 
 }
 
 int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first, uint32_t skip,
-                      uint64_t* d_total, uint32_t reserve) {
+                      uint64_t* d_total) {
   if (!m->total) return SIGMO_OK;
   if (query->max_nodes > kMaxQueryNodes)
     return fail(SIGMO_ERR_DOMAIN, "query graphs of up to %u vertices are supported (largest: %u)", kMaxQueryNodes, query->max_nodes);
@@ -1845,11 +1900,9 @@ int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const Mas
     if (!rc && has_long) rc = allow_max_dynamic_smem(reinterpret_cast<const void*>(dfs_long), q->device);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, q->device);
-    // persistent CTAs; `reserve` slots stay free for a kernel running beside
-    // them.  k_join_dfs keeps at most three resident: a fourth would start its
-    // region only when another CTA has ended
-    const unsigned full = static_cast<unsigned>(sms) * (dfs ? std::min(tn.join_blocks_per_sm, 3u) : tn.join_blocks_per_sm);
-    const unsigned grid = full > reserve + static_cast<unsigned>(sms) ? full - reserve : full;
+    // persistent CTAs; every join kernel keeps at most three resident (a fourth
+    // of k_join_dfs would start its region only when another CTA has ended)
+    const unsigned grid = static_cast<unsigned>(sms) * (dfs ? std::min(tn.join_blocks_per_sm, 3u) : tn.join_blocks_per_sm);
     // fewer pairs than lanes: every pair in up to 16 parts by root candidate
     uint32_t lparts = 0;
     while (dfs && lparts < 4 && (m->total << (lparts + 1)) <= static_cast<uint64_t>(grid) * block) ++lparts;
@@ -1873,17 +1926,6 @@ int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const Mas
           lctr, m->counts, lparts != 0);
       rc = check_launch(q, "k_pair_masks");
       if (!rc && cudaEventRecord(q->ev_masks[par], st) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
-      if (!rc && has_long) {
-        const unsigned lblock = dfs_threads<kPhaseLevels>();
-        if (cudaStreamWaitEvent(long_stream, q->ev_masks[par], 0) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "stream fork failed");
-        if (!rc) {
-          dfs_long<<<static_cast<unsigned>(sms), lblock, dfs_smem<kPhaseLevels>(), long_stream>>>(
-              masks, recs, slot0, cnt, llist, lctr, long_parts, query->qmeta, query->qmeta_id, query->qsel,
-              query->qsel_id, data->adj, find_first, 8u, find_first ? kRefillFirst : kRefillAll, lctr + 1, m->counts, tot, join_limit(q));
-          rc = check_launch(q, "k_join_dfs<long>");
-        }
-        if (!rc && cudaEventRecord(q->ev_long[par], long_stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
-      }
       if (!rc) {
         if (dfs)
           dfs_short<<<grid, block, smem, st>>>(masks, recs, slot0, cnt, nullptr, nullptr, lparts, query->qmeta, query->qmeta_id,
@@ -1893,6 +1935,19 @@ int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const Mas
           join_kernel<<<grid, block, smem, st>>>(masks, recs, slot0, cnt, query->qsel, query->qsel_id, data->adj, find_first,
                                                  tn.join_chunk, cursor, m->counts, tot, join_limit(q));
         rc = check_launch(q, frontier ? "k_join_frontier" : dfs ? "k_join_dfs" : "k_join_masks");
+      }
+      // the long pairs after the short ones: their CTAs take the room that the
+      // persistent CTAs of the short form leave as they end
+      if (!rc && has_long) {
+        const unsigned lblock = dfs_threads<kPhaseLevels>();
+        if (cudaStreamWaitEvent(long_stream, q->ev_masks[par], 0) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "stream fork failed");
+        if (!rc) {
+          dfs_long<<<3u * static_cast<unsigned>(sms), lblock, dfs_smem<kPhaseLevels>(), long_stream>>>(
+              masks, recs, slot0, cnt, llist, lctr, long_parts, query->qmeta, query->qmeta_id, query->qsel,
+              query->qsel_id, data->adj, find_first, 8u, find_first ? kRefillFirst : kRefillAll, lctr + 1, m->counts, tot, join_limit(q));
+          rc = check_launch(q, "k_join_dfs<long>");
+        }
+        if (!rc && cudaEventRecord(q->ev_long[par], long_stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
       }
       // the chunk's buffers are free again once its long pairs are joined too
       if (has_long && cudaStreamWaitEvent(st, q->ev_long[par], 0) != cudaSuccess) rc = rc ? rc : fail(SIGMO_ERR_CUDA, "stream join failed");
@@ -1940,23 +1995,20 @@ int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const Mas
 int launch_join(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first, uint32_t literal,
                 uint64_t* d_total, const uint32_t* ranges, uint32_t nranges) {
   if (!m->total) return SIGMO_OK;
-  uint32_t reserve = 0;
+  SIGMO_TRY(launch_query_order(const_cast<Graph*>(query)));  // before the fork: both streams read it
   int rc = SIGMO_OK;
   if (literal) {
-    // the persistent join leaves one CTA slot per literal block free, so that
-    // the literal join does not wait behind it
     if (cudaEventRecord(q->ev_fork, q->stream) != cudaSuccess || cudaStreamWaitEvent(q->side, q->ev_fork, 0) != cudaSuccess)
       return fail(SIGMO_ERR_CUDA, "stream fork failed");
     const cudaStream_t main_stream = q->stream;
     q->stream = q->side;
-    reserve = std::min<uint32_t>(literal, 148u);
     if (!ranges || nranges == 0)
       rc = launch_join_literal(q, query, data, src, m, find_first, 0, literal, d_total, 0, 0xFFFFFFFFu);
     for (uint32_t r = 0; ranges && r < nranges && !rc; ++r)
       rc = launch_join_literal(q, query, data, src, m, find_first, 0, literal, d_total, ranges[r], ranges[r + 1]);
     q->stream = main_stream;
   }
-  if (!rc && literal < data->num_graphs) rc = launch_join_pairs(q, query, data, src, m, find_first, literal, d_total, reserve);
+  if (!rc && literal < data->num_graphs) rc = launch_join_pairs(q, query, data, src, m, find_first, literal, d_total);
   // join the side stream back (only when this call forked it: a CUDA-graph
   // capture may wait only on events of streams that joined the capture)
   if (literal && (cudaEventRecord(q->ev_join, q->side) != cudaSuccess || cudaStreamWaitEvent(q->stream, q->ev_join, 0) != cudaSuccess))
