@@ -20,9 +20,8 @@ void free_groups(Queue* q, PlaneProgram* pp) {
     dev_free(q, g.spec);
     dev_free(q, g.r_begin);
     dev_free(q, g.row_of);
-    dev_free(q, g.prog);
-    dev_free(q, g.qc_off);
-    dev_free(q, g.qc);
+    dev_free(q, g.quads);
+    dev_free(q, g.q_off);
   }
   pp->groups.clear();
 }
@@ -32,12 +31,11 @@ void free_program(Queue* q, PlaneProgram* pp) {
   dev_free(q, pp->spec);
   dev_free(q, pp->prog_off);
   dev_free(q, pp->prog);
+  dev_free(q, pp->quads);
   dev_free(q, pp->cls);
   dev_free(q, pp->r_begin);
-  dev_free(q, pp->qc_off);
-  dev_free(q, pp->qc);
+  dev_free(q, pp->q_off);
   dev_free(q, pp->qsig_all);
-  pp->qc_off = pp->qc = nullptr;
   *pp = PlaneProgram{};
 }
 
@@ -61,6 +59,18 @@ void parallel_ranges(uint64_t n, unsigned parts, F&& f, int force_serial = 0) {
   for (unsigned p = 1; p < parts; ++p) th.emplace_back([&, p] { f(p, n * p / parts, n * (p + 1) / parts); });
   f(0, 0, n / parts);
   for (auto& t : th) t.join();
+}
+
+// A class program (plane ids below 2^15) appended to `quads`, four ids per
+// entry, its last id repeated to fill the last entry, whose bit 63 is set.
+template <class F>
+void append_quads(size_t n, F&& id, std::vector<uint64_t>* quads) {
+  for (size_t i = 0; i < n; i += 4) {
+    uint64_t x = 0;
+    for (size_t j = 0; j < 4; ++j) x |= static_cast<uint64_t>(id(std::min(i + j, n - 1))) << (16 * j);
+    quads->push_back(x);
+  }
+  quads->back() |= 1ull << 63;
 }
 
 int upload(Queue* q, void** dst, const void* src, size_t bytes) {
@@ -315,42 +325,31 @@ int plan_groups(Queue* q, Graph* query, uint32_t AW, const std::vector<uint32_t>
     }
     r_begin[R] = static_cast<uint32_t>(spec.size());
     for (int r = static_cast<int>(R) - 1; r >= 0; --r) r_begin[r] = std::min(r_begin[r], r_begin[r + 1]);
-    // local programs; qc: per query entry, its class's local program range
-    std::vector<uint32_t> loc_class(C, 0xFFFFFFFFu), prog_off{0}, qc_off{0}, qc;
-    std::vector<uint16_t> prog;
+    // the queries' programs in local ids
+    std::vector<uint32_t> q_off{0};
+    std::vector<uint64_t> quads;
+    if (spec.size() >= 32768u) return fail(SIGMO_ERR_DOMAIN, "group %zu needs %zu planes (limit 32767)", gi, spec.size());
     for (uint32_t qg = grp.q0; qg < grp.q1; ++qg) {
       for (uint32_t e = off[qg]; e < off[qg + 1]; ++e) {
-        const uint32_t c = list[e];
-        if (loc_class[c] == 0xFFFFFFFFu) {
-          loc_class[c] = static_cast<uint32_t>(prog_off.size() - 1);
-          for (uint32_t i = pp.h_prog_off[c]; i < pp.h_prog_off[c + 1]; ++i)
-            prog.push_back(static_cast<uint16_t>(loc_plane[pp.h_prog[i]]));
-          prog_off.push_back(static_cast<uint32_t>(prog.size()));
-        }
-        qc.push_back(prog_off[loc_class[c]]);
-        qc.push_back(prog_off[loc_class[c] + 1]);
+        const uint32_t b = pp.h_prog_off[list[e]], n = pp.h_prog_off[list[e] + 1] - b;
+        // every local id the kernel will index with must be inside its array
+        for (uint32_t i = 0; i < n; ++i)
+          if (loc_plane[pp.h_prog[b + i]] >= spec.size())
+            return fail(SIGMO_ERR_INVALID, "internal: group %zu plane %u outside its %zu planes", gi, loc_plane[pp.h_prog[b + i]], spec.size());
+        append_quads(n, [&](size_t i) { return loc_plane[pp.h_prog[b + i]]; }, &quads);
       }
-      qc_off.push_back(static_cast<uint32_t>(qc.size() / 2));
+      q_off.push_back(static_cast<uint32_t>(quads.size()));
     }
     grp.K = static_cast<uint32_t>(spec.size());
-    grp.C = static_cast<uint32_t>(prog_off.size() - 1);
-    // every local id and range the kernel will index with must be inside its array
-    for (uint16_t k : prog)
-      if (k >= grp.K) return fail(SIGMO_ERR_INVALID, "internal: group %zu plane %u outside its %u planes", gi, k, grp.K);
-    for (size_t i = 0; i < qc.size(); i += 2)
-      if (qc[i] > qc[i + 1] || qc[i + 1] > prog.size())
-        return fail(SIGMO_ERR_INVALID, "internal: group %zu program range outside its %zu entries", gi, prog.size());
     if (planes_admit_smem(grp.K, AW) > 200u * 1024u)
       return fail(SIGMO_ERR_DOMAIN, "group %zu needs more than one admission tile of shared memory", gi);
     grp.nlab = nlab;
-    grp.n_qc = qc.size() / 2;
-    grp.n_prog = prog.size();
+    grp.n_quads = quads.size();
     SIGMO_TRY(upload(q, reinterpret_cast<void**>(&grp.spec), spec.data(), 4 * spec.size()));
     SIGMO_TRY(upload(q, reinterpret_cast<void**>(&grp.r_begin), r_begin.data(), 4 * r_begin.size()));
     SIGMO_TRY(upload(q, reinterpret_cast<void**>(&grp.row_of), row_of.data(), 4 * row_of.size()));
-    SIGMO_TRY(upload(q, reinterpret_cast<void**>(&grp.prog), prog.data(), 2 * prog.size()));
-    SIGMO_TRY(upload(q, reinterpret_cast<void**>(&grp.qc_off), qc_off.data(), 4 * qc_off.size()));
-    SIGMO_TRY(upload(q, reinterpret_cast<void**>(&grp.qc), qc.data(), 4 * qc.size()));
+    SIGMO_TRY(upload(q, reinterpret_cast<void**>(&grp.quads), quads.data(), 8 * quads.size()));
+    SIGMO_TRY(upload(q, reinterpret_cast<void**>(&grp.q_off), q_off.data(), 4 * q_off.size()));
     SIGMO_CUDA_TRY(cudaStreamSynchronize(q->stream));  // host vectors go out of scope
     pp.groups.push_back(grp);
   }
@@ -363,7 +362,7 @@ int plan_groups(Queue* q, Graph* query, uint32_t AW, const std::vector<uint32_t>
 // query that a graph cannot admit is usually rejected by its first class.
 int order_classes(Queue* q, Graph* query, Graph* data) {
   PlaneProgram& pp = query->pp;
-  if (pp.qc && pp.qc_for == data && pp.qc_stamp == data->stamp) return SIGMO_OK;
+  if (pp.q_off && pp.qc_for == data && pp.qc_stamp == data->stamp) return SIGMO_OK;
   SIGMO_TRY(ensure_label_hist(q, data));
   const uint32_t QG = query->num_graphs;
   uint64_t all = 0;
@@ -393,21 +392,29 @@ int order_classes(Queue* q, Graph* query, Graph* data) {
     list.insert(list.end(), per[qg].begin(), per[qg].end());
     off.push_back(static_cast<uint32_t>(list.size()));
   }
-  dev_free(q, pp.qc_off);
-  dev_free(q, pp.qc);
-  pp.qc_off = pp.qc = nullptr;
-  // the kernel reads each entry as its class's program range [begin, end) in prog
-  std::vector<uint32_t> ranges(2 * list.size());
-  for (size_t e = 0; e < list.size(); ++e) {
-    ranges[2 * e] = pp.h_prog_off[list[e]];
-    ranges[2 * e + 1] = pp.h_prog_off[list[e] + 1];
-  }
-  SIGMO_TRY(upload(q, reinterpret_cast<void**>(&pp.qc_off), off.data(), 4 * off.size()));
-  SIGMO_TRY(upload(q, reinterpret_cast<void**>(&pp.qc), ranges.data(), 4 * ranges.size()));
-  pp.h_qc_n = list.size();
+  dev_free(q, pp.q_off);
+  dev_free(q, pp.quads);
+  pp.q_off = nullptr;
+  pp.quads = nullptr;
   free_groups(q, &pp);
   const uint32_t AW = data->adj_words;
-  if (planes_admit_smem(pp.K, AW) > kGroupSmemBudget) SIGMO_TRY(plan_groups(q, query, AW, off, list));
+  // the queries' programs as the kernel reads them: the batch's, and per group
+  // when the batch's planes do not fit one tile
+  std::vector<uint32_t> q_off(QG + 1, 0);
+  std::vector<uint64_t> quads;
+  const bool one_tile = planes_admit_smem(pp.K, AW) <= kGroupSmemBudget;
+  if (pp.K < 32768u)
+    for (uint32_t qg = 0; qg < QG; ++qg) {
+      for (uint32_t e = off[qg]; e < off[qg + 1]; ++e) {
+        const uint32_t b = pp.h_prog_off[list[e]];
+        append_quads(pp.h_prog_off[list[e] + 1] - b, [&](size_t i) { return pp.h_prog[b + i]; }, &quads);
+      }
+      q_off[qg + 1] = static_cast<uint32_t>(quads.size());
+    }
+  pp.n_quads = quads.size();
+  SIGMO_TRY(upload(q, reinterpret_cast<void**>(&pp.q_off), q_off.data(), 4 * q_off.size()));
+  SIGMO_TRY(upload(q, reinterpret_cast<void**>(&pp.quads), quads.data(), 8 * quads.size()));
+  if (!one_tile) SIGMO_TRY(plan_groups(q, query, AW, off, list));
   SIGMO_CUDA_TRY(cudaStreamSynchronize(q->stream));  // host vectors go out of scope
   pp.qc_for = data;
   pp.qc_stamp = data->stamp;
@@ -480,7 +487,7 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
   const uint32_t L = exact ? 0u : std::min(data->low_offset_graphs, G);
   auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
   const ResidentPlanes* rp = run.resident;
-  const uint64_t b_dsig = run.dsig ? 0 : 8ull * R * N, b_planes = rp ? 0 : 8ull * GW * pp.K * AW * 32,
+  const uint64_t b_dsig = run.dsig ? 0 : 8ull * R * N, b_planes = rp ? 0 : 8ull * G * pp.K * AW,
                  b_ne = 4ull * query->num_graphs * GW + 4ull * G;
   // resident planes: the batch's plane k is resident row row_map[k], and the
   // class programs are rewritten as resident rows for the join
@@ -542,6 +549,7 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
   src.prof = q->opts.profile;
   src.planes = rp ? rp->planes : planes;
   src.K = rp ? rp->rows : pp.K;
+  src.tiled = rp != nullptr;
   src.prog_off = pp.prog_off;
   src.prog = rp ? d_rprog : pp.prog;
   src.cls = pp.cls;

@@ -93,10 +93,9 @@ struct PlaneGroup {
   uint32_t* spec = nullptr;      // [K]
   uint32_t* r_begin = nullptr;   // [R + 1]
   uint32_t* row_of = nullptr;    // [K] plane row in the batch
-  uint16_t* prog = nullptr;      // the group's class programs, local plane ids
-  uint32_t* qc_off = nullptr;    // [q1 - q0 + 1]
-  uint32_t* qc = nullptr;        // per entry in evaluation order, its local program range (begin, end)
-  size_t n_qc = 0, n_prog = 0;
+  uint64_t* quads = nullptr;     // the group's query programs, local plane ids (PlaneProgram::quads)
+  uint32_t* q_off = nullptr;     // [q1 - q0 + 1]
+  size_t n_quads = 0;
 };
 
 // Per-query-batch plane program of the batched form (kernels_planes.cu).
@@ -116,11 +115,13 @@ struct PlaneProgram {
   // host copies (class evaluation order)
   std::vector<uint32_t> h_spec, h_prog_off, h_cls, h_qgoff;
   std::vector<uint16_t> h_prog;
-  // per query graph, its distinct classes in evaluation order for one data
-  // graph's label frequencies (rebuilt when the data graph changes)
-  uint32_t* qc_off = nullptr;     // [query graphs + 1]
-  uint32_t* qc = nullptr;         // per entry, its class's program range in prog: (begin, end) u32 pairs
-  size_t h_qc_n = 0;              // entries of qc
+  // per query graph, the programs of its distinct classes in evaluation order
+  // for one data graph's label frequencies (rebuilt when the data graph
+  // changes): four plane ids of 15 bits per entry, a class's last id repeated
+  // to fill its last entry, bit 63 set in it
+  uint64_t* quads = nullptr;
+  uint32_t* q_off = nullptr;      // [query graphs + 1] entries of quads
+  size_t n_quads = 0;
   std::vector<PlaneGroup> groups; // empty: the whole batch fits one tile
   const void* qc_for = nullptr;   // the data graph the order was built for
   uint64_t qc_stamp = 0;
@@ -248,14 +249,16 @@ int launch_fused_filter(Queue* q, const Graph* query, const Graph* data, uint32_
 int launch_gmcr(Queue* q, const Graph* query, const Graph* data, const Candidates* c, Gmcr* m, bool sync_total,
                 uint64_t capacity_hint);
 // Where a join takes a pair's candidate sets from: the candidate bitset, or
-// the batched form's planes (planes: [graph / 32][K][AW][32]; prog: the class
-// programs as row indices into it, pp.prog for the per-batch planes).
+// the batched form's planes ([graph][K][AW], or tiled: [graph / 32][K][AW][32],
+// the resident planes; prog: the class programs as row indices into it, pp.prog
+// for the per-batch planes).
 struct MaskSource {
   const uint32_t* bits = nullptr;
   uint64_t Wp = 0;
   int prof = 0;  // range masks of the bitset's words
   const uint64_t* planes = nullptr;
   uint32_t K = 0;
+  bool tiled = false;
   const uint32_t* prog_off = nullptr;
   const uint16_t* prog = nullptr;
   const uint32_t* cls = nullptr;
@@ -290,6 +293,7 @@ constexpr size_t kGroupSmemBudget = 96u * 1024u;
 // (row_map[k] = resident row of the batch's plane k).
 int launch_planes_admit_resident(Queue* q, const Graph* query, const Graph* data, const ResidentPlanes& rp,
                                  const PlaneProgram& pp, const uint32_t* row_map, uint32_t* admit, uint32_t* counts);
+// Shared memory of a tile of 32 graphs and K planes.
 size_t planes_admit_smem(uint32_t K, uint32_t AW);
 // GMCR from admission words admit[query graph][data graph / 32] and the
 // admitted count of every data graph (scan, total, sorted fill).

@@ -118,14 +118,16 @@ __device__ __forceinline__ void source_mask(const MaskSource& src, uint32_t dAW,
     extract_local<AW>(src.bits + static_cast<uint64_t>(v) * src.Wp, s, e, src.prof, out);
     return;
   }
-  const uint64_t* base = src.planes + static_cast<uint64_t>(g >> 5) * src.K * dAW * 32 + (g & 31u);
+  const uint64_t* base = src.planes + (src.tiled ? static_cast<uint64_t>(g >> 5) * src.K * dAW * 32 + (g & 31u)
+                                                 : static_cast<uint64_t>(g) * src.K * dAW);
+  const uint32_t step = src.tiled ? 32u : 1u;
 #pragma unroll
   for (int w = 0; w < AW; ++w) out[w] = ~0ull;
   const uint32_t c = src.cls[v], e1 = src.prog_off[c + 1];
   for (uint32_t i = src.prog_off[c]; i < e1; ++i) {
-    const uint64_t* row = base + static_cast<uint64_t>(src.prog[i]) * dAW * 32;
+    const uint64_t* row = base + static_cast<uint64_t>(src.prog[i]) * dAW * step;
 #pragma unroll
-    for (int w = 0; w < AW; ++w) out[w] &= row[32 * w];
+    for (int w = 0; w < AW; ++w) out[w] &= row[step * w];
   }
 }
 
@@ -1114,9 +1116,11 @@ __global__ void __launch_bounds__(256) k_pair_masks(
       // one word: the graph's vertex set fits it (word 0 of each plane)
       uint64_t m = ~0ull;
       if (FROM_PLANES) {
-        const uint64_t* pb = src.planes + static_cast<uint64_t>(o_g >> 5) * src.K * AW * 32 + (o_g & 31u);
+        const uint64_t* pb = src.planes + (src.tiled ? static_cast<uint64_t>(o_g >> 5) * src.K * AW * 32 + (o_g & 31u)
+                                                     : static_cast<uint64_t>(o_g) * src.K * AW);
+        const uint32_t step = src.tiled ? AW * 32u : AW;
         const uint32_t c = src.cls[v], e1 = src.prog_off[c + 1];
-        for (uint32_t e = src.prog_off[c]; e < e1; ++e) m &= pb[static_cast<uint64_t>(src.prog[e]) * AW * 32];
+        for (uint32_t e = src.prog_off[c]; e < e1; ++e) m &= pb[src.prog[e] * step];
       } else {
         extract_local<1>(src.bits + static_cast<uint64_t>(v) * src.Wp, o_s, o_e, src.prof, &m);
       }

@@ -12,9 +12,13 @@
 // candidates.hpp:98) is folded into the label planes.  Identical query
 // vertices share one program ("class").
 //
-// Plane layout: planes[((g / 32) * K + k) * AW + w][g % 32] (u64), so the
-// planes of 32 consecutive graphs form one contiguous tile that a CTA copies
-// to shared memory and reads with lane = graph, conflict-free.
+// Plane layouts in memory (u64 words): a batch's planes are graph-major,
+// planes[g][k][AW], so the join's level masks of one molecule read one run of
+// K words (k_pair_masks, whose lanes hold levels of a few molecules: 0.85 ->
+// 0.67 ms for 6.86 M pairs against tile-major rows); the serving loop's resident
+// planes are tile-major, planes[g / 32][k][AW][g % 32], so that the rows of a
+// tile that a batch uses are gathered in 256-byte runs.  In shared memory a
+// tile is [k][AW][32], read with lane = graph, conflict-free.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,118 +33,138 @@ namespace {
 // Label planes come first, then thresholds in (r, l, c) order;
 // r_begin[r] .. r_begin[r + 1] are the thresholds of iteration r.
 
-// One graph's planes into column `gl` of a shared-memory tile [K * AW][32]:
-// the warp's lanes hold vertices lane + 32 p, every plane is a ballot per
-// 32-vertex chunk, and the plane word is stored by a single lane.  Chunks
-// beyond the graph's last vertex are skipped (the warp handles one graph, so
-// that test is uniform).
+// One graph's planes into column `col` of a shared-memory tile whose rows are
+// `row_words` words apart, by one warp.  With `out`, the words also go to
+// out[k][AW] (row row_of[k] when given).
+//
+// Label planes: the lanes hold vertices lane + 32 p, a plane is a ballot per
+// 32-vertex chunk.  Threshold planes: the lanes hold 32 planes (consecutive
+// planes share an iteration, so a load of a vertex's counters is a broadcast of
+// two or three words) and walk the vertices from the last to the first, shifting
+// each comparison's carry into the lane's word: a load, a shift and two
+// additions per vertex for 32 planes, where a ballot per plane took a
+// load, the extraction, a vote and a select for 32 vertices of molecules with
+// 35 (k_planes_admit 1.36 -> 1.09 ms on 100,000 molecules x 600 queries, 0.93 ->
+// 0.51 ms on 60,013 x 500 with sets of two words).
+//
+// plane_test: what a plane compares.  Labels: {value, -}.  Thresholds:
+// {2^32 - (c << 28), left shift that brings the counter's four bits to the top
+// of its 32-bit half | 0x100 for the high half | iteration << 16}: count >= c
+// exactly when the shifted half >= c << 28 (the bits below the counter only add
+// to it), i.e. when adding 2^32 - (c << 28) carries out.
+__device__ __forceinline__ uint2 plane_test(uint32_t sp) {
+  if (sp & 0x80000000u) return make_uint2(sp & 0xFFu, 0u);
+  const uint32_t l = (sp >> 8) & 0xFFu;
+  return make_uint2(0u - ((sp & 0xFFu) << 28), (28u - 4u * (l & 7u)) | (l >= 8u ? 0x100u : 0u) | (sp & 0xFF0000u));
+}
+
+// 2 * acc + the carry of x + y
+__device__ __forceinline__ uint32_t shift_in_carry(uint32_t acc, uint32_t x, uint32_t y) {
+  uint32_t r;
+  asm("{\n .reg .u32 t;\n add.cc.u32 t, %2, %3;\n addc.u32 %0, %1, %1;\n}\n" : "=r"(r) : "r"(acc), "r"(x), "r"(y));
+  return r;
+}
+
 template <int AW>
-__device__ __forceinline__ void build_graph_planes(uint64_t* tile, uint32_t gl, uint32_t s, uint32_t e, unsigned lane,
+__device__ __forceinline__ void build_graph_planes(uint64_t* col, uint32_t row_words, uint32_t s, uint32_t e, unsigned lane,
                                                    const uint8_t* __restrict__ lab, const uint64_t* __restrict__ sig_all,
-                                                   uint64_t N, uint32_t R, uint32_t nlab, const uint32_t* __restrict__ spec,
-                                                   const uint32_t* __restrict__ r_begin, int prof, uint32_t base) {
+                                                   uint64_t N, uint32_t K, uint32_t nlab, const uint2* tests, int prof,
+                                                   uint32_t base, uint64_t* __restrict__ out,
+                                                   const uint32_t* __restrict__ row_of) {
   constexpr int P = 2 * AW;  // 32-vertex chunks per graph
   const uint32_t n = e - s;
-  const uint32_t chunks = (n + 31u) / 32u;
-  uint8_t lb[P];
-  bool vis[P];
-#pragma unroll
-  for (int p = 0; p < P; ++p) {
-    const uint32_t t = lane + 32u * p;
-    const bool in = t < n;
-    const uint32_t v = s + t;
-    lb[p] = in ? lab[v] : 0;
-    // visibility follows global ids (base + local id): the range-mask rule
-    // depends on where the graph ends relative to 32-vertex words
-    const uint32_t gv = base + v;
-    vis[p] = in && ((range_mask(gv >> 5, base + s, base + e, prof) >> (gv & 31u)) & 1u);
-  }
-  auto put = [&](uint32_t k, const uint32_t (&chunk)[P]) {
-#pragma unroll
-    for (int w = 0; w < AW; ++w) {
-      const uint64_t word = static_cast<uint64_t>(chunk[2 * w]) | (static_cast<uint64_t>(chunk[2 * w + 1]) << 32);
-      if (lane == ((k * AW + w) & 31u)) tile[(k * AW + w) * 32 + gl] = word;
-    }
-  };
-  for (uint32_t k = 0; k < nlab; ++k) {
-    const uint32_t val = spec[k] & 0xFFu;
-    uint32_t chunk[P];
-#pragma unroll
-    for (int p = 0; p < P; ++p)
-      chunk[p] = static_cast<uint32_t>(p) < chunks ? __ballot_sync(0xFFFFFFFFu, vis[p] && (val == kWildcard || lb[p] == val)) : 0u;
-    put(k, chunk);
-  }
-  for (uint32_t r = 0; r < R; ++r) {
-    const uint32_t k0 = r_begin[r], k1 = r_begin[r + 1];
-    if (k0 == k1) continue;
-    uint64_t sg[P];
+  {
+    uint8_t lb[P];
+    bool vis[P];
 #pragma unroll
     for (int p = 0; p < P; ++p) {
       const uint32_t t = lane + 32u * p;
-      sg[p] = (static_cast<uint32_t>(p) < chunks && t < n) ? sig_all[static_cast<uint64_t>(r) * N + s + t] : 0ull;
+      const bool in = t < n;
+      const uint32_t v = s + t;
+      lb[p] = in ? lab[v] : 0;
+      // visibility follows global ids (base + local id): the range-mask rule
+      // depends on where the graph ends relative to 32-vertex words
+      const uint32_t gv = base + v;
+      vis[p] = in && ((range_mask(gv >> 5, base + s, base + e, prof) >> (gv & 31u)) & 1u);
     }
-    for (uint32_t k = k0; k < k1; ++k) {
-      const uint32_t sp = spec[k];
-      const uint32_t sh = 4u * ((sp >> 8) & 0xFFu), c = sp & 0xFFu;
+    for (uint32_t k = 0; k < nlab; ++k) {
+      const uint32_t val = tests[k].x;
       uint32_t chunk[P];
 #pragma unroll
-      for (int p = 0; p < P; ++p)
-        chunk[p] = static_cast<uint32_t>(p) < chunks
-                       ? __ballot_sync(0xFFFFFFFFu, static_cast<uint32_t>((sg[p] >> sh) & 0xFull) >= c)
-                       : 0u;
-      put(k, chunk);
+      for (int p = 0; p < P; ++p) chunk[p] = __ballot_sync(0xFFFFFFFFu, vis[p] && (val == kWildcard || lb[p] == val));
+#pragma unroll
+      for (int w = 0; w < AW; ++w)
+        if (lane == static_cast<unsigned>(w)) {
+          const uint64_t word = static_cast<uint64_t>(chunk[2 * w]) | (static_cast<uint64_t>(chunk[2 * w + 1]) << 32);
+          col[k * row_words + w * 32] = word;
+          if (out) out[static_cast<uint64_t>(row_of ? row_of[k] : k) * AW + w] = word;
+        }
     }
   }
-}
-
-// Per 32-graph tile (one CTA per tile, grid-stride): build the tile's planes
-// in shared memory from the data signatures, write the tile out (coalesced;
-// the join reads it), then decide the GMCR admission of every query graph
-// for the tile's 32 graphs (gmcr.hpp:33-128: every query vertex has a
-// candidate in the graph):
-//     admit[q][tile] = AND over q's classes c of NE(c),
-//     NE(c) = ballot over the tile's graphs of "AND of c's program planes != 0".
-// Warps take query graphs; a query's classes are visited in the order the
-// host chose (rarest label first, longer programs first), so most queries
-// are rejected for all 32 graphs after one or two classes and stop there.
-// A class's AND chain stops as soon as it is zero in all 32 graphs.  NE(c)
-// is evaluated for each query that reaches it: classes are rarely shared
-// between queries, and without a per-class cache in shared memory four CTAs
-// fit on an SM instead of three.  The per-graph admitted counts (the GMCR
-// segment lengths) are summed in shared memory.  Queries of one vertex are
-// never admitted (the reference's mapping skips them, gmcr.hpp:100): their
-// class lists are empty.
-constexpr uint32_t kAdmitWarps = 16;
-
-// The tile's planes: built from the data signatures (and written out for the
-// join), or gathered from resident planes (rows row_map[k] of the tile).
-template <int AW, bool GATHER>
-__device__ __forceinline__ void fill_tile(uint64_t* tile, uint32_t gw, uint32_t G, const uint32_t* __restrict__ goff,
-                                          const uint8_t* __restrict__ lab, const uint64_t* __restrict__ sig_all, uint64_t N,
-                                          uint32_t R, uint32_t K, uint32_t nlab, const uint32_t* __restrict__ spec,
-                                          const uint32_t* __restrict__ r_begin, int prof, uint32_t base,
-                                          const uint64_t* __restrict__ rplanes, uint32_t rrows,
-                                          const uint32_t* __restrict__ row_map) {
-  constexpr uint32_t kRow = AW * 32u;
-  const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (GATHER) {
-    const uint64_t* src = rplanes + static_cast<uint64_t>(gw) * rrows * kRow;
-    for (uint32_t k = wid; k < K; k += nw) {
-      const uint64_t* row = src + static_cast<uint64_t>(row_map[k]) * kRow;
+  for (uint32_t k0 = nlab; k0 < K; k0 += 32) {
+    const uint32_t k = k0 + lane;
+    const uint2 ts = tests[k < K ? k : K - 1u];
+    const uint32_t sh = ts.y & 31u, bound = ts.x;
+    const uint32_t* sg = reinterpret_cast<const uint32_t*>(sig_all + static_cast<uint64_t>((ts.y >> 16) & 0xFFu) * N + s) + ((ts.y >> 8) & 1u);
+    uint64_t word[AW];
 #pragma unroll
-      for (int w = 0; w < AW; ++w) tile[k * kRow + 32 * w + lane] = row[32 * w + lane];
+    for (int w = 0; w < AW; ++w) {
+      uint32_t acc[2] = {0, 0};
+#pragma unroll
+      for (int h = 1; h >= 0; --h) {
+        const uint32_t v0 = 64u * w + 32u * h;
+        if (n <= v0) continue;
+        uint32_t v = n - v0 < 32u ? n : v0 + 32u;
+        for (; (v & 7u) && v > v0; --v) acc[h] = shift_in_carry(acc[h], __ldg(sg + 2 * (v - 1)) << sh, bound);
+        for (; v > v0; v -= 8) {  // eight loads in flight
+          uint32_t x[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[i] = __ldg(sg + 2 * (v - 1 - i));
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[h] = shift_in_carry(acc[h], x[i] << sh, bound);
+        }
+      }
+      word[w] = static_cast<uint64_t>(acc[0]) | (static_cast<uint64_t>(acc[1]) << 32);
     }
-  } else {
-    for (uint32_t gl = wid; gl < 32; gl += nw) {
-      const uint32_t g = gw * 32u + gl;
-      if (g < G) {
-        build_graph_planes<AW>(tile, gl, goff[g], goff[g + 1], lane, lab, sig_all, N, R, nlab, spec, r_begin, prof, base);
-      } else {
-        for (uint32_t i = lane; i < K * AW; i += 32) tile[i * 32 + gl] = 0;
+    if (k < K) {
+      const uint64_t row = row_of && out ? row_of[k] : k;
+#pragma unroll
+      for (int w = 0; w < AW; ++w) {
+        col[k * row_words + w * 32] = word[w];
+        if (out) out[row * AW + w] = word[w];
       }
     }
   }
 }
+
+// Per tile of 32 * H graphs (one CTA per tile, grid-stride): build the tile's
+// planes in shared memory from the data signatures (and write them out; the
+// join reads them), then decide the GMCR admission of every query graph for
+// the tile's graphs (gmcr.hpp:33-128: every query vertex has a candidate in
+// the graph):
+//     admit[q][tile] = AND over q's classes c of NE(c),
+//     NE(c) = ballot over the tile's graphs of "AND of c's program planes != 0".
+// Warps take query graphs; a query's classes are visited in the order the
+// host chose (rarest label first, longer programs first), so most queries
+// are rejected for all graphs after one or two classes and stop there.  A
+// class's AND chain starts with the graphs the classes before it left and
+// stops once it is zero in all of them (at every four planes: one 8-byte load
+// gives four plane ids).  NE(c) is evaluated for each query that reaches it:
+// classes are rarely shared between queries.  The per-graph admitted counts
+// (the GMCR segment lengths) are summed in shared memory.  Queries of one
+// vertex are never admitted (the reference's mapping skips them, gmcr.hpp:100):
+// their class lists are empty.
+//
+// Bound by instruction issue (63 % of the slots, 58 % of the shared-memory
+// wavefronts).  H = 2: a lane carries two graphs through the
+// chain, so the program, its addresses and the votes are paid once for 64
+// graphs instead of twice (a model of 1,024 molecules x 600 queries: 4.1
+// classes of 6.5 planes per 32-graph tile and query; 1.35 -> 1.09 ms on 100,000
+// x 600, 0.533 -> 0.512 ms on 200,000 x 60); it needs twice the shared memory,
+// so it is taken where two CTAs of 512 threads still fit an SM, and enough tiles
+// to fill the chip (eight per SM).  A tile whose graphs all have at most 64
+// atoms works on word 0 alone in a batch of wider sets.
+constexpr uint32_t kAdmitWarps = 16;
 
 // 16-byte asynchronous global -> shared copies (no registers in between).
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
@@ -150,33 +174,37 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// Resident rows row_map[k] of tile gw into dst (K rows of AW x 32 words),
-// as 16-byte asynchronous copies spread over the block.
-template <int AW>
+// Resident rows s_map[k] of the 32-graph tiles gw * H .. into dst
+// [K][H][AW * 32], as 16-byte asynchronous copies spread over the block (tiles
+// past the last one: zeros).
+template <int AW, int H>
 __device__ __forceinline__ void gather_tile_async(uint64_t* dst, const uint64_t* __restrict__ rplanes, uint32_t rrows,
-                                                  uint32_t gw, uint32_t K, const uint32_t* s_map) {
-  constexpr uint32_t kRow = AW * 32u, kChunks = AW * 16u;  // 16-byte chunks per row
-  const uint64_t* src = rplanes + static_cast<uint64_t>(gw) * rrows * kRow;
+                                                  uint32_t gw, uint32_t GW, uint32_t K, const uint32_t* s_map) {
+  constexpr uint32_t kRow = AW * 32u, kChunks = AW * 16u * H;  // 16-byte chunks per row of the tile
   for (uint32_t i = threadIdx.x; i < K * kChunks; i += blockDim.x) {
-    const uint32_t k = i / kChunks, c = i % kChunks;
-    cp_async16(dst + k * kRow + 2 * c, src + static_cast<uint64_t>(s_map[k]) * kRow + 2 * c);
+    const uint32_t k = i / kChunks, c = i % kChunks, h = c / (AW * 16u), tile = gw * H + h;
+    uint64_t* at = dst + static_cast<size_t>(k) * (H * kRow) + 2 * c;
+    if (tile < GW) {
+      cp_async16(at, rplanes + (static_cast<uint64_t>(tile) * rrows + s_map[k]) * kRow + 2 * (c % (AW * 16u)));
+    } else {
+      at[0] = at[1] = 0;
+    }
   }
   cp_async_commit();
 }
 
-// Shared-memory layout of k_planes_admit (in u64 units for the tiles):
-//   tile buffer [K * AW * 32] u64, s_map[K] (gather), then the
-//   staged class lists when they fit:
-//   qc[n_qc] (uint2 program ranges), qc_off[QG + 1] (u32), prog[n_prog] (u16).
+// Shared-memory layout of k_planes_admit: tile buffer [K][H][AW * 32] u64, the
+// planes' tests [K] (uint2) or, for a gathered tile, their resident rows [K]
+// (u32), then the queries' programs when they fit: prog[n_quads] (u64: four
+// plane ids), q_off[QG + 1] (u32).
 struct AdmitSmem {
-  size_t tiles, map, lists, total;
+  size_t specs, lists, total;
 };
-__host__ __device__ inline AdmitSmem admit_smem_layout(uint32_t K, uint32_t AW, bool gather, size_t list_bytes) {
+__host__ __device__ inline AdmitSmem admit_smem_layout(uint32_t K, uint32_t AW, uint32_t H, bool gather, size_t list_bytes) {
   AdmitSmem l{};
-  l.tiles = 0;
-  size_t off = static_cast<size_t>(K) * AW * 32 * 8;
-  l.map = off;
-  off += gather ? 4ull * K : 0;
+  size_t off = static_cast<size_t>(K) * H * AW * 32 * 8;
+  l.specs = off;
+  off += (gather ? 4ull : 8ull) * K;
   off = (off + 15) & ~static_cast<size_t>(15);
   l.lists = off;
   off += list_bytes;
@@ -184,125 +212,148 @@ __host__ __device__ inline AdmitSmem admit_smem_layout(uint32_t K, uint32_t AW, 
   return l;
 }
 
-template <int AW, bool GATHER>
-__global__ void __launch_bounds__(kAdmitWarps * 32) k_planes_admit(
+// The admission words of every query graph for one tile, on W of the AW words.
+// A query's program is one run of quads, prog[q_off[qg], q_off[qg + 1]): its
+// classes one after the other, bit 15 of a quad's last id marking a class's
+// end.
+template <int AW, int H, int W>
+__device__ __forceinline__ void admit_tile(const uint64_t* tile, uint32_t QG, const uint32_t* q_off, const uint2* prog,
+                                           const uint32_t (&valid)[H], uint32_t tile0, uint32_t GW,
+                                           uint32_t* __restrict__ admit, uint32_t (&my_cnt)[H]) {
+  constexpr uint32_t kRow = H * AW * 32u;
+  const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const uint64_t* tl = tile + lane;
+  uint32_t i0 = wid < QG ? q_off[wid] : 0u;
+  for (uint32_t qg = wid; qg < QG; qg += nw) {
+    const uint32_t i1 = q_off[qg + 1];
+    uint64_t m[H][W];
+    bool left = i1 > i0;  // an empty program: a query of at most one vertex
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+#pragma unroll
+      for (int w = 0; w < W; ++w) m[h][w] = left && ((valid[h] >> lane) & 1u) ? ~0ull : 0ull;
+    uint2 ids = left ? prog[i0] : make_uint2(0, 0);
+    for (uint32_t i = i0; i < i1;) {
+      const uint2 cur = ids;
+      if (++i < i1) ids = prog[i];  // one entry ahead
+      const uint64_t* a = tl + (cur.x & 0xFFFFu) * kRow;
+      const uint64_t* b = tl + (cur.x >> 16) * kRow;
+      const uint64_t* c = tl + (cur.y & 0xFFFFu) * kRow;
+      const uint64_t* d = tl + ((cur.y >> 16) & 0x7FFFu) * kRow;
+      uint64_t some = 0;
+#pragma unroll
+      for (int h = 0; h < H; ++h)
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          const int o = (h * AW + w) * 32;
+          m[h][w] &= (a[o] & b[o]) & (c[o] & d[o]);
+          some |= m[h][w];
+        }
+      if (!__any_sync(0xFFFFFFFFu, some != 0)) {  // no graph has a candidate: the query is out
+        left = false;
+        break;
+      }
+      if (cur.y & 0x80000000u) {  // the class's end: the next one starts with the graphs that are left
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+          uint64_t x = 0;
+#pragma unroll
+          for (int w = 0; w < W; ++w) x |= m[h][w];
+#pragma unroll
+          for (int w = 0; w < W; ++w) m[h][w] = x ? ~0ull : 0ull;
+        }
+      }
+    }
+    if (qg + nw < QG) i0 = q_off[qg + nw];
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const uint32_t alive = __ballot_sync(0xFFFFFFFFu, left && m[h][0] != 0);
+      if (lane == 0 && tile0 + h < GW) admit[static_cast<uint64_t>(qg) * GW + tile0 + h] = alive;
+      my_cnt[h] += (alive >> lane) & 1u;
+    }
+  }
+}
+
+template <int AW, bool GATHER, int H>
+__global__ void __launch_bounds__(kAdmitWarps * 32, AW == 1 ? (H == 1 ? 4 : 3) : 2) k_planes_admit(
     uint32_t G, const uint32_t* __restrict__ goff, const uint8_t* __restrict__ lab, const uint64_t* __restrict__ sig_all,
     uint64_t N, uint32_t R, uint32_t K, uint32_t nlab, const uint32_t* __restrict__ spec, const uint32_t* __restrict__ r_begin,
     int prof, uint32_t base, const uint64_t* __restrict__ rplanes, uint32_t rrows, const uint32_t* __restrict__ row_map,
-    uint32_t QG,
-    const uint16_t* __restrict__ g_prog, const uint32_t* __restrict__ g_qc_off,
-    const uint2* __restrict__ g_qc, uint32_t n_qc, uint32_t n_prog, int stage_lists,
-    const uint32_t* __restrict__ row_of, uint32_t out_rows, int accumulate, uint64_t* __restrict__ planes,
-    uint32_t* __restrict__ admit, uint32_t* __restrict__ counts) {
+    uint32_t QG, const uint2* __restrict__ g_prog, const uint32_t* __restrict__ g_q_off, uint32_t n_quads, int stage_lists, const uint32_t* __restrict__ row_of, uint32_t out_rows, int accumulate,
+    uint64_t* __restrict__ planes, uint32_t* __restrict__ admit, uint32_t* __restrict__ counts) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ uint32_t tile_cnt[32];
-  constexpr uint32_t kRow = AW * 32u;
+  __shared__ uint32_t tile_cnt[32 * H];
+  constexpr uint32_t kRow = H * AW * 32u;
   const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const uint32_t GW = (G + 31u) / 32u;
-  const uint32_t words = K * AW;
-  const size_t list_bytes = stage_lists ? 8ull * n_qc + 4ull * (QG + 1) + 2ull * n_prog : 0;
-  const AdmitSmem L = admit_smem_layout(K, AW, GATHER, list_bytes);
-  uint64_t* tiles = reinterpret_cast<uint64_t*>(smem_raw);
-  uint32_t* s_map = reinterpret_cast<uint32_t*>(smem_raw + L.map);
-  // per-batch constants: the row map and (when they fit) the class lists
-  const uint32_t* qc_off = g_qc_off;
-  const uint2* qc = g_qc;
-  const uint16_t* prog = g_prog;
-  if (GATHER)
-    for (uint32_t i = threadIdx.x; i < K; i += blockDim.x) s_map[i] = row_map[i];
+  const uint32_t GW = (G + 31u) / 32u, tiles = (GW + H - 1u) / H;
+  const size_t list_bytes = stage_lists ? 8ull * n_quads + 4ull * (QG + 1) : 0;
+  const AdmitSmem L = admit_smem_layout(K, AW, H, GATHER, list_bytes);
+  uint64_t* tile = reinterpret_cast<uint64_t*>(smem_raw);
+  uint32_t* s_map = reinterpret_cast<uint32_t*>(smem_raw + L.specs);
+  uint2* s_test = reinterpret_cast<uint2*>(smem_raw + L.specs);
+  // per-batch constants: the row map or the planes' tests, and (when they fit) the programs
+  const uint32_t* q_off = g_q_off;
+  const uint2* prog = g_prog;
+  for (uint32_t i = threadIdx.x; i < K; i += blockDim.x) {
+    if (GATHER) s_map[i] = row_map[i];
+    else s_test[i] = plane_test(spec[i]);
+  }
   if (stage_lists) {
-    uint2* p2 = reinterpret_cast<uint2*>(smem_raw + L.lists);
-    for (uint32_t i = threadIdx.x; i < n_qc; i += blockDim.x) p2[i] = g_qc[i];
-    uint32_t* p = reinterpret_cast<uint32_t*>(p2 + n_qc);
-    for (uint32_t i = threadIdx.x; i <= QG; i += blockDim.x) p[i] = g_qc_off[i];
-    uint16_t* p16 = reinterpret_cast<uint16_t*>(p + QG + 1);
-    for (uint32_t i = threadIdx.x; i < n_prog; i += blockDim.x) p16[i] = g_prog[i];
-    qc = p2;
-    qc_off = p;
-    prog = p16;
+    uint2* pp = reinterpret_cast<uint2*>(smem_raw + L.lists);
+    for (uint32_t i = threadIdx.x; i < n_quads; i += blockDim.x) pp[i] = g_prog[i];
+    uint32_t* p = reinterpret_cast<uint32_t*>(pp + n_quads);
+    for (uint32_t i = threadIdx.x; i <= QG; i += blockDim.x) p[i] = g_q_off[i];
+    prog = pp;
+    q_off = p;
   }
   __syncthreads();
-  for (uint32_t gw = blockIdx.x; gw < GW; gw += gridDim.x) {
-    uint64_t* tile = tiles;
+  for (uint32_t gw = blockIdx.x; gw < tiles; gw += gridDim.x) {
+    __syncthreads();  // the previous tile is no longer read
+    // every graph of the tile has at most 64 vertices (uniform: all threads vote)
+    bool narrow = AW == 1;
+    if (AW > 1) {
+      bool wide = false;
+      for (uint32_t i = threadIdx.x; i < 32u * H; i += blockDim.x) {
+        const uint32_t g = gw * (32u * H) + i;
+        if (g < G) wide |= goff[g + 1] - goff[g] > 64u;
+      }
+      narrow = !__syncthreads_or(wide);
+    }
     if (GATHER) {
-      // one tile buffer (not two, double-buffered): at 35 KB instead of 70 KB
-      // per CTA more CTAs share an SM and hide each other's gathers
-      __syncthreads();  // every warp is done with the previous tile
-      gather_tile_async<AW>(tile, rplanes, rrows, gw, K, s_map);
+      // one tile buffer (not two, double-buffered): more CTAs share an SM and
+      // hide each other's gathers
+      gather_tile_async<AW, H>(tile, rplanes, rrows, gw, GW, K, s_map);
       cp_async_wait_all();  // this thread's copies; the barrier below covers the others'
     } else {
-      __syncthreads();  // the previous tile is no longer read
-      fill_tile<AW, false>(tile, gw, G, goff, lab, sig_all, N, R, K, nlab, spec, r_begin, prof, base, nullptr, 0, nullptr);
-    }
-    if (threadIdx.x < 32) tile_cnt[threadIdx.x] = 0;
-    __syncthreads();
-    if (!GATHER) {
-      if (!row_of) {  // the batch's planes: this tile's rows, contiguous
-        uint4* dst = reinterpret_cast<uint4*>(planes + static_cast<uint64_t>(gw) * words * 32);
-        const uint4* src = reinterpret_cast<const uint4*>(tile);
-        for (uint32_t i = threadIdx.x; i < words * 16; i += blockDim.x) dst[i] = src[i];
-      } else {  // one group of the batch: local row k goes to row row_of[k] of out_rows
-        constexpr uint32_t kChunks = AW * 16u;  // 16-byte chunks per row
-        uint64_t* dst = planes + static_cast<uint64_t>(gw) * out_rows * kRow;
-        for (uint32_t i = threadIdx.x; i < K * kChunks; i += blockDim.x) {
-          const uint32_t k = i / kChunks, c = i % kChunks;
-          reinterpret_cast<uint4*>(dst + static_cast<uint64_t>(row_of[k]) * kRow)[c] =
-              reinterpret_cast<const uint4*>(tile + k * kRow)[c];
+      for (uint32_t gl = wid; gl < 32u * H; gl += nw) {
+        const uint32_t g = gw * (32u * H) + gl;
+        uint64_t* col = tile + (gl >> 5) * (AW * 32u) + (gl & 31u);
+        if (g < G) {
+          build_graph_planes<AW>(col, kRow, goff[g], goff[g + 1], lane, lab, sig_all, N, K, nlab, s_test, prof, base,
+                                 planes + static_cast<uint64_t>(g) * out_rows * AW, row_of);
+        } else {
+          for (uint32_t i = lane; i < K * AW; i += 32) col[(i / AW) * kRow + (i % AW) * 32] = 0;
         }
       }
     }
-    const uint64_t* tl = tile + lane;
-    const uint32_t in_tile = G - gw * 32u;
-    const uint32_t valid_lanes = in_tile >= 32u ? 0xFFFFFFFFu : ((1u << in_tile) - 1u);
-    uint32_t my_cnt = 0;
-    for (uint32_t qg = wid; qg < QG; qg += nw) {
-      const uint32_t e0 = qc_off[qg], e1 = qc_off[qg + 1];
-      uint32_t alive = e1 > e0 ? valid_lanes : 0u;  // an empty list: a query of at most one vertex
-      for (uint32_t e = e0; e < e1 && alive; ++e) {
-        const uint2 pr = qc[e];  // the class's program: prog[pr.x, pr.y)
-        uint64_t m[AW];
-#pragma unroll
-        for (int w = 0; w < AW; ++w) m[w] = ~0ull;
-        bool any = true;
-        const uint32_t k1 = pr.y;
-        // four planes per step between the warp votes
-        uint32_t k = pr.x;
-        bool live = true;
-        for (; k + 4 <= k1; k += 4) {
-          const uint32_t off0 = static_cast<uint32_t>(prog[k]) * kRow, off1 = static_cast<uint32_t>(prog[k + 1]) * kRow;
-          const uint32_t off2 = static_cast<uint32_t>(prog[k + 2]) * kRow, off3 = static_cast<uint32_t>(prog[k + 3]) * kRow;
-          any = false;
-#pragma unroll
-          for (int w = 0; w < AW; ++w) {
-            m[w] &= (tl[off0 + 32 * w] & tl[off1 + 32 * w]) & (tl[off2 + 32 * w] & tl[off3 + 32 * w]);
-            any |= m[w] != 0;
-          }
-          if (!__any_sync(0xFFFFFFFFu, any)) {
-            live = false;
-            break;
-          }
-        }
-        if (live && k < k1) {
-          any = false;
-          for (; k < k1; ++k) {
-            const uint32_t off = static_cast<uint32_t>(prog[k]) * kRow;
-#pragma unroll
-            for (int w = 0; w < AW; ++w) m[w] &= tl[off + 32 * w];
-          }
-#pragma unroll
-          for (int w = 0; w < AW; ++w) any |= m[w] != 0;
-        }
-        const uint32_t word = __ballot_sync(0xFFFFFFFFu, any);
-        alive &= word;
-      }
-      if (lane == 0) admit[static_cast<uint64_t>(qg) * GW + gw] = alive;
-      my_cnt += (alive >> lane) & 1u;
-    }
-    atomicAdd(&tile_cnt[lane], my_cnt);
+    if (threadIdx.x < 32u * H) tile_cnt[threadIdx.x] = 0;
     __syncthreads();
-    if (threadIdx.x < 32 && gw * 32u + threadIdx.x < G) {
-      if (accumulate) atomicAdd(&counts[gw * 32u + threadIdx.x], tile_cnt[threadIdx.x]);
-      else counts[gw * 32u + threadIdx.x] = tile_cnt[threadIdx.x];
+    uint32_t valid[H], my_cnt[H];
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const uint32_t g0 = (gw * H + h) * 32u, in = g0 < G ? G - g0 : 0u;
+      valid[h] = in >= 32u ? 0xFFFFFFFFu : ((1u << in) - 1u);
+      my_cnt[h] = 0;
+    }
+    if (AW > 1 && narrow) admit_tile<AW, H, 1>(tile, QG, q_off, prog, valid, gw * H, GW, admit, my_cnt);
+    else admit_tile<AW, H, AW>(tile, QG, q_off, prog, valid, gw * H, GW, admit, my_cnt);
+#pragma unroll
+    for (int h = 0; h < H; ++h) atomicAdd(&tile_cnt[32 * h + lane], my_cnt[h]);
+    __syncthreads();
+    const uint32_t g = gw * (32u * H) + threadIdx.x;
+    if (threadIdx.x < 32u * H && g < G) {
+      if (accumulate) atomicAdd(&counts[g], tile_cnt[threadIdx.x]);
+      else counts[g] = tile_cnt[threadIdx.x];
     }
   }
   if (GATHER) cp_async_wait_all();
@@ -315,11 +366,21 @@ __global__ void __launch_bounds__(kAdmitWarps * 32) k_build_planes(
     uint32_t G, const uint32_t* __restrict__ goff, const uint8_t* __restrict__ lab, const uint64_t* __restrict__ sig_all,
     uint64_t N, uint32_t R, uint32_t K, uint32_t nlab, const uint32_t* __restrict__ spec, const uint32_t* __restrict__ r_begin,
     int prof, uint32_t base, uint32_t out_rows, uint64_t* __restrict__ out) {
-  extern __shared__ uint64_t tile[];  // [K * AW][32]
+  extern __shared__ uint64_t tile[];  // [K * AW][32], then the planes' tests [K]
   const uint32_t GW = (G + 31u) / 32u;
+  uint2* tests = reinterpret_cast<uint2*>(tile + static_cast<size_t>(K) * AW * 32);
+  for (uint32_t i = threadIdx.x; i < K; i += blockDim.x) tests[i] = plane_test(spec[i]);
   for (uint32_t gw = blockIdx.x; gw < GW; gw += gridDim.x) {
     __syncthreads();
-    fill_tile<AW, false>(tile, gw, G, goff, lab, sig_all, N, R, K, nlab, spec, r_begin, prof, base, nullptr, 0, nullptr);
+    for (uint32_t gl = threadIdx.x >> 5; gl < 32; gl += blockDim.x >> 5) {
+      const uint32_t g = gw * 32u + gl, lane = threadIdx.x & 31u;
+      if (g < G) {
+        build_graph_planes<AW>(tile + gl, AW * 32u, goff[g], goff[g + 1], lane, lab, sig_all, N, K, nlab, tests, prof, base,
+                               nullptr, nullptr);
+      } else {
+        for (uint32_t i = lane; i < K * AW; i += 32) tile[i * 32 + gl] = 0;
+      }
+    }
     __syncthreads();
     uint4* dst = reinterpret_cast<uint4*>(out + static_cast<uint64_t>(gw) * out_rows * AW * 32);
     const uint4* src = reinterpret_cast<const uint4*>(tile);
@@ -384,7 +445,7 @@ int ensure_label_hist(Queue* q, Graph* g) {
 }
 
 size_t planes_admit_smem(uint32_t K, uint32_t AW) {
-  return admit_smem_layout(K, AW, false, 0).total;
+  return static_cast<size_t>(K) * AW * 32 * 8;
 }
 
 namespace {
@@ -394,44 +455,53 @@ namespace {
 struct AdmitView {
   uint32_t K, nlab, QG;
   const uint32_t *spec, *r_begin;
-  const uint32_t* qc_off;  // [QG + 1] entries of qc per query graph
-  const uint32_t* qc;      // per entry, its class's program range in prog (u32 pairs)
+  const uint32_t* q_off;   // [QG + 1] entries of prog per query graph
   const uint32_t* row_of;  // group launches: local plane row -> row of the batch's plane array
-  const uint16_t* prog;
-  size_t n_qc, n_prog;
+  const uint64_t* prog;    // four plane ids per entry
+  size_t n_quads;
   uint32_t out_rows;
   int accumulate;
 };
 
-template <int AW, bool GATHER>
-int admit_launch(Queue* q, const Graph* data, const uint64_t* sig_all, uint32_t R, const AdmitView& v, const uint64_t* rplanes,
-                 uint32_t rrows, const uint32_t* row_map, uint64_t* planes, uint32_t* admit, uint32_t* counts) {
+template <int AW, bool GATHER, int H>
+int admit_launch_h(Queue* q, const Graph* data, const uint64_t* sig_all, uint32_t R, const AdmitView& v, const uint64_t* rplanes,
+                   uint32_t rrows, const uint32_t* row_map, uint64_t* planes, uint32_t* admit, uint32_t* counts, unsigned sms) {
   const uint32_t G = data->num_graphs, GW = (G + 31u) / 32u, QG = v.QG;
-  const uint32_t n_qc = static_cast<uint32_t>(v.n_qc), n_prog = static_cast<uint32_t>(v.n_prog);
-  const size_t list_bytes = 8ull * n_qc + 4ull * (QG + 1) + 2ull * n_prog;
-  const size_t base = admit_smem_layout(v.K, AW, GATHER, 0).total;
-  // stage the class lists when the block still fits three to an SM
+  const uint32_t n_quads = static_cast<uint32_t>(v.n_quads);
+  const size_t list_bytes = 8ull * n_quads + 4ull * (QG + 1);
+  const size_t base = admit_smem_layout(v.K, AW, H, GATHER, 0).total;
+  // stage the programs when the block still fits three to an SM
   const int stage = base + list_bytes <= 72u * 1024u ? 1 : 0;
-  const size_t smem = admit_smem_layout(v.K, AW, GATHER, stage ? list_bytes : 0).total;
+  const size_t smem = admit_smem_layout(v.K, AW, H, GATHER, stage ? list_bytes : 0).total;
   if (smem > 220u * 1024u) return fail(SIGMO_ERR_DOMAIN, "k_planes_admit needs %zu bytes of shared memory", smem);
   const unsigned block = 32u * kAdmitWarps;
-  int per_sm = 0, sms = 0;
-  SIGMO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, q->device));
-  SIGMO_TRY(allow_max_dynamic_smem(reinterpret_cast<const void*>(k_planes_admit<AW, GATHER>), q->device));
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_planes_admit<AW, GATHER>, block, smem);
+  int per_sm = 0;
+  SIGMO_TRY(allow_max_dynamic_smem(reinterpret_cast<const void*>(k_planes_admit<AW, GATHER, H>), q->device));
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_planes_admit<AW, GATHER, H>, block, smem);
   if (e != cudaSuccess) return fail(SIGMO_ERR_CUDA, "k_planes_admit shared-memory setup failed: %s", cudaGetErrorString(e));
-  const uint64_t grid = std::min<uint64_t>(GW, static_cast<uint64_t>(std::max(per_sm, 1)) * sms);
-  k_planes_admit<AW, GATHER><<<grid, block, smem, q->stream>>>(
+  const uint64_t grid = std::min<uint64_t>((GW + H - 1u) / H, static_cast<uint64_t>(std::max(per_sm, 1)) * sms);
+  k_planes_admit<AW, GATHER, H><<<grid, block, smem, q->stream>>>(
       G, data->graph_offsets, data->node_labels, sig_all, data->total_nodes, R, v.K, v.nlab, v.spec, v.r_begin, q->opts.profile,
-      data->vertex_base, rplanes, rrows, row_map, QG, v.prog, v.qc_off, reinterpret_cast<const uint2*>(v.qc), n_qc,
-      n_prog, stage,
-      v.row_of, v.out_rows, v.accumulate, planes, admit, counts);
+      data->vertex_base, rplanes, rrows, row_map, QG, reinterpret_cast<const uint2*>(v.prog), v.q_off, n_quads,
+      stage, v.row_of, v.out_rows, v.accumulate, planes, admit, counts);
   return check_launch(q, "k_planes_admit");
 }
 
+template <int AW, bool GATHER>
+int admit_launch(Queue* q, const Graph* data, const uint64_t* sig_all, uint32_t R, const AdmitView& v, const uint64_t* rplanes,
+                 uint32_t rrows, const uint32_t* row_map, uint64_t* planes, uint32_t* admit, uint32_t* counts) {
+  int sms = 0;
+  SIGMO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, q->device));
+  // two graphs per lane: see k_planes_admit
+  const uint32_t GW = (data->num_graphs + 31u) / 32u;
+  if constexpr (AW == 1)
+    if (admit_smem_layout(v.K, AW, 2, GATHER, 0).total <= 110u * 1024u && GW >= 8u * static_cast<unsigned>(sms))
+      return admit_launch_h<AW, GATHER, 2>(q, data, sig_all, R, v, rplanes, rrows, row_map, planes, admit, counts, sms);
+  return admit_launch_h<AW, GATHER, 1>(q, data, sig_all, R, v, rplanes, rrows, row_map, planes, admit, counts, sms);
+}
+
 AdmitView whole_batch(const Graph* query, const PlaneProgram& pp) {
-  return AdmitView{pp.K, pp.nlab, query->num_graphs, pp.spec, pp.r_begin, pp.qc_off, pp.qc, nullptr, pp.prog, pp.h_qc_n,
-                   pp.h_prog.size(), pp.K, 0};
+  return AdmitView{pp.K, pp.nlab, query->num_graphs, pp.spec, pp.r_begin, pp.q_off, nullptr, pp.quads, pp.n_quads, pp.K, 0};
 }
 
 }  // namespace
@@ -451,8 +521,8 @@ int launch_planes_admit_group(Queue* q, const Graph* query, const Graph* data, c
                               const PlaneGroup& grp, uint32_t K_total, uint64_t* planes, uint32_t* admit, uint32_t* counts) {
   if (!data->num_graphs || grp.q1 <= grp.q0) return SIGMO_OK;
   const uint32_t GW = (data->num_graphs + 31u) / 32u;
-  const AdmitView v{grp.K,      grp.nlab, grp.q1 - grp.q0, grp.spec, grp.r_begin, grp.qc_off, grp.qc, grp.row_of, grp.prog,
-                    grp.n_qc, grp.n_prog, K_total, 1};
+  const AdmitView v{grp.K,      grp.nlab, grp.q1 - grp.q0, grp.spec, grp.r_begin, grp.q_off, grp.row_of, grp.quads, grp.n_quads,
+                    K_total, 1};
   uint32_t* adm = admit + static_cast<uint64_t>(grp.q0) * GW;
   switch (data->adj_words) {
     case 1: return admit_launch<1, false>(q, data, sig_all, R, v, nullptr, 0, nullptr, planes, adm, counts);
@@ -521,8 +591,8 @@ int build_resident_planes(Queue* q, Graph* data, const uint64_t* sig_all, uint32
     if (!data->label_hist[l] && l != kWildcard) out->label_row[l] = K;
   out->rows = K + 1;
   out->R = R;
-  const size_t smem = static_cast<size_t>(K) * AW * 32 * 8;
-  if (smem > 200u * 1024u) return fail(SIGMO_ERR_DOMAIN, "the database needs %u resident planes (too many for one tile)", K);
+  const size_t smem = static_cast<size_t>(K) * (AW * 32 * 8 + 8);
+  if (static_cast<size_t>(K) * AW * 32 * 8 > 200u * 1024u) return fail(SIGMO_ERR_DOMAIN, "the database needs %u resident planes (too many for one tile)", K);
   void* dspec = nullptr;
   void* drb = nullptr;
   SIGMO_TRY(dev_alloc(q, &dspec, 4ull * K));

@@ -114,3 +114,29 @@ def test_bond_label_join_sizes(qlo, qhi, dlo, dhi, count, prof, ff):
     total = np.zeros(1, np.uint64)
     _, per = sb.joinWildcardCandidates(queue, qg, dg, cand, gm, total, ff, per_pair=True)
     assert len(idx) > 0 and np.array_equal(per, want_per) and int(total[0]) == want_total
+
+
+@pytest.mark.parametrize("count", [37_887, 37_888, 37_921, 40_033])
+@pytest.mark.parametrize("serve", [False, True])
+def test_admission_with_two_graphs_per_lane(count, serve):
+    """From 1,184 tiles of 32 graphs on, the admission carries two graphs per
+    lane: tile counts on both sides, odd and even, ragged last tiles."""
+    d = sb.generate_molecules(count, 3, 9, seed=3301)
+    q = sb.generate_queries(10, 2, 6, seed=3302)
+    ref = oracle.run_pipeline(q, d, 2, oracle.REF_PTX, False)
+    if serve:  # resident planes, gathered
+        with sb.Server(d, iterations=2, find_first=False) as srv:
+            t = srv.submit(q)
+            srv.wait(t)
+            matched, total = srv.query_totals(t, q.num_graphs)
+        want = np.zeros(q.num_graphs, np.uint64)
+        np.add.at(want, ref["indices"].astype(np.int64), ref["per_pair"])
+        hits = np.bincount(ref["indices"][ref["per_pair"] > 0], minlength=q.num_graphs)
+        assert np.array_equal(total, want) and np.array_equal(matched, hits.astype(np.uint64))
+        return
+    queue = sb.Queue(0)
+    gm = sb.GMCR(queue)
+    res = sb.match_batched(queue, sb.createDeviceCSRGraph(queue, q), sb.createDeviceCSRGraph(queue, d), 2, False, None, gm)
+    off, idx = gm.getGMCR()
+    assert np.array_equal(off, ref["offsets"]) and np.array_equal(idx, ref["indices"])
+    assert np.array_equal(gm.getPairCounts(), ref["per_pair"]) and res["total_matches"] == ref["total"]
