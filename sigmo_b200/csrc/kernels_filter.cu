@@ -198,6 +198,7 @@ __global__ void k_sig_planes(const uint64_t* __restrict__ sig, uint64_t n, uint6
   }
 }
 
+// `rows` (<= kTabRows, a multiple of kBatch) rows per block.
 // refineCandidates: C[q][w] &= AND over q's non-zero counters (l, c) of
 // "counter l of vertex >= c", evaluated from the bit-sliced data signatures
 // (planes[l][w], see k_sig_planes).  Thread t owns the two words 2t, 2t+1 of
@@ -213,7 +214,7 @@ __device__ __forceinline__ uint2 ge_pair(const uint4* __restrict__ planes, uint6
 
 __global__ void __launch_bounds__(kTabThreads) k_refine(const uint64_t* __restrict__ qsig, uint64_t Qn,
                                                         const uint4* __restrict__ planes, uint64_t Wp,
-                                                        uint32_t* __restrict__ bits) {
+                                                        uint32_t* __restrict__ bits, uint32_t rows) {
   __shared__ uint32_t present[8];  // threshold p = 15 l + c - 1 (240 bits)
   __shared__ uint8_t slot_of[256];
   __shared__ uint8_t slot_p[kRefineSlots];
@@ -223,8 +224,8 @@ __global__ void __launch_bounds__(kTabThreads) k_refine(const uint64_t* __restri
   __shared__ uint2 T[kRefineSlots][kTabThreads];
   const unsigned tid = threadIdx.x;
   const uint64_t w0 = (static_cast<uint64_t>(blockIdx.x) * kTabThreads + tid) * 2u;
-  const uint64_t q0 = static_cast<uint64_t>(blockIdx.y) * kTabRows;
-  const uint32_t nrows = static_cast<uint32_t>(Qn - q0 < kTabRows ? Qn - q0 : kTabRows);
+  const uint64_t q0 = static_cast<uint64_t>(blockIdx.y) * rows;
+  const uint32_t nrows = static_cast<uint32_t>(Qn - q0 < rows ? Qn - q0 : rows);
   if (tid < 8) present[tid] = 0;
   __syncthreads();
   uint64_t qs = 0;
@@ -367,9 +368,14 @@ int launch_sig_planes(Queue* q, const uint64_t* sig, uint64_t n, uint64_t Wp, ui
 
 int launch_refine(Queue* q, const uint64_t* qsig, const uint32_t* planes, Candidates* c) {
   if (!c->rows || !c->W) return SIGMO_OK;
-  dim3 grid(grid_for(c->Wp, 2u * kTabThreads), static_cast<unsigned>((c->rows + kTabRows - 1) / kTabRows));
+  // rows per block: kTabRows, fewer while the blocks do not fill the chip (1,000
+  // molecules x 160 query vertices: 12 blocks of 64 rows took 21 us, 8 now)
+  uint32_t rows = kTabRows;
+  const uint64_t span = grid_for(c->Wp, 2u * kTabThreads);
+  while (rows > 8u && span * ((c->rows + rows - 1) / rows) < 2u * 148u) rows /= 2;
+  dim3 grid(static_cast<unsigned>(span), static_cast<unsigned>((c->rows + rows - 1) / rows));
   if (grid.y > 65535u) return fail(SIGMO_ERR_DOMAIN, "too many query vertices (%llu)", (unsigned long long)c->rows);
-  k_refine<<<grid, kTabThreads, 0, q->stream>>>(qsig, c->rows, reinterpret_cast<const uint4*>(planes), c->Wp, c->bits);
+  k_refine<<<grid, kTabThreads, 0, q->stream>>>(qsig, c->rows, reinterpret_cast<const uint4*>(planes), c->Wp, c->bits, rows);
   return check_launch(q, "k_refine");
 }
 
