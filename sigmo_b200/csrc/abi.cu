@@ -214,6 +214,10 @@ void queue_free(Queue* q) {
   if (q->ev_start) cudaEventDestroy(q->ev_start);
   if (q->ev_end) cudaEventDestroy(q->ev_end);
   if (q->pinned) cudaFreeHost(q->pinned);
+  if (q->stage) cudaFreeHost(q->stage);
+  if (q->ev_stage) cudaEventDestroy(q->ev_stage);
+  for (cudaEvent_t e : q->ev_match)
+    if (e) cudaEventDestroy(e);
   if (q->d_status) cudaFree(q->d_status);
   delete static_cast<sigmo_queue_t>(q);
 }
@@ -269,6 +273,8 @@ int sigmo_queue_create(int device, const sigmo_options* opts, sigmo_queue_t* out
   if (st == cudaSuccess) st = cudaEventCreate(&q->ev_start);
   if (st == cudaSuccess) st = cudaEventCreate(&q->ev_end);
   if (st == cudaSuccess) st = cudaMallocHost(&q->pinned, 4096);
+  if (st == cudaSuccess) st = cudaMallocHost(&q->stage, 1 << 18);
+  if (st == cudaSuccess) q->stage_bytes = 1 << 18;
   if (st == cudaSuccess) st = cudaMalloc(reinterpret_cast<void**>(&q->d_status), 256);
   if (st == cudaSuccess) st = cudaMemset(q->d_status, 0, 256);
   if (st == cudaSuccess) st = cudaStreamCreateWithFlags(&q->side, cudaStreamNonBlocking);
@@ -279,6 +285,8 @@ int sigmo_queue_create(int device, const sigmo_options* opts, sigmo_queue_t* out
   if (st == cudaSuccess) st = cudaEventCreateWithFlags(&q->ev_aux_join, cudaEventDisableTiming);
   for (int i = 0; i < 2 && st == cudaSuccess; ++i) st = cudaEventCreateWithFlags(&q->ev_masks[i], cudaEventDisableTiming);
   for (int i = 0; i < 2 && st == cudaSuccess; ++i) st = cudaEventCreateWithFlags(&q->ev_long[i], cudaEventDisableTiming);
+  if (st == cudaSuccess) st = cudaEventCreateWithFlags(&q->ev_stage, cudaEventDisableTiming);
+  for (int i = 0; i < 5 && st == cudaSuccess; ++i) st = cudaEventCreate(&q->ev_match[i]);
   if (st == cudaSuccess) {
     // Keep freed stream-ordered allocations cached in the device's default pool
     // (per-call scratch is then reused instead of being remapped every call).

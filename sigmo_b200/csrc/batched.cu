@@ -16,25 +16,14 @@ namespace sigmo_b200 {
 namespace {
 
 void free_groups(Queue* q, PlaneProgram* pp) {
-  for (PlaneGroup& g : pp->groups) {
-    dev_free(q, g.spec);
-    dev_free(q, g.r_begin);
-    dev_free(q, g.row_of);
-    dev_free(q, g.quads);
-    dev_free(q, g.q_off);
-  }
+  for (PlaneGroup& g : pp->groups) dev_free(q, g.blob);
   pp->groups.clear();
+  pp->groups_aw = 0;
 }
 
 void free_program(Queue* q, PlaneProgram* pp) {
   free_groups(q, pp);
-  dev_free(q, pp->spec);
-  dev_free(q, pp->prog_off);
-  dev_free(q, pp->prog);
-  dev_free(q, pp->quads);
-  dev_free(q, pp->cls);
-  dev_free(q, pp->r_begin);
-  dev_free(q, pp->q_off);
+  dev_free(q, pp->blob);
   dev_free(q, pp->qsig_all);
   *pp = PlaneProgram{};
 }
@@ -73,19 +62,71 @@ void append_quads(size_t n, F&& id, std::vector<uint64_t>* quads) {
   quads->back() |= 1ull << 63;
 }
 
-int upload(Queue* q, void** dst, const void* src, size_t bytes) {
-  SIGMO_TRY(dev_alloc(q, dst, bytes ? bytes : 4));
-  if (bytes) SIGMO_CUDA_TRY(cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, q->stream));
+// The queue's pinned staging buffer, at least `bytes` large and free to write.
+int stage_buffer(Queue* q, size_t bytes, void** p) {
+  SIGMO_CUDA_TRY(cudaEventSynchronize(q->ev_stage));  // the last copy from it is done
+  if (bytes > q->stage_bytes) {
+    if (q->stage) cudaFreeHost(q->stage);
+    q->stage = nullptr;
+    q->stage_bytes = 0;
+    const size_t want = std::max<size_t>(2 * bytes, 1 << 18);
+    SIGMO_CUDA_TRY(cudaMallocHost(&q->stage, want));
+    q->stage_bytes = want;
+  }
+  *p = q->stage;
   return SIGMO_OK;
 }
+
+// Host arrays packed into the staging buffer and copied to one device block:
+// add() them all, then send().  at(i): the device address of array i.
+struct Blob {
+  std::vector<std::pair<const void*, size_t>> parts;
+  std::vector<size_t> offs;
+  size_t bytes = 0;
+  char* dev = nullptr;
+  template <class T>
+  size_t add(const std::vector<T>& v) {
+    offs.push_back(bytes);
+    parts.emplace_back(v.data(), v.size() * sizeof(T));
+    bytes += (v.size() * sizeof(T) + 255) & ~static_cast<size_t>(255);
+    return parts.size() - 1;
+  }
+  // On q->stream; ev_stage is recorded after the copy.
+  int send(Queue* q, void** block) {
+    void* host = nullptr;
+    SIGMO_TRY(stage_buffer(q, bytes, &host));
+    for (size_t i = 0; i < parts.size(); ++i)
+      if (parts[i].second) std::memcpy(static_cast<char*>(host) + offs[i], parts[i].first, parts[i].second);
+    SIGMO_TRY(dev_alloc(q, block, bytes + 256));
+    dev = static_cast<char*>(*block);
+    SIGMO_CUDA_TRY(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, q->stream));
+    SIGMO_CUDA_TRY(cudaEventRecord(q->ev_stage, q->stream));
+    return SIGMO_OK;
+  }
+  template <class T>
+  const T* at(size_t i) const {
+    return reinterpret_cast<const T*>(dev + offs[i]);
+  }
+};
 
 }  // namespace
 
 // Builds (or reuses) the plane program of a query batch for R iterations:
 // query signatures of iterations 1..R on the device, then on the host the
 // distinct labels and (r, l, c) thresholds (the planes), the classes of
-// identical (label, signature_1..R) vertices, and each class's program
-// (label plane first, then its thresholds).
+// identical (label, signature_1..R) vertices, each class's program (label plane
+// first, then its thresholds), and per query graph its distinct classes in the
+// order the admission kernel evaluates them: rarest label first (by the query
+// batch's own vertices, whose labels are distributed like the molecules': a
+// model of 1,024 molecules x 600 queries evaluates 4.04 classes per tile and
+// query in this order, 4.09 by the molecules' histogram, which took a kernel and
+// a read-back per data graph), then longer programs first, so a query that a
+// graph cannot admit is usually rejected by its first class.
+//
+// One pass over the vertices with a hash table of classes, everything sent in
+// one copy that the device waits for by an event: the sorted, threaded form
+// with an upload and a wait per array took 0.9 ms of a call with 300 new
+// queries, this one 0.5.
 int build_plane_program(Queue* q, Graph* query, uint32_t R) {
   PlaneProgram& pp = query->pp;
   if (pp.valid && pp.R == R && pp.profile == q->opts.profile) return SIGMO_OK;
@@ -101,142 +142,164 @@ int build_plane_program(Queue* q, Graph* query, uint32_t R) {
   if (query->ready) SIGMO_CUDA_TRY(cudaStreamWaitEvent(q->side, query->ready, 0));
   q->stream = q->side;
   const uint64_t Qn = query->total_nodes;
+  const uint32_t QG = query->num_graphs;
   SIGMO_TRY(dev_alloc(q, reinterpret_cast<void**>(&pp.qsig_all), 8ull * (R ? R : 1) * (Qn ? Qn : 1)));
   SIGMO_TRY(launch_sig_all(q, query, R, pp.qsig_all));
-  std::vector<uint64_t> sig(static_cast<size_t>(R) * Qn);
+  std::vector<uint64_t> sig(static_cast<size_t>(R) * Qn);  // [vertex][R]
   std::vector<uint8_t> lab(Qn);
   if (Qn) {
-    if (R) SIGMO_CUDA_TRY(cudaMemcpyAsync(sig.data(), pp.qsig_all, 8ull * R * Qn, cudaMemcpyDeviceToHost, q->stream));
-    SIGMO_CUDA_TRY(cudaMemcpyAsync(lab.data(), query->node_labels, Qn, cudaMemcpyDeviceToHost, q->stream));
+    void* host = nullptr;
+    SIGMO_TRY(stage_buffer(q, 8ull * R * Qn + Qn, &host));
+    auto* h_sig = static_cast<uint64_t*>(host);
+    auto* h_lab = reinterpret_cast<uint8_t*>(h_sig + static_cast<size_t>(R) * Qn);
+    if (R) SIGMO_CUDA_TRY(cudaMemcpyAsync(h_sig, pp.qsig_all, 8ull * R * Qn, cudaMemcpyDeviceToHost, q->stream));
+    SIGMO_CUDA_TRY(cudaMemcpyAsync(h_lab, query->node_labels, Qn, cudaMemcpyDeviceToHost, q->stream));
+    SIGMO_CUDA_TRY(cudaStreamSynchronize(q->stream));
+    for (uint32_t r = 0; r < R; ++r)
+      for (uint64_t v = 0; v < Qn; ++v) sig[v * R + r] = h_sig[static_cast<size_t>(r) * Qn + v];
+    std::memcpy(lab.data(), h_lab, Qn);
   }
-  SIGMO_CUDA_TRY(cudaStreamSynchronize(q->stream));
 
-  // One pass over the signatures (vertex ranges in parallel): every vertex's
-  // program as raw codes (its label, then (r << 8 | l << 4 | c) for each
-  // non-zero counter in (r, l) order, rows of a fixed stride of 1 + 16 R
-  // entries), marking the labels and thresholds that occur.  Plane ids are
-  // assigned in label and (r, l, c) order, so raw codes sort like the plane
-  // ids they map to.
-  const uint32_t stride = 1 + 16 * R;
-  std::vector<uint16_t> vraw(static_cast<size_t>(Qn) * stride);
-  std::vector<uint32_t> vlen(Qn);
-  const unsigned nt = host_threads(Qn);
-  std::vector<std::vector<uint16_t>> thr_part(nt, std::vector<uint16_t>(static_cast<size_t>(R) * 16, 0));
-  std::vector<std::vector<uint8_t>> lab_part(nt, std::vector<uint8_t>(256, 0));
-  parallel_ranges(Qn, nt, [&](unsigned t, uint64_t v0, uint64_t v1) {
-    uint16_t* tm = thr_part[t].data();
-    uint8_t* lu = lab_part[t].data();
-    for (uint64_t v = v0; v < v1; ++v) {
-      uint16_t* row = vraw.data() + v * stride;
-      uint32_t n = 0;
-      lu[lab[v]] = 1;
-      row[n++] = lab[v];
-      for (uint32_t r = 0; r < R; ++r)
-        for (uint64_t sv = sig[static_cast<size_t>(r) * Qn + v]; sv;) {
-          const uint32_t l = static_cast<uint32_t>(__builtin_ctzll(sv)) >> 2, c = (sv >> (4 * l)) & 0xFu;
-          tm[r * 16 + l] |= static_cast<uint16_t>(1u << c);
-          row[n++] = static_cast<uint16_t>((r << 8) | (l << 4) | c);
-          sv &= ~(0xFull << (4 * l));
+  // classes, in order of their first vertex: an open-addressing table of first
+  // vertices, compared exactly
+  std::vector<uint32_t> cls(Qn), first;
+  std::vector<uint64_t> label_count(256, 0);
+  // a class's thresholds as raw codes r << 8 | l << 4 | c, back to back, and
+  // which codes occur
+  std::vector<uint16_t> raw(Qn * 16);
+  std::vector<uint32_t> raw_off{0};
+  std::vector<uint8_t> occurs(static_cast<size_t>(R) * 256, 0);
+  size_t raw_n = 0;
+  first.reserve(Qn);
+  raw_off.reserve(Qn + 1);
+  {
+    size_t size = 16;
+    while (size < 2 * Qn) size *= 2;
+    std::vector<uint32_t> table(size, 0);  // class + 1, 0: free
+    for (uint64_t v = 0; v < Qn; ++v) {
+      const uint64_t* sv = sig.data() + v * R;
+      ++label_count[lab[v]];
+      uint64_t h = 0x9E3779B97F4A7C15ull * (lab[v] + 1u);
+      for (uint32_t r = 0; r < R; ++r) {
+        h ^= sv[r];
+        h *= 0xFF51AFD7ED558CCDull;
+        h ^= h >> 32;
+      }
+      size_t at = h & (size - 1);
+      for (;; at = (at + 1) & (size - 1)) {
+        const uint32_t c = table[at];
+        if (!c) {
+          table[at] = static_cast<uint32_t>(first.size() + 1);
+          cls[v] = static_cast<uint32_t>(first.size());
+          first.push_back(static_cast<uint32_t>(v));
+          if (raw.size() < raw_n + 16ull * R) raw.resize(2 * raw.size() + 16ull * R);
+          for (uint32_t r = 0; r < R; ++r)
+            for (uint64_t x = sv[r]; x;) {
+              const uint32_t l = static_cast<uint32_t>(__builtin_ctzll(x)) >> 2;
+              const uint32_t code = (r << 8) | (l << 4) | static_cast<uint32_t>((x >> (4 * l)) & 0xFu);
+              raw[raw_n++] = static_cast<uint16_t>(code);
+              occurs[code] = 1;
+              x &= ~(0xFull << (4 * l));
+            }
+          raw_off.push_back(static_cast<uint32_t>(raw_n));
+          break;
         }
-      vlen[v] = n;
+        const uint64_t f = first[c - 1];
+        if (lab[f] == lab[v] && std::equal(sv, sv + R, sig.data() + f * R)) {
+          cls[v] = c - 1;
+          break;
+        }
+      }
     }
-  });
-  std::vector<uint8_t> label_used(256, 0);
-  std::vector<uint16_t> thr_mask(static_cast<size_t>(R) * 16, 0);  // [r][l]: bit c = count c occurs
-  for (unsigned t = 0; t < nt; ++t) {
-    for (size_t i = 0; i < thr_mask.size(); ++i) thr_mask[i] |= thr_part[t][i];
-    for (size_t i = 0; i < 256; ++i) label_used[i] |= lab_part[t][i];
   }
+  const uint32_t C = static_cast<uint32_t>(first.size());
   // planes: label values used by queries (ascending), then the thresholds
   // (r, l, c) that occur, in (r, l, c) order
   std::vector<uint32_t> spec;
   std::vector<uint32_t> label_idx(256, 0), thr_idx(static_cast<size_t>(R) * 256, 0);
   for (uint32_t l = 0; l < 256; ++l)
-    if (label_used[l]) {
+    if (label_count[l]) {
       label_idx[l] = static_cast<uint32_t>(spec.size());
       spec.push_back(0x80000000u | l);
     }
   const uint32_t nlab = static_cast<uint32_t>(spec.size());
-  for (uint32_t r = 0; r < R; ++r)
-    for (uint32_t l = 0; l < 16; ++l)
-      for (uint32_t c = 1; c < 16; ++c)
-        if ((thr_mask[r * 16 + l] >> c) & 1u) {
-          thr_idx[(r << 8) | (l << 4) | c] = static_cast<uint32_t>(spec.size());
-          spec.push_back((r << 16) | (l << 8) | c);
-        }
+  for (uint32_t code = 0; code < R * 256u; ++code)
+    if (occurs[code]) {
+      thr_idx[code] = static_cast<uint32_t>(spec.size());
+      spec.push_back(((code >> 8) << 16) | (((code >> 4) & 0xFu) << 8) | (code & 0xFu));
+    }
   if (spec.size() >= 65535) return fail(SIGMO_ERR_DOMAIN, "query batch needs %zu candidate planes (limit 65535)", spec.size());
-
-  // classes: distinct (label, sig_1..sig_R), numbered in lexicographic program
-  // order: the vertices sorted by (the first four raw codes packed high to low,
-  // a shorter program's missing codes 0 so it sorts first; ties: the full
-  // comparison), in parallel ranges merged pairwise
-  struct Key {
-    uint64_t k;
-    uint32_t v;
+  // the classes' programs, and their place in the evaluation order
+  std::vector<uint32_t> prog_off(C + 1, 0);
+  std::vector<uint16_t> prog(raw_n + C);
+  std::vector<uint64_t> rank(C);  // vertices with the label, then longer programs first
+  size_t n_prog = 0;
+  for (uint32_t c = 0; c < C; ++c) {
+    const uint8_t l = lab[first[c]];
+    prog[n_prog++] = static_cast<uint16_t>(label_idx[l]);
+    for (uint32_t i = raw_off[c]; i < raw_off[c + 1]; ++i) prog[n_prog++] = static_cast<uint16_t>(thr_idx[raw[i]]);
+    prog_off[c + 1] = static_cast<uint32_t>(n_prog);
+    rank[c] = ((l == kWildcard ? Qn : label_count[l]) << 16) | (0xFFFFu - (prog_off[c + 1] - prog_off[c]));
+  }
+  // query graphs in parallel ranges, each range's lists on their own, then
+  // concatenated in query order
+  const std::vector<uint32_t>& qgoff = query->host_graph_offsets;
+  const unsigned nt = host_threads(Qn / 8);
+  struct Part {
+    std::vector<uint32_t> order, order_n, quads_n;
+    std::vector<uint64_t> quads;
   };
-  std::vector<Key> keys(Qn);
-  auto row_of = [&](uint32_t v) { return vraw.data() + static_cast<size_t>(v) * stride; };
-  auto key_less = [&](const Key& x, const Key& y) {
-    if (x.k != y.k) return x.k < y.k;
-    return std::lexicographical_compare(row_of(x.v), row_of(x.v) + vlen[x.v], row_of(y.v), row_of(y.v) + vlen[y.v]);
-  };
-  std::vector<uint64_t> cut(nt + 1);
-  for (unsigned t = 0; t <= nt; ++t) cut[t] = Qn * t / nt;
-  parallel_ranges(Qn, nt, [&](unsigned, uint64_t v0, uint64_t v1) {
-    for (uint64_t v = v0; v < v1; ++v) {
-      const uint16_t* row = row_of(static_cast<uint32_t>(v));
-      uint64_t k = 0;
-      for (uint32_t i = 0; i < 4; ++i) k = (k << 16) | (i < vlen[v] ? row[i] : 0u);
-      keys[v] = Key{k, static_cast<uint32_t>(v)};
-    }
-    std::sort(keys.begin() + v0, keys.begin() + v1, key_less);
-  });
-  for (unsigned w = 1; w < nt; w *= 2)  // pairwise merges of the sorted ranges
-    parallel_ranges(nt, (nt + 2 * w - 1) / (2 * w), [&](unsigned, uint64_t g0, uint64_t g1) {
-      for (uint64_t g = g0; g < g1; ++g) {
-        const uint64_t a = 2 * w * g, m = std::min<uint64_t>(a + w, nt), b = std::min<uint64_t>(a + 2 * w, nt);
-        if (m < b) std::inplace_merge(keys.begin() + cut[a], keys.begin() + cut[m], keys.begin() + cut[b], key_less);
+  std::vector<Part> parts(nt);
+  const bool with_quads = spec.size() < 32768u;
+  parallel_ranges(QG, nt, [&](unsigned t, uint64_t q0, uint64_t q1) {
+    Part& p = parts[t];
+    std::vector<std::pair<uint64_t, uint32_t>> list;
+    for (uint64_t qg = q0; qg < q1; ++qg) {
+      list.clear();
+      // queries of one vertex are never admitted (gmcr.hpp:100): an empty list
+      // tells the kernel so
+      if (qgoff[qg + 1] - qgoff[qg] > 1)
+        for (uint32_t v = qgoff[qg]; v < qgoff[qg + 1]; ++v) list.emplace_back(rank[cls[v]], cls[v]);
+      std::sort(list.begin(), list.end());
+      list.erase(std::unique(list.begin(), list.end()), list.end());
+      const size_t before = p.quads.size();
+      for (const auto& x : list) {
+        p.order.push_back(x.second);
+        const uint32_t b = prog_off[x.second];
+        if (with_quads) append_quads(prog_off[x.second + 1] - b, [&](size_t i) { return prog[b + i]; }, &p.quads);
       }
-    }, 1);
-  std::vector<uint32_t> cls(Qn), prog_off{0};
-  std::vector<uint16_t> prog;
-  prog.reserve(static_cast<size_t>(Qn) * 8);
-  uint32_t max_len = 0;
-  for (uint64_t i = 0; i < Qn; ++i) {
-    const uint32_t v = keys[i].v;
-    if (i == 0 || keys[i - 1].k != keys[i].k || vlen[keys[i - 1].v] != vlen[v] ||
-        !std::equal(row_of(v), row_of(v) + vlen[v], row_of(keys[i - 1].v))) {
-      const uint16_t* row = row_of(v);
-      prog.push_back(static_cast<uint16_t>(label_idx[row[0]]));
-      for (uint32_t j = 1; j < vlen[v]; ++j) prog.push_back(static_cast<uint16_t>(thr_idx[row[j]]));
-      prog_off.push_back(static_cast<uint32_t>(prog.size()));
-      max_len = std::max<uint32_t>(max_len, vlen[v]);
+      p.order_n.push_back(static_cast<uint32_t>(list.size()));
+      p.quads_n.push_back(static_cast<uint32_t>(p.quads.size() - before));
     }
-    cls[v] = static_cast<uint32_t>(prog_off.size() - 2);
+  });
+  std::vector<uint32_t> q_off{0};
+  std::vector<uint64_t> quads;
+  pp.order.clear();
+  pp.order_off.assign(1, 0);
+  for (const Part& p : parts) {
+    pp.order.insert(pp.order.end(), p.order.begin(), p.order.end());
+    quads.insert(quads.end(), p.quads.begin(), p.quads.end());
+    for (uint32_t n : p.order_n) pp.order_off.push_back(pp.order_off.back() + n);
+    for (uint32_t n : p.quads_n) q_off.push_back(q_off.back() + n);
   }
-  const uint32_t C = static_cast<uint32_t>(prog_off.size() - 1);
-  std::vector<uint32_t> r_begin(R + 1, static_cast<uint32_t>(spec.size()));
-  for (uint32_t k = nlab; k < spec.size(); ++k) {
-    const uint32_t r = (spec[k] >> 16) & 0xFFu;
-    r_begin[r] = std::min(r_begin[r], k);
-  }
-  for (int r = static_cast<int>(R) - 1; r >= 0; --r) r_begin[r] = std::min(r_begin[r], r_begin[r + 1]);
+  Blob blob;
+  const size_t i_spec = blob.add(spec), i_off = blob.add(prog_off), i_prog = blob.add(prog), i_cls = blob.add(cls),
+               i_qoff = blob.add(q_off), i_quads = blob.add(quads);
+  SIGMO_TRY(blob.send(q, &pp.blob));
+  SIGMO_CUDA_TRY(cudaStreamWaitEvent(on_side.main, q->ev_stage, 0));
+  pp.spec = blob.at<uint32_t>(i_spec);
+  pp.prog_off = blob.at<uint32_t>(i_off);
+  pp.prog = blob.at<uint16_t>(i_prog);
+  pp.cls = blob.at<uint32_t>(i_cls);
+  pp.q_off = blob.at<uint32_t>(i_qoff);
+  pp.quads = blob.at<uint64_t>(i_quads);
+  pp.n_quads = quads.size();
   pp.K = static_cast<uint32_t>(spec.size());
   pp.C = C;
   pp.nlab = nlab;
-  SIGMO_TRY(upload(q, reinterpret_cast<void**>(&pp.spec), spec.data(), 4 * spec.size()));
-  SIGMO_TRY(upload(q, reinterpret_cast<void**>(&pp.prog_off), prog_off.data(), 4 * prog_off.size()));
-  SIGMO_TRY(upload(q, reinterpret_cast<void**>(&pp.prog), prog.data(), 2 * prog.size()));
-  SIGMO_TRY(upload(q, reinterpret_cast<void**>(&pp.cls), cls.data(), 4 * cls.size()));
-  SIGMO_TRY(upload(q, reinterpret_cast<void**>(&pp.r_begin), r_begin.data(), 4 * r_begin.size()));
-  pp.h_spec = spec;
-  pp.h_prog = prog;
-  pp.h_prog_off = prog_off;
-  pp.h_cls = cls;
-  pp.h_qgoff = query->host_graph_offsets;
-  pp.qc_for = nullptr;
-  pp.max_len = max_len;
-  SIGMO_CUDA_TRY(cudaStreamSynchronize(q->stream));  // host vectors go out of scope
+  pp.h_spec = std::move(spec);
+  pp.h_prog = std::move(prog);
+  pp.h_prog_off = std::move(prog_off);
   pp.R = R;
   pp.profile = q->opts.profile;
   pp.valid = true;
@@ -245,11 +308,18 @@ int build_plane_program(Queue* q, Graph* query, uint32_t R) {
 
 // Splits the query graphs into contiguous groups whose planes and classes fit
 // one admission tile (kGroupSmemBudget), greedily in query order, and uploads
-// each group's program in local plane / class ids.  off/list: every query
-// graph's classes in evaluation order (global class ids).
-int plan_groups(Queue* q, Graph* query, uint32_t AW, const std::vector<uint32_t>& off, const std::vector<uint32_t>& list) {
+// each group's program in local plane ids.  Planned once per set width AW;
+// SIGMO_ERR_DOMAIN when a query graph alone does not fit a tile.
+int plan_groups(Queue* q, Graph* query, uint32_t AW) {
   PlaneProgram& pp = query->pp;
-  const uint32_t QG = query->num_graphs, K = pp.K, C = pp.C, R = pp.R;
+  if (pp.groups_aw == AW) return SIGMO_OK;
+  free_groups(q, &pp);
+  if (planes_admit_smem(pp.K, AW) <= kGroupSmemBudget) {
+    pp.groups_aw = AW;
+    return SIGMO_OK;
+  }
+  const std::vector<uint32_t>&off = pp.order_off, &list = pp.order;
+  const uint32_t QG = query->num_graphs, K = pp.K, C = pp.C;
   std::vector<uint32_t> plane_mark(K, 0), class_mark(C, 0);  // stamp = group number + 1
   uint32_t stamp = 0, Kg = 0, q0 = 0;
   std::vector<std::pair<uint32_t, uint32_t>> ranges;
@@ -307,7 +377,7 @@ int plan_groups(Queue* q, Graph* query, uint32_t AW, const std::vector<uint32_t>
     for (uint32_t qg = grp.q0; qg < grp.q1; ++qg)
       for (uint32_t e = off[qg]; e < off[qg + 1]; ++e)
         for (uint32_t i = pp.h_prog_off[list[e]]; i < pp.h_prog_off[list[e] + 1]; ++i) in_group[pp.h_prog[i]] = 1;
-    std::vector<uint32_t> loc_plane(K, 0xFFFFFFFFu), spec, row_of, r_begin(R + 1, 0xFFFFFFFFu);
+    std::vector<uint32_t> loc_plane(K, 0xFFFFFFFFu), spec, row_of;
     for (uint32_t k = 0; k < K; ++k)
       if (in_group[k]) {
         loc_plane[k] = static_cast<uint32_t>(spec.size());
@@ -315,16 +385,7 @@ int plan_groups(Queue* q, Graph* query, uint32_t AW, const std::vector<uint32_t>
         row_of.push_back(k);
       }
     uint32_t nlab = 0;
-    for (uint32_t i = 0; i < spec.size(); ++i) {
-      if (spec[i] & 0x80000000u) {
-        ++nlab;
-      } else {
-        const uint32_t r = (spec[i] >> 16) & 0xFFu;
-        r_begin[r] = std::min(r_begin[r], i);
-      }
-    }
-    r_begin[R] = static_cast<uint32_t>(spec.size());
-    for (int r = static_cast<int>(R) - 1; r >= 0; --r) r_begin[r] = std::min(r_begin[r], r_begin[r + 1]);
+    for (uint32_t x : spec) nlab += (x & 0x80000000u) != 0;
     // the queries' programs in local ids
     std::vector<uint32_t> q_off{0};
     std::vector<uint64_t> quads;
@@ -345,79 +406,16 @@ int plan_groups(Queue* q, Graph* query, uint32_t AW, const std::vector<uint32_t>
       return fail(SIGMO_ERR_DOMAIN, "group %zu needs more than one admission tile of shared memory", gi);
     grp.nlab = nlab;
     grp.n_quads = quads.size();
-    SIGMO_TRY(upload(q, reinterpret_cast<void**>(&grp.spec), spec.data(), 4 * spec.size()));
-    SIGMO_TRY(upload(q, reinterpret_cast<void**>(&grp.r_begin), r_begin.data(), 4 * r_begin.size()));
-    SIGMO_TRY(upload(q, reinterpret_cast<void**>(&grp.row_of), row_of.data(), 4 * row_of.size()));
-    SIGMO_TRY(upload(q, reinterpret_cast<void**>(&grp.quads), quads.data(), 8 * quads.size()));
-    SIGMO_TRY(upload(q, reinterpret_cast<void**>(&grp.q_off), q_off.data(), 4 * q_off.size()));
-    SIGMO_CUDA_TRY(cudaStreamSynchronize(q->stream));  // host vectors go out of scope
+    Blob blob;
+    const size_t i_spec = blob.add(spec), i_row = blob.add(row_of), i_quads = blob.add(quads), i_off = blob.add(q_off);
+    SIGMO_TRY(blob.send(q, &grp.blob));
+    grp.spec = blob.at<uint32_t>(i_spec);
+    grp.row_of = blob.at<uint32_t>(i_row);
+    grp.quads = blob.at<uint64_t>(i_quads);
+    grp.q_off = blob.at<uint32_t>(i_off);
     pp.groups.push_back(grp);
   }
-  return SIGMO_OK;
-}
-
-// Per query graph, its distinct classes in the order the admission kernel
-// evaluates them for `data`: rarest label first (the data graphs' vertex
-// counts per label), then longer programs (more thresholds) first, so a
-// query that a graph cannot admit is usually rejected by its first class.
-int order_classes(Queue* q, Graph* query, Graph* data) {
-  PlaneProgram& pp = query->pp;
-  if (pp.q_off && pp.qc_for == data && pp.qc_stamp == data->stamp) return SIGMO_OK;
-  SIGMO_TRY(ensure_label_hist(q, data));
-  const uint32_t QG = query->num_graphs;
-  uint64_t all = 0;
-  for (uint64_t x : data->label_hist) all += x;
-  // query graphs in parallel ranges, each query's list on its own, then
-  // concatenated in query order
-  std::vector<std::vector<uint32_t>> per(QG);
-  auto key = [&](uint32_t c) {
-    const uint32_t lab = pp.h_spec[pp.h_prog[pp.h_prog_off[c]]] & 0xFFu;
-    const uint64_t freq = lab == kWildcard ? all : data->label_hist[lab];
-    return std::make_tuple(freq, 0u - (pp.h_prog_off[c + 1] - pp.h_prog_off[c]), c);
-  };
-  parallel_ranges(QG, host_threads(query->total_nodes), [&](unsigned, uint64_t q0, uint64_t q1) {
-    for (uint64_t qg = q0; qg < q1; ++qg) {
-      std::vector<uint32_t>& tmp = per[qg];
-      // queries of one vertex are never admitted (gmcr.hpp:100): an empty list
-      // tells the kernel so
-      if (pp.h_qgoff[qg + 1] - pp.h_qgoff[qg] <= 1) continue;
-      tmp.assign(pp.h_cls.begin() + pp.h_qgoff[qg], pp.h_cls.begin() + pp.h_qgoff[qg + 1]);
-      std::sort(tmp.begin(), tmp.end());
-      tmp.erase(std::unique(tmp.begin(), tmp.end()), tmp.end());
-      std::sort(tmp.begin(), tmp.end(), [&](uint32_t a, uint32_t b) { return key(a) < key(b); });
-    }
-  });
-  std::vector<uint32_t> off{0}, list;
-  for (uint32_t qg = 0; qg < QG; ++qg) {
-    list.insert(list.end(), per[qg].begin(), per[qg].end());
-    off.push_back(static_cast<uint32_t>(list.size()));
-  }
-  dev_free(q, pp.q_off);
-  dev_free(q, pp.quads);
-  pp.q_off = nullptr;
-  pp.quads = nullptr;
-  free_groups(q, &pp);
-  const uint32_t AW = data->adj_words;
-  // the queries' programs as the kernel reads them: the batch's, and per group
-  // when the batch's planes do not fit one tile
-  std::vector<uint32_t> q_off(QG + 1, 0);
-  std::vector<uint64_t> quads;
-  const bool one_tile = planes_admit_smem(pp.K, AW) <= kGroupSmemBudget;
-  if (pp.K < 32768u)
-    for (uint32_t qg = 0; qg < QG; ++qg) {
-      for (uint32_t e = off[qg]; e < off[qg + 1]; ++e) {
-        const uint32_t b = pp.h_prog_off[list[e]];
-        append_quads(pp.h_prog_off[list[e] + 1] - b, [&](size_t i) { return pp.h_prog[b + i]; }, &quads);
-      }
-      q_off[qg + 1] = static_cast<uint32_t>(quads.size());
-    }
-  pp.n_quads = quads.size();
-  SIGMO_TRY(upload(q, reinterpret_cast<void**>(&pp.q_off), q_off.data(), 4 * q_off.size()));
-  SIGMO_TRY(upload(q, reinterpret_cast<void**>(&pp.quads), quads.data(), 8 * quads.size()));
-  if (!one_tile) SIGMO_TRY(plan_groups(q, query, AW, off, list));
-  SIGMO_CUDA_TRY(cudaStreamSynchronize(q->stream));  // host vectors go out of scope
-  pp.qc_for = data;
-  pp.qc_stamp = data->stamp;
+  pp.groups_aw = AW;
   return SIGMO_OK;
 }
 
@@ -431,19 +429,11 @@ using namespace sigmo_b200;
 
 namespace {
 
-struct Events {
-  cudaEvent_t e[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-  ~Events() {
-    for (auto& x : e)
-      if (x) cudaEventDestroy(x);
-  }
-};
-
 // The bitset route: fused filter writes the final bitset (all words), GMCR
 // and the join read it.  Used when the caller asks for the bitset, or when a
 // batch does not fit the plane route.
 int batched_bitset(Queue* q, Graph* query, Graph* data, uint32_t R, int find_first, Candidates* c, Gmcr* m,
-                   uint64_t* d_total, Events& ev, const BatchedRun& run) {
+                   uint64_t* d_total, const BatchedRun& run) {
   PlaneProgram& pp = query->pp;
   const uint64_t N = data->total_nodes;
   void* buf = nullptr;
@@ -455,11 +445,11 @@ int batched_bitset(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
   int rc = run.dsig ? SIGMO_OK : launch_sig_all(q, data, R, dsig);
   for (uint32_t r = 0; r < R && !rc; ++r)
     rc = launch_sig_planes(q, dsig + static_cast<uint64_t>(r) * N, N, c->Wp, planes + static_cast<uint64_t>(r) * 16 * 4 * c->Wp);
-  if (!rc && cudaEventRecord(ev.e[1], q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
+  if (!rc && cudaEventRecord(q->ev_match[1], q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
   if (!rc) rc = launch_fused_filter(q, query, data, R, pp.qsig_all, planes, c);
-  if (!rc && cudaEventRecord(ev.e[2], q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
+  if (!rc && cudaEventRecord(q->ev_match[2], q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
   if (!rc) rc = launch_gmcr(q, query, data, c, m, true, 0);
-  if (!rc && cudaEventRecord(ev.e[3], q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
+  if (!rc && cudaEventRecord(q->ev_match[3], q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
   const bool exact = q->opts.profile == kProfileExact;
   MaskSource src;
   src.bits = c->bits;
@@ -473,12 +463,12 @@ int batched_bitset(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
 }
 
 // The plane route (no full bitset in HBM).
-int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_first, Gmcr* m, uint64_t* d_total, Events& ev,
+int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_first, Gmcr* m, uint64_t* d_total,
                    const BatchedRun& run) {
   // stage events are not recorded while the work is captured into a graph
   auto mark = [&](int i) -> int {
     if (run.capture) return SIGMO_OK;
-    return cudaEventRecord(ev.e[i], q->stream) == cudaSuccess ? SIGMO_OK : fail(SIGMO_ERR_CUDA, "event record failed");
+    return cudaEventRecord(q->ev_match[i], q->stream) == cudaSuccess ? SIGMO_OK : fail(SIGMO_ERR_CUDA, "event record failed");
   };
   PlaneProgram& pp = query->pp;
   const uint64_t N = data->total_nodes;
@@ -528,15 +518,14 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
       rc = fail(SIGMO_ERR_CUDA, "H2D copy failed");
   }
   if (!rc) rc = mark(1);
-  if (!rc) rc = order_classes(q, query, data);
   if (!rc && !rp && !pp.groups.empty()) {
     // a batch too large for one tile: group by group into the batch's planes
     if (cudaMemsetAsync(adm_counts, 0, 4ull * G, q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "memset failed");
     for (size_t gi = 0; gi < pp.groups.size() && !rc; ++gi)
-      rc = launch_planes_admit_group(q, query, data, dsig, R, pp.groups[gi], pp.K, planes, admit, adm_counts);
+      rc = launch_planes_admit_group(q, query, data, dsig, pp.groups[gi], pp.K, planes, admit, adm_counts);
   } else if (!rc) {
     rc = rp ? launch_planes_admit_resident(q, query, data, *rp, pp, d_row_map, admit, adm_counts)
-            : launch_planes_admit(q, query, data, dsig, R, pp, planes, admit, adm_counts);
+            : launch_planes_admit(q, query, data, dsig, pp, planes, admit, adm_counts);
   }
   if (!rc) rc = mark(2);
   // captured: the admitted total of the run that built the graph sizes the
@@ -575,9 +564,7 @@ void drop_graph(Gmcr* m) {
 // queue's pinned buffer.  Returns SIGMO_ERR_INVALID (and drops the graph)
 // when the admitted total differs from the one the graph was sized for.
 int replay_graph(Queue* q, Graph* query, Graph* data, Gmcr* m, sigmo_match_result* out) {
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  SIGMO_CUDA_TRY(cudaEventCreate(&e0));
-  SIGMO_CUDA_TRY(cudaEventCreate(&e1));
+  const cudaEvent_t e0 = q->ev_match[0], e1 = q->ev_match[1];
   cudaError_t e = cudaEventRecord(e0, q->stream);
   if (e == cudaSuccess) e = cudaGraphLaunch(m->graph, q->stream);
   if (e == cudaSuccess) q->launches += m->graph_launches;
@@ -585,8 +572,6 @@ int replay_graph(Queue* q, Graph* query, Graph* data, Gmcr* m, sigmo_match_resul
   if (e == cudaSuccess) e = cudaStreamSynchronize(q->stream);
   float f = 0;
   if (e == cudaSuccess) cudaEventElapsedTime(&f, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
   if (e != cudaSuccess) return fail(SIGMO_ERR_CUDA, "graph replay failed: %s", cudaGetErrorString(e));
   SIGMO_TRY(join_status_result(q));  // the graph read the status word back
   const uint64_t* pin = static_cast<const uint64_t*>(q->pinned);
@@ -610,14 +595,13 @@ int capture_graph(Queue* q, Graph* query, Graph* data, uint32_t R, int find_firs
   drop_graph(m);
   BatchedRun run = run0;
   run.capture = true;
-  Events ev;  // unused while capturing
   const uint64_t launches0 = q->launches;
   SIGMO_CUDA_TRY(cudaStreamBeginCapture(q->stream, cudaStreamCaptureModeThreadLocal));
   uint64_t* d_total = nullptr;
   int rc = join_status_reset(q);
   if (!rc) rc = tmp_alloc(q, reinterpret_cast<void**>(&d_total), 8);
   if (!rc && cudaMemsetAsync(d_total, 0, 8, q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "memset failed");
-  if (!rc) rc = batched_planes(q, query, data, R, find_first, m, d_total, ev, run);
+  if (!rc) rc = batched_planes(q, query, data, R, find_first, m, d_total, run);
   uint64_t* pin = static_cast<uint64_t*>(q->pinned);
   if (!rc && (cudaMemcpyAsync(pin, d_total, 8, cudaMemcpyDeviceToHost, q->stream) != cudaSuccess ||
               cudaMemcpyAsync(pin + 1, m->offsets + data->num_graphs, 4, cudaMemcpyDeviceToHost, q->stream) != cudaSuccess))
@@ -669,9 +653,7 @@ int match_batched(Queue* q, Graph* query, Graph* data, uint32_t R, int find_firs
   drop_graph(m);  // this run may replace the arrays a captured batch refers to
   std::memset(out, 0, sizeof(*out));
   SIGMO_TRY(join_status_reset(q));
-  Events ev;
-  for (auto& e : ev.e) SIGMO_CUDA_TRY(cudaEventCreate(&e));
-  SIGMO_CUDA_TRY(cudaEventRecord(ev.e[0], q->stream));
+  SIGMO_CUDA_TRY(cudaEventRecord(q->ev_match[0], q->stream));
   // the data graph's signatures do not depend on the query batch: launched
   // first, they run while the host builds the query batch's plane program
   BatchedRun prun = run;
@@ -697,11 +679,12 @@ int match_batched(Queue* q, Graph* query, Graph* data, uint32_t R, int find_firs
   // the planes route takes any batch whose query graphs each fit an admission
   // tile (larger batches are admitted in groups); planes take 8 B per
   // (plane, graph, word) in device memory
-  int prc = order_classes(q, query, data);
-  if (prc == SIGMO_ERR_DOMAIN) prc = SIGMO_OK;  // a query graph too large for a tile: bitset route
-  else if (prc) return prc;
-  const bool planes_fit = query->pp.qc_for == data && (!query->pp.groups.empty() ||
-                                                       planes_admit_smem(query->pp.K, data->adj_words) <= 200u * 1024u);
+  const size_t tile_bytes = planes_admit_smem(query->pp.K, data->adj_words);
+  // (resident planes are gathered for the whole batch as long as they fit a tile)
+  const int prc = run.resident && tile_bytes <= 200u * 1024u ? SIGMO_OK : plan_groups(q, query, data->adj_words);
+  // SIGMO_ERR_DOMAIN: a query graph too large for a tile, bitset route
+  if (prc && prc != SIGMO_ERR_DOMAIN) rc = prc;
+  const bool planes_fit = !prc && (!query->pp.groups.empty() || tile_bytes <= 200u * 1024u);
   const bool bitset_route = materialize || !planes_fit;
   if (!rc && bitset_route && data->vertex_base)
     rc = fail(SIGMO_ERR_DOMAIN, "a shard (vertex base %u) runs on the planes route only; this batch needs the bitset route",
@@ -710,13 +693,13 @@ int match_batched(Queue* q, Graph* query, Graph* data, uint32_t R, int find_firs
     if (bitset_route) {
       sigmo_candidates_t cc = static_cast<sigmo_candidates_t>(c);
       if (!cc) rc = sigmo_candidates_create(static_cast<sigmo_queue_t>(q), query->total_nodes, data->total_nodes, &cc);
-      if (!rc) rc = batched_bitset(q, query, data, R, find_first, cc, m, d_total, ev, prun);
+      if (!rc) rc = batched_bitset(q, query, data, R, find_first, cc, m, d_total, prun);
       if (cc != c) sigmo_candidates_destroy(cc);
     } else {
-      rc = batched_planes(q, query, data, R, find_first, m, d_total, ev, prun);
+      rc = batched_planes(q, query, data, R, find_first, m, d_total, prun);
     }
   }
-  if (!rc && cudaEventRecord(ev.e[4], q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
+  if (!rc && cudaEventRecord(q->ev_match[4], q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "event record failed");
   if (!rc) rc = join_status_fetch(q);
   if (!rc) {
     cudaError_t e = cudaMemcpyAsync(q->pinned, d_total, 8, cudaMemcpyDeviceToHost, q->stream);
@@ -729,15 +712,15 @@ int match_batched(Queue* q, Graph* query, Graph* data, uint32_t R, int find_firs
     out->admitted_pairs = m->total;
     out->pairs = static_cast<uint64_t>(query->num_graphs) * data->num_graphs;
     float f;
-    cudaEventElapsedTime(&f, ev.e[0], ev.e[1]);
+    cudaEventElapsedTime(&f, q->ev_match[0], q->ev_match[1]);
     out->ms_signatures = f;
-    cudaEventElapsedTime(&f, ev.e[1], ev.e[2]);
+    cudaEventElapsedTime(&f, q->ev_match[1], q->ev_match[2]);
     out->ms_filter = f;
-    cudaEventElapsedTime(&f, ev.e[2], ev.e[3]);
+    cudaEventElapsedTime(&f, q->ev_match[2], q->ev_match[3]);
     out->ms_mapping = f;
-    cudaEventElapsedTime(&f, ev.e[3], ev.e[4]);
+    cudaEventElapsedTime(&f, q->ev_match[3], q->ev_match[4]);
     out->ms_join = f;
-    cudaEventElapsedTime(&f, ev.e[0], ev.e[4]);
+    cudaEventElapsedTime(&f, q->ev_match[0], q->ev_match[4]);
     out->ms_total = f;
     m->counts_valid = true;
   }

@@ -41,6 +41,12 @@ struct Queue {
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
   void* pinned = nullptr;  // small pinned host buffer for scalar read-backs
+  // Pinned staging of query programs (grown on demand) and the event after the
+  // last copy from it: it is written again only once that copy is done.
+  void* stage = nullptr;
+  size_t stage_bytes = 0;
+  cudaEvent_t ev_stage = nullptr;
+  cudaEvent_t ev_match[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // stages of a batched match
   cudaStream_t side = nullptr;  // second stream for work that overlaps the main one
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // third stream: the join's odd chunks (level masks of one chunk overlap the
@@ -89,12 +95,12 @@ int join_status_result(Queue* q);
 // plane to its row in the batch's plane array.
 struct PlaneGroup {
   uint32_t q0 = 0, q1 = 0;
-  uint32_t K = 0, C = 0, nlab = 0;
-  uint32_t* spec = nullptr;      // [K]
-  uint32_t* r_begin = nullptr;   // [R + 1]
-  uint32_t* row_of = nullptr;    // [K] plane row in the batch
-  uint64_t* quads = nullptr;     // the group's query programs, local plane ids (PlaneProgram::quads)
-  uint32_t* q_off = nullptr;     // [q1 - q0 + 1]
+  uint32_t K = 0, nlab = 0;
+  void* blob = nullptr;               // the device arrays below
+  const uint32_t* spec = nullptr;     // [K]
+  const uint32_t* row_of = nullptr;   // [K] plane row in the batch
+  const uint64_t* quads = nullptr;    // the group's query programs, local plane ids (PlaneProgram::quads)
+  const uint32_t* q_off = nullptr;    // [q1 - q0 + 1]
   size_t n_quads = 0;
 };
 
@@ -103,29 +109,27 @@ struct PlaneProgram {
   bool valid = false;
   uint32_t R = 0;
   int profile = 0;
-  uint32_t K = 0;                 // planes per data graph
-  uint32_t C = 0;                 // classes of identical query vertices
-  uint32_t* spec = nullptr;       // [K] plane definitions
-  uint32_t* prog_off = nullptr;   // [C + 1]
-  uint16_t* prog = nullptr;       // plane indices of each class's program
-  uint32_t* cls = nullptr;        // [query vertices] class of each vertex
-  uint32_t nlab = 0;              // label planes (spec[0 .. nlab))
-  uint32_t* r_begin = nullptr;    // [R + 1] first threshold plane of each iteration
-  uint32_t max_len = 0;           // longest program
-  // host copies (class evaluation order)
-  std::vector<uint32_t> h_spec, h_prog_off, h_cls, h_qgoff;
-  std::vector<uint16_t> h_prog;
-  // per query graph, the programs of its distinct classes in evaluation order
-  // for one data graph's label frequencies (rebuilt when the data graph
-  // changes): four plane ids of 15 bits per entry, a class's last id repeated
-  // to fill its last entry, bit 63 set in it
-  uint64_t* quads = nullptr;
-  uint32_t* q_off = nullptr;      // [query graphs + 1] entries of quads
+  uint32_t K = 0;                     // planes per data graph
+  uint32_t C = 0;                     // classes of identical query vertices
+  uint32_t nlab = 0;                  // label planes (spec[0 .. nlab))
+  void* blob = nullptr;               // the device arrays below
+  const uint32_t* spec = nullptr;     // [K] plane definitions
+  const uint32_t* prog_off = nullptr; // [C + 1]
+  const uint16_t* prog = nullptr;     // plane indices of each class's program
+  const uint32_t* cls = nullptr;      // [query vertices] class of each vertex
+  // per query graph, the programs of its distinct classes in evaluation order:
+  // four plane ids of 15 bits per entry, a class's last id repeated to fill its
+  // last entry, bit 63 set in it
+  const uint64_t* quads = nullptr;
+  const uint32_t* q_off = nullptr;    // [query graphs + 1] entries of quads
   size_t n_quads = 0;
-  std::vector<PlaneGroup> groups; // empty: the whole batch fits one tile
-  const void* qc_for = nullptr;   // the data graph the order was built for
-  uint64_t qc_stamp = 0;
-  uint64_t* qsig_all = nullptr;   // [R][query vertices] signatures, iterations 1..R
+  // host copies; order[order_off[q] .. order_off[q + 1]): query graph q's
+  // distinct classes in evaluation order
+  std::vector<uint32_t> h_spec, h_prog_off, order, order_off;
+  std::vector<uint16_t> h_prog;
+  std::vector<PlaneGroup> groups;     // for sets of groups_aw words; empty: the whole batch fits one tile
+  uint32_t groups_aw = 0;             // 0: not planned
+  uint64_t* qsig_all = nullptr;       // [R][query vertices] signatures, iterations 1..R
 };
 
 struct Graph {
@@ -156,7 +160,7 @@ struct Graph {
   uint16_t* qmeta = nullptr;       // [num_graphs][16]
   uint16_t* qmeta_id = nullptr;    // [num_graphs][16] same, identity order
   std::vector<uint32_t> host_graph_offsets;  // host copy (sizes, dispatch)
-  std::vector<uint64_t> label_hist;          // vertices per label (filled on first use, 256 entries)
+  std::vector<uint64_t> label_hist;          // vertices per label (filled on first use by the resident planes, 256 entries)
   uint64_t stamp = 0;                        // unique per graph object (cache keys)
   cudaEvent_t ready = nullptr;               // recorded after the creation work on the queue's stream
   PlaneProgram pp;                 // when this graph is the query side of a batched match
@@ -280,13 +284,13 @@ int launch_join(Queue* q, const Graph* query, const Graph* data, const MaskSourc
                 uint64_t* d_total, const uint32_t* ranges = nullptr, uint32_t nranges = 0);
 int launch_gmcr_from_ne(Queue* q, const Graph* query, const Graph* data, const uint32_t* NE, const uint32_t* cls, Gmcr* m,
                         bool sync_total, uint64_t capacity_hint);
-int launch_planes_admit(Queue* q, const Graph* query, const Graph* data, const uint64_t* sig_all, uint32_t R,
-                        const PlaneProgram& pp, uint64_t* planes, uint32_t* admit, uint32_t* counts);
+int launch_planes_admit(Queue* q, const Graph* query, const Graph* data, const uint64_t* sig_all, const PlaneProgram& pp,
+                        uint64_t* planes, uint32_t* admit, uint32_t* counts);
 // One group of a batch: its planes go to their rows of the batch's planes
 // (K_total rows per tile), its admission words to its query graphs' rows, and
 // its per-graph admitted counts are added to counts.
-int launch_planes_admit_group(Queue* q, const Graph* query, const Graph* data, const uint64_t* sig_all, uint32_t R,
-                              const PlaneGroup& grp, uint32_t K_total, uint64_t* planes, uint32_t* admit, uint32_t* counts);
+int launch_planes_admit_group(Queue* q, const Graph* query, const Graph* data, const uint64_t* sig_all, const PlaneGroup& grp,
+                              uint32_t K_total, uint64_t* planes, uint32_t* admit, uint32_t* counts);
 // Shared memory of one k_planes_admit tile budgeted for a query group's planes.
 constexpr size_t kGroupSmemBudget = 96u * 1024u;
 // The same admission with the tile's planes gathered from resident planes

@@ -30,8 +30,7 @@ namespace {
 
 // spec[k]: bit 31 set = label plane (bits 0..7 = label value, 255 = any);
 // otherwise r = bits 16..23, l = bits 8..15, c = bits 0..7 (count >= c).
-// Label planes come first, then thresholds in (r, l, c) order;
-// r_begin[r] .. r_begin[r + 1] are the thresholds of iteration r.
+// Label planes come first, then thresholds in (r, l, c) order.
 
 // One graph's planes into column `col` of a shared-memory tile whose rows are
 // `row_words` words apart, by one warp.  With `out`, the words also go to
@@ -277,8 +276,8 @@ __device__ __forceinline__ void admit_tile(const uint64_t* tile, uint32_t QG, co
 template <int AW, bool GATHER, int H>
 __global__ void __launch_bounds__(kAdmitWarps * 32, AW == 1 ? (H == 1 ? 4 : 3) : 2) k_planes_admit(
     uint32_t G, const uint32_t* __restrict__ goff, const uint8_t* __restrict__ lab, const uint64_t* __restrict__ sig_all,
-    uint64_t N, uint32_t R, uint32_t K, uint32_t nlab, const uint32_t* __restrict__ spec, const uint32_t* __restrict__ r_begin,
-    int prof, uint32_t base, const uint64_t* __restrict__ rplanes, uint32_t rrows, const uint32_t* __restrict__ row_map,
+    uint64_t N, uint32_t K, uint32_t nlab, const uint32_t* __restrict__ spec, int prof, uint32_t base,
+    const uint64_t* __restrict__ rplanes, uint32_t rrows, const uint32_t* __restrict__ row_map,
     uint32_t QG, const uint2* __restrict__ g_prog, const uint32_t* __restrict__ g_q_off, uint32_t n_quads, int stage_lists, const uint32_t* __restrict__ row_of, uint32_t out_rows, int accumulate,
     uint64_t* __restrict__ planes, uint32_t* __restrict__ admit, uint32_t* __restrict__ counts) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -364,8 +363,8 @@ __global__ void __launch_bounds__(kAdmitWarps * 32, AW == 1 ? (H == 1 ? 4 : 3) :
 template <int AW>
 __global__ void __launch_bounds__(kAdmitWarps * 32) k_build_planes(
     uint32_t G, const uint32_t* __restrict__ goff, const uint8_t* __restrict__ lab, const uint64_t* __restrict__ sig_all,
-    uint64_t N, uint32_t R, uint32_t K, uint32_t nlab, const uint32_t* __restrict__ spec, const uint32_t* __restrict__ r_begin,
-    int prof, uint32_t base, uint32_t out_rows, uint64_t* __restrict__ out) {
+    uint64_t N, uint32_t K, uint32_t nlab, const uint32_t* __restrict__ spec, int prof, uint32_t base, uint32_t out_rows,
+    uint64_t* __restrict__ out) {
   extern __shared__ uint64_t tile[];  // [K * AW][32], then the planes' tests [K]
   const uint32_t GW = (G + 31u) / 32u;
   uint2* tests = reinterpret_cast<uint2*>(tile + static_cast<size_t>(K) * AW * 32);
@@ -454,7 +453,7 @@ namespace {
 // group's (local ids; planes scattered to row_of).
 struct AdmitView {
   uint32_t K, nlab, QG;
-  const uint32_t *spec, *r_begin;
+  const uint32_t* spec;
   const uint32_t* q_off;   // [QG + 1] entries of prog per query graph
   const uint32_t* row_of;  // group launches: local plane row -> row of the batch's plane array
   const uint64_t* prog;    // four plane ids per entry
@@ -464,7 +463,7 @@ struct AdmitView {
 };
 
 template <int AW, bool GATHER, int H>
-int admit_launch_h(Queue* q, const Graph* data, const uint64_t* sig_all, uint32_t R, const AdmitView& v, const uint64_t* rplanes,
+int admit_launch_h(Queue* q, const Graph* data, const uint64_t* sig_all, const AdmitView& v, const uint64_t* rplanes,
                    uint32_t rrows, const uint32_t* row_map, uint64_t* planes, uint32_t* admit, uint32_t* counts, unsigned sms) {
   const uint32_t G = data->num_graphs, GW = (G + 31u) / 32u, QG = v.QG;
   const uint32_t n_quads = static_cast<uint32_t>(v.n_quads);
@@ -481,14 +480,14 @@ int admit_launch_h(Queue* q, const Graph* data, const uint64_t* sig_all, uint32_
   if (e != cudaSuccess) return fail(SIGMO_ERR_CUDA, "k_planes_admit shared-memory setup failed: %s", cudaGetErrorString(e));
   const uint64_t grid = std::min<uint64_t>((GW + H - 1u) / H, static_cast<uint64_t>(std::max(per_sm, 1)) * sms);
   k_planes_admit<AW, GATHER, H><<<grid, block, smem, q->stream>>>(
-      G, data->graph_offsets, data->node_labels, sig_all, data->total_nodes, R, v.K, v.nlab, v.spec, v.r_begin, q->opts.profile,
+      G, data->graph_offsets, data->node_labels, sig_all, data->total_nodes, v.K, v.nlab, v.spec, q->opts.profile,
       data->vertex_base, rplanes, rrows, row_map, QG, reinterpret_cast<const uint2*>(v.prog), v.q_off, n_quads,
       stage, v.row_of, v.out_rows, v.accumulate, planes, admit, counts);
   return check_launch(q, "k_planes_admit");
 }
 
 template <int AW, bool GATHER>
-int admit_launch(Queue* q, const Graph* data, const uint64_t* sig_all, uint32_t R, const AdmitView& v, const uint64_t* rplanes,
+int admit_launch(Queue* q, const Graph* data, const uint64_t* sig_all, const AdmitView& v, const uint64_t* rplanes,
                  uint32_t rrows, const uint32_t* row_map, uint64_t* planes, uint32_t* admit, uint32_t* counts) {
   int sms = 0;
   SIGMO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, q->device));
@@ -496,38 +495,38 @@ int admit_launch(Queue* q, const Graph* data, const uint64_t* sig_all, uint32_t 
   const uint32_t GW = (data->num_graphs + 31u) / 32u;
   if constexpr (AW == 1)
     if (admit_smem_layout(v.K, AW, 2, GATHER, 0).total <= 110u * 1024u && GW >= 8u * static_cast<unsigned>(sms))
-      return admit_launch_h<AW, GATHER, 2>(q, data, sig_all, R, v, rplanes, rrows, row_map, planes, admit, counts, sms);
-  return admit_launch_h<AW, GATHER, 1>(q, data, sig_all, R, v, rplanes, rrows, row_map, planes, admit, counts, sms);
+      return admit_launch_h<AW, GATHER, 2>(q, data, sig_all, v, rplanes, rrows, row_map, planes, admit, counts, sms);
+  return admit_launch_h<AW, GATHER, 1>(q, data, sig_all, v, rplanes, rrows, row_map, planes, admit, counts, sms);
 }
 
 AdmitView whole_batch(const Graph* query, const PlaneProgram& pp) {
-  return AdmitView{pp.K, pp.nlab, query->num_graphs, pp.spec, pp.r_begin, pp.q_off, nullptr, pp.quads, pp.n_quads, pp.K, 0};
+  return AdmitView{pp.K, pp.nlab, query->num_graphs, pp.spec, pp.q_off, nullptr, pp.quads, pp.n_quads, pp.K, 0};
 }
 
 }  // namespace
 
-int launch_planes_admit(Queue* q, const Graph* query, const Graph* data, const uint64_t* sig_all, uint32_t R,
-                        const PlaneProgram& pp, uint64_t* planes, uint32_t* admit, uint32_t* counts) {
+int launch_planes_admit(Queue* q, const Graph* query, const Graph* data, const uint64_t* sig_all, const PlaneProgram& pp,
+                        uint64_t* planes, uint32_t* admit, uint32_t* counts) {
   if (!data->num_graphs) return SIGMO_OK;
   const AdmitView v = whole_batch(query, pp);
   switch (data->adj_words) {
-    case 1: return admit_launch<1, false>(q, data, sig_all, R, v, nullptr, 0, nullptr, planes, admit, counts);
-    case 2: return admit_launch<2, false>(q, data, sig_all, R, v, nullptr, 0, nullptr, planes, admit, counts);
-    default: return admit_launch<4, false>(q, data, sig_all, R, v, nullptr, 0, nullptr, planes, admit, counts);
+    case 1: return admit_launch<1, false>(q, data, sig_all, v, nullptr, 0, nullptr, planes, admit, counts);
+    case 2: return admit_launch<2, false>(q, data, sig_all, v, nullptr, 0, nullptr, planes, admit, counts);
+    default: return admit_launch<4, false>(q, data, sig_all, v, nullptr, 0, nullptr, planes, admit, counts);
   }
 }
 
-int launch_planes_admit_group(Queue* q, const Graph* query, const Graph* data, const uint64_t* sig_all, uint32_t R,
-                              const PlaneGroup& grp, uint32_t K_total, uint64_t* planes, uint32_t* admit, uint32_t* counts) {
+int launch_planes_admit_group(Queue* q, const Graph* query, const Graph* data, const uint64_t* sig_all, const PlaneGroup& grp,
+                              uint32_t K_total, uint64_t* planes, uint32_t* admit, uint32_t* counts) {
   if (!data->num_graphs || grp.q1 <= grp.q0) return SIGMO_OK;
   const uint32_t GW = (data->num_graphs + 31u) / 32u;
-  const AdmitView v{grp.K,      grp.nlab, grp.q1 - grp.q0, grp.spec, grp.r_begin, grp.q_off, grp.row_of, grp.quads, grp.n_quads,
+  const AdmitView v{grp.K,      grp.nlab, grp.q1 - grp.q0, grp.spec, grp.q_off, grp.row_of, grp.quads, grp.n_quads,
                     K_total, 1};
   uint32_t* adm = admit + static_cast<uint64_t>(grp.q0) * GW;
   switch (data->adj_words) {
-    case 1: return admit_launch<1, false>(q, data, sig_all, R, v, nullptr, 0, nullptr, planes, adm, counts);
-    case 2: return admit_launch<2, false>(q, data, sig_all, R, v, nullptr, 0, nullptr, planes, adm, counts);
-    default: return admit_launch<4, false>(q, data, sig_all, R, v, nullptr, 0, nullptr, planes, adm, counts);
+    case 1: return admit_launch<1, false>(q, data, sig_all, v, nullptr, 0, nullptr, planes, adm, counts);
+    case 2: return admit_launch<2, false>(q, data, sig_all, v, nullptr, 0, nullptr, planes, adm, counts);
+    default: return admit_launch<4, false>(q, data, sig_all, v, nullptr, 0, nullptr, planes, adm, counts);
   }
 }
 
@@ -536,9 +535,9 @@ int launch_planes_admit_resident(Queue* q, const Graph* query, const Graph* data
   if (!data->num_graphs) return SIGMO_OK;
   const AdmitView v = whole_batch(query, pp);
   switch (data->adj_words) {
-    case 1: return admit_launch<1, true>(q, data, nullptr, 0, v, rp.planes, rp.rows, row_map, nullptr, admit, counts);
-    case 2: return admit_launch<2, true>(q, data, nullptr, 0, v, rp.planes, rp.rows, row_map, nullptr, admit, counts);
-    default: return admit_launch<4, true>(q, data, nullptr, 0, v, rp.planes, rp.rows, row_map, nullptr, admit, counts);
+    case 1: return admit_launch<1, true>(q, data, nullptr, v, rp.planes, rp.rows, row_map, nullptr, admit, counts);
+    case 2: return admit_launch<2, true>(q, data, nullptr, v, rp.planes, rp.rows, row_map, nullptr, admit, counts);
+    default: return admit_launch<4, true>(q, data, nullptr, v, rp.planes, rp.rows, row_map, nullptr, admit, counts);
   }
 }
 
@@ -572,11 +571,9 @@ int build_resident_planes(Queue* q, Graph* data, const uint64_t* sig_all, uint32
       spec.push_back(0x80000000u | l);
     }
   const uint32_t nlab = static_cast<uint32_t>(spec.size());
-  std::vector<uint32_t> r_begin(R + 1, 0);
   out->base_row.assign(16ull * R, 0);
   out->cmax.assign(16ull * R, 0);
   for (uint32_t r = 0; r < R; ++r) {
-    r_begin[r] = static_cast<uint32_t>(spec.size());
     for (uint32_t l = 0; l < 16; ++l) {
       const uint32_t cm = cmax[r * 16 + l];
       out->cmax[r * 16 + l] = static_cast<uint8_t>(cm);
@@ -584,7 +581,6 @@ int build_resident_planes(Queue* q, Graph* data, const uint64_t* sig_all, uint32
       for (uint32_t c = 1; c <= cm; ++c) spec.push_back((r << 16) | (l << 8) | c);
     }
   }
-  r_begin[R] = static_cast<uint32_t>(spec.size());
   const uint32_t K = static_cast<uint32_t>(spec.size());
   out->zero_row = K;
   for (uint32_t l = 0; l < 256; ++l)
@@ -594,12 +590,9 @@ int build_resident_planes(Queue* q, Graph* data, const uint64_t* sig_all, uint32
   const size_t smem = static_cast<size_t>(K) * (AW * 32 * 8 + 8);
   if (static_cast<size_t>(K) * AW * 32 * 8 > 200u * 1024u) return fail(SIGMO_ERR_DOMAIN, "the database needs %u resident planes (too many for one tile)", K);
   void* dspec = nullptr;
-  void* drb = nullptr;
   SIGMO_TRY(dev_alloc(q, &dspec, 4ull * K));
-  SIGMO_TRY(dev_alloc(q, &drb, 4ull * (R + 1)));
   int rc = SIGMO_OK;
-  if (cudaMemcpyAsync(dspec, spec.data(), 4ull * K, cudaMemcpyHostToDevice, q->stream) != cudaSuccess ||
-      cudaMemcpyAsync(drb, r_begin.data(), 4ull * (R + 1), cudaMemcpyHostToDevice, q->stream) != cudaSuccess)
+  if (cudaMemcpyAsync(dspec, spec.data(), 4ull * K, cudaMemcpyHostToDevice, q->stream) != cudaSuccess)
     rc = fail(SIGMO_ERR_CUDA, "H2D copy failed");
   if (!rc) rc = dev_alloc(q, reinterpret_cast<void**>(&out->planes), 8ull * GW * out->rows * AW * 32 + 8);
   if (!rc && GW) {
@@ -613,9 +606,8 @@ int build_resident_planes(Queue* q, Graph* data, const uint64_t* sig_all, uint32
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_build_planes<AWV>, block, smem);  \
   if (e == cudaSuccess)                                                                                              \
     k_build_planes<AWV><<<std::min<uint64_t>(GW, static_cast<uint64_t>(std::max(per_sm, 1)) * sms), block, smem,      \
-                          q->stream>>>(G, data->graph_offsets, data->node_labels, sig_all, N, R, K, nlab,            \
-                                       static_cast<const uint32_t*>(dspec), static_cast<const uint32_t*>(drb),        \
-                                       q->opts.profile, data->vertex_base, out->rows, out->planes)
+                          q->stream>>>(G, data->graph_offsets, data->node_labels, sig_all, N, K, nlab,               \
+                                       static_cast<const uint32_t*>(dspec), q->opts.profile, data->vertex_base, out->rows, out->planes)
     switch (AW) {
       case 1: SIGMO_BUILD(1); break;
       case 2: SIGMO_BUILD(2); break;
@@ -627,7 +619,6 @@ int build_resident_planes(Queue* q, Graph* data, const uint64_t* sig_all, uint32
   }
   if (!rc && cudaStreamSynchronize(q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "resident plane build failed");
   dev_free(q, dspec);
-  dev_free(q, drb);
   return rc;
 }
 
