@@ -602,9 +602,10 @@ __device__ __forceinline__ uint8_t csr_edge_label(uint32_t a, uint32_t b, const 
 // backtracking.  find_first ends a lane's DFS at its first match.  mapping[]
 // (per query vertex) starts zeroed per lane and carries over between its DFS
 // runs, as the reference's private array does.  Like the driver's join, the
-// count depends on these steps only where the visited set is live: this kernel
-// takes the graphs starting below vertex 256 (REF_PTX) and those over 256
-// vertices; k_join_wide<.., BONDS> takes the others.
+// count depends on these steps only where the visited set is live.  This kernel
+// takes batches with graphs over 256 vertices; in the others
+// k_join_wildcard_sets takes the graphs starting below vertex 256 (REF_PTX) and
+// k_join_wide<.., BONDS> the rest.
 template <bool EXACT>
 __global__ void k_join_wildcard(const uint32_t* __restrict__ bits, uint64_t Wp, int prof, const uint32_t* __restrict__ qgoff,
                                 const uint64_t* __restrict__ qadj, const uint32_t* __restrict__ qroff,
@@ -794,6 +795,174 @@ __device__ __forceinline__ void bond_row(const BondGraphs& bg, uint32_t a, uint3
       seen[w] |= bit;
     }
   }
+}
+
+// k_join_wildcard (REF_PTX) for graphs of at most 64 * AW vertices, on
+// graph-local sets: the same searches in the same order, a warp per sub-group
+// of a graph (sub-group sg of nsg takes the segment's slots sg, sg + nsg, ...),
+// its slot's masks built once by all lanes, and per lane and level the
+// candidates left and the neighbour counts in shared memory, as in
+// k_join_literal_sets.  With the walk over the earlier levels and CSR rows per
+// candidate: 1.53 ms for the first ten molecules of 2,003 x 40 pairs, this
+// @@.
+inline size_t wildcard_smem(uint32_t aw, uint32_t levels) {
+  return 32ull * levels * (24ull * aw + 1u) + 8ull * levels * aw;
+}
+
+template <int AW>
+__global__ void __launch_bounds__(32) k_join_wildcard_sets(MaskSource src, BondGraphs bg, const uint32_t* __restrict__ qgoff,
+                                                           const uint64_t* __restrict__ qsel_id,
+                                                           const uint32_t* __restrict__ dgoff,
+                                                           const uint64_t* __restrict__ dadj,
+                                                           const uint32_t* __restrict__ indices, uint32_t graphs, uint32_t nsg,
+                                                           uint32_t levels, int find_first, uint64_t* __restrict__ counts,
+                                                           unsigned long long* __restrict__ d_total) {
+  extern __shared__ uint64_t wild_sm[];
+  constexpr unsigned kAll = 0xFFFFFFFFu;
+  const uint32_t lane = threadIdx.x, L = levels;
+  uint64_t* M = wild_sm;                          // [vertex][AW]
+  uint64_t* rem = wild_sm + L * AW + lane;        // [level][AW][32]
+  uint64_t* p0 = rem + 32u * L * AW;
+  uint64_t* p1 = p0 + 32u * L * AW;
+  uint8_t* map = reinterpret_cast<uint8_t*>(wild_sm + L * AW + 96u * L * AW) + lane;  // [vertex][32] local ids
+#define LVL(arr, d, w) arr[((d) * AW + (w)) * 32u]
+  uint64_t my_total = 0;
+  for (uint32_t blk = blockIdx.x; blk < graphs * nsg; blk += gridDim.x) {
+    const uint32_t g = blk / nsg, sg = blk % nsg;
+    const uint32_t s = dgoff[g], e = dgoff[g + 1];
+    const uint32_t seg0 = bg.doffsets[g], seglen = bg.doffsets[g + 1] - seg0;
+    const uint64_t low = s >= 256u ? 0ull : (256u - s >= 64u ? ~0ull : ((1ull << (256u - s)) - 1ull));
+    auto bit_of = [&](uint32_t t) -> uint64_t { return t < 64u ? (1ull << t) & low : 0ull; };
+    // mapping[] of a fresh work-item: global vertex 0
+#pragma unroll 1
+    for (uint32_t k = 0; k < L; ++k) map[k * 32u] = s == 0 ? 0 : kLitOutside;
+    for (uint32_t it = sg; it < seglen; it += nsg) {
+      const uint32_t qg = indices[seg0 + it];
+      const uint32_t v0 = qgoff[qg], n = qgoff[qg + 1] - v0;
+      __syncwarp();
+      for (uint32_t j = lane; j < n; j += 32u) source_mask<AW>(src, AW, v0 + j, g, s, e, M + j * AW);
+      __syncwarp();
+      uint32_t mine = 0;
+      if (lane < n)
+#pragma unroll
+        for (int w = 0; w < AW; ++w) mine += __popcll(M[lane * AW + w]);
+      const uint32_t max_c = __reduce_max_sync(kAll, mine);
+      const uint32_t root = __reduce_max_sync(kAll, lane < n && mine == max_c ? lane : 0u);
+      const uint64_t below = (1ull << root) - 1ull;
+      uint64_t found = 0;
+      for (uint32_t sc = lane; sc < max_c; sc += 32u) {
+        uint32_t t0 = 0, skip = sc;  // the sc-th candidate of the root
+#pragma unroll
+        for (int w = 0; w < AW; ++w) {
+          uint64_t m = M[root * AW + w];
+          const uint32_t c = __popcll(m);
+          if (skip < c) {
+            for (; skip; --skip) m &= m - 1;
+            t0 = 64u * w + __ffsll(static_cast<long long>(m)) - 1u;
+            skip = 0xFFFFFFFFu;
+          } else if (skip != 0xFFFFFFFFu) {
+            skip -= c;
+          }
+        }
+        map[root * 32u] = static_cast<uint8_t>(t0);
+        uint64_t visited = bit_of(t0);
+        uint32_t d = 0, t = t0;  // t was placed at level d: find the candidates of level d + 1
+        for (bool placed = true;;) {
+          if (placed) {
+            const uint32_t v = d + 1u <= root ? d : d + 1u;
+            uint64_t sel = qsel_id[v0 + v];
+            sel = ((bg.qadj[v0 + root] >> v) & 1ull) | ((sel & below) << 1) | (sel & ~((below << 1) | 1ull));
+            const uint32_t cn = __popcll(sel);
+            uint64_t n0[AW], n1[AW], f[AW];
+#pragma unroll
+            for (int w = 0; w < AW; ++w) {
+              const uint64_t r = dadj[static_cast<uint64_t>(s + t) * AW + w];
+              const uint64_t b0 = d ? LVL(p0, d, w) : 0ull, b1 = d ? LVL(p1, d, w) : 0ull;
+              n0[w] = (b0 ^ r) | (b1 & b0);
+              n1[w] = b1 | (b0 & r);
+              f[w] = M[v * AW + w];
+            }
+            for (uint64_t m = sel; m; m &= m - 1) {
+              const uint32_t i = __ffsll(static_cast<long long>(m)) - 1;
+              const uint32_t u = i == 0 ? root : (i <= root ? i - 1u : i);
+              uint64_t row[AW];
+              bond_row<AW>(bg, s + map[u * 32u], s, csr_edge_label(v0 + u, v0 + v, bg.qroff, bg.qcol, bg.qel), row);
+#pragma unroll
+              for (int w = 0; w < AW; ++w) f[w] &= row[w];
+            }
+            if (cn <= 2u) {
+              const uint64_t e0 = cn == 1u ? ~0ull : 0ull, e1 = cn == 2u ? ~0ull : 0ull;
+#pragma unroll
+              for (int w = 0; w < AW; ++w) f[w] &= ~((n0[w] ^ e0) | (n1[w] ^ e1));
+            } else {
+              for (uint32_t i = 0; i <= d; ++i) {
+                const uint32_t u = i == 0 ? root : (i <= root ? i - 1u : i);
+                const uint64_t* row = dadj + static_cast<uint64_t>(s + map[u * 32u]) * AW;
+                const uint64_t want = 0ull - ((sel >> i) & 1ull);
+#pragma unroll
+                for (int w = 0; w < AW; ++w) f[w] &= ~(row[w] ^ want);
+              }
+            }
+            ++d;
+#pragma unroll
+            for (int w = 0; w < AW; ++w) {
+              LVL(rem, d, w) = f[w];
+              LVL(p0, d, w) = n0[w];
+              LVL(p1, d, w) = n1[w];
+            }
+            placed = false;
+          }
+          const uint32_t v = d <= root ? d - 1u : d;  // the frame's query vertex
+          if (d + 1u == n) {  // the last one in one step, as in k_join_literal_sets
+            uint32_t c = 0, first = 0, final = 0;
+#pragma unroll
+            for (int w = 0; w < AW; ++w) {
+              const uint64_t p = LVL(rem, d, w) & (w ? ~0ull : ~visited);
+              if (!p) continue;
+              if (!c) first = 64u * w + __ffsll(static_cast<long long>(p)) - 1u;
+              c += __popcll(p);
+              final = 64u * w + 63u - __clzll(static_cast<long long>(p));
+              if (w == 0 && !find_first) visited |= p & low;
+            }
+            if (c) {
+              map[v * 32u] = static_cast<uint8_t>(find_first ? first : final);
+              found += find_first ? 1u : c;
+              if (find_first) break;
+            }
+          } else {
+            t = 0xFFFFFFFFu;
+#pragma unroll
+            for (int w = 0; w < AW; ++w) {
+              const uint64_t r = LVL(rem, d, w);
+              if (t == 0xFFFFFFFFu && r) {
+                t = 64u * w + __ffsll(static_cast<long long>(r)) - 1u;
+                LVL(rem, d, w) = r & (r - 1);
+              }
+            }
+            if (t != 0xFFFFFFFFu) {
+              if (!(visited & bit_of(t))) {
+                map[v * 32u] = static_cast<uint8_t>(t);
+                visited |= bit_of(t);
+                placed = true;
+              }
+              continue;
+            }
+          }
+          // the frame is used up
+          visited &= ~bit_of(map[v * 32u]);  // mapping[], perhaps stale
+          if (--d == 0) break;
+          if (d == 1u) visited = bit_of(t0);  // back at the first frame: the root alone
+        }
+      }
+      my_total += found;
+      uint64_t slot_total = found;
+      for (int o = 16; o; o >>= 1) slot_total += __shfl_xor_sync(kAll, slot_total, o);
+      if (lane == 0) counts[seg0 + it] = slot_total;
+    }
+  }
+#undef LVL
+  for (int o = 16; o; o >>= 1) my_total += __shfl_xor_sync(kAll, my_total, o);
+  if (lane == 0 && my_total) atomicAdd(d_total, static_cast<unsigned long long>(my_total));
 }
 
 template <int AW, bool EXACT, bool BONDS>
@@ -1297,7 +1466,7 @@ template <uint32_t LV>
 constexpr uint32_t dfs_threads() { return LV <= kDfsLevels ? 160u : 96u; }
 template <uint32_t LV>
 constexpr size_t dfs_smem() { return dfs_threads<LV>() * (LV * 3 * 8 + (LV - 1) * (2 * 8 + 2)); }
-constexpr uint32_t kDfsAhead = 1024;  // slots ahead of the one taken that are brought to L2
+constexpr uint32_t kDfsAhead = 256;  // slots ahead of the one taken that are brought to L2
 constexpr uint32_t kRefillAll = 12, kRefillFirst = 20;
 
 template <uint32_t LV, bool EXACT, uint32_t DAW>
@@ -1778,9 +1947,25 @@ int launch_join_wildcard(Queue* q, const Graph* query, const Graph* data, const 
   const uint32_t G = data->num_graphs;
   if (!G || !m->total) return SIGMO_OK;
   auto* tot = reinterpret_cast<unsigned long long*>(d_total);
-  // graphs [0, literal): step by step, on the side stream; the others by sets
+  MaskSource src;
+  src.bits = c->bits;
+  src.Wp = c->Wp;
+  src.prof = q->opts.profile;
+  BondGraphs bg;
+  bg.qadj = query->adj;
+  bg.qroff = query->row_offsets;
+  bg.qcol = query->column_indices;
+  bg.qel = query->edge_labels;
+  bg.droff = data->row_offsets;
+  bg.dcol = data->column_indices;
+  bg.del = data->edge_labels;
+  bg.doffsets = m->offsets;
+  bg.total_slots = m->total;
+  // graphs [0, literal): step by step, on the side stream; the others in any order
   uint32_t literal = G;
-  if (data->max_nodes <= 64u * kMaxAdjWords) {
+  const bool sets = data->max_nodes <= 64u * kMaxAdjWords;
+  if (sets) {
+    SIGMO_TRY(launch_query_order(const_cast<Graph*>(query)));  // before the fork: both streams read it
     literal = 0;
     while (!exact && literal < G && data->host_graph_offsets[literal] < kLowOffsetLimit) ++literal;
   }
@@ -1788,34 +1973,28 @@ int launch_join_wildcard(Queue* q, const Graph* query, const Graph* data, const 
     if (cudaEventRecord(q->ev_fork, q->stream) != cudaSuccess || cudaStreamWaitEvent(q->side, q->ev_fork, 0) != cudaSuccess)
       return fail(SIGMO_ERR_CUDA, "stream fork failed");
     const unsigned grid = std::min<uint32_t>(literal, 148u * 64u);
-    auto kern = exact ? k_join_wildcard<true> : k_join_wildcard<false>;
-    kern<<<grid, wg, 0, q->side>>>(c->bits, c->Wp, q->opts.profile, query->graph_offsets, query->adj, query->row_offsets,
+    const size_t smem = wildcard_smem(data->adj_words, query->max_nodes);
+    if (sets) {
+      auto kern = data->adj_words == 1 ? k_join_wildcard_sets<1> : data->adj_words == 2 ? k_join_wildcard_sets<2> : k_join_wildcard_sets<4>;
+      SIGMO_TRY(allow_max_dynamic_smem(reinterpret_cast<const void*>(kern), q->device));
+      kern<<<grid_for(static_cast<uint64_t>(literal) * (wg / 32u), 1, 148u * 64u), 32, smem, q->side>>>(
+          src, bg, query->graph_offsets, query->qsel_id, data->graph_offsets, data->adj, m->indices, literal, wg / 32u,
+          query->max_nodes, find_first, m->counts, tot);
+    } else {
+      auto kern = exact ? k_join_wildcard<true> : k_join_wildcard<false>;
+      kern<<<grid, wg, 0, q->side>>>(c->bits, c->Wp, q->opts.profile, query->graph_offsets, query->adj, query->row_offsets,
                                    query->column_indices, query->edge_labels, data->graph_offsets, data->adj, data->adj_words,
                                    data->row_offsets, data->column_indices, data->edge_labels, m->offsets, m->indices, literal,
                                    find_first, m->counts, tot);
+    }
     SIGMO_TRY(check_launch(q, "k_join_wildcard"));
   }
   int rc = SIGMO_OK;
   if (literal < G) {
-    rc = launch_query_order(const_cast<Graph*>(query));
     void* cursor = nullptr;
-    if (!rc) rc = tmp_alloc(q, &cursor, 8);
+    rc = tmp_alloc(q, &cursor, 8);
     if (!rc && cudaMemsetAsync(cursor, 0, 8, q->stream) != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "memset failed");
-    MaskSource src;
-    src.bits = c->bits;
-    src.Wp = c->Wp;
-    src.prof = q->opts.profile;
-    BondGraphs bg;
-    bg.qadj = query->adj;
-    bg.qroff = query->row_offsets;
-    bg.qcol = query->column_indices;
-    bg.qel = query->edge_labels;
-    bg.droff = data->row_offsets;
-    bg.dcol = data->column_indices;
-    bg.del = data->edge_labels;
-    bg.doffsets = m->offsets;
     bg.first_graph = literal;
-    bg.total_slots = m->total;
     const uint32_t aw = data->adj_words, stride = query->max_nodes * aw;
     const uint32_t batch = std::max(1u, std::min<uint32_t>(kWideBatch, static_cast<uint32_t>(kWideMaskBytes / (8ull * stride))));
     const size_t smem = wide_smem(batch, aw, stride);
