@@ -241,6 +241,18 @@ int build_plane_program(Queue* q, Graph* query, uint32_t R) {
     prog_off[c + 1] = static_cast<uint32_t>(n_prog);
     rank[c] = ((l == kWildcard ? Qn : label_count[l]) << 16) | (0xFFFFu - (prog_off[c + 1] - prog_off[c]));
   }
+  std::vector<uint64_t> cquads;  // the classes' programs, four ids per entry
+  std::vector<uint32_t> cquad_off(C + 1, 0);
+  cquads.reserve(n_prog / 4 + C);
+  for (uint32_t c = 0; c < C; ++c) {
+    const uint32_t b = prog_off[c], n = prog_off[c + 1] - b;
+    for (uint32_t i = 0; i < n; i += 4) {
+      uint64_t x = 0;
+      for (uint32_t j = 0; j < 4; ++j) x |= static_cast<uint64_t>(prog[b + std::min(i + j, n - 1)]) << (16 * j);
+      cquads.push_back(x);
+    }
+    cquad_off[c + 1] = static_cast<uint32_t>(cquads.size());
+  }
   // query graphs in parallel ranges, each range's lists on their own, then
   // concatenated in query order
   const std::vector<uint32_t>& qgoff = query->host_graph_offsets;
@@ -265,8 +277,9 @@ int build_plane_program(Queue* q, Graph* query, uint32_t R) {
       const size_t before = p.quads.size();
       for (const auto& x : list) {
         p.order.push_back(x.second);
-        const uint32_t b = prog_off[x.second];
-        if (with_quads) append_quads(prog_off[x.second + 1] - b, [&](size_t i) { return prog[b + i]; }, &p.quads);
+        if (!with_quads) continue;
+        p.quads.insert(p.quads.end(), cquads.begin() + cquad_off[x.second], cquads.begin() + cquad_off[x.second + 1]);
+        p.quads.back() |= 1ull << 63;
       }
       p.order_n.push_back(static_cast<uint32_t>(list.size()));
       p.quads_n.push_back(static_cast<uint32_t>(p.quads.size() - before));
@@ -283,13 +296,13 @@ int build_plane_program(Queue* q, Graph* query, uint32_t R) {
     for (uint32_t n : p.quads_n) q_off.push_back(q_off.back() + n);
   }
   Blob blob;
-  const size_t i_spec = blob.add(spec), i_off = blob.add(prog_off), i_prog = blob.add(prog), i_cls = blob.add(cls),
+  const size_t i_spec = blob.add(spec), i_off = blob.add(cquad_off), i_prog = blob.add(cquads), i_cls = blob.add(cls),
                i_qoff = blob.add(q_off), i_quads = blob.add(quads);
   SIGMO_TRY(blob.send(q, &pp.blob));
   SIGMO_CUDA_TRY(cudaStreamWaitEvent(on_side.main, q->ev_stage, 0));
   pp.spec = blob.at<uint32_t>(i_spec);
   pp.prog_off = blob.at<uint32_t>(i_off);
-  pp.prog = blob.at<uint16_t>(i_prog);
+  pp.prog = blob.at<uint64_t>(i_prog);
   pp.cls = blob.at<uint32_t>(i_cls);
   pp.q_off = blob.at<uint32_t>(i_qoff);
   pp.quads = blob.at<uint64_t>(i_quads);
@@ -299,6 +312,7 @@ int build_plane_program(Queue* q, Graph* query, uint32_t R) {
   pp.nlab = nlab;
   pp.h_spec = std::move(spec);
   pp.h_prog = std::move(prog);
+  pp.h_quads = std::move(cquads);
   pp.h_prog_off = std::move(prog_off);
   pp.R = R;
   pp.profile = q->opts.profile;
@@ -482,7 +496,7 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
   // resident planes: the batch's plane k is resident row row_map[k], and the
   // class programs are rewritten as resident rows for the join
   std::vector<uint32_t> row_map;
-  std::vector<uint16_t> rprog;
+  std::vector<uint64_t> rprog;
   if (rp) {
     if (rp->R != R) return fail(SIGMO_ERR_INVALID, "resident planes hold %u iterations, the batch asks for %u", rp->R, R);
     row_map.resize(pp.K);
@@ -495,10 +509,13 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
         row_map[k] = c <= rp->cmax[r * 16 + l] ? rp->base_row[r * 16 + l] + c - 1 : rp->zero_row;
       }
     }
-    rprog.resize(pp.h_prog.size());
-    for (size_t i = 0; i < rprog.size(); ++i) rprog[i] = static_cast<uint16_t>(row_map[pp.h_prog[i]]);
+    rprog.resize(pp.h_quads.size());
+    for (size_t i = 0; i < rprog.size(); ++i) {
+      const uint64_t x = pp.h_quads[i];
+      for (int j = 0; j < 4; ++j) rprog[i] |= static_cast<uint64_t>(row_map[(x >> (16 * j)) & 0xFFFFu] & 0xFFFFu) << (16 * j);
+    }
   }
-  const uint64_t b_map = 4ull * row_map.size() + 2ull * rprog.size();
+  const uint64_t b_map = al(4ull * row_map.size()) + 8ull * rprog.size();
   void* buf = nullptr;
   SIGMO_TRY(tmp_alloc(q, &buf, al(b_dsig) + al(b_planes) + al(b_ne) + al(b_map) + 256));
   char* p = static_cast<char*>(buf);
@@ -510,11 +527,11 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
   uint32_t* adm_counts = admit + static_cast<uint64_t>(query->num_graphs) * GW;
   p += al(b_ne);
   uint32_t* d_row_map = reinterpret_cast<uint32_t*>(p);
-  uint16_t* d_rprog = reinterpret_cast<uint16_t*>(d_row_map + row_map.size());
+  uint64_t* d_rprog = reinterpret_cast<uint64_t*>(p + al(4ull * row_map.size()));
   int rc = run.dsig ? SIGMO_OK : launch_sig_all(q, data, R, dsig);
   if (!rc && rp) {
     if (cudaMemcpyAsync(d_row_map, row_map.data(), 4ull * row_map.size(), cudaMemcpyHostToDevice, q->stream) != cudaSuccess ||
-        cudaMemcpyAsync(d_rprog, rprog.data(), 2ull * rprog.size(), cudaMemcpyHostToDevice, q->stream) != cudaSuccess)
+        cudaMemcpyAsync(d_rprog, rprog.data(), 8ull * rprog.size(), cudaMemcpyHostToDevice, q->stream) != cudaSuccess)
       rc = fail(SIGMO_ERR_CUDA, "H2D copy failed");
   }
   if (!rc) rc = mark(1);

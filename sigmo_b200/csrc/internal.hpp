@@ -114,8 +114,10 @@ struct PlaneProgram {
   uint32_t nlab = 0;                  // label planes (spec[0 .. nlab))
   void* blob = nullptr;               // the device arrays below
   const uint32_t* spec = nullptr;     // [K] plane definitions
-  const uint32_t* prog_off = nullptr; // [C + 1]
-  const uint16_t* prog = nullptr;     // plane indices of each class's program
+  // each class's program, four plane ids per entry (the last one repeated to
+  // fill the last entry)
+  const uint32_t* prog_off = nullptr; // [C + 1] entries of prog
+  const uint64_t* prog = nullptr;
   const uint32_t* cls = nullptr;      // [query vertices] class of each vertex
   // per query graph, the programs of its distinct classes in evaluation order:
   // four plane ids of 15 bits per entry, a class's last id repeated to fill its
@@ -126,7 +128,8 @@ struct PlaneProgram {
   // host copies; order[order_off[q] .. order_off[q + 1]): query graph q's
   // distinct classes in evaluation order
   std::vector<uint32_t> h_spec, h_prog_off, order, order_off;
-  std::vector<uint16_t> h_prog;
+  std::vector<uint16_t> h_prog;       // h_prog_off: classes' ids in h_prog
+  std::vector<uint64_t> h_quads;      // prog
   std::vector<PlaneGroup> groups;     // for sets of groups_aw words; empty: the whole batch fits one tile
   uint32_t groups_aw = 0;             // 0: not planned
   uint64_t* qsig_all = nullptr;       // [R][query vertices] signatures, iterations 1..R
@@ -254,8 +257,8 @@ int launch_gmcr(Queue* q, const Graph* query, const Graph* data, const Candidate
                 uint64_t capacity_hint);
 // Where a join takes a pair's candidate sets from: the candidate bitset, or
 // the batched form's planes ([graph][K][AW], or tiled: [graph / 32][K][AW][32],
-// the resident planes; prog: the class programs as row indices into it, pp.prog
-// for the per-batch planes).
+// the resident planes; prog: the class programs, four row indices into it per
+// entry, pp.prog for the per-batch planes).
 struct MaskSource {
   const uint32_t* bits = nullptr;
   uint64_t Wp = 0;
@@ -264,7 +267,7 @@ struct MaskSource {
   uint32_t K = 0;
   bool tiled = false;
   const uint32_t* prog_off = nullptr;
-  const uint16_t* prog = nullptr;
+  const uint64_t* prog = nullptr;
   const uint32_t* cls = nullptr;
 };
 // Query graphs [q_begin, q_end) of each segment only (the full range: 0, ~0u).
