@@ -231,6 +231,45 @@ __global__ void k_gmcr_admit(const uint32_t* __restrict__ NE, uint32_t GW, const
   }
 }
 
+// Segment offsets of up to kScanSmall data graphs in one launch (offsets[0] = 0,
+// then the inclusive sums of counts): a block, a run of graphs per thread.  The
+// general scan takes a memset and two launches, 12 us of a small call's chain
+// against 5.
+constexpr uint32_t kScanSmall = 8192, kScanThreads = 1024;
+__global__ void __launch_bounds__(kScanThreads) k_gmcr_scan(const uint32_t* __restrict__ counts, uint32_t G,
+                                                            uint32_t* __restrict__ offsets) {
+  __shared__ uint32_t s_warp[32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t per = (G + kScanThreads - 1u) / kScanThreads;
+  const uint32_t g0 = threadIdx.x * per, g1 = g0 + per < G ? g0 + per : G;
+  uint32_t sum = 0;
+  for (uint32_t g = g0; g < g1; ++g) sum += counts[g];
+  uint32_t incl = sum;
+#pragma unroll
+  for (unsigned o = 1; o < 32; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    uint32_t w = s_warp[lane];
+#pragma unroll
+    for (unsigned o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, w, o);
+      if (lane >= o) w += v;
+    }
+    s_warp[lane] = w;
+  }
+  __syncthreads();
+  uint32_t at = incl - sum + (warp ? s_warp[warp - 1] : 0u);
+  if (threadIdx.x == 0) offsets[0] = 0;
+  for (uint32_t g = g0; g < g1; ++g) {
+    at += counts[g];
+    offsets[g + 1] = at;
+  }
+}
+
 // Segment fill.  A warp owns 32 consecutive data graphs (one admission word
 // column) and walks the query graphs 32 at a time: lane l loads the word of
 // query q0 + l, then for each of the 32 graphs a vote gives the chunk's
@@ -296,14 +335,18 @@ int launch_gmcr_from_admit(Queue* q, const Graph* query, const Graph* data, cons
   if (!m->offsets) SIGMO_TRY(dev_alloc(q, reinterpret_cast<void**>(&m->offsets), sizeof(uint32_t) * (G + 1ull)));
   m->num_data_graphs = G;
   m->counts_valid = false;
-  SIGMO_CUDA_TRY(cudaMemsetAsync(m->offsets, 0, sizeof(uint32_t) * (G + 1ull), q->stream));
+  const bool small = G && QG && G <= kScanSmall;
+  if (!small) SIGMO_CUDA_TRY(cudaMemsetAsync(m->offsets, 0, sizeof(uint32_t) * (G + 1ull), q->stream));
   size_t cub_bytes = 0;
-  if (G) cub::DeviceScan::InclusiveSum(nullptr, cub_bytes, static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
+  if (G && !small) cub::DeviceScan::InclusiveSum(nullptr, cub_bytes, static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
                                        static_cast<int>(G), q->stream);
   void* cub_tmp = nullptr;
-  SIGMO_TRY(tmp_alloc(q, &cub_tmp, cub_bytes + 256));
+  if (!small) SIGMO_TRY(tmp_alloc(q, &cub_tmp, cub_bytes + 256));
   int rc = SIGMO_OK;
-  if (G && QG) {
+  if (small) {
+    k_gmcr_scan<<<1, kScanThreads, 0, q->stream>>>(counts, G, m->offsets);
+    rc = check_launch(q, "k_gmcr_scan");
+  } else if (G && QG) {
     cudaError_t e = cub::DeviceScan::InclusiveSum(cub_tmp, cub_bytes, counts, m->offsets + 1, static_cast<int>(G), q->stream);
     if (e != cudaSuccess) rc = fail(SIGMO_ERR_CUDA, "device scan failed: %s", cudaGetErrorString(e));
     q->launches += 2;

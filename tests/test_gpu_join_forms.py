@@ -140,3 +140,12 @@ def test_admission_with_two_graphs_per_lane(count, serve):
     off, idx = gm.getGMCR()
     assert np.array_equal(off, ref["offsets"]) and np.array_equal(idx, ref["indices"])
     assert np.array_equal(gm.getPairCounts(), ref["per_pair"]) and res["total_matches"] == ref["total"]
+
+
+@pytest.mark.parametrize("count", [1, 31, 33, 1024, 1025, 8191, 8192, 8193])
+def test_segment_offsets_by_graph_count(count):
+    """One-launch offsets up to 8,192 data graphs: fewer graphs than threads,
+    one per thread, ragged runs, the largest count and the one past it."""
+    d = sb.generate_molecules(count, 8, 14, seed=3401)
+    q = sb.generate_queries(6, 2, 4, seed=3402).concat(sb.io.parse(_graph(2, [(0, 1)], [1, 1]) + "\n"))
+    _check(q, d, 1, "ref-ptx", True)
