@@ -87,7 +87,7 @@ __device__ __forceinline__ uint32_t dominance_word(uint64_t qs, const uint4* __r
 constexpr unsigned kTabThreads = 128;
 constexpr unsigned kTabRows = 64;
 constexpr unsigned kFilterSlots = 16;   // distinct labels tabulated per block
-constexpr unsigned kRefineSlots = 32;   // distinct (label, count) thresholds tabulated per block
+constexpr unsigned kRefineSlots = 12;   // distinct (label, count) thresholds tabulated per block
 constexpr uint16_t kNoSlot = 0x8000u;   // row entry computed directly (beyond the table)
 
 // Exclusive ranks of the set bits of a shared bitmap of `nwords` words (<= 32),
@@ -204,7 +204,13 @@ __global__ void k_sig_planes(const uint64_t* __restrict__ sig, uint64_t n, uint6
 // (planes[l][w], see k_sig_planes).  Thread t owns the two words 2t, 2t+1 of
 // the block's 256-word span; the block's distinct thresholds (kRefineSlots at
 // most, about ten for molecule queries) are tabulated per thread, and a word
-// is written back only when it changed.
+// is written back only when it changed.  Bound by the bitset's traffic: one read
+// and the changed words' write.  What matters below that is warps in flight, and
+// the table's shared memory set their number: six passes over 100,000 molecules
+// x 600 take 5.12 ms with 32 slots (6 blocks per SM), 3.94 with 16 (7, by
+// registers) and 3.71 with 12 (10); four words per thread took 4.16, eight
+// slots 3.70.  A threshold beyond the table is computed from the planes, which
+// the block's other rows have brought to L1.
 __device__ __forceinline__ uint2 ge_pair(const uint4* __restrict__ planes, uint64_t Wp, uint64_t w0, uint32_t p) {
   const uint32_t l = p / 15u, c = p % 15u + 1u;
   const uint4 a = __ldg(planes + static_cast<uint64_t>(l) * Wp + w0);
@@ -212,7 +218,7 @@ __device__ __forceinline__ uint2 ge_pair(const uint4* __restrict__ planes, uint6
   return make_uint2(ge_sliced(a.x, a.y, a.z, a.w, c), ge_sliced(b.x, b.y, b.z, b.w, c));
 }
 
-__global__ void __launch_bounds__(kTabThreads) k_refine(const uint64_t* __restrict__ qsig, uint64_t Qn,
+__global__ void __launch_bounds__(kTabThreads, 10) k_refine(const uint64_t* __restrict__ qsig, uint64_t Qn,
                                                         const uint4* __restrict__ planes, uint64_t Wp,
                                                         uint32_t* __restrict__ bits, uint32_t rows) {
   __shared__ uint32_t present[8];  // threshold p = 15 l + c - 1 (240 bits)
