@@ -161,7 +161,10 @@ __device__ __forceinline__ void build_graph_planes(uint64_t* col, uint32_t row_w
 // classes of 6.5 planes per 32-graph tile and query; 1.35 -> 1.09 ms on 100,000
 // x 600, 0.533 -> 0.512 ms on 200,000 x 60); it needs twice the shared memory,
 // so it is taken where two CTAs of 512 threads still fit an SM, and enough tiles
-// to fill the chip (eight per SM).  A tile whose graphs all have at most 64
+// for the CTAs that one graph per lane would keep on the chip (four per SM): the
+// filter stage of 37,000 / 30,000 / 25,000 / 20,000 / 10,000 molecules x 300
+// takes 0.314 / 0.253 / 0.222 / 0.189 / 0.119 ms with one, 0.283 / 0.238 / 0.197
+// / 0.189 / 0.148 with two.  A tile whose graphs all have at most 64
 // atoms works on word 0 alone in a batch of wider sets.
 constexpr uint32_t kAdmitWarps = 16;
 
@@ -494,7 +497,7 @@ int admit_launch(Queue* q, const Graph* data, const uint64_t* sig_all, const Adm
   // two graphs per lane: see k_planes_admit
   const uint32_t GW = (data->num_graphs + 31u) / 32u;
   if constexpr (AW == 1)
-    if (admit_smem_layout(v.K, AW, 2, GATHER, 0).total <= 110u * 1024u && GW >= 8u * static_cast<unsigned>(sms))
+    if (admit_smem_layout(v.K, AW, 2, GATHER, 0).total <= 110u * 1024u && GW >= 4u * static_cast<unsigned>(sms))
       return admit_launch_h<AW, GATHER, 2>(q, data, sig_all, v, rplanes, rrows, row_map, planes, admit, counts, sms);
   return admit_launch_h<AW, GATHER, 1>(q, data, sig_all, v, rplanes, rrows, row_map, planes, admit, counts, sms);
 }

@@ -116,10 +116,10 @@ def test_bond_label_join_sizes(qlo, qhi, dlo, dhi, count, prof, ff):
     assert len(idx) > 0 and np.array_equal(per, want_per) and int(total[0]) == want_total
 
 
-@pytest.mark.parametrize("count", [37_887, 37_888, 37_921, 40_033])
+@pytest.mark.parametrize("count", [18_912, 18_913, 18_945, 37_887, 37_888, 37_921, 40_033])
 @pytest.mark.parametrize("serve", [False, True])
 def test_admission_with_two_graphs_per_lane(count, serve):
-    """From 1,184 tiles of 32 graphs on, the admission carries two graphs per
+    """From 592 tiles of 32 graphs on, the admission carries two graphs per
     lane: tile counts on both sides, odd and even, ragged last tiles."""
     d = sb.generate_molecules(count, 3, 9, seed=3301)
     q = sb.generate_queries(10, 2, 6, seed=3302)
