@@ -149,3 +149,28 @@ def test_segment_offsets_by_graph_count(count):
     d = sb.generate_molecules(count, 8, 14, seed=3401)
     q = sb.generate_queries(6, 2, 4, seed=3402).concat(sb.io.parse(_graph(2, [(0, 1)], [1, 1]) + "\n"))
     _check(q, d, 1, "ref-ptx", True)
+
+
+@pytest.mark.parametrize("prof", ["ref-ptx", "exact"])
+@pytest.mark.parametrize("count", [1, 2, 9, 130, 1_111])
+def test_bit_sliced_signatures_by_vertex_count(count, prof):
+    """Refinement against the oracle's bitset after every pass: vertex counts
+    short of one word, of a word group and of a row's padding, and queries with
+    more thresholds than a block's table holds."""
+    d = sb.generate_molecules(count, 5, 40, seed=3501)
+    q = sb.generate_queries(24, 3, 20, seed=3502)
+    queue = sb.Queue(0, profile=prof)
+    qg, dg = sb.createDeviceCSRGraph(queue, q), sb.createDeviceCSRGraph(queue, d)
+    cand = sb.Candidates(queue, qg.total_nodes, dg.total_nodes)
+    sig = sb.Signature(queue, dg.total_nodes, qg.total_nodes)
+    sig.generateDataSignatures(dg)
+    sig.generateQuerySignatures(qg)
+    sb.filterCandidates(queue, qg, dg, sig, cand)
+    bits = oracle.filter_candidates(q, d)
+    assert np.array_equal(cand.getHostCandidates(), bits)
+    for r in range(1, 4):
+        sig.refineDataSignatures(dg, r)
+        sig.refineQuerySignatures(qg, r)
+        sb.refineCandidates(queue, qg, dg, sig, cand)
+        bits = oracle.refine_candidates(q, d, sig.getQuerySignatures(), sig.getDataSignatures(), bits)
+        assert np.array_equal(cand.getHostCandidates(), bits), r
