@@ -237,8 +237,11 @@ class ClockSampler:
             self.path.parent.mkdir(parents=True, exist_ok=True)
             self.f = open(self.path, "w")
             self.proc = subprocess.Popen(["nvidia-smi", f"--id={self.index}", f"--query-gpu={self.QUERY}", "--format=csv,noheader,nounits",
-                                          "-lms", "200"], stdout=self.f, stderr=subprocess.DEVNULL)
-            time.sleep(0.3)
+                                          "-lms", "50"], stdout=self.f, stderr=subprocess.DEVNULL)
+            # the timed region can be as short as 50 ms: it begins once samples arrive (5 s at most)
+            deadline = time.monotonic() + 5.0
+            while time.monotonic() < deadline and not self.path.stat().st_size:
+                time.sleep(0.02)
         except Exception:
             self.proc = None
         return self
