@@ -83,6 +83,7 @@ int dev_alloc(Queue* q, void** p, size_t bytes) {
 void dev_free(Queue* q, void* p) {
   if (p) cudaFreeAsync(p, q->stream);
 }
+DeviceBlock::~DeviceBlock() { dev_free(q, p); }
 
 namespace {
 // One pool per device for per-call temporaries; its release threshold is
@@ -755,7 +756,7 @@ int sigmo_gmcr_create(sigmo_queue_t q, sigmo_gmcr_t* out) {
 int sigmo_gmcr_destroy(sigmo_gmcr_t m) {
   if (!m) return SIGMO_OK;
   cudaSetDevice(m->q->device);
-  if (m->graph) cudaGraphExecDestroy(m->graph);
+  drop_graph(m);
   dev_free(m->q, m->offsets);
   dev_free(m->q, m->indices);
   dev_free(m->q, m->pair_graph);
@@ -768,11 +769,7 @@ int sigmo_gmcr_destroy(sigmo_gmcr_t m) {
 
 int sigmo_gmcr_generate(sigmo_gmcr_t m, sigmo_graph_t query, sigmo_graph_t data, sigmo_candidates_t c) {
   if (!m || !query || !data || !c) return fail(SIGMO_ERR_INVALID, "null argument");
-  if (m->graph) {  // the captured batch refers to the arrays this call may replace
-    cudaGraphExecDestroy(m->graph);
-    m->graph = nullptr;
-    for (auto& k : m->graph_key) k = 0;
-  }
+  drop_graph(m);  // the captured batch refers to the arrays this call may replace
   if (c->rows != query->total_nodes || c->targets != data->total_nodes)
     return fail(SIGMO_ERR_INVALID, "candidate bitset does not match the graphs");
   Queue* q = m->q;

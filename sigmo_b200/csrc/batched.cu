@@ -15,15 +15,12 @@
 namespace sigmo_b200 {
 namespace {
 
-void free_groups(Queue* q, PlaneProgram* pp) {
-  for (PlaneGroup& g : pp->groups) dev_free(q, g.blob);
+void free_groups(PlaneProgram* pp) {
   pp->groups.clear();
   pp->groups_aw = 0;
 }
 
 void free_program(Queue* q, PlaneProgram* pp) {
-  free_groups(q, pp);
-  dev_free(q, pp->blob);
   dev_free(q, pp->qsig_all);
   *pp = PlaneProgram{};
 }
@@ -92,13 +89,15 @@ struct Blob {
     return parts.size() - 1;
   }
   // On q->stream; ev_stage is recorded after the copy.
-  int send(Queue* q, void** block) {
+  int send(Queue* q, std::shared_ptr<DeviceBlock>* block) {
     void* host = nullptr;
     SIGMO_TRY(stage_buffer(q, bytes, &host));
     for (size_t i = 0; i < parts.size(); ++i)
       if (parts[i].second) std::memcpy(static_cast<char*>(host) + offs[i], parts[i].first, parts[i].second);
-    SIGMO_TRY(dev_alloc(q, block, bytes + 256));
-    dev = static_cast<char*>(*block);
+    void* p = nullptr;
+    SIGMO_TRY(dev_alloc(q, &p, bytes + 256));
+    *block = std::make_shared<DeviceBlock>(q, p);
+    dev = static_cast<char*>(p);
     SIGMO_CUDA_TRY(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, q->stream));
     SIGMO_CUDA_TRY(cudaEventRecord(q->ev_stage, q->stream));
     return SIGMO_OK;
@@ -327,7 +326,7 @@ int build_plane_program(Queue* q, Graph* query, uint32_t R) {
 int plan_groups(Queue* q, Graph* query, uint32_t AW) {
   PlaneProgram& pp = query->pp;
   if (pp.groups_aw == AW) return SIGMO_OK;
-  free_groups(q, &pp);
+  free_groups(&pp);
   if (planes_admit_smem(pp.K, AW) <= kGroupSmemBudget) {
     pp.groups_aw = AW;
     return SIGMO_OK;
@@ -568,13 +567,14 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
 
 namespace sigmo_b200 {
 
-namespace {
-
 void drop_graph(Gmcr* m) {
   if (m->graph) cudaGraphExecDestroy(m->graph);
   m->graph = nullptr;
+  m->graph_reads.clear();
   for (auto& k : m->graph_key) k = 0;
 }
+
+namespace {
 
 // Replays the captured batch: the device work of the planes route (no host
 // synchronisation inside), then the match total and the GMCR total to the
@@ -637,6 +637,10 @@ int capture_graph(Queue* q, Graph* query, Graph* data, uint32_t R, int find_firs
   }
   if (g) cudaGraphDestroy(g);
   cudaGetLastError();
+  if (!rc) {
+    m->graph_reads.push_back(query->pp.blob);
+    for (const PlaneGroup& grp : query->pp.groups) m->graph_reads.push_back(grp.blob);
+  }
   m->graph_launches = q->launches - launches0;
   q->launches = launches0;  // nothing ran during the capture
   m->counts_valid = true;   // the counts of the run before the capture are still in place

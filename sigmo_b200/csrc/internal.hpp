@@ -5,6 +5,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <memory>
 #include <vector>
 
 #include "common.hpp"
@@ -89,6 +90,16 @@ int join_status_reset(Queue* q);
 int join_status_fetch(Queue* q);
 int join_status_result(Queue* q);
 
+// Device memory with several owners, freed on the queue's stream by the last.
+struct DeviceBlock {
+  Queue* q;
+  void* p;
+  DeviceBlock(Queue* queue, void* ptr) : q(queue), p(ptr) {}
+  DeviceBlock(const DeviceBlock&) = delete;
+  DeviceBlock& operator=(const DeviceBlock&) = delete;
+  ~DeviceBlock();
+};
+
 // A contiguous range of query graphs whose planes fit one k_planes_admit
 // tile in shared memory (a batch too large for one tile is admitted group by
 // group).  Device arrays are in group-local plane ids; row_of maps a local
@@ -96,7 +107,7 @@ int join_status_result(Queue* q);
 struct PlaneGroup {
   uint32_t q0 = 0, q1 = 0;
   uint32_t K = 0, nlab = 0;
-  void* blob = nullptr;               // the device arrays below
+  std::shared_ptr<DeviceBlock> blob;  // the device arrays below
   const uint32_t* spec = nullptr;     // [K]
   const uint32_t* row_of = nullptr;   // [K] plane row in the batch
   const uint64_t* quads = nullptr;    // the group's query programs, local plane ids (PlaneProgram::quads)
@@ -112,7 +123,7 @@ struct PlaneProgram {
   uint32_t K = 0;                     // planes per data graph
   uint32_t C = 0;                     // classes of identical query vertices
   uint32_t nlab = 0;                  // label planes (spec[0 .. nlab))
-  void* blob = nullptr;               // the device arrays below
+  std::shared_ptr<DeviceBlock> blob;  // the device arrays below
   const uint32_t* spec = nullptr;     // [K] plane definitions
   // each class's program, four plane ids per entry (the last one repeated to
   // fill the last entry)
@@ -206,7 +217,13 @@ struct Gmcr {
   cudaGraphExec_t graph = nullptr;
   uint64_t graph_key[7] = {0, 0, 0, 0, 0, 0, 0};  // inputs, mode, profile, tuning, join budget
   uint64_t graph_launches = 0;  // kernels in the captured batch
+  // The query program blocks that the captured kernels read: the query graph may
+  // replace its program (another R, another set width) between replays.
+  std::vector<std::shared_ptr<DeviceBlock>> graph_reads;
 };
+
+// Gives up the captured batch and what it holds.
+void drop_graph(Gmcr* m);
 
 // Stage timing: every public stage brackets its launches with these.
 int stage_begin(Queue* q);
