@@ -215,7 +215,7 @@ struct Gmcr {
   bool counts_valid = false;
   // CUDA graph of the last batched match run in graph mode, and what it was built for
   cudaGraphExec_t graph = nullptr;
-  uint64_t graph_key[7] = {0, 0, 0, 0, 0, 0, 0};  // inputs, mode, profile, tuning, join budget
+  uint64_t graph_key[7] = {0, 0, 0, 0, 0, 0, 0};  // inputs, vertex base, mode, profile, tuning, join budget
   uint64_t graph_launches = 0;  // kernels in the captured batch
   // The query program blocks that the captured kernels read: the query graph may
   // replace its program (another R, another set width) between replays.

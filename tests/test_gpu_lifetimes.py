@@ -53,3 +53,24 @@ def test_replay_after_the_query_graph_was_grouped_for_another_set_width():
             res = sb.match_batched(queue, qg, dg[i], R, True, None, gm[i], graph=True)
             assert (res["ms_signatures"] == 0.0) == (call > 0)
             _equal(gm[i], res, want[i])
+
+
+def test_replay_after_the_shard_moved():
+    """The range masks and the literal join follow a shard's first global
+    vertex: a batch captured for one is not replayed for another."""
+    d, q = sb.generate_molecules(700, 10, 40, seed=3621), sb.generate_queries(40, 3, 12, seed=3622)
+    queue = sb.Queue(0)
+    qg, dg = sb.createDeviceCSRGraph(queue, q), sb.createDeviceCSRGraph(queue, d)
+    gm, totals = sb.GMCR(queue), []
+    for base in (0, 100_003, 100_017):
+        dg.set_vertex_base(base)
+        plain = sb.GMCR(queue)
+        want = sb.match_batched(queue, qg, dg, 4, False, None, plain)
+        for call in range(2):
+            res = sb.match_batched(queue, qg, dg, 4, False, None, gm, graph=True)
+            assert (res["ms_signatures"] == 0.0) == (call > 0)
+            assert res["total_matches"] == want["total_matches"] and res["admitted_pairs"] == want["admitted_pairs"]
+            assert all(np.array_equal(x, y) for x, y in zip(gm.getGMCR(), plain.getGMCR()))
+            assert np.array_equal(gm.getPairCounts(), plain.getPairCounts())
+        totals.append(want["total_matches"])
+    assert len(set(totals)) == 3
