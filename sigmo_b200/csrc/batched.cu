@@ -660,10 +660,10 @@ int match_batched(Queue* q, Graph* query, Graph* data, uint32_t R, int find_firs
     return fail(SIGMO_ERR_DOMAIN, "the batched form runs the REF_PTX and EXACT profiles; REF_X86 runs the stage-per-launch calls");
   SIGMO_CUDA_TRY(cudaSetDevice(q->device));
   const sigmo_tuning& tn = q->tune;
+  // (overflow_split has no effect on the device work)
   const uint64_t key[7] = {query->stamp, data->stamp, R | (static_cast<uint64_t>(data->vertex_base) << 32),
                            static_cast<uint64_t>(find_first),
                            static_cast<uint64_t>(q->opts.profile) | (static_cast<uint64_t>(tn.overflow_serial) << 8) |
-                               (static_cast<uint64_t>(tn.overflow_split) << 16) |
                                (static_cast<uint64_t>(tn.join_kernel) << 24) | (static_cast<uint64_t>(tn.join_pool) << 32),
                            (static_cast<uint64_t>(tn.join_blocks_per_sm) << 48) | (static_cast<uint64_t>(tn.join_chunk) << 40) |
                                (static_cast<uint64_t>(tn.mask_chunk_slots) << 32) | tn.overflow_blocks,

@@ -74,3 +74,14 @@ def test_replay_after_the_shard_moved():
             assert np.array_equal(gm.getPairCounts(), plain.getPairCounts())
         totals.append(want["total_matches"])
     assert len(set(totals)) == 3
+
+
+def test_replay_across_a_tuning_field_without_effect():
+    d, q = sb.generate_molecules(500, 10, 40, seed=3631), sb.generate_queries(20, 3, 20, seed=3632)
+    queue = sb.Queue(0)
+    qg, dg, gm = sb.createDeviceCSRGraph(queue, q), sb.createDeviceCSRGraph(queue, d), sb.GMCR(queue)
+    first = sb.match_batched(queue, qg, dg, 3, False, None, gm, graph=True)
+    for field, replays in (("overflow_split", True), ("overflow_blocks", False)):
+        queue.set_tuning(**{field: 5})
+        res = sb.match_batched(queue, qg, dg, 3, False, None, gm, graph=True)
+        assert (res["ms_signatures"] == 0.0) == replays and res["total_matches"] == first["total_matches"]
