@@ -374,7 +374,7 @@ int plan_groups(Queue* q, Graph* query, uint32_t AW) {
       q0 = qg;
     }
     take(qg);
-    if (planes_admit_smem(Kg, AW) > 200u * 1024u)
+    if (planes_admit_smem(Kg, AW) > kTileSmemLimit)
       return fail(SIGMO_ERR_DOMAIN, "query graph %u alone needs more than one admission tile of shared memory", qg);
   }
   ranges.emplace_back(q0, QG);
@@ -415,7 +415,7 @@ int plan_groups(Queue* q, Graph* query, uint32_t AW) {
       q_off.push_back(static_cast<uint32_t>(quads.size()));
     }
     grp.K = static_cast<uint32_t>(spec.size());
-    if (planes_admit_smem(grp.K, AW) > 200u * 1024u)
+    if (planes_admit_smem(grp.K, AW) > kTileSmemLimit)
       return fail(SIGMO_ERR_DOMAIN, "group %zu needs more than one admission tile of shared memory", gi);
     grp.nlab = nlab;
     grp.n_quads = quads.size();
@@ -493,9 +493,13 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
   const uint64_t b_dsig = run.dsig ? 0 : 8ull * R * N, b_planes = rp ? 0 : 8ull * G * pp.K * AW,
                  b_ne = 4ull * query->num_graphs * GW + 4ull * G;
   // resident planes: the batch's plane k is resident row row_map[k], and the
-  // class programs are rewritten as resident rows for the join
-  std::vector<uint32_t> row_map;
-  std::vector<uint64_t> rprog;
+  // class programs are rewritten as resident rows for the join.  Where the
+  // batch's planes exceed a tile, those with the same row (thresholds and labels
+  // that the database does not reach all have the zero row) become one plane of
+  // the tile, and the query programs follow: a tile then holds at most the
+  // database's rows, which were built to fit one.
+  std::vector<uint32_t> row_map, rq_off;
+  std::vector<uint64_t> rprog, rquads;
   if (rp) {
     if (rp->R != R) return fail(SIGMO_ERR_INVALID, "resident planes hold %u iterations, the batch asks for %u", rp->R, R);
     row_map.resize(pp.K);
@@ -513,8 +517,27 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
       const uint64_t x = pp.h_quads[i];
       for (int j = 0; j < 4; ++j) rprog[i] |= static_cast<uint64_t>(row_map[(x >> (16 * j)) & 0xFFFFu] & 0xFFFFu) << (16 * j);
     }
+    if (planes_admit_smem(pp.K, AW) > kTileSmemLimit) {
+      std::vector<uint32_t> tile_of(rp->rows, 0xFFFFFFFFu), rows;
+      for (uint32_t row : row_map)
+        if (tile_of[row] == 0xFFFFFFFFu) {
+          tile_of[row] = static_cast<uint32_t>(rows.size());
+          rows.push_back(row);
+        }
+      rq_off.push_back(0);
+      for (uint32_t qg = 0; qg < query->num_graphs; ++qg) {
+        for (uint32_t e = pp.order_off[qg]; e < pp.order_off[qg + 1]; ++e) {
+          const uint32_t b = pp.h_prog_off[pp.order[e]], n = pp.h_prog_off[pp.order[e] + 1] - b;
+          append_quads(n, [&](size_t i) { return tile_of[row_map[pp.h_prog[b + i]]]; }, &rquads);
+        }
+        rq_off.push_back(static_cast<uint32_t>(rquads.size()));
+      }
+      row_map = std::move(rows);
+    }
+    pp.gathered = static_cast<uint32_t>(row_map.size());
   }
-  const uint64_t b_map = al(4ull * row_map.size()) + 8ull * rprog.size();
+  const uint64_t b_rows = al(4ull * row_map.size()), b_rprog = al(8ull * rprog.size()), b_rquads = al(8ull * rquads.size());
+  const uint64_t b_map = b_rows + b_rprog + b_rquads + 4ull * rq_off.size();
   void* buf = nullptr;
   SIGMO_TRY(tmp_alloc(q, &buf, al(b_dsig) + al(b_planes) + al(b_ne) + al(b_map) + 256));
   char* p = static_cast<char*>(buf);
@@ -526,11 +549,17 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
   uint32_t* adm_counts = admit + static_cast<uint64_t>(query->num_graphs) * GW;
   p += al(b_ne);
   uint32_t* d_row_map = reinterpret_cast<uint32_t*>(p);
-  uint64_t* d_rprog = reinterpret_cast<uint64_t*>(p + al(4ull * row_map.size()));
+  uint64_t* d_rprog = reinterpret_cast<uint64_t*>(p + b_rows);
+  uint64_t* d_rquads = reinterpret_cast<uint64_t*>(p + b_rows + b_rprog);
+  uint32_t* d_rq_off = reinterpret_cast<uint32_t*>(p + b_rows + b_rprog + b_rquads);
   int rc = run.dsig ? SIGMO_OK : launch_sig_all(q, data, R, dsig);
   if (!rc && rp) {
     if (cudaMemcpyAsync(d_row_map, row_map.data(), 4ull * row_map.size(), cudaMemcpyHostToDevice, q->stream) != cudaSuccess ||
         cudaMemcpyAsync(d_rprog, rprog.data(), 8ull * rprog.size(), cudaMemcpyHostToDevice, q->stream) != cudaSuccess)
+      rc = fail(SIGMO_ERR_CUDA, "H2D copy failed");
+    if (!rc && !rq_off.empty() &&
+        (cudaMemcpyAsync(d_rquads, rquads.data(), 8ull * rquads.size(), cudaMemcpyHostToDevice, q->stream) != cudaSuccess ||
+         cudaMemcpyAsync(d_rq_off, rq_off.data(), 4ull * rq_off.size(), cudaMemcpyHostToDevice, q->stream) != cudaSuccess))
       rc = fail(SIGMO_ERR_CUDA, "H2D copy failed");
   }
   if (!rc) rc = mark(1);
@@ -540,8 +569,11 @@ int batched_planes(Queue* q, Graph* query, Graph* data, uint32_t R, int find_fir
     for (size_t gi = 0; gi < pp.groups.size() && !rc; ++gi)
       rc = launch_planes_admit_group(q, query, data, dsig, pp.groups[gi], pp.K, planes, admit, adm_counts);
   } else if (!rc) {
-    rc = rp ? launch_planes_admit_resident(q, query, data, *rp, pp, d_row_map, admit, adm_counts)
-            : launch_planes_admit(q, query, data, dsig, pp, planes, admit, adm_counts);
+    rc = !rp              ? launch_planes_admit(q, query, data, dsig, pp, planes, admit, adm_counts)
+         : rq_off.empty() ? launch_planes_admit_resident(q, query, data, *rp, pp.gathered, pp.quads, pp.n_quads, pp.q_off,
+                                                         d_row_map, admit, adm_counts)
+                          : launch_planes_admit_resident(q, query, data, *rp, pp.gathered, d_rquads, rquads.size(), d_rq_off,
+                                                         d_row_map, admit, adm_counts);
   }
   if (!rc) rc = mark(2);
   // captured: the admitted total of the run that built the graph sizes the
@@ -702,11 +734,11 @@ int match_batched(Queue* q, Graph* query, Graph* data, uint32_t R, int find_firs
   // tile (larger batches are admitted in groups); planes take 8 B per
   // (plane, graph, word) in device memory
   const size_t tile_bytes = planes_admit_smem(query->pp.K, data->adj_words);
-  // (resident planes are gathered for the whole batch as long as they fit a tile)
-  const int prc = run.resident && tile_bytes <= 200u * 1024u ? SIGMO_OK : plan_groups(q, query, data->adj_words);
+  // (resident planes: a tile holds at most the database's rows, whatever the batch)
+  const int prc = run.resident ? SIGMO_OK : plan_groups(q, query, data->adj_words);
   // SIGMO_ERR_DOMAIN: a query graph too large for a tile, bitset route
   if (prc && prc != SIGMO_ERR_DOMAIN) rc = prc;
-  const bool planes_fit = !prc && (!query->pp.groups.empty() || tile_bytes <= 200u * 1024u);
+  const bool planes_fit = run.resident || (!prc && (!query->pp.groups.empty() || tile_bytes <= kTileSmemLimit));
   const bool bitset_route = materialize || !planes_fit;
   if (!rc && bitset_route && data->vertex_base)
     rc = fail(SIGMO_ERR_DOMAIN, "a shard (vertex base %u) runs on the planes route only; this batch needs the bitset route",

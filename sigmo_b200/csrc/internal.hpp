@@ -136,6 +136,7 @@ struct PlaneProgram {
   const uint64_t* quads = nullptr;
   const uint32_t* q_off = nullptr;    // [query graphs + 1] entries of quads
   size_t n_quads = 0;
+  uint32_t gathered = 0;              // planes of the last run's admission tile when gathered from resident planes
   // host copies; order[order_off[q] .. order_off[q + 1]): query graph q's
   // distinct classes in evaluation order
   std::vector<uint32_t> h_spec, h_prog_off, order, order_off;
@@ -313,10 +314,14 @@ int launch_planes_admit_group(Queue* q, const Graph* query, const Graph* data, c
                               uint32_t K_total, uint64_t* planes, uint32_t* admit, uint32_t* counts);
 // Shared memory of one k_planes_admit tile budgeted for a query group's planes.
 constexpr size_t kGroupSmemBudget = 96u * 1024u;
-// The same admission with the tile's planes gathered from resident planes
-// (row_map[k] = resident row of the batch's plane k).
-int launch_planes_admit_resident(Queue* q, const Graph* query, const Graph* data, const ResidentPlanes& rp,
-                                 const PlaneProgram& pp, const uint32_t* row_map, uint32_t* admit, uint32_t* counts);
+// Planes of one tile at most (the kernel's tests or row map come on top).
+constexpr size_t kTileSmemLimit = 200u * 1024u;
+// The same admission with the tile's K planes gathered from resident planes
+// (row_map[k] = resident row of the tile's plane k; the query programs quads,
+// q_off in the tile's plane ids).
+int launch_planes_admit_resident(Queue* q, const Graph* query, const Graph* data, const ResidentPlanes& rp, uint32_t K,
+                                 const uint64_t* quads, size_t n_quads, const uint32_t* q_off, const uint32_t* row_map,
+                                 uint32_t* admit, uint32_t* counts);
 // Shared memory of a tile of 32 graphs and K planes.
 size_t planes_admit_smem(uint32_t K, uint32_t AW);
 // GMCR from admission words admit[query graph][data graph / 32] and the

@@ -533,10 +533,11 @@ int launch_planes_admit_group(Queue* q, const Graph* query, const Graph* data, c
   }
 }
 
-int launch_planes_admit_resident(Queue* q, const Graph* query, const Graph* data, const ResidentPlanes& rp,
-                                 const PlaneProgram& pp, const uint32_t* row_map, uint32_t* admit, uint32_t* counts) {
+int launch_planes_admit_resident(Queue* q, const Graph* query, const Graph* data, const ResidentPlanes& rp, uint32_t K,
+                                 const uint64_t* quads, size_t n_quads, const uint32_t* q_off, const uint32_t* row_map,
+                                 uint32_t* admit, uint32_t* counts) {
   if (!data->num_graphs) return SIGMO_OK;
-  const AdmitView v = whole_batch(query, pp);
+  const AdmitView v{K, 0, query->num_graphs, nullptr, q_off, nullptr, quads, n_quads, 0, 0};
   switch (data->adj_words) {
     case 1: return admit_launch<1, true>(q, data, nullptr, v, rp.planes, rp.rows, row_map, nullptr, admit, counts);
     case 2: return admit_launch<2, true>(q, data, nullptr, v, rp.planes, rp.rows, row_map, nullptr, admit, counts);
@@ -591,7 +592,7 @@ int build_resident_planes(Queue* q, Graph* data, const uint64_t* sig_all, uint32
   out->rows = K + 1;
   out->R = R;
   const size_t smem = static_cast<size_t>(K) * (AW * 32 * 8 + 8);
-  if (static_cast<size_t>(K) * AW * 32 * 8 > 200u * 1024u) return fail(SIGMO_ERR_DOMAIN, "the database needs %u resident planes (too many for one tile)", K);
+  if (planes_admit_smem(K, AW) > kTileSmemLimit) return fail(SIGMO_ERR_DOMAIN, "the database needs %u resident planes (too many for one tile)", K);
   void* dspec = nullptr;
   SIGMO_TRY(dev_alloc(q, &dspec, 4ull * K));
   int rc = SIGMO_OK;

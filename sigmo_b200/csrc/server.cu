@@ -282,7 +282,7 @@ void Server::run_batch(Worker* w, std::vector<Request*>& batch) {
     run.nranges = static_cast<uint32_t>(batch.size());
     note(match_batched(q, qg, data, so.iterations, so.find_first, false, nullptr, w->m, &mr, run));
     if (!rc && rp.planes)
-      gathered = 8ull * ((data->num_graphs + 31ull) / 32ull) * 32ull * qg->pp.K * data->adj_words;
+      gathered = 8ull * ((data->num_graphs + 31ull) / 32ull) * 32ull * qg->pp.gathered * data->adj_words;
   }
   // per-query totals (and the matched pairs when a request asked for them)
   if (!rc && QG) {
