@@ -499,16 +499,28 @@ int launch_graph_derive(Graph* g) {
 int launch_query_order(Graph* g) {
   Queue* q = g->q;
   if (g->qorder) return SIGMO_OK;
-  SIGMO_TRY(dev_alloc(q, reinterpret_cast<void**>(&g->qorder), g->total_nodes ? g->total_nodes : 1));
-  SIGMO_TRY(dev_alloc(q, reinterpret_cast<void**>(&g->qsel), sizeof(uint64_t) * (g->total_nodes ? g->total_nodes : 1)));
-  SIGMO_TRY(dev_alloc(q, reinterpret_cast<void**>(&g->qsel_id), sizeof(uint64_t) * (g->total_nodes ? g->total_nodes : 1)));
-  SIGMO_TRY(dev_alloc(q, reinterpret_cast<void**>(&g->qmeta), 32ull * (g->num_graphs ? g->num_graphs : 1)));
-  SIGMO_TRY(dev_alloc(q, reinterpret_cast<void**>(&g->qmeta_id), 32ull * (g->num_graphs ? g->num_graphs : 1)));
-  if (g->num_graphs && g->adj_words == 1) {
+  // the graph takes the arrays once all of them are there and filled: a call
+  // that ran short of memory is made again as if it had not been made
+  const uint64_t N = g->total_nodes ? g->total_nodes : 1, G = g->num_graphs ? g->num_graphs : 1;
+  void* p[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // qorder, qsel, qsel_id, qmeta, qmeta_id
+  const uint64_t bytes[5] = {N, 8 * N, 8 * N, 32 * G, 32 * G};
+  int rc = SIGMO_OK;
+  for (int i = 0; i < 5 && !rc; ++i) rc = dev_alloc(q, &p[i], bytes[i]);
+  if (!rc && g->num_graphs && g->adj_words == 1) {
     k_query_order<<<grid_for(32ull * g->num_graphs, 128, 4096u), 128, 0, q->stream>>>(
-        g->num_graphs, g->graph_offsets, g->adj, g->qorder, g->qsel, g->qsel_id, g->qmeta, g->qmeta_id);
-    SIGMO_TRY(check_launch(q, "k_query_order"));
+        g->num_graphs, g->graph_offsets, g->adj, static_cast<uint8_t*>(p[0]), static_cast<uint64_t*>(p[1]),
+        static_cast<uint64_t*>(p[2]), static_cast<uint16_t*>(p[3]), static_cast<uint16_t*>(p[4]));
+    rc = check_launch(q, "k_query_order");
   }
+  if (rc) {
+    for (void* x : p) dev_free(q, x);
+    return rc;
+  }
+  g->qorder = static_cast<uint8_t*>(p[0]);
+  g->qsel = static_cast<uint64_t*>(p[1]);
+  g->qsel_id = static_cast<uint64_t*>(p[2]);
+  g->qmeta = static_cast<uint16_t*>(p[3]);
+  g->qmeta_id = static_cast<uint16_t*>(p[4]);
   return SIGMO_OK;
 }
 

@@ -1,5 +1,8 @@
 """Calls at the limits of a tile, of device memory and of the forms' sizes:
 served, and with the oracle's results (whole numbers: equal)."""
+import contextlib
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -28,6 +31,76 @@ def _thresholds(q, R):
         sig = oracle.refine_signatures(q, r, oracle.REF_PTX, sig, reach)
         out.update((r, l, (v >> (4 * l)) & 15) for v in sig.tolist() for l in range(16) if (v >> (4 * l)) & 15)
     return out
+
+
+class _PoolProps(ctypes.Structure):  # CUmemPoolProps
+    _fields_ = [("alloc_type", ctypes.c_int), ("handle_types", ctypes.c_int), ("location_type", ctypes.c_int),
+                ("location_id", ctypes.c_int), ("security", ctypes.c_void_p), ("max_size", ctypes.c_size_t),
+                ("usage", ctypes.c_ushort), ("reserved", ctypes.c_ubyte * 54)]
+
+
+@contextlib.contextmanager
+def _short_of_memory(free):
+    """Stream-ordered allocations come from a pool of 64 MB of which about
+    `free` MB are left."""
+    cu = ctypes.CDLL("libcuda.so.1")
+    ok = lambda rc: rc == 0 or pytest.fail(f"CUDA driver error {rc}")  # noqa: E731
+    before, pool = ctypes.c_void_p(), ctypes.c_void_p()
+    ok(cu.cuDeviceGetMemPool(ctypes.byref(before), 0))
+    ok(cu.cuMemPoolCreate(ctypes.byref(pool), ctypes.byref(_PoolProps(1, 0, 1, 0, None, 64 << 20, 0))))
+    blocks = []
+    while len(blocks) < 1024:
+        p = ctypes.c_uint64()
+        if cu.cuMemAllocFromPoolAsync(ctypes.byref(p), ctypes.c_size_t(1 << 20), pool, None):
+            break
+        blocks.append(p)
+    assert free < len(blocks) < 1024
+    for _ in range(free):
+        ok(cu.cuMemFreeAsync(blocks.pop(), None))
+    ok(cu.cuStreamSynchronize(None))
+    ok(cu.cuDeviceSetMemPool(0, pool))
+    try:
+        yield
+    finally:
+        ok(cu.cuDeviceSetMemPool(0, before))
+        for p in blocks:
+            ok(cu.cuMemFreeAsync(p, None))
+        ok(cu.cuStreamSynchronize(None))
+        ok(cu.cuMemPoolDestroy(pool))
+
+
+def _filtered(queue, qg, dg, R):
+    cand = sb.Candidates(queue, qg.total_nodes, dg.total_nodes)
+    sig = sb.Signature(queue, dg.total_nodes, qg.total_nodes)
+    sig.generateDataSignatures(dg)
+    sig.generateQuerySignatures(qg)
+    sb.filterCandidates(queue, qg, dg, sig, cand)
+    for r in range(1, R + 1):
+        sig.refineDataSignatures(dg, r)
+        sig.refineQuerySignatures(qg, r)
+        sb.refineCandidates(queue, qg, dg, sig, cand)
+    queue.wait()
+    return cand
+
+
+def test_join_after_the_matching_order_ran_out_of_memory():
+    """The matching order's first array fits, its second does not: the call
+    fails, and the next one starts over."""
+    d, q = sb.generate_molecules(20, 10, 40, seed=3711), sb.generate_queries(60_000, 4, 14, seed=3712)
+    assert q.total_nodes * 8 > 3 << 20 > q.total_nodes
+    ref = oracle.run_pipeline(q, d, 2, oracle.REF_PTX, True)
+    queue = sb.Queue(0)
+    qg, dg = sb.createDeviceCSRGraph(queue, q), sb.createDeviceCSRGraph(queue, d)
+    cand = _filtered(queue, qg, dg, 2)
+    gm = sb.GMCR(queue)
+    gm.generateGMCR(qg, dg, cand)
+    with _short_of_memory(3):
+        with pytest.raises(sb.SigmoError) as ei:
+            sb.joinCandidates(queue, qg, dg, cand, gm, np.zeros(1, np.uint64), True)
+        assert ei.value.code == 3
+    total = np.zeros(1, np.uint64)
+    _, per = sb.joinCandidates(queue, qg, dg, cand, gm, total, True, per_pair=True)
+    assert np.array_equal(per, ref["per_pair"]) and int(total[0]) == ref["total"]
 
 
 @pytest.mark.parametrize("wide", [False, True])
