@@ -380,6 +380,10 @@ int launch_gmcr_from_admit(Queue* q, const Graph* query, const Graph* data, cons
                                                                                 m->pair_graph, m->capacity);
     rc = check_launch(q, "k_gmcr_fill");
   }
+  if (rc) {  // no mapping: the calls that read one refuse it
+    m->total = 0;
+    m->num_data_graphs = 0;
+  }
   dev_free(q, cub_tmp);
   return rc;
 }

@@ -39,15 +39,19 @@ class _PoolProps(ctypes.Structure):  # CUmemPoolProps
                 ("usage", ctypes.c_ushort), ("reserved", ctypes.c_ubyte * 54)]
 
 
+_small_pool = ctypes.c_void_p()  # kept: objects that outlive a test may hold memory of it
+
+
 @contextlib.contextmanager
 def _short_of_memory(free):
     """Stream-ordered allocations come from a pool of 64 MB of which about
     `free` MB are left."""
     cu = ctypes.CDLL("libcuda.so.1")
     ok = lambda rc: rc == 0 or pytest.fail(f"CUDA driver error {rc}")  # noqa: E731
-    before, pool = ctypes.c_void_p(), ctypes.c_void_p()
+    before, pool = ctypes.c_void_p(), _small_pool
     ok(cu.cuDeviceGetMemPool(ctypes.byref(before), 0))
-    ok(cu.cuMemPoolCreate(ctypes.byref(pool), ctypes.byref(_PoolProps(1, 0, 1, 0, None, 64 << 20, 0))))
+    if not pool:
+        ok(cu.cuMemPoolCreate(ctypes.byref(pool), ctypes.byref(_PoolProps(1, 0, 1, 0, None, 64 << 20, 0))))
     blocks = []
     while len(blocks) < 1024:
         p = ctypes.c_uint64()
@@ -66,7 +70,6 @@ def _short_of_memory(free):
         for p in blocks:
             ok(cu.cuMemFreeAsync(p, None))
         ok(cu.cuStreamSynchronize(None))
-        ok(cu.cuMemPoolDestroy(pool))
 
 
 def _filtered(queue, qg, dg, R):
@@ -99,6 +102,29 @@ def test_join_after_the_matching_order_ran_out_of_memory():
             sb.joinCandidates(queue, qg, dg, cand, gm, np.zeros(1, np.uint64), True)
         assert ei.value.code == 3
     total = np.zeros(1, np.uint64)
+    _, per = sb.joinCandidates(queue, qg, dg, cand, gm, total, True, per_pair=True)
+    assert np.array_equal(per, ref["per_pair"]) and int(total[0]) == ref["total"]
+
+
+def test_join_after_the_mapping_ran_out_of_memory():
+    """A mapping whose arrays did not all fit is refused by the join."""
+    d, q = sb.generate_molecules(20, 10, 40, seed=3711), sb.generate_queries(60_000, 4, 14, seed=3712)
+    ref = oracle.run_pipeline(q, d, 2, oracle.REF_PTX, True)
+    assert len(ref["indices"]) * 16 > 3 << 20 > len(ref["indices"]) * 4
+    queue = sb.Queue(0)
+    qg, dg = sb.createDeviceCSRGraph(queue, q), sb.createDeviceCSRGraph(queue, d)
+    cand = _filtered(queue, qg, dg, 2)
+    gm, total = sb.GMCR(queue), np.zeros(1, np.uint64)
+    with _short_of_memory(3):
+        with pytest.raises(sb.SigmoError) as ei:
+            gm.generateGMCR(qg, dg, cand)
+        assert ei.value.code == 3
+    with pytest.raises(sb.SigmoError) as ei:
+        sb.joinCandidates(queue, qg, dg, cand, gm, total, True)
+    assert ei.value.code == 1 and int(total[0]) == 0
+    gm.generateGMCR(qg, dg, cand)
+    off, idx = gm.getGMCR()
+    assert np.array_equal(off, ref["offsets"]) and np.array_equal(idx, ref["indices"])
     _, per = sb.joinCandidates(queue, qg, dg, cand, gm, total, True, per_pair=True)
     assert np.array_equal(per, ref["per_pair"]) and int(total[0]) == ref["total"]
 
