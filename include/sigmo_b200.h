@@ -299,7 +299,15 @@ SIGMO_API int sigmo_gmcr_generate_noalloc(sigmo_queue_t q, sigmo_graph_t query, 
 /* Adds the number of matches to *num_matches (host, caller-zeroed, like the
  * reference's USM counter, sigmo.cpp:145-146).  find_first: at most one match
  * per (query, data graph) pair.  per_pair (nullable, host) receives the count
- * of every GMCR slot (total_query_indices entries). */
+ * of every GMCR slot (total_query_indices entries).
+ * Device memory beside the arguments, for the call: level masks of up to
+ * sigmo_tuning.mask_chunk_slots slots at a time, 144 bytes each (two such
+ * buffers when there are more slots), and 4 bytes per slot for each of two
+ * lists when the queries reach 11 vertices or the pairs need wider sets.
+ * Where that does not fit the slots are joined in smaller runs, down to 4,096
+ * of them (0.6 MB).  The memory comes from the pool of per-call temporaries,
+ * which keeps it for later calls and gives it back when another allocation of
+ * the library does not fit. */
 SIGMO_API int sigmo_join_candidates(sigmo_queue_t q, sigmo_graph_t query, sigmo_graph_t data, sigmo_candidates_t c,
                           sigmo_gmcr_t m, uint64_t* num_matches, int find_first, uint64_t* per_pair);
 /* joinWildcardCandidates (isomorphism.hpp:435-560, with defineMatchingOrder

@@ -68,23 +68,6 @@ int stage_end(Queue* q) {
   return SIGMO_OK;
 }
 
-int dev_alloc(Queue* q, void** p, size_t bytes) {
-  *p = nullptr;
-  if (bytes == 0) bytes = 1;
-  cudaError_t e = cudaMallocAsync(p, bytes, q->stream);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    *p = nullptr;
-    return fail(e == cudaErrorMemoryAllocation ? SIGMO_ERR_OOM : SIGMO_ERR_CUDA, "device allocation of %zu bytes failed: %s",
-                bytes, cudaGetErrorString(e));
-  }
-  return SIGMO_OK;
-}
-void dev_free(Queue* q, void* p) {
-  if (p) cudaFreeAsync(p, q->stream);
-}
-DeviceBlock::~DeviceBlock() { dev_free(q, p); }
-
 namespace {
 // One pool per device for per-call temporaries; its release threshold is
 // unlimited, so freed blocks stay mapped for the next call.
@@ -109,23 +92,52 @@ int tmp_pool(int device, cudaMemPool_t* out) {
   *out = pool;
   return SIGMO_OK;
 }
+
+// Both pools keep what was freed to them (the device's own one too, see
+// sigmo_queue_create): unused memory of one is given back when an allocation
+// from the other does not fit.
+void release_unused(Queue* q) {
+  cudaStreamSynchronize(q->stream);  // the frees queued so far
+  cudaMemPool_t pool = nullptr;
+  if (tmp_pool(q->device, &pool) == SIGMO_OK) cudaMemPoolTrimTo(pool, 0);
+  if (cudaDeviceGetMemPool(&pool, q->device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+  cudaGetLastError();
+}
+
+// `pool` null: the device's current one.
+int alloc_from(Queue* q, cudaMemPool_t pool, void** p, size_t bytes) {
+  if (bytes == 0) bytes = 1;
+  cudaError_t e = cudaSuccess;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    *p = nullptr;
+    e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, q->stream) : cudaMallocAsync(p, bytes, q->stream);
+    if (e == cudaSuccess) return SIGMO_OK;
+    cudaGetLastError();
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (attempt || e != cudaErrorMemoryAllocation || cudaStreamIsCapturing(q->stream, &cs) != cudaSuccess ||
+        cs != cudaStreamCaptureStatusNone)
+      break;
+    release_unused(q);
+  }
+  *p = nullptr;
+  return fail(e == cudaErrorMemoryAllocation ? SIGMO_ERR_OOM : SIGMO_ERR_CUDA, "device allocation of %zu bytes failed: %s", bytes,
+              cudaGetErrorString(e));
+}
 }  // namespace
 
+int dev_alloc(Queue* q, void** p, size_t bytes) { return alloc_from(q, nullptr, p, bytes); }
+void dev_free(Queue* q, void* p) {
+  if (p) cudaFreeAsync(p, q->stream);
+}
+DeviceBlock::~DeviceBlock() { dev_free(q, p); }
+
 int tmp_alloc(Queue* q, void** p, size_t bytes) {
+  *p = nullptr;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   SIGMO_CUDA_TRY(cudaStreamIsCapturing(q->stream, &cs));
-  if (cs != cudaStreamCaptureStatusNone) return dev_alloc(q, p, bytes);
-  *p = nullptr;
   cudaMemPool_t pool = nullptr;
-  SIGMO_TRY(tmp_pool(q->device, &pool));
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, q->stream);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    *p = nullptr;
-    return fail(e == cudaErrorMemoryAllocation ? SIGMO_ERR_OOM : SIGMO_ERR_CUDA, "device allocation of %zu bytes failed: %s",
-                bytes, cudaGetErrorString(e));
-  }
-  return SIGMO_OK;
+  if (cs == cudaStreamCaptureStatusNone) SIGMO_TRY(tmp_pool(q->device, &pool));
+  return alloc_from(q, pool, p, bytes);
 }
 int queue_scratch(Queue* q, size_t bytes, void** p) {
   if (bytes > q->scratch_bytes) {

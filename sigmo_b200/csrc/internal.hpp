@@ -298,6 +298,8 @@ int launch_join_wildcard(Queue* q, const Graph* query, const Graph* data, const 
 // count does not depend on the order of its search).
 int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first, uint32_t skip,
                       uint64_t* d_total);
+// Device memory that it takes for `slots` pairs at once (less where that is short).
+uint64_t join_pairs_bytes(const Queue* q, const Graph* query, const Graph* data, uint64_t slots);
 // Every pair: the literal join of data graphs [0, literal) on the side stream
 // (once per range of query graphs when `ranges` holds nranges + 1 boundaries),
 // beside launch_join_pairs for the rest; the main stream waits for both.

@@ -1207,7 +1207,7 @@ __global__ void __launch_bounds__(256) k_pair_masks(
       const bool lng = !generic && n > kDfsLevels;
       rec[local] = make_uint4(ds, n | (ident ? 0x100u : 0u) | (generic ? 0x200u : 0u) | (lng ? 0x400u : 0u) |
                                       (g < skip_below ? 0x800u : 0u), qoff, qg);
-      if (lng && g >= skip_below) {  // joined by k_join_dfs's long form, in parts
+      if (longs && lng && g >= skip_below) {  // joined by k_join_dfs's long form, in parts
         longs[atomicAdd(longs_len, 1ull)] = static_cast<uint32_t>(slot);
         counts[slot] = 0;
       }
@@ -1984,42 +1984,64 @@ int launch_join_wildcard(Queue* q, const Graph* query, const Graph* data, const 
   return rc;
 }
 
-int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first, uint32_t skip,
-                      uint64_t* d_total) {
-  if (!m->total) return SIGMO_OK;
-  if (query->max_nodes > kMaxQueryNodes)
-    return fail(SIGMO_ERR_DOMAIN, "query graphs of up to %u vertices are supported (largest: %u)", kMaxQueryNodes, query->max_nodes);
+namespace {
+
+// Device memory of the pair join for `slots` slots.
+struct PairScratch {
+  void *buf = nullptr, *mbuf[2] = {nullptr, nullptr};
+  uint64_t chunk = 0;  // slots per mask buffer
+  bool two = false;    // several chunks: two mask buffers
+  bool has_long = false, has_overflow = false;
+  size_t lists = 0;    // counters, overflow list, long-pair lists
+  size_t masks = 0;    // one mask buffer
+};
+PairScratch pair_scratch(const sigmo_tuning& tn, uint32_t query_nodes, uint32_t data_nodes, uint64_t slots) {
+  PairScratch p;
+  p.chunk = std::min<uint64_t>(slots, static_cast<uint64_t>(tn.mask_chunk_slots) << 20);
+  p.two = slots > p.chunk;
+  p.has_long = tn.join_kernel == 2 && query_nodes > kDfsLevels;
+  p.has_overflow = query_nodes > kPhaseLevels || data_nodes > 64u;
+  p.lists = 256 + (p.has_overflow ? 4ull * slots : 0) + (p.has_long ? 4ull * p.chunk * (p.two ? 2 : 1) : 0);
+  p.masks = 8ull * kPhaseLevels * p.chunk + 16ull * p.chunk;
+  return p;
+}
+
+int alloc_scratch(Queue* q, PairScratch* p) {
+  int rc = tmp_alloc(q, &p->buf, p->lists);
+  if (!rc) rc = tmp_alloc(q, &p->mbuf[0], p->masks);
+  if (!rc && p->two) rc = tmp_alloc(q, &p->mbuf[1], p->masks);
+  if (rc) {
+    dev_free(q, p->mbuf[0]);
+    dev_free(q, p->buf);
+  }
+  return rc;
+}
+
+// The pairs in slots [first, first + slots); frees the scratch.
+int join_slots(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first, uint32_t skip,
+               uint64_t* d_total, uint64_t first, uint64_t slots, const PairScratch& sc) {
   const bool exact = q->opts.profile == kProfileExact;
-  SIGMO_TRY(launch_query_order(const_cast<Graph*>(query)));
   const sigmo_tuning& tn = q->tune;
-  const uint64_t chunk = std::min<uint64_t>(m->total, static_cast<uint64_t>(tn.mask_chunk_slots) << 20);
-  void* buf = nullptr;
-  SIGMO_TRY(tmp_alloc(q, &buf, 256 + 4ull * m->total + 8ull * chunk));
+  void *buf = sc.buf, *mbuf[2] = {sc.mbuf[0], sc.mbuf[1]};
+  const uint64_t chunk = sc.chunk;
+  // several chunks: even ones on the main stream, odd ones on the aux stream,
+  // each stream with its own mask buffer and work cursor, so one chunk's level
+  // masks run beside the previous chunk's persistent join
+  const bool two = sc.two, has_long = sc.has_long, has_overflow = sc.has_overflow;
   // [0] work cursor of the even chunks, [1] generic-join cursor, [2] overflow
   // length, [3] odd chunks' cursor; then per chunk parity the long pairs'
   // list length [4 + 2 i] and cursor [5 + 2 i]
   auto* ctr = static_cast<unsigned long long*>(buf);
   uint32_t* overflow = reinterpret_cast<uint32_t*>(static_cast<char*>(buf) + 256);
-  uint32_t* longs = overflow + m->total;  // [2][chunk]
-  SIGMO_CUDA_TRY(cudaMemsetAsync(ctr, 0, 256, q->stream));
+  uint32_t* longs = has_long ? overflow + (has_overflow ? slots : 0) : nullptr;  // [two ? 2 : 1][chunk]
+  int rc = cudaMemsetAsync(ctr, 0, 256, q->stream) == cudaSuccess ? SIGMO_OK : fail(SIGMO_ERR_CUDA, "memset failed");
   auto* tot = reinterpret_cast<unsigned long long*>(d_total);
   // two-phase join, in chunks of slots, for the pairs of queries of <= 16
   // vertices and molecules of <= 64 atoms; the rest go to the overflow list
-  int rc = SIGMO_OK;
   const bool frontier = tn.join_kernel == 1, dfs = tn.join_kernel == 2;
-  const bool has_long = dfs && query->max_nodes > kDfsLevels;
-  const bool has_overflow = query->max_nodes > kPhaseLevels || data->max_nodes > 64u;
-  // several chunks: even ones on the main stream, odd ones on the aux stream,
-  // each stream with its own mask buffer and work cursor, so one chunk's level
-  // masks run beside the previous chunk's persistent join
-  const bool two = m->total > chunk;
   // the long pairs run beside the short ones
   const cudaStream_t long_stream = two ? q->side : q->aux;
   {
-    const size_t mbytes = 8ull * kPhaseLevels * chunk + 16ull * chunk;
-    void* mbuf[2] = {nullptr, nullptr};
-    rc = tmp_alloc(q, &mbuf[0], mbytes);
-    if (!rc && two) rc = tmp_alloc(q, &mbuf[1], mbytes);
     const cudaStream_t streams[2] = {q->stream, q->aux};
     if (!rc && two &&
         (cudaEventRecord(q->ev_aux_fork, q->stream) != cudaSuccess || cudaStreamWaitEvent(q->aux, q->ev_aux_fork, 0) != cudaSuccess))
@@ -2056,18 +2078,18 @@ int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const Mas
     const unsigned grid = static_cast<unsigned>(sms) * (dfs ? std::min(tn.join_blocks_per_sm, 3u) : tn.join_blocks_per_sm);
     // fewer pairs than lanes: every pair in up to 16 parts by root candidate
     uint32_t lparts = 0;
-    while (dfs && lparts < 4 && (m->total << (lparts + 1)) <= static_cast<uint64_t>(grid) * block) ++lparts;
+    while (dfs && lparts < 4 && (slots << (lparts + 1)) <= static_cast<uint64_t>(grid) * block) ++lparts;
     const uint32_t long_parts = find_first ? lparts : std::max(lparts, 1u);
     uint64_t c = 0;
-    for (uint64_t slot0 = 0; slot0 < m->total && !rc; slot0 += chunk, ++c) {
-      const uint64_t cnt = std::min<uint64_t>(chunk, m->total - slot0);
+    for (uint64_t slot0 = first; slot0 < first + slots && !rc; slot0 += chunk, ++c) {
+      const uint64_t cnt = std::min<uint64_t>(chunk, first + slots - slot0);
       const uint32_t par = c & 1;
       const cudaStream_t st = streams[par];
       auto* masks = static_cast<uint64_t*>(mbuf[par]);
       auto* recs = reinterpret_cast<uint4*>(masks + kPhaseLevels * chunk);
       unsigned long long* cursor = ctr + (par ? 3 : 0);
       unsigned long long* lctr = ctr + 4 + 2 * par;
-      uint32_t* llist = longs + par * chunk;
+      uint32_t* llist = has_long ? longs + par * chunk : nullptr;
       if (c >= 2 && (cudaMemsetAsync(cursor, 0, 8, st) != cudaSuccess || cudaMemsetAsync(lctr, 0, 16, st) != cudaSuccess))
         rc = fail(SIGMO_ERR_CUDA, "memset failed");
       if (rc) break;
@@ -2141,6 +2163,40 @@ int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const Mas
   if (side && cudaEventRecord(q->ev_join, q->side) == cudaSuccess) cudaStreamWaitEvent(q->stream, q->ev_join, 0);
   dev_free(q, buf);
   return rc;
+}
+
+// Smallest number of slots that the pair join is cut down to: 0.6 MB of masks.
+constexpr uint64_t kMinJoinSlots = 4096;
+
+}  // namespace
+
+uint64_t join_pairs_bytes(const Queue* q, const Graph* query, const Graph* data, uint64_t slots) {
+  const PairScratch sc = pair_scratch(q->tune, query->max_nodes, data->max_nodes, slots);
+  return sc.lists + sc.masks * (sc.two ? 2 : 1);
+}
+
+// All slots at once; where the device memory does not allow that, runs of half
+// as many one after the other, and so on.
+int launch_join_pairs(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first, uint32_t skip,
+                      uint64_t* d_total) {
+  if (!m->total) return SIGMO_OK;
+  if (query->max_nodes > kMaxQueryNodes)
+    return fail(SIGMO_ERR_DOMAIN, "query graphs of up to %u vertices are supported (largest: %u)", kMaxQueryNodes, query->max_nodes);
+  SIGMO_TRY(launch_query_order(const_cast<Graph*>(query)));
+  uint64_t run = m->total;
+  for (uint64_t first = 0; first < m->total;) {
+    const uint64_t slots = std::min(run, m->total - first);
+    PairScratch sc = pair_scratch(q->tune, query->max_nodes, data->max_nodes, slots);
+    const int rc = alloc_scratch(q, &sc);
+    if (rc == SIGMO_ERR_OOM && slots > kMinJoinSlots) {
+      run = std::max((slots + 1) / 2, kMinJoinSlots);
+      continue;
+    }
+    SIGMO_TRY(rc);
+    SIGMO_TRY(join_slots(q, query, data, src, m, find_first, skip, d_total, first, slots, sc));
+    first += slots;
+  }
+  return SIGMO_OK;
 }
 
 int launch_join(Queue* q, const Graph* query, const Graph* data, const MaskSource& src, Gmcr* m, int find_first, uint32_t literal,

@@ -2,6 +2,9 @@
 served, and with the oracle's results (whole numbers: equal)."""
 import contextlib
 import ctypes
+import subprocess
+import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -127,6 +130,61 @@ def test_join_after_the_mapping_ran_out_of_memory():
     assert np.array_equal(off, ref["offsets"]) and np.array_equal(idx, ref["indices"])
     _, per = sb.joinCandidates(queue, qg, dg, cand, gm, total, True, per_pair=True)
     assert np.array_equal(per, ref["per_pair"]) and int(total[0]) == ref["total"]
+
+
+_IN_LITTLE_MEMORY = """
+import sys
+import numpy as np
+import torch
+import sigmo_b200 as sb
+sys.path.insert(0, "tests")
+from test_gpu_limits import _filtered
+
+def stage_join(cand, gm, ff):
+    total = np.zeros(1, np.uint64)
+    return sb.joinCandidates(queue, qg, dg, cand, gm, total, ff, per_pair=True)[1], int(total[0])
+
+def fill(left):
+    torch.cuda.synchronize()
+    return torch.empty(torch.cuda.mem_get_info()[0] - (left << 20), dtype=torch.uint8, device="cuda")
+
+profile, long = sys.argv[1], sys.argv[2] == "long"
+queue = sb.Queue(0, profile=profile)
+hi = 30 if long else 9
+for count in (400, 30_000):  # the kernels are loaded before the memory is short
+    q = sb.generate_queries(300, 3, hi, seed=3722, skew_lo=6, skew_hi=min(hi, 15))
+    qg, dg = sb.createDeviceCSRGraph(queue, q), sb.createDeviceCSRGraph(queue, sb.generate_molecules(count, 10, 60, seed=3721))
+    cand, gm = _filtered(queue, qg, dg, 3), sb.GMCR(queue)
+    gm.generateGMCR(qg, dg, cand)
+    if count == 400:
+        stage_join(cand, gm, False)
+pairs = gm.total_query_indices
+assert pairs * 144 > 128 << 20, pairs  # the pair join's masks
+rest = fill(64)
+short = [stage_join(cand, gm, ff) for ff in (False, True)]
+del rest
+torch.cuda.empty_cache()
+plenty = sb.GMCR(queue)
+for (per, total), ff in zip(short, (False, True)):
+    res = sb.match_batched(queue, qg, dg, 3, ff, None, plenty)
+    assert np.array_equal(per, plenty.getPairCounts()) and total == res["total_matches"] > 0
+# what the temporaries kept is given back to an allocation that needs it
+rest = fill(64)
+more = sb.Candidates(queue, 1000, 8 * 100_000 * 8 // 5)
+print("ok", pairs)
+"""
+
+
+@pytest.mark.parametrize("queries", ["short", "long"])
+@pytest.mark.parametrize("profile", ["ref-ptx", "exact"])
+def test_stage_join_in_little_memory(profile, queries):
+    """The stage join beside its bitset, on a card that is otherwise full: runs
+    of fewer pairs, with the counts of the batched form.  In a process of its
+    own, whose memory pools hold nothing yet."""
+    root = Path(__file__).resolve().parent.parent
+    r = subprocess.run([sys.executable, "-c", _IN_LITTLE_MEMORY, profile, queries], cwd=root, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and r.stdout.startswith("ok"), r.stdout + r.stderr
 
 
 @pytest.mark.parametrize("wide", [False, True])
