@@ -145,22 +145,20 @@ struct Server {
 namespace {
 
 // Device footprint of a batch once its plane program is known: planes (none
-// when the database's planes are resident), the
-// non-empty matrix, the GMCR arrays for every (query, data graph) pair, the
-// join's per-chunk level masks and the result arrays.
-uint64_t projected_bytes(const Graph* query, const Graph* data, bool resident) {
+// when the database's planes are resident), admission words and counts, the
+// GMCR arrays for every (query, data graph) pair, the join's level masks and
+// lists for as many, the result arrays, and 16 MB for the query graphs, their
+// programs and scan storage.
+uint64_t projected_bytes(const Queue* q, const Graph* query, const Graph* data, bool resident) {
   const PlaneProgram& pp = query->pp;
   const uint64_t G = data->num_graphs, GW = (G + 31) / 32, QG = query->num_graphs;
   const uint64_t pairs = QG * G;
   const uint64_t planes = resident ? 0 : 8ull * GW * 32 * pp.K * data->adj_words;
-  const uint64_t ne = 4ull * pp.C * GW + 4ull * QG * GW;
+  const uint64_t admission = 4ull * QG * GW + 4ull * G;
   const uint64_t gmcr = 4ull * (G + 1) + pairs * (4 + 4 + 8);
-  // level masks + setup records per chunk of slots (two chunk buffers, one per
-  // stream, once the pairs exceed one chunk), and the overflow list
-  const uint64_t chunk = std::min<uint64_t>(pairs, 8ull << 20);
-  const uint64_t join = (pairs > chunk ? 2 : 1) * chunk * (8ull * 16 + 16) + 4ull * pairs;
+  const uint64_t join = join_pairs_bytes(q, query, data, pairs);
   const uint64_t results = pairs * (4 + 4 + 4 + 8);
-  return planes + ne + gmcr + join + results + (16ull << 20);
+  return planes + admission + gmcr + join + results + (16ull << 20);
 }
 
 }  // namespace
@@ -259,7 +257,7 @@ void Server::run_batch(Worker* w, std::vector<Request*>& batch) {
   if (!rc) note(build_plane_program(q, qg, so.iterations));
   // admission by the batch's projected device footprint
   if (!rc) {
-    const uint64_t need = projected_bytes(qg, data, rp.planes != nullptr);
+    const uint64_t need = projected_bytes(q, qg, data, rp.planes != nullptr);
     std::unique_lock<std::mutex> lk(mu);
     if (need > so.memory_budget) {
       note(fail(SIGMO_ERR_OOM, "batch of %llu query graphs needs %llu bytes, above the serving memory budget (%llu bytes)",

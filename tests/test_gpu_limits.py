@@ -215,3 +215,18 @@ def test_serving_a_batch_with_more_planes_than_a_tile(wide, profile):
             np.add.at(want, ref["indices"].astype(np.int64), ref["per_pair"])
             assert np.array_equal(total, want) and keep.any()
             assert np.array_equal(matched, np.bincount(ref["indices"][keep], minlength=request.num_graphs).astype(np.uint64))
+
+
+@pytest.mark.parametrize("hi,lists", [(10, 0), (16, 1), (30, 2)])
+def test_serving_estimate_holds_the_joins_lists(hi, lists):
+    """A batch's projected device bytes: mapping, level masks and, by the
+    queries' sizes, the lists of long and of wide pairs, for every pair, the
+    result lists and 16 MB."""
+    d = sb.generate_molecules(20_000, 10, 40, seed=3731)
+    q = sb.generate_queries(12, 3, 8, seed=3732).concat(sb.generate_queries(1, hi, hi, seed=3733))
+    assert q.sizes().max() == hi
+    pairs = d.num_graphs * q.num_graphs
+    with sb.Server(d, iterations=3, max_inflight=1) as srv:
+        projected = srv.wait(srv.submit(q))["projected_bytes"]
+    need = 4 * d.num_graphs + pairs * (16 + 144 + 4 * lists + 20) + (16 << 20)
+    assert need <= projected <= need + (1 << 20)
