@@ -26,15 +26,41 @@ namespace {
 // row, so nothing waits for the adjacency rows.  (Three kernels before, the
 // graph-per-thread ones with a serial chain per graph: 121 us for 100,000
 // molecules, 45 us for the two uploads of a small search; this one 67 and 11.)
-constexpr uint32_t kDeriveRange = 256;
+//
+// Looking an edge's reverse up costs the neighbour's degree, so a block with a
+// vertex of more than kDeriveDegree entries tests bits instead: it stages the
+// rows of all graphs that its vertices belong to (those of the first and the last
+// one that lie outside its range are built a second time) and a vertex looks its
+// own bit up in each neighbour's row.  Creation of 2,000 complete graphs of 256
+// vertices 8.4 -> 1.0 ms, 10,000 of 64 0.85 -> 0.16, 50,000 of 16 0.20 -> 0.14,
+// of 80,000 of 10 vertices 0.19 and 0.18 ms; molecules have no such vertex.
+constexpr uint32_t kDeriveRange = 256, kDeriveDegree = 8;
+
+// The local adjacency row of a vertex, CSR entries [i0, i1), of the graph
+// [prev, prev + n), into shared memory.
+template <int AW>
+__device__ __forceinline__ void stage_row(uint32_t i0, uint32_t i1, uint32_t prev, uint32_t n, const uint32_t* __restrict__ col,
+                                          uint64_t* row) {
+#pragma unroll
+  for (int k = 0; k < AW; ++k) row[k] = 0;
+  if (n > 64u * AW) n = 64u * AW;
+  for (uint32_t i = i0; i < i1; ++i) {
+    const uint32_t t = col[i] - prev;  // neighbours outside the graph set no bit
+    if (t < n) row[t >> 6] |= 1ull << (t & 63u);
+  }
+}
+
 template <int AW>
 __global__ void __launch_bounds__(kDeriveRange) k_graph_derive(uint64_t N, uint32_t G, const uint32_t* __restrict__ goff,
                                                                const uint32_t* __restrict__ roff,
                                                                const uint32_t* __restrict__ col,
                                                                uint32_t* __restrict__ node_graph, uint64_t* __restrict__ adj,
                                                                uint8_t* __restrict__ sym) {
+  constexpr uint32_t kMax = 64u * AW;  // vertices of a graph whose rows are complete
   __shared__ uint32_t s_off[kDeriveRange + 1];
   __shared__ uint32_t s_first;
+  __shared__ uint32_t s_lo, s_hi, s_last;  // staged vertices [s_lo, s_hi); first vertex of the last one's graph
+  __shared__ uint64_t s_rows[kDeriveRange + 2 * kMax][AW];
   for (uint64_t v0 = static_cast<uint64_t>(blockIdx.x) * kDeriveRange; v0 < N; v0 += static_cast<uint64_t>(gridDim.x) * kDeriveRange) {
     if (threadIdx.x < 32) {  // the last graph that starts at or before v0: in [lo, hi)
       uint32_t lo = 0, hi = G;
@@ -52,9 +78,9 @@ __global__ void __launch_bounds__(kDeriveRange) k_graph_derive(uint64_t N, uint3
     const uint32_t first = s_first, have = G - first < kDeriveRange ? G - first : kDeriveRange;  // graphs staged
     for (uint32_t i = threadIdx.x; i <= have; i += blockDim.x) s_off[i] = goff[first + i];
     __syncthreads();
-    const uint64_t v = v0 + threadIdx.x;
+    const uint64_t v = v0 + threadIdx.x, v1 = v0 + kDeriveRange < N ? v0 + kDeriveRange : N;
+    uint32_t g = 0, prev = 0, end = 0, i0 = 0, i1 = 0;
     if (v < N) {
-      uint32_t g, prev, end;
       if (s_off[have] > v) {
         uint32_t lo = 0, hi = have;  // the last staged graph that starts at or before v
         while (hi - lo > 1) {
@@ -76,18 +102,49 @@ __global__ void __launch_bounds__(kDeriveRange) k_graph_derive(uint64_t N, uint3
         prev = goff[g];
         end = goff[g + 1];
       }
-      const uint32_t n = end - prev;
+      i0 = roff[v];
+      i1 = roff[v + 1];
+    }
+    const uint32_t n = end - prev;
+    bool mirrored = n <= kMax && static_cast<uint32_t>(v) - prev < n && end <= N;
+    if (__syncthreads_or(i1 - i0 > kDeriveDegree)) {
+      if (v == v0) s_lo = mirrored ? prev : static_cast<uint32_t>(v0);
+      if (v + 1 == v1) {
+        s_hi = mirrored ? end : static_cast<uint32_t>(v1);
+        s_last = prev;
+      }
+      __syncthreads();
+      const uint32_t lo = s_lo, before = static_cast<uint32_t>(v0) - lo, after = s_hi - static_cast<uint32_t>(v1);
+      uint64_t* mine = s_rows[before + threadIdx.x];
+      if (v < N) stage_row<AW>(i0, i1, prev, n, col, mine);
+      // the vertices outside the range: of its first graph and of its last one
+      // (bits past a graph's end are not read)
+      for (uint32_t i = threadIdx.x; i < before + after; i += blockDim.x) {
+        const uint32_t u = i < before ? lo + i : static_cast<uint32_t>(v1) + (i - before);
+        stage_row<AW>(roff[u], roff[u + 1], i < before ? lo : s_last, kMax, col, s_rows[u - lo]);
+      }
+      __syncthreads();
+      if (v < N) {
+#pragma unroll
+        for (int k = 0; k < AW; ++k) {
+          const uint64_t bits = mine[k];
+          adj[v * AW + k] = bits;
+          for (uint64_t m = bits; m && mirrored; m &= m - 1) {
+            const uint32_t at = prev + 64u * k + __ffsll(static_cast<long long>(m)) - 1u - lo, me = static_cast<uint32_t>(v) - prev;
+            mirrored = at < s_hi - lo && ((s_rows[at][me >> 6] >> (me & 63u)) & 1ull);
+          }
+        }
+      }
+    } else if (v < N) {
       uint64_t row[AW];
 #pragma unroll
       for (int k = 0; k < AW; ++k) row[k] = 0;
-      bool mirrored = n <= 64u * AW;
-      const uint32_t i1 = roff[v + 1];
-      for (uint32_t i = roff[v]; i < i1; ++i) {
+      for (uint32_t i = i0; i < i1; ++i) {
         const uint32_t t = col[i] - prev;  // neighbours outside the graph set no bit
-        if (t >= n || t >= 64u * AW) continue;
+        if (t >= n || t >= kMax) continue;
+        const uint64_t bit = 1ull << (t & 63u);
 #pragma unroll
-        for (int k = 0; k < AW; ++k)
-          if ((t >> 6) == static_cast<uint32_t>(k)) row[k] |= 1ull << (t & 63u);
+        for (int k = 0; k < AW; ++k) row[k] |= (t >> 6) == static_cast<uint32_t>(k) ? bit : 0ull;
         if (mirrored) {
           const uint32_t j1 = roff[prev + t + 1];
           bool back = false;
@@ -95,9 +152,11 @@ __global__ void __launch_bounds__(kDeriveRange) k_graph_derive(uint64_t N, uint3
           mirrored = back;
         }
       }
-      node_graph[v] = g;
 #pragma unroll
       for (int k = 0; k < AW; ++k) adj[v * AW + k] = row[k];
+    }
+    if (v < N) {
+      node_graph[v] = g;
       if (!mirrored) sym[g] = 0;
     }
     __syncthreads();  // the offsets are no longer read

@@ -230,3 +230,40 @@ def test_serving_estimate_holds_the_joins_lists(hi, lists):
         projected = srv.wait(srv.submit(q))["projected_bytes"]
     need = 4 * d.num_graphs + pairs * (16 + 144 + 4 * lists + 20) + (16 << 20)
     assert need <= projected <= need + (1 << 20)
+
+
+def _dense(n, degree, seed, loops=()):
+    """A random graph; a vertex of `loops` gets a self-loop, whose second CSR
+    entry names vertex 0 (an edge that vertex 0 does not have back)."""
+    rng = np.random.default_rng(seed)
+    u, v = np.nonzero(np.triu(rng.random((n, n)) < degree / n, 1))
+    order = rng.permutation(len(u))
+    edges = [(int(u[i]), int(v[i])) for i in order] + [(x, x) for x in loops]
+    return _graph(n, edges, rng.choice([0, 7, 8], n).tolist())
+
+
+@pytest.mark.parametrize("profile", [oracle.REF_PTX, oracle.EXACT])
+@pytest.mark.parametrize("widest", [64, 128, 256])
+def test_graph_creation_by_degree_and_position(widest, profile):
+    """Adjacency rows and the mirrored flag (an unmirrored graph is joined in
+    identity order): vertices of 8, 9 and more entries beside molecules, graphs
+    that lie in one, two and three ranges of 256 vertices, more than 256 empty
+    graphs in a row, unmirrored graphs of every kind."""
+    from test_gpu_join_forms import _check
+
+    sizes = [n for n in (9, 10, 63, 64, 65, 127, 128, 129, 200, 255, 256) if n <= widest]
+    lines = [_graph(n, [(i, j) for i in range(n) for j in range(i + 1, n)], [8] * n) for n in (9, 10)]
+    for k, n in enumerate(sizes):
+        lines += [_dense(n, 6, k), _dense(n, 14, 100 + k), _dense(n, 14, 200 + k, loops=(3, n - 1)), _dense(n, 3, 300 + k, loops=(5,))]
+    lines += ["n#0 l#0 e#0"] * 600 + [_graph(n, [(0, i) for i in range(1, n)], [8] * n) for n in sizes]
+    lines += ["n#0 l#0 e#0"] * 300
+    molecules = sb.generate_molecules(40, 5, 40, seed=3741)
+    dense = sb.io.parse("\n".join(lines) + "\n")
+    assert dense.num_graphs > 900 and dense.sizes().max() == widest
+    d = dense.concat(molecules).concat(dense).concat(molecules)
+    queries = [_graph(2, [(0, 1)], [8, 7]), _graph(3, [(0, 1), (1, 2)], [8, 7, 8]), _graph(3, [(0, 1), (1, 2), (2, 0)], [8, 8, 8]),
+               _graph(4, [(0, 1), (0, 2), (0, 3)], [8, 0, 7, 7]), _graph(4, [(0, 1), (1, 2), (2, 3), (3, 0)], [8, 7, 8, 0]),
+               _graph(3, [(0, 1), (1, 2), (1, 1)], [8, 7, 8])]
+    for ff in (False, True):
+        ref = _check(sb.io.parse("\n".join(queries) + "\n"), d, 1, {oracle.REF_PTX: "ref-ptx", oracle.EXACT: "exact"}[profile], ff)
+        assert (ref["per_pair"] > 0).sum() > 100
