@@ -379,18 +379,22 @@ __global__ void k_join_literal(const uint32_t* __restrict__ bits, uint64_t Wp, i
 // has them (writing them as bitset words first took seven more launches, 130 us
 // before the join of a batch of any size), the graph's rows are staged in
 // shared memory, a round's masks are built by the whole block, and the
-// work-items of a graph are spread over blocks of kLitItems: a warp steps through its lanes' different moves in turn, so four
-// lanes take less time than 32, and blocks of 9 KB fit beside the persistent
-// join's.  (One block of 128 work-items per graph, walking the earlier rows at
-// each step: 1.02 ms for the first ten molecules of 100,000 x 600 pairs, 112 us
-// of 1,000 x 20; this form 190 and 74 us.)  Launches over many graphs (REF_X86)
-// keep one block per graph.  Molecules over 64 atoms and queries over
-// 32 vertices used to take k_join_literal's candidate-by-candidate form: 3.7 ms
-// for the first ten molecules of 60,000 x 500 uneven pairs.
+// work-items of a graph are spread over blocks of kLitItems: a warp steps through
+// its lanes' different moves in turn, so four lanes take less time than 32, and
+// blocks of up to 4 KB fit beside the persistent join's.  (One block of 128
+// work-items per graph, walking the earlier rows at each step: 1.02 ms for the
+// first ten molecules of 100,000 x 600 pairs, 112 us of 1,000 x 20; this form
+// 190 and 74 us.)  Launches over many graphs (REF_X86) take kLitItemsMany
+// work-items per block, whose state (33 bytes per work-item and level of the
+// batch's longest query) leaves room for many blocks: 1,000 x 20 and 5,000 x 100
+// pairs take 420 / 1,467 us with 4, 263 / 758 with 16, 279 / 778 with 32 and 263 /
+// 2,571 with the 128 of one block per graph.  Molecules over 64 atoms and queries
+// over 32 vertices used to take k_join_literal's candidate-by-candidate form: 3.7
+// ms for the first ten molecules of 60,000 x 500 uneven pairs.
 constexpr uint32_t kLitLevels = 32;
 constexpr uint8_t kLitOutside = 0xFFu;
-constexpr uint32_t kLitItems = 4;
-constexpr size_t kLitBytesPerThread = kLitLevels * (4 * sizeof(uint64_t) + 1);
+constexpr uint32_t kLitItems = 4, kLitItemsMany = 16;
+constexpr size_t kLitBytesPerLevel = 4 * sizeof(uint64_t) + 1;  // of a thread
 
 // wg: work-items of a graph (the reference's work-group size); bt of them per
 // block, one thread each.  With SMEM the block may have more threads, which only
@@ -399,16 +403,17 @@ template <int AW, bool SMEM>
 __global__ void k_join_literal_sets(MaskSource src, int prof, const uint32_t* __restrict__ qgoff, const uint64_t* __restrict__ qsel_id,
                                     const uint32_t* __restrict__ dgoff, const uint64_t* __restrict__ dadj, uint32_t dAW,
                                     const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ indices, uint32_t g0,
-                                    uint32_t g1, uint32_t wg, uint32_t bt, uint32_t q_begin, uint32_t q_end, int find_first,
-                                    uint64_t* __restrict__ counts, unsigned long long* __restrict__ d_total, JoinLimit lim) {
+                                    uint32_t g1, uint32_t wg, uint32_t bt, uint32_t levels, uint32_t q_begin, uint32_t q_end,
+                                    int find_first, uint64_t* __restrict__ counts,
+                                    unsigned long long* __restrict__ d_total, JoinLimit lim) {
   extern __shared__ uint64_t lit_sm[];
   __shared__ uint64_t s_row[SMEM ? 64 : 1];  // the graph's adjacency rows (word 0)
   const uint32_t tid = threadIdx.x;
   uint64_t* cm_s = lit_sm + tid;  // the threads past bt - 1 do not search
-  uint64_t* rem_s = lit_sm + kLitLevels * bt + tid;
-  uint64_t* p0_s = lit_sm + 2 * kLitLevels * bt + tid;
-  uint64_t* p1_s = lit_sm + 3 * kLitLevels * bt + tid;
-  uint8_t* map_s = reinterpret_cast<uint8_t*>(lit_sm + 4 * kLitLevels * bt) + tid;
+  uint64_t* rem_s = lit_sm + levels * bt + tid;
+  uint64_t* p0_s = lit_sm + 2 * levels * bt + tid;
+  uint64_t* p1_s = lit_sm + 3 * levels * bt + tid;
+  uint8_t* map_s = reinterpret_cast<uint8_t*>(lit_sm + 4 * levels * bt) + tid;
   constexpr uint32_t kLocal = SMEM ? 1 : kMaxQueryNodes;
   uint64_t cm_l[kLocal * AW], rem_l[kLocal * AW], p0_l[kLocal * AW], p1_l[kLocal * AW];
   uint8_t map_l[kLocal];
@@ -417,7 +422,6 @@ __global__ void k_join_literal_sets(MaskSource src, int prof, const uint32_t* __
 #define P0(j, w) (SMEM ? p0_s[(j) * bt] : p0_l[(j) * AW + (w)])
 #define P1(j, w) (SMEM ? p1_s[(j) * bt] : p1_l[(j) * AW + (w)])
 #define MAP(j) (SMEM ? map_s[(j) * bt] : map_l[(j)])
-  constexpr uint32_t kLevels = SMEM ? kLitLevels : kMaxQueryNodes;
   const uint32_t parts = (wg + bt - 1u) / bt;  // blocks per graph
   const uint64_t blocks = static_cast<uint64_t>(g1 - g0) * parts;
   uint64_t my_total = 0, steps = 0;
@@ -454,7 +458,7 @@ __global__ void k_join_literal_sets(MaskSource src, int prof, const uint32_t* __
     }
     const uint8_t map0 = s == 0 ? 0 : kLitOutside;
 #pragma unroll 1
-    for (uint32_t k = 0; searches && k < kLevels; ++k) MAP(k) = map0;  // mapping[] of a fresh work-item
+    for (uint32_t k = 0; searches && k < levels; ++k) MAP(k) = map0;  // mapping[] of a fresh work-item
     // graph-local bits the reference's uint8-indexed visited set can hold:
     // under REF_PTX those whose global id is below 256; under REF_X86 all
     // (the count modulo 64 is the local id).  A fresh work-item's mapping[]
@@ -466,7 +470,7 @@ __global__ void k_join_literal_sets(MaskSource src, int prof, const uint32_t* __
     for (uint32_t it = lid; lid0 < wg && it - tid < seg1 - seg0; it += wg) {
       if (SMEM) {  // the masks of the round's pairs, (work-item, level) per thread
         __syncthreads();  // the round before is done
-        for (uint32_t x = tid; x < bt * kLitLevels; x += blockDim.x) {
+        for (uint32_t x = tid; x < bt * levels; x += blockDim.x) {
           const uint32_t i = x % bt, j = x / bt, slot = it - tid + i;
           if (lid0 + i >= wg || slot >= seg1 - seg0) continue;
           const uint32_t q0 = qgoff[indices[seg0 + slot]];
@@ -1877,15 +1881,17 @@ int launch_join_literal(Queue* q, const Graph* query, const Graph* data, const M
     for (uint32_t g = graph_begin; g < graph_end; ++g)
       range_max = std::max(range_max, data->host_graph_offsets[g + 1] - data->host_graph_offsets[g]);
   }
-  // one word per set where the range's graphs allow it; its state fits shared
-  // memory up to kLitLevels levels and 256 threads
+  // one word per set where the range's graphs allow it; its state is in shared
+  // memory up to kLitLevels levels
   const bool one = range_max <= 64u;
-  // few graphs (those below vertex 256): small blocks, else a block per graph
-  const uint32_t block = graphs <= kLowOffsetLimit ? kLitItems : wg;
-  const bool smem_fits = one && query->max_nodes <= kLitLevels && kLitBytesPerThread * block <= 200u * 1024u;
+  const uint32_t levels = query->max_nodes;
+  const bool smem_fits = one && levels <= kLitLevels;
+  // few graphs (those below vertex 256): the smallest blocks; else small ones where
+  // a block's threads share the masks, and a block per graph where they do not
+  const uint32_t block = graphs <= kLowOffsetLimit ? kLitItems : smem_fits ? kLitItemsMany : wg;
   const uint64_t want = static_cast<uint64_t>(graphs) * ((wg + block - 1u) / block);
   if (one || (q->opts.profile == kProfilePtx && range_max <= 64u * kMaxAdjWords)) {
-    const size_t smem = smem_fits ? kLitBytesPerThread * block : 0;
+    const size_t smem = smem_fits ? kLitBytesPerLevel * levels * block : 0;
     auto kern = smem_fits ? k_join_literal_sets<1, true>
                 : one     ? k_join_literal_sets<1, false>
                 : data->adj_words == 2 ? k_join_literal_sets<2, false>
@@ -1893,7 +1899,7 @@ int launch_join_literal(Queue* q, const Graph* query, const Graph* data, const M
     if (smem) SIGMO_TRY(allow_max_dynamic_smem(reinterpret_cast<const void*>(kern), q->device));
     kern<<<grid_for(want, 1, 148u * 64u), smem_fits ? std::max(block, 32u) : block, smem, q->stream>>>(
         src, q->opts.profile, query->graph_offsets, query->qsel_id, data->graph_offsets, data->adj, data->adj_words, m->offsets,
-        m->indices, graph_begin, graph_end, wg, block, q_begin, q_end, find_first, m->counts, tot, join_limit(q));
+        m->indices, graph_begin, graph_end, wg, block, levels, q_begin, q_end, find_first, m->counts, tot, join_limit(q));
     return check_launch(q, "k_join_literal_sets");
   }
   if (!src.bits) return fail(SIGMO_ERR_INVALID, "internal: the literal join of graphs over %u vertices reads the bitset", 64u * kMaxAdjWords);

@@ -267,3 +267,25 @@ def test_graph_creation_by_degree_and_position(widest, profile):
     for ff in (False, True):
         ref = _check(sb.io.parse("\n".join(queries) + "\n"), d, 1, {oracle.REF_PTX: "ref-ptx", oracle.EXACT: "exact"}[profile], ff)
         assert (ref["per_pair"] > 0).sum() > 100
+
+
+@pytest.mark.parametrize("wg", [32, 128, 1024])
+@pytest.mark.parametrize("hi", [9, 32, 33])
+def test_literal_search_over_many_graphs(hi, wg):
+    """REF_X86 takes the literal search for every molecule: more of them than
+    the small blocks are for, work-groups of fewer and more items than a block,
+    queries up to the levels that shared memory holds and one past it."""
+    d = sb.generate_molecules(300, 5, 64, seed=3751)
+    q = sb.generate_queries(60, 2, 9, seed=3752).concat(sb.generate_queries(3, hi, hi, seed=3753))
+    assert q.sizes().max() == hi
+    queue = sb.Queue(0, profile="ref-x86", join_work_group_size=wg)
+    qg, dg = sb.createDeviceCSRGraph(queue, q), sb.createDeviceCSRGraph(queue, d)
+    cand, gm = _filtered(queue, qg, dg, 2), sb.GMCR(queue)
+    gm.generateGMCR(qg, dg, cand)
+    off, idx = gm.getGMCR()
+    for ff in (False, True):
+        ref = oracle.run_pipeline(q, d, 2, oracle.REF_X86, ff, wg=wg)
+        assert np.array_equal(off, ref["offsets"]) and np.array_equal(idx, ref["indices"]) and np.diff(off.astype(int)).max() > 32
+        total = np.zeros(1, np.uint64)
+        _, per = sb.joinCandidates(queue, qg, dg, cand, gm, total, ff, per_pair=True)
+        assert np.array_equal(per, ref["per_pair"]) and int(total[0]) == ref["total"] > 0
