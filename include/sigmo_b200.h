@@ -137,7 +137,9 @@ typedef struct sigmo_tuning {
                                     candidate each, neighbour counts instead of a walk over the
                                     earlier levels) with CTA-local slot regions; 0: per-lane DFS
                                     with one work cursor; 1: warp-cooperative frontier join
-                                    (32 candidate tries per round, one per lane)                 */
+                                    (32 candidate tries per round, one per lane).  2 was the
+                                    fastest on every workload measured; the others stay for
+                                    callers that set them                                        */
   uint32_t join_pool;            /* join_kernel 2: sixteenths of the slots in the pool shared by
                                     all CTAs after their own regions, 1..16 (2)                  */
 } sigmo_tuning;

@@ -32,12 +32,11 @@ unsigned host_threads(uint64_t n) {
   return static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>({n / 1024, 8, hw})));
 }
 // f(part, begin, end) over `parts` contiguous ranges of [0, n), part 0 on the
-// calling thread; parts <= 1 (or `force_serial`) runs inline.
+// calling thread; parts <= 1 runs inline.
 template <class F>
-void parallel_ranges(uint64_t n, unsigned parts, F&& f, int force_serial = 0) {
-  if (parts <= 1 || force_serial) {
-    for (unsigned p = 0; p < parts; ++p) f(p, n * p / parts, n * (p + 1) / parts);
-    if (parts == 0) f(0, 0, n);
+void parallel_ranges(uint64_t n, unsigned parts, F&& f) {
+  if (parts <= 1) {
+    f(0, 0, n);
     return;
   }
   std::vector<std::thread> th;
@@ -160,7 +159,8 @@ int build_plane_program(Queue* q, Graph* query, uint32_t R) {
   }
 
   // classes, in order of their first vertex: an open-addressing table of first
-  // vertices, compared exactly
+  // vertices, compared exactly (hashed by the multiply and xor-shift step of
+  // MurmurHash3's 64-bit finaliser)
   std::vector<uint32_t> cls(Qn), first;
   std::vector<uint64_t> label_count(256, 0);
   // a class's thresholds as raw codes r << 8 | l << 4 | c, back to back, and
@@ -319,7 +319,7 @@ int build_plane_program(Queue* q, Graph* query, uint32_t R) {
   return SIGMO_OK;
 }
 
-// Splits the query graphs into contiguous groups whose planes and classes fit
+// Splits the query graphs into contiguous groups whose planes fit
 // one admission tile (kGroupSmemBudget), greedily in query order, and uploads
 // each group's program in local plane ids.  Planned once per set width AW;
 // SIGMO_ERR_DOMAIN when a query graph alone does not fit a tile.

@@ -220,19 +220,7 @@ __global__ void k_sig_planes(const uint64_t* __restrict__ sig, uint64_t n, uint6
   }
 }
 
-// `rows` (<= kTabRows, a multiple of kBatch) rows per block.
-// refineCandidates: C[q][w] &= AND over q's non-zero counters (l, c) of
-// "counter l of vertex >= c", evaluated from the bit-sliced data signatures
-// (planes[l][w], see k_sig_planes).  Thread t owns the two words 2t, 2t+1 of
-// the block's 256-word span; the block's distinct thresholds (kRefineSlots at
-// most, about ten for molecule queries) are tabulated per thread, and a word
-// is written back only when it changed.  Bound by the bitset's traffic: one read
-// and the changed words' write.  What matters below that is warps in flight, and
-// the table's shared memory set their number: six passes over 100,000 molecules
-// x 600 take 5.12 ms with 32 slots (6 blocks per SM), 3.94 with 16 (7, by
-// registers) and 3.71 with 12 (10); four words per thread took 4.16, eight
-// slots 3.70.  A threshold beyond the table is computed from the planes, which
-// the block's other rows have brought to L1.
+// "Counter l >= c" of two words, for threshold p = 15 l + c - 1.
 __device__ __forceinline__ uint2 ge_pair(const uint4* __restrict__ planes, uint64_t Wp, uint64_t w0, uint32_t p) {
   const uint32_t l = p / 15u, c = p % 15u + 1u;
   const uint4 a = __ldg(planes + static_cast<uint64_t>(l) * Wp + w0);
@@ -240,6 +228,21 @@ __device__ __forceinline__ uint2 ge_pair(const uint4* __restrict__ planes, uint6
   return make_uint2(ge_sliced(a.x, a.y, a.z, a.w, c), ge_sliced(b.x, b.y, b.z, b.w, c));
 }
 
+// refineCandidates: C[q][w] &= AND over q's non-zero counters (l, c) of
+// "counter l of vertex >= c", evaluated from the bit-sliced data signatures
+// (planes[l][w], see k_sig_planes).  Thread t owns the two words 2t, 2t+1 of
+// the block's 256-word span; the block's distinct thresholds (kRefineSlots at
+// most, about ten for molecule queries) are tabulated per thread, and a word
+// is written back only when it changed.  `rows` (<= kTabRows, a multiple of
+// kBatch) rows per block.  Bound by the bitset's traffic: one read and the changed
+// words' write (a first pass over 100,000 molecules x 600 reaches 93 % of the
+// copy bandwidth), with issue close behind (73 % of the slots, 69 % of the warps;
+// 20,000 x 600: 245 us, 321 with 32 slots).  What matters below that is warps in flight, and
+// the table's shared memory set their number: six passes over 100,000 molecules
+// x 600 take 5.12 ms with 32 slots (6 blocks per SM), 3.94 with 16 (7, by
+// registers) and 3.71 with 12 (10); four words per thread took 4.16, eight
+// slots 3.70.  A threshold beyond the table is computed from the planes, which
+// the block's other rows have brought to L1.
 __global__ void __launch_bounds__(kTabThreads, 10) k_refine(const uint64_t* __restrict__ qsig, uint64_t Qn,
                                                         const uint4* __restrict__ planes, uint64_t Wp,
                                                         uint32_t* __restrict__ bits, uint32_t rows) {

@@ -1161,12 +1161,8 @@ __global__ void __launch_bounds__(kWideWarps * 32) k_join_wide(
 // set of the query vertex placed at level j = AND of its class's plane program
 // for the slot's data graph, stored [slot-in-chunk][level] (coalesced: one
 // 128-byte line per slot, so a pair's later levels hit in cache).
-// Phase B (k_join_masks): the DFS as a flat per-lane state machine whose pair
-// setup is just the load of those masks (issued one pair ahead, so the DRAM
-// latency of a refill overlaps the current pair's DFS), with the per-level
-// state in shared memory ([level][thread]).  Trying a candidate t at level k is O(1):
-// next = base[k+1] & (row(t) or ~row(t)) [& ~used]; base[k+2] is computed
-// once per descent.
+// Phase B: the DFS on those masks, k_join_dfs by default (k_join_masks and
+// k_join_frontier for callers that set sigmo_tuning.join_kernel).
 constexpr uint32_t kPhaseLevels = 16;
 constexpr uint32_t kDfsLevels = 10;  // most vertices of a query in k_join_dfs's short form
 constexpr uint32_t kPhaseThreads = 256;
@@ -1271,6 +1267,12 @@ __global__ void __launch_bounds__(256) k_pair_masks(
   }
 }
 
+// Phase B with sigmo_tuning.join_kernel = 0: the DFS as a flat per-lane state
+// machine whose pair setup is just the load of the masks (issued one pair ahead,
+// so the DRAM latency of a refill overlaps the current pair's DFS), with the
+// per-level state in shared memory ([level][thread]).  Trying a candidate t at
+// level k is O(1): next = base[k+1] & (row(t) or ~row(t)) [& ~used]; base[k+2] is
+// computed once per descent.
 // DAW: words per adjacency row of the data batch (the pairs here use word 0).
 template <bool EXACT, uint32_t DAW>
 __global__ void __launch_bounds__(kPhaseThreads) k_join_masks(
@@ -1394,14 +1396,14 @@ __global__ void __launch_bounds__(kPhaseThreads) k_join_masks(
 // Trying candidates from the highest vertex down needs no bit reversal.
 //
 // Bound by the latency of the chain level -> candidate -> row -> candidates of
-// the next level at 15 warps per SM (ncu, 5.2 M pairs of queries up to 10
-// vertices: 55 % of the issue slots, 48 % of the integer pipe, 24 of 32 lanes
-// per instruction); the state is kept per level in shared memory rather than
+// the next level at 15 warps per SM (ncu, 60,000 molecules x 600 queries, 4.0 M
+// pairs: 56 % of the issue slots, 53 % of the integer pipe, 23 of 32 lanes per
+// instruction); the state is kept per level in shared memory rather than
 // recomputed because those loads use a pipe that is idle otherwise.  The form
 // before this one walked the earlier rows and went back level by level: 7 of 32
-// lanes per instruction; join stage of 100,000 molecules x 600 queries (6.86 M
-// pairs) 9.26 -> 4.79 ms find-all, of 10,007 ring systems x 100 automorphic
-// queries 14.8 -> 5.5 ms.
+// lanes per instruction, 6.2 ms for the pairs of 100,000 molecules x 600 queries
+// where the short form takes 2.4 and the long one 0.6 beside it; the join stage of
+// 10,007 ring systems x 100 automorphic queries went from 14.8 to 3.8 ms.
 //
 // A lane that ends its pair waits until `refill` lanes of its warp are idle, so
 // the (divergent) setup of new pairs is shared by several lanes.  Work: each
@@ -1416,8 +1418,8 @@ __global__ void __launch_bounds__(kPhaseThreads) k_join_masks(
 // items are its entries.  Queries of up to kDfsLevels vertices are 93 % of the
 // pairs and 97 % of the turns of the mixed query set, so the short form's
 // lanes carry 402 B instead of 654.  Its CTAs have 160 threads so that three
-// leave 60 KB of an SM to L1: with 192 (28 KB of L1) the rows fall out of it,
-// 5.9 instead of 4.8 ms.
+// leave 60 KB of an SM to L1: with 192 (28 KB of L1) the rows fall out of it (an
+// early state of this form: 5.9 instead of 4.8 ms).
 // Loads of data that is read once, kept out of L1 (which holds the adjacency
 // rows), and a hint that brings a later pair's data to L2.
 __device__ __forceinline__ uint4 load_once(const uint4* p) {

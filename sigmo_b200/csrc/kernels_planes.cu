@@ -154,8 +154,8 @@ __device__ __forceinline__ void build_graph_planes(uint64_t* col, uint32_t row_w
 // vertex are never admitted (the reference's mapping skips them, gmcr.hpp:100):
 // their class lists are empty.
 //
-// Bound by instruction issue (63 % of the slots, 58 % of the shared-memory
-// wavefronts).  H = 2: a lane carries two graphs through the
+// Bound by instruction issue (60,000 molecules x 600 queries: 63 % of the slots,
+// 66 % of the integer pipe, 56 % of the shared-memory wavefronts).  H = 2: a lane carries two graphs through the
 // chain, so the program, its addresses and the votes are paid once for 64
 // graphs instead of twice (a model of 1,024 molecules x 600 queries: 4.1
 // classes of 6.5 planes per 32-graph tile and query; 1.35 -> 1.09 ms on 100,000
