@@ -704,13 +704,44 @@ __global__ void k_join_wildcard(const uint32_t* __restrict__ bits, uint64_t Wp, 
   if (lane == 0 && my_total) atomicAdd(d_total, static_cast<unsigned long long>(my_total));
 }
 
+// Position of the r-th (0-based) set bit of m; m has more than r set bits.
+__device__ __forceinline__ uint32_t nth_set32(uint32_t m, uint32_t r) {
+  uint32_t pos = 0, c = __popc(m & 0xFFFFu);
+  if (r >= c) { r -= c; pos += 16; m >>= 16; }
+  c = __popc(m & 0xFFu);
+  if (r >= c) { r -= c; pos += 8; m >>= 8; }
+  c = __popc(m & 0xFu);
+  if (r >= c) { r -= c; pos += 4; m >>= 4; }
+  c = __popc(m & 0x3u);
+  if (r >= c) { r -= c; pos += 2; m >>= 2; }
+  if (r >= (m & 1u)) pos += 1;
+  return pos;
+}
+__device__ __forceinline__ uint32_t nth_set64(uint64_t m, uint32_t r) {
+  const uint32_t lo = static_cast<uint32_t>(m), c = __popc(lo);
+  const bool up = r >= c;
+  return (up ? 32u : 0u) + nth_set32(up ? static_cast<uint32_t>(m >> 32) : lo, up ? r - c : r);
+}
+
+// The set's members whose rank is `share` modulo 1 << log2n.
+__device__ __forceinline__ uint64_t share_of(uint64_t set, uint32_t share, uint32_t log2n) {
+  if (!log2n) return set;
+  uint64_t keep = 0;
+  for (uint32_t r = 0; set; ++r, set &= set - 1)
+    if ((r & ((1u << log2n) - 1u)) == share) keep |= set & (0ull - set);
+  return keep;
+}
+
 // The join of the pairs listed by k_pair_masks as too large for the two-phase
 // join: queries of up to kMaxQueryNodes vertices, molecules of up to 64 * AW
 // atoms.  A warp takes a batch of up to `batch` pairs, builds their level masks
 // in shared memory with all lanes busy (an item per (pair, level), as in
 // k_pair_masks), and then its lanes run k_join_dfs's turns, each lane on one
-// root candidate of one pair at a time, so a heavy pair is spread over the
-// warp.  The per-level state is in local memory (the pairs are few).  The
+// root candidate of one pair at a time (or, where a pair has few, on a share of one
+// candidate's searches, by the next level's candidates), so a heavy pair is spread
+// over the warp.  (A star of four in a star of 100 atoms: 2.25 ms by one lane, 0.20
+// so; the first turn of a share is taken with the item, so the turns are as before.)
+// The per-level state is in local memory (the pairs are few).  The
 // one-lane-per-part form that this replaced rebuilt every mask in every part:
 // 1.43 ms for the 0.4 % of 6.86 M pairs with queries over 16 vertices.
 constexpr uint32_t kWideWarps = 4;
@@ -719,7 +750,9 @@ constexpr size_t kWideMaskBytes = 8192;  // level masks of one warp's batch, at 
 struct WideEntry {
   uint64_t cnt;
   uint32_t qoff, n, s, slot;  // qoff: identity-order flag in bit 31
-  uint32_t root, pad;         // BONDS: the query vertex placed first
+  uint32_t root;              // BONDS: the query vertex placed first
+  uint32_t items, log2n;      // root candidates x shares of the next level's candidates (2^log2n)
+  uint32_t next;              // items taken
 };
 // [batch] entries, [batch][AW] root candidates, [batch][stride] masks per warp
 inline size_t wide_smem(uint32_t batch, uint32_t aw, uint32_t stride) {
@@ -971,7 +1004,7 @@ __global__ void __launch_bounds__(kWideWarps * 32) k_join_wide(
       s = dgoff[g];
       e = dgoff[g + 1];
       ident = BONDS || !(qsym[qg] && dsym[g]);
-      ent[lane] = WideEntry{0, qoff | (ident ? 0x80000000u : 0u), n, s, slot, 0, 0};
+      ent[lane] = WideEntry{0, qoff | (ident ? 0x80000000u : 0u), n, s, slot, 0, 0, 0, 0};
     }
     uint32_t incl = n;
 #pragma unroll
@@ -1007,6 +1040,23 @@ __global__ void __launch_bounds__(kWideWarps * 32) k_join_wide(
     for (uint32_t i = lane; i < ne * AW; i += 32)
       roots[i] = masks[(i / AW) * stride + (BONDS ? ent[i / AW].root * AW : 0u) + i % AW];
     __syncwarp();
+    // an item is a root candidate, or a share of its searches (by the next
+    // level's candidates) where a pair has fewer of them than its part of the
+    // warp's lanes (BONDS: the root has the most candidates of all)
+    if (lane < ne) {
+      WideEntry& en = ent[lane];
+      uint32_t c0 = 0, c1 = 0;
+#pragma unroll
+      for (int w = 0; w < AW; ++w) {
+        c0 += __popcll(roots[lane * AW + w]);
+        c1 += __popcll(masks[lane * stride + AW + w]);
+      }
+      uint32_t log2n = 0;
+      while (!BONDS && ((c0 * ne) << log2n) < 32u && (2u << log2n) <= c1) ++log2n;
+      en.log2n = log2n;
+      en.items = c0 << log2n;
+    }
+    __syncwarp();
     // the lanes' searches
     uint64_t alive = 0, cnt = 0;  // alive: levels with untried candidates
     uint32_t my = 0;              // this lane's pair within the batch
@@ -1014,44 +1064,77 @@ __global__ void __launch_bounds__(kWideWarps * 32) k_join_wide(
     const uint64_t* M = masks;
     const uint64_t* arow = dadj;
     uint32_t root = 0, v0 = 0;    // BONDS: the root, and the query's first vertex
-    bool dry = false;  // no root candidate left for this lane
+    bool dry = false;  // no item left for this lane
+    auto flush = [&]() {
+      auto* at = reinterpret_cast<unsigned long long*>(&ent[my].cnt);
+      if (find_first && !BONDS) atomicExch(at, 1ull);
+      else atomicAdd(at, static_cast<unsigned long long>(find_first ? 1ull : cnt));
+      cnt = 0;
+    };
     for (;;) {
-      if (!alive && cnt) {
-        auto* at = reinterpret_cast<unsigned long long*>(&ent[my].cnt);
-        if (find_first && !BONDS) atomicExch(at, 1ull);
-        else atomicAdd(at, static_cast<unsigned long long>(find_first ? 1ull : cnt));
-        cnt = 0;
-      }
-      if (!alive && !dry) {
+      if (!alive && cnt) flush();
+      while (!alive && !dry) {
         dry = true;
+        uint32_t item = 0;
         for (uint32_t i = 0; i < ne && dry; ++i) {
-          const uint32_t c = (lane + i) % ne;
+          const uint32_t c = (lane + i) % ne, items = ent[c].items;
           if (find_first && !BONDS && *reinterpret_cast<volatile uint64_t*>(&ent[c].cnt)) continue;
-          for (uint32_t w = 0; w < AW && dry; ++w) {
-            unsigned long long v = *reinterpret_cast<volatile unsigned long long*>(&roots[c * AW + w]);
-            while (v && dry) {
-              const unsigned long long bit = v & (0ull - v);
-              const unsigned long long old = atomicAnd(&roots[c * AW + w], ~bit);
-              if (old & bit) {
-                dry = false;
-                my = c;
-#pragma unroll
-                for (uint32_t x = 0; x < AW; ++x) rest[0][x] = x == w ? bit : 0ull;
-              }
-              v = old & ~bit;
-            }
+          if (*reinterpret_cast<volatile uint32_t*>(&ent[c].next) >= items) continue;
+          item = atomicAdd(&ent[c].next, 1u);
+          if (item < items) {
+            dry = false;
+            my = c;
           }
         }
-        if (!dry) {
-          const WideEntry& en = ent[my];
-          n = en.n;
-          selp = ((en.qoff >> 31) ? qsel_id : qsel) + (en.qoff & 0x7FFFFFFFu);
-          arow = dadj + static_cast<uint64_t>(en.s) * AW;
-          M = masks + my * stride;
-          root = en.root;
-          v0 = en.qoff & 0x7FFFFFFFu;
-          s = en.s;
+        if (dry) break;
+        const WideEntry& en = ent[my];
+        n = en.n;
+        selp = ((en.qoff >> 31) ? qsel_id : qsel) + (en.qoff & 0x7FFFFFFFu);
+        arow = dadj + static_cast<uint64_t>(en.s) * AW;
+        M = masks + my * stride;
+        root = en.root;
+        v0 = en.qoff & 0x7FFFFFFFu;
+        s = en.s;
+        // the item's root candidate
+        uint32_t skip = item >> en.log2n, t = 0;
+        bool found = false;
+#pragma unroll
+        for (int w = 0; w < AW; ++w) {
+          const uint64_t v = roots[my * AW + w];
+          const uint32_t c = __popcll(v);
+          const bool here = !found && skip < c;
+          if (here) t = 64u * w + nth_set64(v, skip);
+          found |= here;
+          skip -= found ? 0u : c;
+        }
+        if (BONDS || !en.log2n) {
+#pragma unroll
+          for (int w = 0; w < AW; ++w) rest[0][w] = (t >> 6) == static_cast<uint32_t>(w) ? 1ull << (t & 63u) : 0ull;
           alive = 1;
+          continue;
+        }
+        // a share: its first turn here, with the share of level 1's candidates
+        const uint32_t mod = (1u << en.log2n) - 1u;
+        const uint64_t next_to = 0ull - (selp[1] & 1ull);
+        pick[0] = static_cast<uint8_t>(t);
+        uint32_t rank = 0, c = 0;
+        for (uint32_t w = 0; w < AW; ++w) {
+          uint64_t keep = 0;
+          for (uint64_t x = M[AW + w]; x; x &= x - 1, ++rank)
+            if ((rank & mod) == (item & mod)) keep |= x & (0ull - x);
+          const uint64_t r = arow[t * AW + w];
+          const uint64_t bit = EXACT && (t >> 6) == w ? 1ull << (t & 63u) : 0ull;
+          keep &= ~(r ^ next_to) & ~bit;
+          rest[1][w] = keep;
+          p0[1][w] = r | bit;
+          p1[1][w] = bit;
+          c += __popcll(keep);
+        }
+        if (n > 2u) {
+          alive = c ? 2u : 0u;
+        } else if (c) {  // level 1 is the last
+          cnt = c;
+          flush();
         }
       }
       if (!__any_sync(kAll, alive != 0)) break;
@@ -1410,8 +1493,10 @@ __global__ void __launch_bounds__(kPhaseThreads) k_join_masks(
 // CTA first takes items from its own contiguous region of the chunk, so its
 // lanes join neighbouring molecules whose adjacency rows stay in L1, then from
 // a tail pool shared by all CTAs (pool16 sixteenths of the chunk).  An item is
-// one of the 1 << lparts parts of a pair (every 2^lparts-th root candidate):
-// pairs are split when there are fewer of them than lanes.
+// one of the 1 << lparts parts of a pair (every 2^lparts-th root candidate, and
+// where the pair has fewer of them, of each a share of the next level's
+// candidates): pairs are split when there are fewer of them than lanes.  (A star of
+// five vertices in a star of 64, one root candidate: 73.7 ms by one lane, 4.8 so.)
 //
 // LV: most vertices of a query (LV - 1 levels of state per lane).  Pairs of
 // longer queries are flagged and listed by k_pair_masks; with a list, the
@@ -1545,12 +1630,11 @@ __global__ void __launch_bounds__(dfs_threads<LV>()) k_join_dfs(
                 nextm[(j - 1) * T] = mm[j / 4].m[j % 4];
                 meta[(j - 1) * T] = static_cast<uint16_t>(qm[j / 2] >> (16u * (j % 2)));
               }
-            if (lparts) {  // this part's root candidates: ranks = part mod 2^lparts
-              const uint32_t part = static_cast<uint32_t>(item) & ((1u << lparts) - 1u);
-              uint64_t keep = 0;
-              for (uint32_t i = 0; root; ++i, root &= root - 1)
-                if ((i & ((1u << lparts) - 1u)) == part) keep |= root & (0ull - root);
-              root = keep;
+            if (lparts) {  // this part's root candidates, and where they are fewer than the parts its share of the next level's
+              const uint32_t part = static_cast<uint32_t>(item) & ((1u << lparts) - 1u), c0 = __popcll(root);
+              const uint32_t by_root = c0 > 1u ? min(lparts, 32u - __clz(c0 - 1u)) : 0u;  // log2
+              root = share_of(root, part & ((1u << by_root) - 1u), by_root);
+              if (by_root < lparts) nextm[0] = share_of(mm[0].m[1], part >> by_root, lparts - by_root);
             }
             rest[0] = root;
             alive = root ? 1u : 0u;
@@ -1611,25 +1695,6 @@ __global__ void __launch_bounds__(dfs_threads<LV>()) k_join_dfs(
   }
   for (int o = 16; o; o >>= 1) my_total += __shfl_xor_sync(kAll, my_total, o);
   if (lane == 0 && my_total) atomicAdd(d_total, static_cast<unsigned long long>(my_total));
-}
-
-// Position of the r-th (0-based) set bit of m; m has more than r set bits.
-__device__ __forceinline__ uint32_t nth_set32(uint32_t m, uint32_t r) {
-  uint32_t pos = 0, c = __popc(m & 0xFFFFu);
-  if (r >= c) { r -= c; pos += 16; m >>= 16; }
-  c = __popc(m & 0xFFu);
-  if (r >= c) { r -= c; pos += 8; m >>= 8; }
-  c = __popc(m & 0xFu);
-  if (r >= c) { r -= c; pos += 4; m >>= 4; }
-  c = __popc(m & 0x3u);
-  if (r >= c) { r -= c; pos += 2; m >>= 2; }
-  if (r >= (m & 1u)) pos += 1;
-  return pos;
-}
-__device__ __forceinline__ uint32_t nth_set64(uint64_t m, uint32_t r) {
-  const uint32_t lo = static_cast<uint32_t>(m), c = __popc(lo);
-  const bool up = r >= c;
-  return (up ? 32u : 0u) + nth_set32(up ? static_cast<uint32_t>(m >> 32) : lo, up ? r - c : r);
 }
 
 // Phase B, warp-cooperative form (k_join_frontier).  A warp keeps up to 32

@@ -118,3 +118,27 @@ def test_budget_spent_among_wide_pairs(prof):
         queue.set_join_budget(0)
         res = sb.match_batched(queue, qg, dg, 2, True, None, gm, graph=graph)
         assert res["total_matches"] == ref["total"] and np.array_equal(gm.getPairCounts(), ref["per_pair"])
+
+
+def _broom(n, leaves, hub):
+    """A chain of n vertices whose last one, of label `hub`, carries `leaves` vertices."""
+    edges = [(i, i + 1) for i in range(n - 1)] + [(n - 1, n + i) for i in range(leaves)]
+    labels = [8] * (n - 1) + [hub] + [8] * leaves
+    return (f"n#{n + leaves} l#1 " + " ".join(f"{i} {x}" for i, x in enumerate(labels)) + f" e#{len(edges)} " +
+            " ".join(f"{u} {v} 1" for u, v in edges))
+
+
+@pytest.mark.parametrize("prof,ff", MODES)
+@pytest.mark.parametrize("chain,leaves,copies", [(1, 40, 1), (9, 30, 6), (16, 30, 2), (1, 100, 6), (5, 120, 2), (14, 190, 1),
+                                                 (3, 9, 300), (3, 9, 1200)])
+def test_pairs_with_one_root_candidate(chain, leaves, copies, prof, ff):
+    """The hub of a star is one candidate: its pair's parts are shares of the
+    next level's.  Patterns of 2 vertices (whose next level is the last), up to
+    10, 11 to 16 and more, molecules of one, two and four words, few pairs and
+    several batches of wide ones, below vertex 256 and above."""
+    patterns = [_broom(1, k, 7) for k in (1, 2, 3)] + [_broom(k, 2, 7) for k in (2, min(chain, 8), chain)]
+    q = sb.io.parse("\n".join(patterns) + "\n")
+    molecules = [_broom(chain, leaves - i, 7) for i in range(3)] + [_broom(2, 3, 7)]
+    d = sb.io.parse("\n".join(molecules * copies + [_broom(30, 3, 0)] * 10 + molecules * copies) + "\n")
+    ref = _check(q, d, 1, prof, ff)
+    assert ref["total"] > 0
